@@ -76,6 +76,8 @@ _SIGNATURES = {
                       I, I, I, I, P],
     "hb_delta_conv_update": [P, I, c_longlong, I, P, c_longlong, c_longlong, P, P, I, I, I, P],
     "hb_delta_recurrence": [P, P, P, P, P, P, c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
+    "hb_delta_recurrence_chunked": [P, P, P, P, P, P, c_longlong, P, P, P, P, I, I, I, I, I, I, I, P],
+    "hb_mlstm_recurrence_chunked": [P, I, c_longlong, I, I, I, F, P, P, P, c_longlong, P, P, P, P, P, I, I, I, I, I, P],
     "hb_delta_out_norm": [P, P, I, P, F, P, I, c_longlong, I, I, c_longlong, I, P],
     "hb_hyper_step": [P, P, P, I, P, I, P, P, P, I, P, P, F, P, P, I, F, P, I, P, P, I, I, I, P],
     "hb_hyper_sum": [P, P, I, I, I, P],
@@ -106,6 +108,8 @@ def lib():
             fn = getattr(handle, name)
             fn.argtypes = sig
             fn.restype = c_int
+        handle.hb_recurrence_chunked_scratch_floats.argtypes = [I, I, I]
+        handle.hb_recurrence_chunked_scratch_floats.restype = c_longlong
         handle.hb_moe_down_tc_scratch_floats.argtypes = [I]
         handle.hb_moe_down_tc_scratch_floats.restype = c_longlong
         _lib = handle
@@ -585,6 +589,19 @@ def delta_conv_update(proj: torch.Tensor, chan_off: int, channels: int, taps_n: 
                                       _stream()), "delta_conv_update")
 
 
+CHUNKED_MIN_TOKENS = 80      # ... and 8 more for every request of the step
+
+
+def _chunked_recurrence(n: int, n_seqs: int, dim: int) -> bool:
+    """Whether a step's recurrence goes sixteen tokens at a time. A chunk costs about what a dozen tokens cost one by one,
+    however few tokens it holds, and there is a launch more."""
+    return dim <= 128 and n >= CHUNKED_MIN_TOKENS + 8 * n_seqs
+
+
+def _chunked_scratch(n: int, n_seqs: int, heads: int, device) -> torch.Tensor:
+    return torch.empty(lib().hb_recurrence_chunked_scratch_floats(n, n_seqs, heads), dtype=torch.float32, device=device)
+
+
 def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Optional[torch.Tensor],
                      decay: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, heads: int,
                      kvh: int, dim: int, vdim: int, general: bool = False, rows: int = 0, single_tokens: bool = False,
@@ -605,6 +622,14 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Op
     if state.dim() != 2 or state.shape[1] < heads * dim * vdim or cu_seqlens.numel() != slots.numel() + 1:
         raise KernelError("the state or the request tables do not fit")
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
+    if not (general or rows or single_tokens) and _chunked_recurrence(n, slots.numel(), dim):
+        scratch = _chunked_scratch(n, slots.numel(), heads, q.device)
+        _check(lib().hb_delta_recurrence_chunked(
+            _ptr(q), _ptr(k), _ptr(v), None if plain else _ptr(beta), _ptr(decay), _ptr(state), state.shape[1],
+            _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(out), n, slots.numel(), heads, kvh, dim, vdim, int(plain),
+            _stream()), "delta_recurrence")
+        LAUNCHES[0] += 1
+        return out
     _check(lib().hb_delta_recurrence(_ptr(q), _ptr(k), _ptr(v), None if plain else _ptr(beta), _ptr(decay), _ptr(state),
                                      state.shape[1], _ptr(cu_seqlens), _ptr(slots), _ptr(out), slots.numel(), heads, kvh,
                                      dim, vdim, 1 if general else int(rows), int(single_tokens), int(plain), _stream()),
@@ -833,6 +858,14 @@ def mlstm_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_s
         raise KernelError("the state row is too short for this memory")
     o = torch.empty((n, heads, vdim), dtype=torch.float32, device=proj.device)
     nq = torch.empty((n, heads), dtype=torch.float32, device=proj.device)
+    if not rows_per_lane and _chunked_recurrence(n, slots.numel(), dim):
+        scratch = _chunked_scratch(n, slots.numel(), heads, proj.device)
+        _check(lib().hb_mlstm_recurrence_chunked(
+            _ptr(proj), _dt(proj), ld, q_off, k_off, v_off, float(q_scale), _ptr(keep), _ptr(take), _ptr(state),
+            state.stride(0), _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(o), _ptr(nq), n, slots.numel(), heads, dim,
+            vdim, _stream()), "mlstm_recurrence")
+        LAUNCHES[0] += 1
+        return o, nq
     _check(lib().hb_mlstm_recurrence(_ptr(proj), _dt(proj), ld, q_off, k_off, v_off, float(q_scale), _ptr(keep),
                                      _ptr(take), _ptr(state), state.stride(0), _ptr(cu_seqlens), _ptr(slots), _ptr(o),
                                      _ptr(nq), slots.numel(), heads, dim, vdim, int(rows_per_lane), _stream()),

@@ -1,0 +1,111 @@
+"""The recurrences sixteen tokens at a time (portions of prompts), against the same recurrences token after token in
+float64: partial chunks, one-token requests beside portions, sizes around the kernels' tiles of 16 rows and columns."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+# outputs and states, largest error over largest value: sums of at most 128 float32 products (sqrt(128) 2^-24 = 7e-7 of their
+# length) whose factors carry a few roundings of 6e-8 each, over memories of some dozens of tokens: 3e-6 with room
+TOL = 3e-6
+LENS = [1, 16, 130, 17, 15, 2]
+
+
+def close(got, want, what):
+    err = float((got.double().cpu() - want.double().cpu()).abs().max() / want.abs().max().clamp_min(1e-30))
+    assert err <= TOL, (what, err)
+
+
+def tables(lens):
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    slots = torch.randperm(len(lens) + 2, generator=torch.Generator().manual_seed(1))[: len(lens)].to(torch.int32)
+    return cu, slots
+
+
+@pytest.mark.parametrize("plain", [False, True])
+@pytest.mark.parametrize("heads,kvh,dim,vdim", [(4, 2, 128, 128), (2, 2, 1, 1), (3, 3, 16, 16), (2, 1, 17, 33), (4, 4, 64, 15),
+                                                (2, 1, 65, 17), (6, 3, 96, 40), (1, 1, 112, 130), (9, 9, 127, 129)])
+def test_delta_rule_and_plain(heads, kvh, dim, vdim, plain):
+    from hi_b200.kernels import ops
+
+    assert ops._chunked_recurrence(sum(LENS), len(LENS), dim)
+    g = torch.Generator().manual_seed(dim)
+    n = sum(LENS)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    q = (F.normalize(rnd(n, kvh, dim), dim=-1) * dim ** -0.5).reshape(n, -1)
+    k = F.normalize(rnd(n, kvh, dim), dim=-1).reshape(n, -1)
+    v, beta = rnd(n, heads * vdim), torch.rand(n, heads, generator=g)
+    decay = torch.exp(-torch.exp(2.0 * rnd(n, heads * dim) - 2.0))       # from almost one to far underflow in a chunk
+    decay[5, :3] = 0.0
+    cu, slots = tables(LENS)
+    state = rnd(len(LENS) + 2, heads * dim * vdim + 3)
+    dev = state.to(DEV)
+    o = ops.delta_recurrence(q.to(DEV), k.to(DEV), v.to(DEV), None if plain else beta.to(DEV), decay.to(DEV), dev, cu.to(DEV),
+                             slots.to(DEV), heads, kvh, dim, vdim, plain=plain)
+    wide = lambda t: t.double().view(n, kvh, dim).repeat_interleave(heads // kvh, dim=1)
+    qd, kd, vd, gd = wide(q), wide(k), v.double().view(n, heads, vdim), decay.double().view(n, heads, dim)
+    for s, slot in enumerate(slots.tolist()):
+        S = state[slot, : heads * dim * vdim].double().view(heads, dim, vdim)
+        want = []
+        for t in range(int(cu[s]), int(cu[s + 1])):
+            S = S * gd[t][:, :, None]
+            u = vd[t] if plain else beta[t].double()[:, None] * (vd[t] - torch.einsum("hdv,hd->hv", S, kd[t]))
+            S = S + kd[t][:, :, None] * u[:, None, :]
+            want.append(torch.einsum("hdv,hd->hv", S, qd[t]).reshape(-1))
+        close(o[int(cu[s]): int(cu[s + 1])], torch.stack(want), f"request {s}")
+        close(dev[slot, : heads * dim * vdim], S.reshape(-1), f"state {s}")
+        assert torch.equal(dev[slot, heads * dim * vdim:].cpu(), state[slot, heads * dim * vdim:])
+    for slot in set(range(len(LENS) + 2)) - set(slots.tolist()):
+        assert torch.equal(dev[slot].cpu(), state[slot])
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim,vdim", [(4, 128, 128), (3, 16, 15), (2, 33, 16), (1, 1, 1), (2, 96, 47), (10, 64, 129)])
+def test_mlstm(heads, dim, vdim, dt):
+    from hi_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(dim)
+    n, off = sum(LENS), 3
+    proj = (0.5 * torch.randn(n, off + heads * (2 * dim + vdim) + 1, generator=g)).to(dt)
+    keep, take = torch.rand(n, heads, generator=g), torch.rand(n, heads, generator=g)
+    cu, slots = tables(LENS)
+    floats = ops.mlstm_state_floats(heads, dim, vdim)
+    state = 0.3 * torch.randn(len(LENS) + 2, floats, generator=g)
+    dev = state.to(DEV)
+    o, nq = ops.mlstm_recurrence(proj.to(DEV), off, off + heads * dim, off + 2 * heads * dim, dim ** -0.5, keep.to(DEV),
+                                 take.to(DEV), dev, cu.to(DEV), slots.to(DEV), heads, dim, vdim)
+    p = proj.double()
+    q, k = (p[:, off + i * heads * dim: off + (i + 1) * heads * dim].view(n, heads, dim) for i in (0, 1))
+    v = torch.cat([p[:, off + 2 * heads * dim: -1].view(n, heads, vdim), torch.ones(n, heads, 1, dtype=torch.float64)], dim=2)
+    for s, slot in enumerate(slots.tolist()):
+        S = state[slot, : heads * (vdim + 1) * dim].double().view(heads, vdim + 1, dim)
+        want = []
+        for t in range(int(cu[s]), int(cu[s + 1])):
+            S = keep[t].double().view(-1, 1, 1) * S + (take[t].double()[:, None] * v[t])[:, :, None] * k[t][:, None, :]
+            want.append(torch.einsum("hvd,hd->hv", S, q[t]) * dim ** -0.5)
+        want, rows = torch.stack(want), slice(int(cu[s]), int(cu[s + 1]))
+        close(o[rows], want[:, :, :vdim], f"request {s}")
+        close(nq[rows], want[:, :, vdim], f"n.q of request {s}")
+        close(dev[slot, : heads * (vdim + 1) * dim], S.reshape(-1), f"state {s}")
+        assert torch.equal(dev[slot, heads * (vdim + 1) * dim:].cpu(), state[slot, heads * (vdim + 1) * dim:])
+
+
+def test_what_is_not_finite_stays_with_later_tokens_and_its_column():
+    from hi_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(0)
+    n, heads, dim, vdim = 200, 2, 64, 48
+    q, k = (F.normalize(torch.randn(n, heads, dim, generator=g), dim=-1).reshape(n, -1).to(DEV) for _ in range(2))
+    v, beta = torch.randn(n, heads * vdim, generator=g).to(DEV), torch.rand(n, heads, generator=g).to(DEV)
+    decay = (0.5 + 0.5 * torch.rand(n, heads * dim, generator=g)).to(DEV)
+    cu, slots = torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    call = lambda: ops.delta_recurrence(q, k, v, beta, decay, torch.zeros(1, heads * dim * vdim, device=DEV), cu, slots, heads,
+                                        heads, dim, vdim)
+    clean = call()
+    v[70, 5] = float("nan")
+    got = call()
+    assert bool(torch.isnan(got[70:, 5]).all())
+    other = torch.ones_like(got, dtype=torch.bool)
+    other[70:, 5] = False
+    assert torch.equal(got[other], clean[other])
