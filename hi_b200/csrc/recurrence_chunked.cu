@@ -13,6 +13,13 @@
 //     NW more warps, in two groups that take turns, prepare the next chunk's rows (decay products) and write the chunk's
 //     outputs, which nothing waits for.
 //
+// Measured (B200, one request of 2,048 tokens, 16 heads of 128 x 128; before: token after token, a chain of 2,048 steps):
+// delta rule 582 -> 230 us (24 of them the matrices), the rule without correction 573 -> 163, mLSTM 437 -> 187; 32 heads of
+// Mamba-2 709 -> 254. Error against 64 bits (2-norm, outputs / states): delta rule 9.1e-8 / 1.3e-7 -> 7.1e-8 / 7.0e-8, without
+// correction 1.4e-7 / 1.1e-7 -> 8.7e-8 / 5.4e-8. A chunk is 1.6 us of a block: 6,000 warp instructions, of which the
+// preparation of its rows is 40 %, between three barriers. Tried: the products as float32 fma (the shared-memory reads of 4 x 4
+// tiles bound it: 293 us); two tf32 pieces a factor (error 1.1e-7, states of Mamba-2 1.9 times as far off: taken back).
+//
 // What is not finite in a token's inputs reaches that token's and later outputs of the request, never an earlier one.
 #include "api.h"
 #include "common.cuh"

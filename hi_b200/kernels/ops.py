@@ -594,7 +594,9 @@ CHUNKED_MIN_TOKENS = 80      # ... and 8 more for every request of the step
 
 def _chunked_recurrence(n: int, n_seqs: int, dim: int) -> bool:
     """Whether a step's recurrence goes sixteen tokens at a time. A chunk costs about what a dozen tokens cost one by one,
-    however few tokens it holds, and there is a launch more."""
+    however few tokens it holds, and there is a launch more. Measured, kernel times of 16 heads of 128 x 128, delta rule:
+    one request of 24 / 48 / 96 tokens 11.4 / 18.0 / 31.5 us one by one against 12.4 / 14.0 / 19.0; 64 requests of 3 tokens
+    132 against 157; 31 single tokens beside 512 214 against 162."""
     return dim <= 128 and n >= CHUNKED_MIN_TOKENS + 8 * n_seqs
 
 
