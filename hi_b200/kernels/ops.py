@@ -36,6 +36,7 @@ _SIGNATURES = {
     "hb_moe_combine": [P, P, P, P, I, P, I, I, I, P],
     "hb_qkv_post": [P, I, P, I, I, I, F, I, F, F, P, P, I, I, F, P, I, I, I, P, P, P, I, P, P, P, I, I, I, I, I, I, P],
     "hb_paged_attention": [P, I, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, F, P, P, I, I, P, P, P],
+    "hb_attention_portions": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, F, P, P, I, P, P, P],
     "hb_attention_merge": [P, P, P, I, I, I, I, I, I, P, P],
     "hb_attention_decode": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P],
     "hb_attention_decode_tma": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P],
@@ -1059,6 +1060,70 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
                                     _ptr(sink_values), ATTENTION_SPLIT, splits, _ptr(part_acc), _ptr(part_ml), _stream()),
            "paged_attention")
     return (part_acc, part_ml) if parts else out
+
+
+PORTION_ROW_LENGTHS = (16, 32, 48, 64, 80, 96, 112, 128, 192)
+
+
+def portion_attention_splits(blocks: int, keys: int) -> int:
+    """How many blocks share a row tile's keys: as few as bring the rounds of blocks (two on each of 148 SMs), times the key
+    tiles of a block and its fixed cost, to their least."""
+    tiles = -(-keys // 32) + 1
+    best = (None, 1)
+    for s in range(1, min(32, max(1, tiles // 2)) + 1):
+        cost = -(-(blocks * s) // 296) * (-(-tiles // s) + 2) + (2 + 0.25 * s if s > 1 else 0)
+        if best[0] is None or cost < best[0]:
+            best = (cost, s)
+    return best[1]
+
+
+def portion_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
+                      cu_seqlens: torch.Tensor, positions: torch.Tensor, n_new, chunk: int, window: int, scale: float,
+                      max_context: int, sink: bool = False, softcap: float = 0.0, slopes: Optional[torch.Tensor] = None,
+                      sink_values: Optional[torch.Tensor] = None, keep: int = 0) -> Optional[torch.Tensor]:
+    """:func:`paged_attention` of float32 portions (request ``s`` brings the ``n_new[s]`` rows ``cu_seqlens[s]`` .. of ``q``,
+    at consecutive positions), or None for what this kernel does not take (head sizes, alignment)."""
+    n, nh, hd = q.shape
+    if q.dtype != torch.float32 or hd not in PORTION_ROW_LENGTHS or not q.is_contiguous():
+        return None
+    _need(q, "q"); _need(k_pages, "k_pages", q.dtype); _need(v_pages, "v_pages", q.dtype)
+    for t, nm in ((block_table, "block_table"), (cu_seqlens, "cu_seqlens"), (positions, "positions")):
+        _need(t, nm, torch.int32)
+    _, nkv, page_size, hd2 = k_pages.shape
+    if hd2 != hd or k_pages.shape != v_pages.shape:
+        raise KernelError("cache pages do not match the query's head_dim")
+    if nh % nkv:
+        raise KernelError(f"{nh} query heads are not a multiple of {nkv} kv heads")
+    if cu_seqlens.numel() != len(n_new) + 1 or block_table.shape[0] < len(n_new):
+        raise KernelError("cu_seqlens / block_table do not match the number of requests")
+    for t, nm in ((slopes, "slopes"), (sink_values, "sink_values")):
+        if t is not None:
+            _need(t, nm, torch.float32)
+            if t.numel() != nh:
+                raise KernelError(f"{nm} needs one number per query head")
+    group, longest = nh // nkv, max(int(max_context), 1)
+    if chunk > 0:
+        longest = min(longest, chunk)
+    if window > 0:
+        longest = min(longest, window + keep + 64 // group)
+    splits = portion_attention_splits(nkv * sum(-(-m * group // 64) for m in n_new), longest)
+    out = torch.empty_like(q)
+    part_acc = part_ml = None
+    if splits > 1:
+        part_acc = torch.empty((n, nh, splits, hd), dtype=torch.float32, device=q.device)
+        part_ml = torch.empty((n, nh, splits, 2), dtype=torch.float32, device=q.device)
+    sink = bool(sink) or sink_values is not None
+    code = lib().hb_attention_portions(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.shape[1],
+                                       _ptr(cu_seqlens), _ptr(positions), _ptr(out), len(n_new), max(n_new), nh, nkv, hd,
+                                       page_size, int(chunk), int(window), int(keep), float(scale), int(sink), float(softcap),
+                                       _ptr(slopes), _ptr(sink_values), splits, _ptr(part_acc), _ptr(part_ml), _stream())
+    if code == _UNSUPPORTED:
+        return None
+    _check(code, "attention_portions")
+    if splits > 1:
+        _check(lib().hb_attention_merge(_ptr(part_acc), _ptr(part_ml), _ptr(out), _dt(out), n * nh, hd, splits, int(sink), nh,
+                                        _ptr(sink_values), _stream()), "attention_merge")
+    return out
 
 
 def sigmoid_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
