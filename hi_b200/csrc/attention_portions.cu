@@ -7,9 +7,13 @@
 // where it does not fit. Maximum, exponentials and sums are float32 as in the general kernel, and so are the rules of what a
 // token may read (see attention.cu); a value that is not finite reaches only the rows that may read it.
 //
-// What bounds it: mma.sync, at 2 cycles of an SM for [16, 16] x [16, 8], six of them a product; two blocks per SM, so one
-// splits its next tile while the other multiplies. The general kernel (a warp per row, 32 rows of keys at once, uncoalesced)
-// read every key once per row: 600 tokens behind 301, 16 heads / 4 kv heads of 128: GENERAL_US -> NEW_US.
+// What bounds it: mma.sync, at 2 cycles of an SM for [16, 16] x [16, 8], six of them a product (0.4 of the time), and the
+// chains between them: a block of four warps splits, multiplies and takes exponentials in turn, two blocks per SM (104 KB of
+// pieces each). The general kernel (a warp per row, uncoalesced rows of keys, every key read once per row) took 1,622 us for
+// 600 tokens behind 301, 16 heads / 4 kv heads of 128, and 18.1 ms for 2,048 tokens, 40 / 8 heads; this one 139 us and
+// 1.16 ms. Steps: keys and values loaded where they are needed, two key tiles of products side by side 187 us; four side by
+// side (the five small terms are a chain) 174; a tile's rows loaded into registers under the products before them 150; the
+// shares of a row tile's keys chosen by fractional rounds 139. Error against 64 bits 4.8e-7 -> 1.8e-7.
 #include "api.h"
 #include "common.cuh"
 #include "mma.cuh"
@@ -145,29 +149,33 @@ __global__ void __launch_bounds__(32 * WARPS, NT <= 8 ? 2 : 1) portion_attention
   const __nv_bfloat16* k_at = ks + ((lane & 7) + (lane >> 4) * 8) * LD + ((lane >> 3) & 1) * 8;
   const __nv_bfloat16* v_at = vs + (lane & 15) * LD + (lane >> 4) * 8;
 
+  // A tile's rows come as registers while the warps multiply something else: its values under its own scores, the next
+  // tile's keys under its weights times values.
+  constexpr int LOADS = KEYS * PER / (32 * WARPS);
+  float4 in[LOADS];
+  auto load = [&](const float* pages, const long long* off_of) {
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {
+      const int e = tid + i * 32 * WARPS;
+      const long long off = off_of[e / PER];
+      in[i] = off >= 0 ? *reinterpret_cast<const float4*>(pages + off + (e % PER) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  auto store = [&](__nv_bfloat16* to) {
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {
+      const int e = tid + i * 32 * WARPS;
+      put4<KP>(to + (e / PER) * LD + (e % PER) * 4, in[i]);
+    }
+  };
+  load(a.k_pages, offs[tile0 & 1]);
+  store(ks);
+  __syncthreads();
   for (int tile = tile0; tile < tile1; ++tile) {
     const int key0 = key0_of(tile);
-    bool odd = false;                       // a value that is not finite
     const long long* off_of = offs[tile & 1];
-#pragma unroll(NT <= 4 ? NT : 4)
-    for (int i = 0; i < KEYS * PER / (32 * WARPS); ++i) {
-      const int e = tid + i * 32 * WARPS, r = e / PER, c = (e % PER) * 4;
-      const long long off = off_of[r];
-      float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-      if (off >= 0) {
-        kv = *reinterpret_cast<const float4*>(a.k_pages + off + c);
-        vv = *reinterpret_cast<const float4*>(a.v_pages + off + c);
-      }
-      if (!(finite(vv.x) && finite(vv.y) && finite(vv.z) && finite(vv.w))) {
-        odd = true;
-        vv.x = finite(vv.x) ? vv.x : 0.f; vv.y = finite(vv.y) ? vv.y : 0.f;
-        vv.z = finite(vv.z) ? vv.z : 0.f; vv.w = finite(vv.w) ? vv.w : 0.f;
-      }
-      put4<KP>(ks + r * LD + c, kv);
-      put4<KP>(vs + r * LD + c, vv);
-    }
+    load(a.v_pages, off_of);
     if (tile + 1 < tile1) find(tile + 1);
-    const int any_odd = __syncthreads_or(odd);
 
     // scores
     float s[4][4], lo_s[4][4];
@@ -180,29 +188,43 @@ __global__ void __launch_bounds__(32 * WARPS, NT <= 8 ? 2 : 1) portion_attention
       unsigned qa[3][4];
 #pragma unroll
       for (int p = 0; p < 3; ++p) hb::ldmatrix_x4(qa[p], q_at + p * QP + kk * 16);
+      // four key tiles side by side: a product's five small terms are a chain
+      unsigned kb[2][3][4];
 #pragma unroll
-      for (int np = 0; np < 2; ++np) {
-        unsigned kb[3][4];
+      for (int np = 0; np < 2; ++np)
 #pragma unroll
-        for (int p = 0; p < 3; ++p) hb::ldmatrix_x4(kb[p], k_at + p * KP + np * 16 * LD + kk * 16);
-        float hi[2][4];
+        for (int p = 0; p < 3; ++p) hb::ldmatrix_x4(kb[np][p], k_at + p * KP + np * 16 * LD + kk * 16);
+      float hi[4][4];
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) hi[n][e] = 0.f;
-          mma16(hi[n], qa[0], kb[0][2 * n], kb[0][2 * n + 1]);
+        for (int e = 0; e < 4; ++e) hi[n][e] = 0.f;
+      constexpr int from[6][2] = {{0, 0}, {2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}};
+#pragma unroll
+      for (int x = 0; x < 6; ++x)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          const unsigned(&kx)[4] = kb[n / 2][from[x][1]];
+          mma16(x == 0 ? hi[n] : lo_s[n], qa[from[x][0]], kx[2 * (n % 2)], kx[2 * (n % 2) + 1]);
         }
-        constexpr int from[5][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}};
 #pragma unroll
-        for (int x = 0; x < 5; ++x)
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
-          for (int n = 0; n < 2; ++n) mma16(lo_s[2 * np + n], qa[from[x][0]], kb[from[x][1]][2 * n], kb[from[x][1]][2 * n + 1]);
+        for (int e = 0; e < 4; ++e) s[n][e] += hi[n][e];
+    }
+    bool odd = false;                       // a value that is not finite
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) s[2 * np + n][e] += hi[n][e];
+    for (int i = 0; i < LOADS; ++i) {
+      float4& v = in[i];
+      if (!(finite(v.x) && finite(v.y) && finite(v.z) && finite(v.w))) {
+        odd = true;
+        v.x = finite(v.x) ? v.x : 0.f; v.y = finite(v.y) ? v.y : 0.f;
+        v.z = finite(v.z) ? v.z : 0.f; v.w = finite(v.w) ? v.w : 0.f;
       }
     }
+    store(vs);                              // read last before the end of the tile before this one
+    const int any_odd = __syncthreads_or(odd);          // ... and all warps are through with the keys
+    if (tile + 1 < tile1) load(a.k_pages, offs[(tile + 1) & 1]);
     float most[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int n = 0; n < 4; ++n)
@@ -247,28 +269,37 @@ __global__ void __launch_bounds__(32 * WARPS, NT <= 8 ? 2 : 1) portion_attention
         for (int x = 0; x < 3; ++x) pa[kk][x][e] = p[x];
       }
 #pragma unroll
-    for (int np = 0; np < NT; ++np) {
-      float hi[2][4], lo_o[2][4];
+    for (int n0 = 0; n0 < 2 * NT; n0 += 4) {
+      constexpr int TILES = 4;
+      const int live = n0 + TILES <= 2 * NT ? TILES : 2;          // 2 NT is even
+      float hi[TILES][4], lo_o[TILES][4];
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int n = 0; n < TILES; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) hi[n][e] = lo_o[n][e] = 0.f;
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk) {
-        unsigned vb[3][4];
+        unsigned vb[2][3][4];
 #pragma unroll
-        for (int p = 0; p < 3; ++p) hb::ldmatrix_x4_trans(vb[p], v_at + p * KP + kk * 16 * LD + np * 16);
-        constexpr int from[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int p = 0; p < 3; ++p)
+            if (2 * h < live) hb::ldmatrix_x4_trans(vb[h][p], v_at + p * KP + kk * 16 * LD + n0 * 8 + h * 16);
+        constexpr int from[6][2] = {{0, 0}, {2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}};
 #pragma unroll
         for (int x = 0; x < 6; ++x)
 #pragma unroll
-          for (int n = 0; n < 2; ++n)
-            mma16(x == 5 ? hi[n] : lo_o[n], pa[kk][from[x][0]], vb[from[x][1]][2 * n], vb[from[x][1]][2 * n + 1]);
+          for (int n = 0; n < TILES; ++n)
+            if (n < live) {
+              const unsigned(&vx)[4] = vb[n / 2][from[x][1]];
+              mma16(x == 0 ? hi[n] : lo_o[n], pa[kk][from[x][0]], vx[2 * (n % 2)], vx[2 * (n % 2) + 1]);
+            }
       }
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int n = 0; n < TILES; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[2 * np + n][e] = fmaf(o[2 * np + n][e], corr[e >> 1], hi[n][e] + lo_o[n][e]);
+        for (int e = 0; e < 4; ++e)
+          if (n < live) o[n0 + n][e] = fmaf(o[n0 + n][e], corr[e >> 1], hi[n][e] + lo_o[n][e]);
     }
     if (any_odd)
       for (int j = 0; j < KEYS; ++j) {
@@ -283,7 +314,8 @@ __global__ void __launch_bounds__(32 * WARPS, NT <= 8 ? 2 : 1) portion_attention
             if (!finite(v) && key <= pos[i] && (key >= lo[i] || key < kept[i])) o[n][e] += v;
           }
       }
-    __syncthreads();                        // the tile is read
+    if (tile + 1 < tile1) store(ks);
+    __syncthreads();                        // the tile is read, the next one's keys are there
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {

@@ -1066,12 +1066,14 @@ PORTION_ROW_LENGTHS = (16, 32, 48, 64, 80, 96, 112, 128, 192)
 
 
 def portion_attention_splits(blocks: int, keys: int) -> int:
-    """How many blocks share a row tile's keys: as few as bring the rounds of blocks (two on each of 148 SMs), times the key
-    tiles of a block and its fixed cost, to their least."""
+    """How many blocks share a row tile's keys: the rounds of blocks (two on each of 148 SMs; later rounds fill up as blocks
+    end) times the key tiles of a block and its fixed cost, plus the merge, at their least. Measured with 1 / 2 / 3 / 8 / 16
+    shares: 152 blocks of up to 29 tiles 174 / 137 / 150 / 147 / 169 us, 28 blocks of 129 tiles 704 / 372 / 256 / 130 / 134 us
+    (111 with 10), 1,280 blocks of up to 65 tiles 1,162 / 1,372 / 1,390 / 1,568 / 1,813 us."""
     tiles = -(-keys // 32) + 1
     best = (None, 1)
     for s in range(1, min(32, max(1, tiles // 2)) + 1):
-        cost = -(-(blocks * s) // 296) * (-(-tiles // s) + 2) + (2 + 0.25 * s if s > 1 else 0)
+        cost = max(1.0, blocks * s / 296) * (-(-tiles // s) + 1.5) + (2 + 0.3 * s if s > 1 else 0)
         if best[0] is None or cost < best[0]:
             best = (cost, s)
     return best[1]
