@@ -113,3 +113,51 @@ def test_shared_keys_holes_and_what_is_not_finite(monkeypatch):
     other = torch.ones_like(got, dtype=torch.bool)
     other[40:, :2, 3] = False
     assert float((got[other].double() - want[other]).abs().max() / want.abs().max()) <= TOL
+
+
+@pytest.mark.parametrize("hd", [64, 128, 192])
+@pytest.mark.parametrize("lens", [[1 + 128, 40], [31, 129 + 64], [97 + 128, 3], [33 + 256, 200]])
+def test_tiles_with_few_tokens_in_the_bfloat16_kernel(hd, lens):
+    """The tcgen05 kernel's warps without a token: the portion before gives what it gives alone, whatever the rows of the
+    next request hold (here NaN), and the last rows of a ragged tile are right (bfloat16 weights and outputs: 2^-8 each)."""
+    from hi_b200.kernels import ops
+
+    portions = [(lens[0], 150), (lens[1], 70)]
+    q, k, v, table, cu, pos = setup(4, 2, hd, 64, portions, seed=3)
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    want = reference(q, k, v, table, portions, 0, 0, 0, hd ** -0.5)[: lens[0]]
+    call = lambda qq: ops.prefill_attention_tc(qq.to(DEV), k.to(DEV), v.to(DEV), table.to(DEV), cu.to(DEV), pos.to(DEV), 2,
+                                               max(lens), 0, 0, hd ** -0.5).cpu()[: lens[0]]
+    got = call(q)
+    assert float((got.double() - want).abs().max() / want.abs().max()) <= 2e-2
+    q[lens[0]:] = float("nan")
+    assert torch.equal(call(q), got)
+    ops.check_tc_status()
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,hd,splits", [(1, 16, 1), (7, 64, 2), (9, 128, 8), (40, 128, 9), (33, 192, 33), (5, 80, 70), (3, 1024, 5)])
+def test_merge(rows, hd, splits, dt):
+    from hi_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(hd + splits)
+    acc, ml = torch.randn(rows, splits, hd, generator=g), torch.randn(rows, splits, 2, generator=g) * 3
+    ml[:, :, 1] = ml[:, :, 1].abs() + 0.1
+    ml[0, (splits + 1) // 2:, 0] = float("-inf")          # splits beyond a token's range: never written
+    acc[0, (splits + 1) // 2:] = float("nan")
+    sinks = torch.randn(1, generator=g)
+    acc_d, ml_d, sinks_d = acc.to(DEV), ml.to(DEV), sinks.to(DEV)
+    for sink in (0, 1):
+        out = torch.empty(rows, hd, dtype=dt, device=DEV)
+        code = ops.lib().hb_attention_merge(acc_d.data_ptr(), ml_d.data_ptr(), out.data_ptr(),
+                                            0 if dt == torch.float32 else 1, rows, hd, splits, sink, 1, sinks_d.data_ptr() if sink else None,
+                                            torch.cuda.current_stream().cuda_stream)
+        assert code == 0
+        m = ml[:, :, 0].double()
+        w = torch.exp(m - m.max(1, keepdim=True).values.clamp_min(-1e30))
+        den = (w * ml[:, :, 1].double()).sum(1)
+        if sink:
+            den = torch.where(den > 0, den + torch.exp(sinks.double() - m.max(1).values), den)
+        want = torch.where(w[:, :, None] > 0, w[:, :, None] * acc.double(), 0.0).sum(1) / den.clamp_min(1e-300)[:, None]
+        err = float((out.cpu().double() - want).abs().max() / want.abs().max())
+        assert err <= (2e-6 if dt == torch.float32 else 4e-3), err
