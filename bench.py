@@ -287,15 +287,15 @@ def long_context_point(engine, cfg, args, pk, vocab, cpu_gen):
     toks = torch.randint(0, vocab, (3 * short,), generator=cpu_gen).tolist()
     times = []
     for i, min_tiles in enumerate((None, None, 1 << 30)):       # the first runs untimed
-        keep = ops.PREFILL_SPLIT_MIN_TILES
+        keep = ops.PREFILL_SPLIT_MIN_TILES, ops.PREFILL_MOST_SHARES
         if min_tiles:
-            ops.PREFILL_SPLIT_MIN_TILES = min_tiles
+            ops.PREFILL_SPLIT_MIN_TILES, ops.PREFILL_MOST_SHARES = min_tiles, 1
         start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
         engine.step([StepEntry("Ls", toks[i * short:(i + 1) * short], [])])
         end.record()
         torch.cuda.synchronize()
-        ops.PREFILL_SPLIT_MIN_TILES = keep
+        ops.PREFILL_SPLIT_MIN_TILES, ops.PREFILL_MOST_SHARES = keep
         times.append(start.elapsed_time(end))
     engine.finish("Ls")
     out["short_portion"] = {"tokens": short, "offset": ctx - 3 * short, "ms": round(times[1], 2),

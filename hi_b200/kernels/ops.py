@@ -7,6 +7,7 @@ on a CUDA device, or a library that cannot be built, raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_longlong, c_uint64, c_void_p
 from typing import Optional, Tuple
 
@@ -1754,6 +1755,55 @@ def prefill_key_splits(blocks: int, key_tiles: int, sms: int) -> int:
     best = max(fill.values())
     choice = min(k for k, f in fill.items() if f >= best - 0.05)
     return choice if fill[choice] > fill[1] else 1
+
+
+PREFILL_MOST_SHARES = 8                # of any query tile's keys
+
+
+def prefill_shares(portions, nh: int, hd: int, chunk: int, window: int, rows: int, sms: int) -> int:
+    """The same question for launches of any mix, from a model of the kernel's time; ``portions`` are (cached, new) tokens,
+    ``rows`` the step's tokens. A block's key tile takes 1.1 us alone on its SM and 1.6 us beside a second block (rows over 128:
+    one block per SM, 1.15 us); blocks run in rounds of their average length, no sooner than any portion's alone or than the longest; shared rows are
+    written and read once in float32 (3 TB/s), and the merge is a launch (4 us). Shares must save a tenth. Measured, 1 share
+    against the choice: 40 heads of 128, 128 tokens behind 1,000 / 3,000 / 7,000 27 / 59 / 125 -> 22 / 30 / 44 us, 700 behind 300
+    beside 150 behind 9,000 196 -> 136; 16 heads, 513 behind 7,000 135 -> 71, 1,024 behind 7,000 143 -> 101; 16 heads of 192,
+    300 behind 2,000 49 -> 34. Whole prompts keep one block (2,048 tokens, 40 heads: 77 us, 153 in two shares)."""
+    per_sm = 2 if hd <= 128 else 1
+    pair = 1.6 if per_sm == 2 else 1.15
+    most, runs = 0, [[0, 0.0]]          # blocks and their tiles: of all, then of every portion
+
+    def tiles(first, last):
+        lo = first // chunk * chunk if chunk else 0
+        if window:
+            lo = max(lo, first - window + 1)
+        return last // 64 - lo // 64 + 1
+
+    for cached, new in portions:
+        count = -(-new // 128)
+        head = tiles(cached, cached + min(new, 128) - 1)
+        tail = tiles(cached + 128 * (count - 1), cached + new - 1)
+        runs.append([nh * count, nh * count * (head + tail) / 2])
+        runs[0] = [runs[0][0] + runs[-1][0], runs[0][1] + runs[-1][1]]
+        most = max(most, head, tail)
+    if not runs[0][0]:
+        return 1
+    return _fewest_us(tuple(tuple(r) for r in runs), most, rows * nh * hd, per_sm, pair, sms, PREFILL_MOST_SHARES)
+
+
+@functools.lru_cache(maxsize=256)                  # a step's layers ask the same
+def _fewest_us(runs, most: int, numbers: int, per_sm: int, pair: float, sms: int, limit: int) -> int:
+    def cost(k):
+        t = -(-most // k) * (1.1 if runs[0][0] * k <= sms else pair)
+        for blocks, work in runs:
+            if blocks:
+                each = work / blocks / k + (0.5 if k > 1 else 0.0)
+                rounds, rest = divmod(blocks * k, per_sm * sms)
+                t = max(t, rounds * each * pair + (each * (1.1 if rest <= sms else pair) if rest else 0.0))
+        return 7.0 + t + (4.0 + numbers * 8.0 * k / 3e6 if k > 1 else 0.0)
+
+    alone = cost(1)
+    best = min(range(1, limit + 1), key=cost)
+    return best if cost(best) < 0.9 * alone else 1
 
 
 # --------------------------------------------------------------------------- experts

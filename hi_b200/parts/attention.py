@@ -17,20 +17,25 @@ DIFF_TC_MIN_TOKENS = 64      # new tokens of a request from which differential a
                              # tile is 64 tokens by two maps)
 
 
-def _key_splits(ctx, nh: int, chunk: int, sliding: int, single: bool, device) -> int:
+def _key_splits(ctx, nh: int, hd: int, chunk: int, sliding: int, keep: int, single: bool, device) -> int:
     """Portions far into long contexts on a layer that sees every key: all blocks of the
     tensor-core prefill kernel then have about the same many key tiles, and a partly filled
-    last round of blocks is worth splitting the keys for (ops.prefill_key_splits)."""
-    if chunk or sliding:
+    last round of blocks is worth splitting the keys for (ops.prefill_key_splits). Everything else: what a model of
+    the kernel's time says (ops.prefill_shares)."""
+    if keep:
         return 1
     portions = [(s, n) for s, n in zip(ctx.start_pos, ctx.n_new) if n > 1 or not single]
     if not portions:
         return 1
-    shortest, longest_new = min(s for s, _n in portions), max(n for _s, n in portions)
-    if shortest < 2 * longest_new:
-        return 1
-    blocks = nh * sum(-(-n // ops.PREFILL_TC_MIN_TOKENS) for _s, n in portions)
-    return ops.prefill_key_splits(blocks, shortest // 64, ops.sm_count(device))
+    sms = ops.sm_count(device)
+    if not chunk and not sliding:
+        shortest, longest_new = min(s for s, _n in portions), max(n for _s, n in portions)
+        if shortest >= 2 * longest_new:
+            blocks = nh * sum(-(-n // ops.PREFILL_TC_MIN_TOKENS) for _s, n in portions)
+            shares = ops.prefill_key_splits(blocks, shortest // 64, sms)
+            if shares > 1:
+                return shares
+    return ops.prefill_shares(portions, nh, hd, chunk, sliding, ctx.n_tokens, sms)
 
 
 def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, hd: int, chunk: int, sliding: int,
@@ -62,7 +67,7 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
         if tc:
             o = ops.prefill_attention_tc(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions,
                                          ctx.n_seqs, ctx.max_new, chunk, sliding, scale, skip_single=single,
-                                         key_splits=_key_splits(ctx, nh, chunk, sliding, single, q.device), sink=sink,
+                                         key_splits=_key_splits(ctx, nh, hd, chunk, sliding, keep, single, q.device), sink=sink,
                                          softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep)
         else:
             o = ops.prefill_attention(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions,

@@ -16,3 +16,18 @@ def test_key_shares_of_the_tensor_core_prefill_attention():
         assert ops.prefill_key_splits(blocks, tiles, sms) == 1, (blocks, tiles)
     # a smaller GPU has fewer places: the same launch is then more than its rounds' worth
     assert ops.prefill_key_splits(160, 1020, 40) == 1
+
+
+def test_key_shares_of_any_mix_of_portions():
+    """Few blocks with long runs of keys share them, chunked and windowed layers too; prompts from the start, launches that
+    fill the GPU and nothing to do keep one block per query tile and head."""
+    shares = lambda portions, nh=40, hd=128, chunk=0, window=0: ops.prefill_shares(portions, nh, hd, chunk, window,
+                                                                                  sum(n for _c, n in portions), 148)
+    assert shares([(7000, 128)]) > 1 and shares([(7000, 128)], chunk=8192) > 1 and shares([(100000, 128)], window=4096) > 1
+    assert shares([(8190, 128)], chunk=8192) > 1                     # the tile reaches back over the chunk's end
+    assert shares([(8192, 128)], chunk=8192) == 1 and shares([(9000, 128)], window=64) == 1
+    assert shares([(9000, 150), (300, 700)]) > 1
+    for portions in ([], [(0, 2048)], [(0, 128)], [(0, 512), (0, 1)], [(20000, 4096)], [(3000, 1024)]):
+        assert shares(portions) == 1, portions
+    for hd in (64, 128, 192):
+        assert 1 <= shares([(50000, 1)], nh=1, hd=hd) <= 8
