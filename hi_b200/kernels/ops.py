@@ -80,6 +80,7 @@ _SIGNATURES = {
     "hb_delta_recurrence": [P, P, P, P, P, P, c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
     "hb_delta_recurrence_chunked": [P, P, P, P, P, P, c_longlong, P, P, P, P, I, I, I, I, I, I, I, P],
     "hb_mlstm_recurrence_chunked": [P, I, c_longlong, I, I, I, F, P, P, P, c_longlong, P, P, P, P, P, I, I, I, I, I, P],
+    "hb_skinny_linear": [P, c_longlong, P, P, P, I, I, I, I, P],
     "hb_delta_out_norm": [P, P, I, P, F, P, I, c_longlong, I, I, c_longlong, I, P],
     "hb_hyper_step": [P, P, P, I, P, I, P, P, P, I, P, P, F, P, P, I, F, P, I, P, P, I, I, I, P],
     "hb_hyper_sum": [P, P, I, I, I, P],
@@ -271,6 +272,28 @@ def embed_position(table: torch.Tensor, tokens: torch.Tensor, positions: torch.T
     out = torch.empty((n, hidden), dtype=torch.float32, device=table.device)
     _check(lib().hb_embed_position(_ptr(table), _dt(table), _ptr(tokens), _ptr(positions), _ptr(turns), _ptr(out), n, hidden,
                                    vocab, float(scale), _stream()), "embed_position")
+    return out
+
+
+SKINNY_MOST_TOKENS = 16      # rows of x up to which the kernel may be the faster one (it says so itself)
+
+
+def skinny_linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
+                  bias: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """``x @ weight.T (+ bias)`` for a few rows of bfloat16 ``x`` (its rows may be a column slice of a wider matrix), with
+    float32 sums, in ``out_dtype``; None for what the kernel does not take (sizes, strides, alignment) or is not the faster one for."""
+    (n, k), (m, k2) = x.shape, weight.shape
+    if not 0 < n <= SKINNY_MOST_TOKENS or k != k2 or k % 8 or k == 0 or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or \
+            x.stride(1) != 1 or (n > 1 and x.stride(0) % 8) or not weight.is_contiguous() or \
+            out_dtype not in (torch.bfloat16, torch.float32) or \
+            (bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != m or not bias.is_contiguous())):
+        return None
+    out = torch.empty((n, m), dtype=out_dtype, device=x.device)
+    code = lib().hb_skinny_linear(_ptr(x), x.stride(0) if n > 1 else k, _ptr(weight), _ptr(bias), _ptr(out), _dt(out), n, m, k,
+                                  _stream())
+    if code == _UNSUPPORTED:
+        return None
+    _check(code, "skinny_linear")
     return out
 
 

@@ -1,6 +1,8 @@
 """Dense matrix products of the product path: the library's (cuBLAS through torch.mm), as
 the reference engine uses a library for every dense projection
-(crates/hi-cuda/src/runtime.rs:1118-1143, cublasGemmEx with float32 accumulation).
+(crates/hi-cuda/src/runtime.rs:1118-1143, cublasGemmEx with float32 accumulation); of a few
+bfloat16 rows (decode steps) a kernel of this tree's own, which streams the weights
+(``ops.skinny_linear``), where it is the faster one.
 
 float32 products run with TF32 and reduced-precision reductions switched off, so the 32-bit
 path is true 32-bit.
@@ -8,6 +10,8 @@ path is true 32-bit.
 from __future__ import annotations
 
 import torch
+
+from ..kernels import ops
 
 
 def configure_matmul_precision() -> None:
@@ -35,6 +39,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
         if bias is not None:
             y += bias.to(torch.float32)
         return y.to(out_dtype or x.dtype)
+    if x.dtype == torch.bfloat16 and x.shape[0] <= ops.SKINNY_MOST_TOKENS:
+        y = ops.skinny_linear(x, weight, out_dtype or x.dtype, None if bias is None else bias.to(x.dtype))
+        if y is not None:
+            return y
     if bias is not None:
         y = torch.addmm(bias.to(x.dtype), x, weight.t())
         return y if out_dtype in (None, x.dtype) else y.to(out_dtype)

@@ -1,0 +1,48 @@
+"""Products of a few bfloat16 rows against the same in float64: edges of the kernel's tiles (16 rows of the weight, 8 tokens,
+32 of K), each of its forms, rows that are a slice of a wider matrix, and what is left to the library."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("n_out,k", [(1, 8), (15, 40), (17, 2048), (2368, 64), (2369, 328), (4737, 264), (6657, 128), (48, 4104)])
+@pytest.mark.parametrize("tokens", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_against_float64(n_out, k, tokens, out_dtype):
+    from hi_b200.kernels import ops
+    from hi_b200.parts.linear import linear
+
+    g = torch.Generator(device=DEV).manual_seed(n_out + k)
+    wide = torch.randn(tokens, k + 24, device=DEV, generator=g).to(torch.bfloat16)
+    x, w = wide[:, 8: 8 + k], (torch.randn(n_out, k, device=DEV, generator=g) * k ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(n_out, device=DEV, generator=g).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    got = ops.skinny_linear(x, w, out_dtype)
+    if tokens > 8 and n_out > 2368:
+        assert got is None
+        return
+    # float32 sums of k exact products of size one in all: a few 2^-24; bfloat16 results: 2^-9 of the value
+    tol = 2e-6 if out_dtype == torch.float32 else 2.0 ** -8
+    assert float((got.double() - want).abs().max()) <= tol * float(want.abs().max())
+    got = linear(x, w, out_dtype=out_dtype, bias=bias)
+    want = want + bias.double()
+    assert got.dtype == out_dtype and float((got.double() - want).abs().max()) <= tol * float(want.abs().max())
+
+
+def test_what_is_left_to_the_library():
+    from hi_b200.kernels import ops
+    from hi_b200.parts.linear import linear
+
+    x, w = torch.randn(4, 72, device=DEV).to(torch.bfloat16), torch.randn(33, 72, device=DEV).to(torch.bfloat16)
+    flat = torch.randn(4 * 72 + 1, device=DEV).to(torch.bfloat16)
+    for a, b in ((x[:, :68], w[:, :68].contiguous()), (x[:, 4:68], w[:, :64].contiguous()), (x, w.t().contiguous().t()),
+                 (torch.randn(17, 72, device=DEV).to(torch.bfloat16), w), (flat[1:].view(4, 72), w), (x[:0], w), (x.t()[:, :4].t(), w)):
+        if a.shape[0] and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and b.is_contiguous() and a.shape[1] % 8 == 0 and a.shape[0] <= 16:
+            continue
+        assert ops.skinny_linear(a, b, torch.bfloat16) is None
+        got, want = linear(a, b), a.double() @ b.double().t()
+        assert got.shape == want.shape and (not got.numel() or float((got.double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max()))
+    with pytest.raises(Exception):
+        linear(x, w[:, :64].contiguous())
