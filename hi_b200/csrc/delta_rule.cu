@@ -6,7 +6,8 @@
 //                      portion's first token come from the request's state), q and k to unit length per head
 //                      (q also times dim^-1/2), beta = sigmoid(.), decay = exp(-exp(A_log) * softplus(a + dt_bias))
 //   delta_conv_update  per request: the last (taps - 1) inputs of the portion replace the state's
-//   delta_recurrence   per (request, head, group of value columns), token after token:
+//   delta_recurrence   per (request, head, group of value columns), token after token (portions of enough tokens:
+//                      recurrence_chunked.cu; single tokens: delta_single_kernel, by whole lines of the state):
 //                        S <- decay * S (rows);  u = beta * (v - S^T k);  S <- S + k u^T;  o = S^T q
 //                      A thread owns one column of S, so nothing is exchanged between threads but k, q and the
 //                      decay of the token, which the block stages in shared memory one token ahead.

@@ -6,7 +6,7 @@
 // in three kernels, all float32:
 //   mlstm_gates       the gates' logarithms for all tokens side by side, the scan of m token after token (adds and
 //                     maxima only), then keep = e^(f + m - m'), take = e^(i - m') and floor = e^(-m') side by side
-//   mlstm_recurrence  S and n token after token. n is one more column of S whose value is always 1, so that
+//   mlstm_recurrence  S and n token after token (portions of enough tokens: recurrence_chunked.cu). n is one more column of S whose value is always 1, so that
 //                     n' . q falls out as one more output. A column lives in the registers of L lanes, R rows each.
 //   mlstm_out_norm    the division, the RMS norm of every head's output, the weight and the sigmoid gate
 // A request's state is one float32 row: [heads][vdim + 1][dim] (column-major S, then n), then m [heads]. It

@@ -311,10 +311,13 @@ router_few_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const floa
 // them, four at a time, so every load is used 4 (weights) or 16 (activations) times from
 // registers and nothing waits on shared memory. Needs hidden % 8 == 0. The partial sums meet in
 // shared memory and are added in part order. With one block column (experts <= ROUTER_EXP) the
-// block also selects; otherwise router_select_kernel does.
-constexpr int ROUTER_TOK = 4, ROUTER_EXP = 16;
+// block also selects; otherwise router_select_kernel does. Up to eight experts take a block of eight
+// columns; the lanes' sums come together by a halving butterfly, which adds the same pairs as a
+// butterfly per logit in a fifth of the shuffles (2,048 tokens of 2,048, 8 experts: ROUTER_US; the products
+// of sixteen columns and 64 butterflies a warp were what it spent its time on).
+constexpr int ROUTER_TOK = 4;
 
-template <typename TW>
+template <typename TW, int ROUTER_EXP>
 __global__ void __launch_bounds__(ROUTER_KPARTS * 32)
 router_logits_tiled_kernel(const float* __restrict__ x, const TW* __restrict__ w, const float* __restrict__ bias, int n, int hidden, int experts,
                            int top_k, int mode, float score_scale, float* __restrict__ logits, int* __restrict__ ids,
@@ -366,13 +369,25 @@ router_logits_tiled_kernel(const float* __restrict__ x, const TW* __restrict__ w
         }
     }
   }
+  {
+    constexpr int N = ROUTER_TOK * ROUTER_EXP;
+    float v[N];
 #pragma unroll
-  for (int tt = 0; tt < ROUTER_TOK; ++tt)
+    for (int i = 0; i < N; ++i) v[i] = acc[i / ROUTER_EXP][i % ROUTER_EXP];
+    int mine = 0;
 #pragma unroll
-    for (int e = 0; e < ROUTER_EXP; ++e) {
-      const float v = hb::warp_sum(acc[tt][e]);
-      if (lane == 0) partial[part][tt][e] = v;
+    for (int half = N / 2, off = 16; off >= 1; half >>= 1, off >>= 1) {
+      const bool up = lane & off;
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const float give = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+      }
+      mine += up ? half : 0;
     }
+#pragma unroll
+    for (int i = 0; i < N / 32; ++i) partial[part][(mine + i) / ROUTER_EXP][(mine + i) % ROUTER_EXP] = v[i];
+  }
   __syncthreads();
   if (threadIdx.x < ROUTER_TOK * ROUTER_EXP) {
     const int tt = threadIdx.x / ROUTER_EXP, e = threadIdx.x % ROUTER_EXP;
@@ -693,15 +708,19 @@ int router_launch(const void* x, int x_dtype, const void* w, int w_dtype, const 
     // many tokens (measured: faster than one block per token from about 100): register tiles of
     // 4 tokens x 16 experts; with more than 16 experts the
     // selection needs the stored logits of all block columns
-    dim3 grid((n + ROUTER_TOK - 1) / ROUTER_TOK, (experts + ROUTER_EXP - 1) / ROUTER_EXP);
+    const int columns = experts <= 8 ? 8 : 16;
+    dim3 grid((n + ROUTER_TOK - 1) / ROUTER_TOK, (experts + columns - 1) / columns);
     if (grid.y > 1 && !logits_out) return HB_ERR_BAD_ARG;
     if (grid.y > 65535) return HB_ERR_UNSUPPORTED;
-    if (w_dtype == HB_DTYPE_F32)
-      router_logits_tiled_kernel<float><<<grid, ROUTER_KPARTS * 32, 0, stream>>>(
-          (const float*)x, (const float*)w, bias, n, hidden, experts, top_k, mode, score_scale, logits_out, ids, scores);
-    else
-      router_logits_tiled_kernel<__nv_bfloat16><<<grid, ROUTER_KPARTS * 32, 0, stream>>>(
-          (const float*)x, (const __nv_bfloat16*)w, bias, n, hidden, experts, top_k, mode, score_scale, logits_out, ids, scores);
+#define HB_ROUTER_TILED(TW, EXP)                                                                                        \
+  router_logits_tiled_kernel<TW, EXP><<<grid, ROUTER_KPARTS * 32, 0, stream>>>(                                         \
+      (const float*)x, (const TW*)w, bias, n, hidden, experts, top_k, mode, score_scale, logits_out, ids, scores)
+    if (w_dtype == HB_DTYPE_F32) {
+      if (columns == 8) HB_ROUTER_TILED(float, 8); else HB_ROUTER_TILED(float, 16);
+    } else {
+      if (columns == 8) HB_ROUTER_TILED(__nv_bfloat16, 8); else HB_ROUTER_TILED(__nv_bfloat16, 16);
+    }
+#undef HB_ROUTER_TILED
     HB_LAUNCH_CHECK();
     if (grid.y > 1) {
       router_select_kernel<<<(n + 127) / 128, 128, 0, stream>>>(logits_out, n, experts, top_k, mode, score_scale, ids, scores);

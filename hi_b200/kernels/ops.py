@@ -637,7 +637,8 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Op
     S <- decay * S (per row); u = beta (v - S^T k); S <- S + k u^T; o = S^T q. Returns o float32 [N, heads*vdim].
     ``general`` forces the kernel that keeps S in shared memory (any dim) instead of registers (dim <= 256);
     ``rows`` (16, 32) forces how many rows of a column a lane holds, else ``single_tokens`` (every request
-    brings one token) decides: the order of the sums differs between the forms, by rounding only.
+    brings one token) decides: the order of the sums differs between the forms, by rounding only. Steps of enough tokens
+    go sixteen tokens at a time (``_chunked_recurrence``; dim <= 128).
     ``plain``: the rule without the correction, S <- decay * S + k v^T; o = S^T q (``beta`` is not read)."""
     for t, nm in ((q, "q"), (k, "k"), (v, "v"), (decay, "decay"), (state, "state")) + (() if plain else ((beta, "beta"),)):
         _need(t, nm, torch.float32)
@@ -1089,6 +1090,7 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
 PORTION_ROW_LENGTHS = (16, 32, 48, 64, 80, 96, 112, 128, 192)
 
 
+@functools.lru_cache(maxsize=256)
 def portion_attention_splits(blocks: int, keys: int) -> int:
     """How many blocks share a row tile's keys: the rounds of blocks (two on each of 148 SMs; later rounds fill up as blocks
     end) times the key tiles of a block and its fixed cost, plus the merge, at their least. Measured with 1 / 2 / 3 / 8 / 16
@@ -1293,6 +1295,7 @@ def sigmoid_prefill_attention_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages
     return sigmoid_merge(part_acc, positions, q.dtype, v_inv_freq, v_interleaved)
 
 
+@functools.lru_cache(maxsize=1024)           # a step's layers ask the same (a search over every number of splits)
 def _decode_splits(longest: int, groups: int) -> Tuple[int, int]:
     """How to cut ``longest`` keys for ``groups`` (token, kv head) pairs: the number of splits
     that minimises waves x (tiles per block + a block's fixed cost) + a cost per split (the
