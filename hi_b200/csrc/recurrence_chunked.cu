@@ -14,7 +14,7 @@
 //     outputs, which nothing waits for.
 //
 // Measured (B200, one request of 2,048 tokens, 16 heads of 128 x 128; before: token after token, a chain of 2,048 steps):
-// delta rule 582 -> 230 us (24 of them the matrices), the rule without correction 573 -> 163, mLSTM 437 -> 187; 32 heads of
+// delta rule 582 -> 230 us (24 of them the matrices), the rule without correction 573 -> 163, mLSTM 437 -> 184; 32 heads of
 // Mamba-2 709 -> 254. Error against 64 bits (2-norm, outputs / states): delta rule 9.1e-8 / 1.3e-7 -> 7.1e-8 / 7.0e-8, without
 // correction 1.4e-7 / 1.1e-7 -> 8.7e-8 / 5.4e-8. A chunk is 1.6 us of a block: 6,000 warp instructions, of which the
 // preparation of its rows is 40 %, between three barriers. Tried: the products as float32 fma (the shared-memory reads of 4 x 4
@@ -457,12 +457,24 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
     const T* kp = k + (size_t)t0 * a.q_ld;
     const T* qp = q + (size_t)t0 * a.q_ld;
     const float* gp = decay + (size_t)t0 * decay_ld;
+    // (one decay a head: most chunks have nothing to ask about; 10 us of the mLSTM's 173 on ragged portions. With a decay a
+    // row the same made the delta rule slower, 244 us for 235.)
+    if (SCALAR && count == C && d < a.dim && a.q_ld < (1 << 26)) {
+      const int ql = (int)a.q_ld, gl = (int)decay_ld;
 #pragma unroll
-    for (int t = 0; t < C; ++t, kp += a.q_ld, qp += a.q_ld, gp += decay_ld) {
-      const bool in = t < count && d < a.dim;
-      kr[t] = in ? *kp : hb::from_f32<T>(0.f);
-      qr[t] = in ? *qp : hb::from_f32<T>(0.f);
-      gr[t] = in ? *gp : 1.f;
+      for (int t = 0; t < C; ++t) {
+        kr[t] = kp[t * ql];
+        qr[t] = qp[t * ql];
+        gr[t] = gp[t * gl];
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < C; ++t, kp += a.q_ld, qp += a.q_ld, gp += decay_ld) {
+        const bool in = t < count && d < a.dim;
+        kr[t] = in ? *kp : hb::from_f32<T>(0.f);
+        qr[t] = in ? *qp : hb::from_f32<T>(0.f);
+        gr[t] = in ? *gp : 1.f;
+      }
     }
     const float4* m = reinterpret_cast<const float4*>(a.matrices + ((size_t)(unit0 + i) * a.heads + head) * (2 * C * C) + (PLAIN ? C * C : 0));
 #pragma unroll
