@@ -108,8 +108,11 @@ extern "C" int hb_skinny_linear(const void* x, long long x_ld, const void* w, co
   //   32000 x 2048 25.5 / 22.0, 202048 x 5120 294.7 / 290.4
   // For 9 to 16 tokens the library's wide kernels are the faster ones (8192 x 2048 8.4 / 9.9), its narrow ones are not
   // (2048 x 8192 13.3 / 11.0, 2048 x 2048 5.6 / 4.7, 128 x 2048 4.7 / 3.2).
+  // One token of wide rows of 4,096 and more: even alone, and beside the expert kernels of a step of one request the library
+  // is the faster one (Scout-sized, eight layers: 1.451 ms a step against 1.459). With 8 tokens it is the other way (routed
+  // experts beside the shared one of 16384 x 5120 and 5120 x 8192: 304 us against 328 with the library).
   const bool narrow = n_out <= 148 * 16;
-  if (tokens > 16 || (tokens > 8 && !narrow)) return HB_ERR_UNSUPPORTED;
+  if (tokens > 16 || (tokens > 8 && !narrow) || (tokens == 1 && n_out > 296 * 16 && K >= 4096)) return HB_ERR_UNSUPPORTED;
   if (tokens > 8)
     return K >= 4096 ? launch_skinny<2, 4, 512>(x, x_ld, w, bias, out, f, tokens, n_out, K, stream)
                      : launch_skinny<2, 2, 512>(x, x_ld, w, bias, out, f, tokens, n_out, K, stream);
