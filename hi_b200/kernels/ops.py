@@ -281,7 +281,13 @@ SKINNY_MOST_TOKENS = 16      # rows of x up to which the kernel may be the faste
 def skinny_linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
                   bias: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """``x @ weight.T (+ bias)`` for a few rows of bfloat16 ``x`` (its rows may be a column slice of a wider matrix), with
-    float32 sums, in ``out_dtype``; None for what the kernel does not take (sizes, strides, alignment) or is not the faster one for."""
+    float32 sums, in ``out_dtype``; None for what the kernel does not take (sizes, strides, alignment, operands on another GPU
+    or on the host beside ``x``, results that need gradients) or is not the faster one for."""
+    if not x.is_cuda:
+        raise KernelError("x must be a CUDA tensor; this engine has no CPU path")
+    if weight.device != x.device or (bias is not None and bias.device != x.device) or x.device.index != torch.cuda.current_device() or \
+            (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad))):
+        return None
     (n, k), (m, k2) = x.shape, weight.shape
     if not 0 < n <= SKINNY_MOST_TOKENS or k != k2 or k % 8 or k == 0 or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or \
             x.stride(1) != 1 or (n > 1 and x.stride(0) % 8) or not weight.is_contiguous() or \

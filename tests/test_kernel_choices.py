@@ -1,4 +1,7 @@
-"""Decisions that the Python side takes for the kernels, as plain functions of sizes. No GPU."""
+"""Decisions that the Python side takes for the kernels, as plain functions of sizes and operands. No GPU."""
+import pytest
+import torch
+
 from hi_b200.kernels import ops
 
 
@@ -31,3 +34,28 @@ def test_key_shares_of_any_mix_of_portions():
         assert shares(portions) == 1, portions
     for hd in (64, 128, 192):
         assert 1 <= shares([(50000, 1)], nh=1, hd=hd) <= 8
+
+
+def test_products_of_a_few_rows_leave_foreign_operands_to_the_library(monkeypatch):
+    """What is not on x's GPU, or x not on the current one, or wants gradients never reaches the kernel as a pointer."""
+    class OnGpu(torch.Tensor):                # a host tensor that says it is on a GPU: no pointer of it may be used
+        where = 0
+        is_cuda = property(lambda self: True)
+        device = property(lambda self: torch.device("cuda", self.where))
+
+    def on(t, where=0):
+        t = t.as_subclass(OnGpu)
+        t.where = where
+        return t
+
+    monkeypatch.setattr(ops, "lib", lambda: pytest.fail("the kernel library was called"))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    bf16 = torch.bfloat16
+    x, w, b = torch.zeros(2, 16, dtype=bf16), torch.zeros(32, 16, dtype=bf16), torch.zeros(32, dtype=bf16)
+    assert ops.skinny_linear(on(x), w, bf16) is None
+    assert ops.skinny_linear(on(x), on(w), bf16, b) is None
+    assert ops.skinny_linear(on(x), on(w, 1), bf16) is None
+    assert ops.skinny_linear(on(x, 1), on(w, 1), bf16, on(b, 1)) is None
+    assert ops.skinny_linear(on(x), on(w).requires_grad_(), bf16) is None
+    with pytest.raises(ops.KernelError):
+        ops.skinny_linear(x, w, bf16)

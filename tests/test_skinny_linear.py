@@ -46,3 +46,16 @@ def test_what_is_left_to_the_library():
         assert got.shape == want.shape and (not got.numel() or float((got.double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max()))
     with pytest.raises(Exception):
         linear(x, w[:, :64].contiguous())
+
+
+def test_operands_on_the_host_are_refused_and_gradients_kept():
+    from hi_b200.parts.linear import linear
+
+    x, w = torch.randn(4, 72, device=DEV).to(torch.bfloat16), torch.randn(33, 72, device=DEV).to(torch.bfloat16)
+    for weight, bias in ((w.cpu(), None), (w, torch.zeros(33, dtype=torch.bfloat16))):
+        with pytest.raises(RuntimeError):
+            linear(x, weight, bias=bias)
+    w.requires_grad_()
+    linear(x, w).float().sum().backward()
+    want = x.double().sum(0).expand_as(w)                # four terms in float32, rounded to bfloat16: 2^-9 of the value
+    assert float((w.grad.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
