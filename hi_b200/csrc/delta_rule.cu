@@ -381,8 +381,8 @@ __global__ void __launch_bounds__(kSingleThreads) delta_single_kernel(const Recu
   __shared__ float4 part[2][GROUPS][LC];          // s'.k and s'.q of a group's rows
   __shared__ float kq_part[GROUPS];
   const int head = blockIdx.y, seq = blockIdx.z, lane = threadIdx.x % LC, group = threadIdx.x / LC;
-  const int t = a.cu_seqlens[seq];
-  if (t >= a.cu_seqlens[seq + 1]) return;
+  const int first = a.cu_seqlens[seq], last = a.cu_seqlens[seq + 1];
+  if (first >= last) return;
   const int kvhead = head / (a.heads / a.kvh), col = blockIdx.x * COLS + lane * 4, row0 = group * ROWS;
   const bool live = col < a.vdim;
   float* S = a.state + (size_t)a.slots[seq] * a.state_stride + (size_t)head * a.dim * a.vdim + col;
@@ -390,66 +390,71 @@ __global__ void __launch_bounds__(kSingleThreads) delta_single_kernel(const Recu
 #pragma unroll
   for (int r = 0; r < ROWS; ++r)
     s[r] = live && row0 + r < a.dim ? __ldcs(reinterpret_cast<const float4*>(S + (size_t)(row0 + r) * a.vdim)) : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float* kp = a.k + (size_t)t * a.kvh * a.dim + (size_t)kvhead * a.dim + row0;
-  const float* qp = a.q + (size_t)t * a.kvh * a.dim + (size_t)kvhead * a.dim + row0;
-  const float* gp = a.decay + (size_t)t * a.heads * a.dim + (size_t)head * a.dim + row0;
-  const size_t at = (size_t)t * a.heads * a.vdim + (size_t)head * a.vdim + col;
-  const float4 v = live ? *reinterpret_cast<const float4*>(a.v + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float beta = a.plain ? 1.f : a.beta[(size_t)t * a.heads + head];
-  float4 sk[2], sq[2];
-  float kq[2] = {0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < 2; ++i) sk[i] = sq[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int r = 0; r < ROWS; ++r) {
-    const bool in = row0 + r < a.dim;
-    const float k = in ? kp[r] : 0.f, q = in ? qp[r] : 0.f, g = in ? gp[r] : 1.f;
-    float4& x = s[r];
-    float4 &d = sk[r & 1], &o = sq[r & 1];
-    x.x *= g; x.y *= g; x.z *= g; x.w *= g;
-    d.x = fmaf(x.x, k, d.x); d.y = fmaf(x.y, k, d.y); d.z = fmaf(x.z, k, d.z); d.w = fmaf(x.w, k, d.w);
-    o.x = fmaf(x.x, q, o.x); o.y = fmaf(x.y, q, o.y); o.z = fmaf(x.z, q, o.z); o.w = fmaf(x.w, q, o.w);
-    kq[r & 1] = fmaf(k, q, kq[r & 1]);
-  }
   auto add = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
-  part[0][group][lane] = add(sk[0], sk[1]);
-  part[1][group][lane] = add(sq[0], sq[1]);
-  if (lane == 0) kq_part[group] = kq[0] + kq[1];
-  __syncthreads();
-  // neighbours first, the same order for every thread
-  auto all = [&](int which) {
-    float4 x[GROUPS];
+  // (one token as a rule: the step says so. A request that brings more of them is right here all the same.)
+#pragma unroll 1
+  for (int t = first; t < last; ++t) {
+    if (t > first) __syncthreads();                // the sums of the token before are read
+    const float* kp = a.k + (size_t)t * a.kvh * a.dim + (size_t)kvhead * a.dim + row0;
+    const float* qp = a.q + (size_t)t * a.kvh * a.dim + (size_t)kvhead * a.dim + row0;
+    const float* gp = a.decay + (size_t)t * a.heads * a.dim + (size_t)head * a.dim + row0;
+    const size_t at = (size_t)t * a.heads * a.vdim + (size_t)head * a.vdim + col;
+    const float4 v = live ? *reinterpret_cast<const float4*>(a.v + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float beta = a.plain ? 1.f : a.beta[(size_t)t * a.heads + head];
+    float4 sk[2], sq[2];
+    float kq[2] = {0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < GROUPS; ++i) x[i] = part[which][i][lane];
+    for (int i = 0; i < 2; ++i) sk[i] = sq[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int step = 1; step < GROUPS; step *= 2)
+    for (int r = 0; r < ROWS; ++r) {
+      const bool in = row0 + r < a.dim;
+      const float k = in ? kp[r] : 0.f, q = in ? qp[r] : 0.f, g = in ? gp[r] : 1.f;
+      float4& x = s[r];
+      float4 &d = sk[r & 1], &o = sq[r & 1];
+      x.x *= g; x.y *= g; x.z *= g; x.w *= g;
+      d.x = fmaf(x.x, k, d.x); d.y = fmaf(x.y, k, d.y); d.z = fmaf(x.z, k, d.z); d.w = fmaf(x.w, k, d.w);
+      o.x = fmaf(x.x, q, o.x); o.y = fmaf(x.y, q, o.y); o.z = fmaf(x.z, q, o.z); o.w = fmaf(x.w, q, o.w);
+      kq[r & 1] = fmaf(k, q, kq[r & 1]);
+    }
+    part[0][group][lane] = add(sk[0], sk[1]);
+    part[1][group][lane] = add(sq[0], sq[1]);
+    if (lane == 0) kq_part[group] = kq[0] + kq[1];
+    __syncthreads();
+    // neighbours first, the same order for every thread
+    auto all = [&](int which) {
+      float4 x[GROUPS];
 #pragma unroll
-      for (int i = 0; i < GROUPS; i += 2 * step) x[i] = add(x[i], x[i + step]);
-    return x[0];
-  };
-  float4 u = v;
-  if (!a.plain) {
-    const float4 d = all(0);
-    u = make_float4(beta * (v.x - d.x), beta * (v.y - d.y), beta * (v.z - d.z), beta * (v.w - d.w));
-  }
+      for (int i = 0; i < GROUPS; ++i) x[i] = part[which][i][lane];
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r) {
-    if (!live || row0 + r >= a.dim) continue;
-    const float k = kp[r];
-    *reinterpret_cast<float4*>(S + (size_t)(row0 + r) * a.vdim) =
-        make_float4(fmaf(k, u.x, s[r].x), fmaf(k, u.y, s[r].y), fmaf(k, u.z, s[r].z), fmaf(k, u.w, s[r].w));
-  }
-  if (group == 0 && live) {
-    float kqs[GROUPS];
+      for (int step = 1; step < GROUPS; step *= 2)
 #pragma unroll
-    for (int i = 0; i < GROUPS; ++i) kqs[i] = kq_part[i];
+        for (int i = 0; i < GROUPS; i += 2 * step) x[i] = add(x[i], x[i + step]);
+      return x[0];
+    };
+    float4 u = v;
+    if (!a.plain) {
+      const float4 d = all(0);
+      u = make_float4(beta * (v.x - d.x), beta * (v.y - d.y), beta * (v.z - d.z), beta * (v.w - d.w));
+    }
 #pragma unroll
-    for (int step = 1; step < GROUPS; step *= 2)
+    for (int r = 0; r < ROWS; ++r) {
+      if (!live || row0 + r >= a.dim) continue;
+      const float k = kp[r];
+      s[r] = make_float4(fmaf(k, u.x, s[r].x), fmaf(k, u.y, s[r].y), fmaf(k, u.z, s[r].z), fmaf(k, u.w, s[r].w));
+      if (t + 1 == last) *reinterpret_cast<float4*>(S + (size_t)(row0 + r) * a.vdim) = s[r];
+    }
+    if (group == 0 && live) {
+      float kqs[GROUPS];
 #pragma unroll
-      for (int i = 0; i < GROUPS; i += 2 * step) kqs[i] += kqs[i + step];
-    const float4 o = all(1);
-    *reinterpret_cast<float4*>(a.out + at) =
-        make_float4(fmaf(u.x, kqs[0], o.x), fmaf(u.y, kqs[0], o.y), fmaf(u.z, kqs[0], o.z), fmaf(u.w, kqs[0], o.w));
+      for (int i = 0; i < GROUPS; ++i) kqs[i] = kq_part[i];
+#pragma unroll
+      for (int step = 1; step < GROUPS; step *= 2)
+#pragma unroll
+        for (int i = 0; i < GROUPS; i += 2 * step) kqs[i] += kqs[i + step];
+      const float4 o = all(1);
+      *reinterpret_cast<float4*>(a.out + at) =
+          make_float4(fmaf(u.x, kqs[0], o.x), fmaf(u.y, kqs[0], o.y), fmaf(u.z, kqs[0], o.z), fmaf(u.w, kqs[0], o.w));
+    }
   }
 }
 

@@ -111,30 +111,34 @@ def test_what_is_not_finite_stays_with_later_tokens_and_its_column():
     assert torch.equal(got[other], clean[other])
 
 
+@pytest.mark.parametrize("lens", [[1] * 5, [3, 0, 1], [2, 40]])
 @pytest.mark.parametrize("plain", [False, True])
 @pytest.mark.parametrize("heads,kvh,dim,vdim", [(4, 2, 128, 128), (3, 1, 48, 4), (2, 2, 64, 64), (6, 2, 100, 68), (2, 1, 127, 132)])
-def test_single_tokens_by_whole_lines(heads, kvh, dim, vdim, plain):
-    """One token of each of five requests, states in rows of whole 16 bytes: outputs and states against float64."""
+def test_single_tokens_by_whole_lines(heads, kvh, dim, vdim, plain, lens):
+    """A step said to bring one token a request, states in rows of whole 16 bytes: outputs and states against float64. What
+    the step is said to bring decides the order of the sums only: requests that bring none or several are right too."""
     from hi_b200.kernels import ops
 
-    n, g = 5, torch.Generator().manual_seed(dim + vdim)
+    n, g = sum(lens), torch.Generator().manual_seed(dim + vdim)
     rnd = lambda *s: torch.randn(*s, generator=g)
     q, k = (F.normalize(rnd(n, kvh, dim), dim=-1).reshape(n, -1) for _ in range(2))
     v, beta, decay = rnd(n, heads * vdim), torch.rand(n, heads, generator=g), torch.rand(n, heads * dim, generator=g)
-    cu, slots = tables([1] * n)
-    state = rnd(n + 2, heads * dim * vdim + 4)
+    cu, slots = tables(lens)
+    state = rnd(len(lens) + 2, heads * dim * vdim + 4)
     dev = state.to(DEV)
     o = ops.delta_recurrence(q.to(DEV), k.to(DEV), v.to(DEV), None if plain else beta.to(DEV), decay.to(DEV), dev, cu.to(DEV),
                              slots.to(DEV), heads, kvh, dim, vdim, single_tokens=True, plain=plain).cpu()
     dev = dev.cpu()
-    for t, slot in enumerate(slots.tolist()):
-        wide = lambda x: x[t].double().view(kvh, dim).repeat_interleave(heads // kvh, dim=0)
-        S = state[slot, : heads * dim * vdim].double().view(heads, dim, vdim) * decay[t].double().view(heads, dim, 1)
-        vt = v[t].double().view(heads, vdim)
-        u = vt if plain else beta[t].double()[:, None] * (vt - torch.einsum("hdv,hd->hv", S, wide(k)))
-        S = S + wide(k)[:, :, None] * u[:, None, :]
-        close(o[t], torch.einsum("hdv,hd->hv", S, wide(q)).reshape(-1), f"output {t}")
-        close(dev[slot, : heads * dim * vdim], S.reshape(-1), f"state {t}")
+    for i, slot in enumerate(slots.tolist()):
+        S = state[slot, : heads * dim * vdim].double().view(heads, dim, vdim)
+        for t in range(int(cu[i]), int(cu[i + 1])):
+            wide = lambda x: x[t].double().view(kvh, dim).repeat_interleave(heads // kvh, dim=0)
+            S = S * decay[t].double().view(heads, dim, 1)
+            vt = v[t].double().view(heads, vdim)
+            u = vt if plain else beta[t].double()[:, None] * (vt - torch.einsum("hdv,hd->hv", S, wide(k)))
+            S = S + wide(k)[:, :, None] * u[:, None, :]
+            close(o[t], torch.einsum("hdv,hd->hv", S, wide(q)).reshape(-1), f"output {t}")
+        close(dev[slot, : heads * dim * vdim], S.reshape(-1), f"state {slot}")
         assert torch.equal(dev[slot, heads * dim * vdim:], state[slot, heads * dim * vdim:])
-    for slot in set(range(n + 2)) - set(slots.tolist()):
+    for slot in set(range(len(lens) + 2)) - set(slots.tolist()):
         assert torch.equal(dev[slot], state[slot])
