@@ -154,20 +154,21 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ x, const void* __rest
 
 // The same for steps of many rows (no row_map): a block walks rows gridDim apart and asks for the rows NORM_AHEAD ahead while
 // it works on one, by cp.async into a place of the thread's own in shared memory (a thread reads back only what it asked for
-// itself, so arrival needs no barrier); the weight stays in registers, and the row's sum takes one barrier. What bounds it is
+// itself, so arrival needs no barrier: its plain loads must stay behind the wait and ahead of the next request, which is what
+// the "memory" of these statements says); the weight stays in registers, and the row's sum takes one barrier. What bounds it is
 // HBM; the kernel above, a row a block, waits for its loads, sums and writes in turn.
 // Measured, 2,048 rows of 5,120, a block a row against this (and the bytes at the copy rate): the norm alone 22.6 / 17.2 us
 // (9.7), with a bfloat16 delta 39.9 / 26.9 (19.4), with two routed rows and the float32 copy too 67.0 / 56.5 (38.7).
 constexpr int NORM_AHEAD = 2, NORM_STREAM_ROWS = 512;
 
 __device__ __forceinline__ void ask16(void* to, const void* from) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
 }
 __device__ __forceinline__ void ask8(void* to, const void* from) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
 }
 __device__ __forceinline__ void ask4(void* to, const void* from) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
 }
 
 struct NormArgs {
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_stream_kernel(const NormArgs 
       if (a.routed && a.routed_weight && lane < a.top_k)
         ask4(st + at_f + (warp * 8 + lane) * 4, a.routed_weight + (size_t)r * a.top_k + lane);
     }
-    asm volatile("cp.async.commit_group;");
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int step = gridDim.x;
   int r = blockIdx.x;
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_stream_kernel(const NormArgs 
   find(r + NORM_AHEAD * step);
   for (int n = 0; r < a.rows; ++n, r += step) {
     unsigned char* st = stages + (size_t)(n % NORM_AHEAD) * stage_bytes;
-    asm volatile("cp.async.wait_group %0;" ::"n"(NORM_AHEAD - 1));
+    asm volatile("cp.async.wait_group %0;" ::"n"(NORM_AHEAD - 1) : "memory");
     if (a.routed_weight) __syncwarp();                          // the factors came by the warp's first lanes
     float4 v[NG];
     float ss = 0.f;
@@ -285,10 +286,10 @@ __global__ void __launch_bounds__(512) add_rmsnorm_stream_kernel(const NormArgs 
       }
     }
   }
-  asm volatile("cp.async.wait_group 0;");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// Shared memory of a block, or 0 where the rows are too long for the streaming form.
+// Blocks of the streaming form: as many an SM as their stages leave room for (at most four).
 template <int NG>
 int launch_norm_stream(const NormArgs& a, int threads, int stage_bytes, cudaStream_t stream) {
   const int smem = NORM_AHEAD * stage_bytes;

@@ -42,3 +42,22 @@ def test_norm_and_combine(rows, hidden, top_k, weighted, dtype):
     many = ops.add_rmsnorm(x0.clone(), delta, w, 1e-5, torch.float32, x_scale=kw["x_scale"], delta2=delta2)
     many = many[: len(one)]
     assert float((one - many).abs().max()) <= 2e-6 * float(one.abs().max())      # the order of a row's squares differs
+
+
+@pytest.mark.parametrize("rows,hidden", [(2048, 2048), (1905, 2048), (513, 8188), (2050, 5120)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_norm_alone(rows, hidden, out_dtype):
+    """Nothing to add: from 3.9 million numbers on the streaming form, which leaves the stream as it is, to the bit."""
+    from hi_b200.kernels import ops
+
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    x0, w = torch.randn(rows, hidden, device=DEV, generator=g), 1 + 0.1 * torch.randn(hidden, device=DEV, generator=g)
+    x0[7, 5], x0[9] = float("inf"), float("nan")               # each stays in its row
+    fine = torch.ones(rows, dtype=torch.bool, device=DEV)
+    fine[7] = fine[9] = False
+    want = x0.double() / torch.sqrt((x0.double() ** 2).mean(1, keepdim=True) + 1e-5) * w.double()
+    x = x0.clone()
+    y, y32 = ops.add_rmsnorm(x, None, w, 1e-5, out_dtype, also_f32=True)
+    assert torch.equal(x.view(torch.int32), x0.view(torch.int32))
+    assert float((y32 - want)[fine].abs().max()) <= 2e-6 * float(want[fine].abs().max())
+    assert torch.equal(y[fine], y32[fine].to(out_dtype)) and bool(torch.isnan(y[9]).all()) and bool(torch.isnan(y[7, 5]))
