@@ -5,7 +5,8 @@
 // three bfloat16 pieces each that sum to them exactly (8 + 8 + 8 bits), and the six products of pieces down to 2^-24 of the
 // whole are summed in float32: the large one by itself and added with float32's own rounding, since a tensor core cuts a sum
 // where it does not fit. Maximum, exponentials and sums are float32 as in the general kernel, and so are the rules of what a
-// token may read (see attention.cu); a value that is not finite reaches only the rows that may read it.
+// token may read (see attention.cu). A value that is not finite reaches only the rows that may read it; a score that comes
+// out not finite (an infinite key may weigh nothing) is worked out again as the general kernel does.
 //
 // What bounds it: mma.sync, at 2 cycles of an SM for [16, 16] x [16, 8], six of them a product (0.4 of the time), and the
 // chains between them: a block of four warps splits, multiplies and takes exponentials in turn, two blocks per SM (104 KB of
@@ -42,15 +43,6 @@ struct PortionArgs {
   float* part_ml;               // [N * nh, splits, 2]
 };
 
-__device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
-  p[0] = hb::pack_bf16(x, y);
-  x -= __uint_as_float(p[0] << 16);
-  y -= __uint_as_float(p[0] & 0xffff0000u);
-  p[1] = hb::pack_bf16(x, y);
-  x -= __uint_as_float(p[1] << 16);
-  y -= __uint_as_float(p[1] & 0xffff0000u);
-  p[2] = hb::pack_bf16(x, y);
-}
 __device__ __forceinline__ void mma16(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -61,8 +53,8 @@ __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466
 template <int PIECE>
 __device__ __forceinline__ void put4(__nv_bfloat16* at, float4 v) {
   uint32_t a[3], b[3];
-  split3(v.x, v.y, a);
-  split3(v.z, v.w, b);
+  hb::split3(v.x, v.y, a);
+  hb::split3(v.z, v.w, b);
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(at + i * PIECE) = make_uint2(a[i], b[i]);
 }
@@ -225,17 +217,41 @@ __global__ void __launch_bounds__(32 * WARPS, NT <= 8 ? 2 : 1) portion_attention
     store(vs);                              // read last before the end of the tile before this one
     const int any_odd = __syncthreads_or(odd);          // ... and all warps are through with the keys
     if (tile + 1 < tile1) load(a.k_pages, offs[(tile + 1) & 1]);
+    auto seen = [&](int i, int at) {
+      const int key = key0 + at;
+      return key <= pos[i] && (key >= lo[i] || key < kept[i]) && off_of[at] >= 0;
+    };
+    bool again = false;                     // a score that is not finite
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s[n][e] = (s[n][e] + lo_s[n][e]) * a.scale;
+        again |= !finite(s[n][e]);
+      }
+    if (again)
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = e >> 1, at = n * 8 + 2 * q4 + (e & 1);
+          if (finite(s[n][e]) || !seen(i, at)) continue;
+          const float *qr = a.q + th[i] * HD, *kr = a.k_pages + off_of[at];
+          float dot = 0.f;
+#pragma unroll 1
+          for (int d = 0; d < HD; ++d) dot += (qr[d] * a.scale) * kr[d];
+          s[n][e] = dot;
+        }
     float most[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int i = e >> 1, at = n * 8 + 2 * q4 + (e & 1), key = key0 + at;
-        float x = (s[n][e] + lo_s[n][e]) * a.scale;
+        const int i = e >> 1, at = n * 8 + 2 * q4 + (e & 1);
+        float x = s[n][e];
         if (a.softcap > 0.f) x = a.softcap * tanhf(x * inv_cap);
-        x -= slope[i] * (float)(pos[i] - key);
-        const bool seen = key <= pos[i] && (key >= lo[i] || key < kept[i]) && off_of[at] >= 0;
-        s[n][e] = seen ? x : -INFINITY;
+        x -= slope[i] * (float)(pos[i] - key0 - at);
+        s[n][e] = seen(i, at) ? x : -INFINITY;
         most[i] = fmaxf(most[i], s[n][e]);
       }
     float corr[2];
@@ -264,7 +280,7 @@ __global__ void __launch_bounds__(32 * WARPS, NT <= 8 ? 2 : 1) portion_attention
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         uint32_t p[3];
-        split3(s[2 * kk + (e >> 1)][2 * (e & 1)], s[2 * kk + (e >> 1)][2 * (e & 1) + 1], p);
+        hb::split3(s[2 * kk + (e >> 1)][2 * (e & 1)], s[2 * kk + (e >> 1)][2 * (e & 1) + 1], p);
 #pragma unroll
         for (int x = 0; x < 3; ++x) pa[kk][x][e] = p[x];
       }

@@ -33,5 +33,25 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<unsigned*>(&v);
 }
+// the same held to bfloat16's largest finite value (a NaN stays one)
+__device__ __forceinline__ unsigned pack_bf16_sat(float lo, float hi) {
+  unsigned r;
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+
+// Two floats as three pairs of bfloat16 that sum to them exactly (8 + 8 + 8 bits): the six products of pieces down to
+// 2^-24 of the whole, on the tensor cores with float32 sums, are a float32 product's. Floats above bfloat16's largest value
+// (3.39e38) would round to infinity: the first piece stops at that value and the other two hold the rest, so any finite
+// float has finite pieces. Of what is not finite at least one piece is NaN, and so is every product of it.
+__device__ __forceinline__ void split3(float x, float y, unsigned (&p)[3]) {
+  p[0] = pack_bf16_sat(x, y);
+  x -= __uint_as_float(p[0] << 16);
+  y -= __uint_as_float(p[0] & 0xffff0000u);
+  p[1] = pack_bf16(x, y);
+  x -= __uint_as_float(p[1] << 16);
+  y -= __uint_as_float(p[1] & 0xffff0000u);
+  p[2] = pack_bf16(x, y);
+}
 
 }  // namespace hb

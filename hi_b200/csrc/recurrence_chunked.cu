@@ -9,7 +9,7 @@
 //   chunk_matrices_kernel   T and B of all chunks and heads, side by side (they need no state)
 //   chunk_recurrence_kernel per (request, head, 16 or 32 columns of S): chunk after chunk. NW warps own 16 rows of S each,
 //     in registers as accumulator tiles; their products run on the tensor cores with every float32 factor as three
-//     bfloat16 pieces (see split3), and the sums over all rows are brought together in shared memory in a fixed order.
+//     bfloat16 pieces (see hb::split3), and the sums over all rows are brought together in shared memory in a fixed order.
 //     NW more warps, in two groups that take turns, prepare the next chunk's rows (decay products) and write the chunk's
 //     outputs, which nothing waits for.
 //
@@ -20,7 +20,8 @@
 // preparation of its rows is 40 %, between three barriers. Tried: the products as float32 fma (the shared-memory reads of 4 x 4
 // tiles bound it: 293 us); two tf32 pieces a factor (error 1.1e-7, states of Mamba-2 1.9 times as far off: taken back).
 //
-// What is not finite in a token's inputs reaches that token's and later outputs of the request, never an earlier one.
+// What is not finite in a token's inputs reaches that token's and later outputs of the request, never an earlier one (an
+// infinite value or state comes out of the products as NaN, where token after token the sum could stay infinite).
 #include "api.h"
 #include "common.cuh"
 #include "mma.cuh"
@@ -201,23 +202,16 @@ __global__ void __launch_bounds__(128) chunk_matrices_kernel(const ChunkArgs a) 
   }
 }
 
-// Two floats as three pairs of bfloat16 that sum to them exactly (8 + 8 + 8 bits): the six products of pieces down to
-// 2^-24 of the whole, on the tensor cores with float32 sums, are a float32 product's.
-__device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
-  p[0] = hb::pack_bf16(x, y);
-  x -= __uint_as_float(p[0] << 16);
-  y -= __uint_as_float(p[0] & 0xffff0000u);
-  p[1] = hb::pack_bf16(x, y);
-  x -= __uint_as_float(p[1] << 16);
-  y -= __uint_as_float(p[1] & 0xffff0000u);
-  p[2] = hb::pack_bf16(x, y);
-}
+// the pieces of hb::split3, of one float
 __device__ __forceinline__ void put_pieces(__nv_bfloat16* at, int step, float x) {
+  unsigned short first;
+  asm("cvt.rn.satfinite.bf16.f32 %0, %1;" : "=h"(first) : "f"(x));
+  __nv_bfloat16 h = __ushort_as_bfloat16(first);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat16 h = __float2bfloat16_rn(x);
     at[i * step] = h;
     x -= __bfloat162float(h);
+    h = __float2bfloat16_rn(x);
   }
 }
 __device__ __forceinline__ void mma16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -319,7 +313,7 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           uint32_t p[3];
-          split3(s[m][e >> 1][2 * (e & 1)], s[m][e >> 1][2 * (e & 1) + 1], p);
+          hb::split3(s[m][e >> 1][2 * (e & 1)], s[m][e >> 1][2 * (e & 1) + 1], p);
 #pragma unroll
           for (int x = 0; x < 3; ++x) sp[m][x][e] = p[x];
         }
@@ -332,7 +326,7 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
           for (int h = 0; h < 2; ++h) {
             const float2 v = *reinterpret_cast<const float2*>(&st.p[row + 8 * n + g][warp * 16 + 8 * h + 2 * q4]);
             uint32_t p[3];
-            split3(v.x, v.y, p);
+            hb::split3(v.x, v.y, p);
 #pragma unroll
             for (int x = 0; x < 3; ++x) pp[n][x][h] = p[x];
           }
@@ -398,7 +392,7 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
         for (int h = 0; h < 2; ++h) {
           const float2 v = *reinterpret_cast<const float2*>(&st.rk[warp * 16 + 8 * n + g][8 * h + 2 * q4]);
           uint32_t p[3];
-          split3(v.x, v.y, p);
+          hb::split3(v.x, v.y, p);
 #pragma unroll
           for (int x = 0; x < 3; ++x) rp[n][x][h] = p[x];
         }

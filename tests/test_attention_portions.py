@@ -115,6 +115,52 @@ def test_shared_keys_holes_and_what_is_not_finite(monkeypatch):
     assert float((got[other].double() - want[other]).abs().max() / want.abs().max()) <= TOL
 
 
+def test_the_ends_of_the_range():
+    """Finite numbers above bfloat16's largest (3.39e38) and infinite keys and queries: hidden ones change nothing for the
+    rows that may not read them, a score of minus infinity weighs nothing, and a query reaches its own row only."""
+    top = 3.4e38
+    portions = [(70, 100)]
+    q, k, v, table, cu, pos = setup(4, 2, 64, 16, portions, seed=5)
+    args = (table, portions, 0, 0, 0, 0.125)
+    at = 140                                              # the key of the 41st new token, hidden from the forty before it
+    page, row = table[0, at // 16].long(), at % 16
+
+    vt = v.clone()
+    vt[page, 0, row, 3], vt[page, 1, row, 7] = top, -top
+    got, want = run((q, k, vt, table, cu, pos), portions), reference(q, k, vt, *args)
+    read = torch.zeros_like(got, dtype=torch.bool)
+    read[40:, :2, 3] = read[40:, 2:, 7] = True
+    assert float((got[read].double() - want[read]).abs().max()) <= TOL * top
+    close(got[~read], want[~read])
+
+    signs = torch.where(q[:, :2, 5].abs() > 0.02, q[:, :2, 5].sign(), torch.zeros(()))
+    for big in (top, float("inf")):                       # the key outweighs everything or weighs nothing, as the query's sign says
+        kt = k.clone()
+        kt[page, 0, row, 5] = big
+        got = run((q, kt, v, table, cu, pos), portions)
+        plain = reference(q, k, v, *args)
+        close(got[:40], plain[:40])
+        close(got[:, 2:], plain[:, 2:])
+        kt[page, 0, row, 5] = 1e30                        # (finite in float64 and in the reference's softmax)
+        want = reference(q, kt, v, *args)
+        nothing, all_of_it = torch.zeros(70, 4, dtype=torch.bool), torch.zeros(70, 4, dtype=torch.bool)
+        nothing[40:, :2], all_of_it[40:, :2] = signs[40:] < 0, signs[40:] > 0
+        assert bool(nothing.any()) and bool(all_of_it.any())
+        close(got[nothing], want[nothing])
+        if big == top:
+            close(got[all_of_it], want[all_of_it])
+        else:
+            assert not bool(torch.isfinite(got[all_of_it]).any())
+
+    qt = q.clone()
+    qt[12, 1, 9] = float("inf")
+    got, want = run((qt, k, v, table, cu, pos), portions), reference(q, k, v, *args)
+    other = torch.ones(70, 4, dtype=torch.bool)
+    other[12, 1] = False
+    close(got[other], want[other])
+    assert not bool(torch.isfinite(got[12, 1]).any())
+
+
 @pytest.mark.parametrize("hd", [64, 128, 192])
 @pytest.mark.parametrize("lens", [[1 + 128, 40], [31, 129 + 64], [97 + 128, 3], [33 + 256, 200]])
 def test_tiles_with_few_tokens_in_the_bfloat16_kernel(hd, lens):

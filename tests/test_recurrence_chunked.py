@@ -111,6 +111,47 @@ def test_what_is_not_finite_stays_with_later_tokens_and_its_column():
     assert torch.equal(got[other], clean[other])
 
 
+@pytest.mark.parametrize("plain", [False, True])
+def test_the_end_of_the_range(plain):
+    """Finite values and states above bfloat16's largest number (3.39e38): their own columns as in float64, the others as
+    without them. Keys of half a unit and decays below a half keep the float32 sums themselves in range."""
+    from hi_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(7)
+    n, heads, dim, vdim, top = 200, 2, 64, 48, 3.4e38
+    q, k = (0.5 * F.normalize(torch.randn(n, heads, dim, generator=g), dim=-1).reshape(n, -1) for _ in range(2))
+    v, beta = torch.randn(n, heads * vdim, generator=g), torch.rand(n, heads, generator=g)
+    decay = 0.1 + 0.3 * torch.rand(n, heads * dim, generator=g)
+    cu, slots = torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    state = torch.zeros(1, heads * dim * vdim)
+
+    def call():
+        s = state.to(DEV)
+        o = ops.delta_recurrence(q.to(DEV), k.to(DEV), v.to(DEV), None if plain else beta.to(DEV), decay.to(DEV), s, cu, slots, heads,
+                                 heads, dim, vdim, plain=plain)
+        return o.cpu(), s.cpu()
+
+    clean, clean_state = call()
+    v[70, 5], v[71, vdim + 3] = top, -top                 # head 0 column 5, head 1 column 3
+    state.view(heads, dim, vdim)[1, 2, 9] = top
+    got, got_state = call()
+    S, want = state.double().view(heads, dim, vdim).clone(), []
+    for t in range(n):
+        kt, qt, vt = (x[t].double().view(heads, -1) for x in (k, q, v))
+        S = S * decay[t].double().view(heads, dim, 1)
+        u = vt if plain else beta[t].double()[:, None] * (vt - torch.einsum("hdv,hd->hv", S, kt))
+        S = S + kt[:, :, None] * u[:, None, :]
+        want.append(torch.einsum("hdv,hd->hv", S, qt).reshape(-1))
+    want, touched = torch.stack(want), torch.zeros(heads * vdim, dtype=torch.bool)
+    touched[[5, vdim + 3, vdim + 9]] = True
+    for c in touched.nonzero().flatten().tolist():
+        close(got[:, c], want[:, c], f"column {c}")
+    assert torch.equal(got[:, ~touched], clean[:, ~touched])
+    rows = lambda s: s.view(heads, dim, vdim).permute(0, 2, 1).reshape(heads * vdim, dim)
+    assert torch.equal(rows(got_state)[~touched], rows(clean_state)[~touched])
+    close(rows(got_state)[touched], rows(S.float())[touched], "state")
+
+
 @pytest.mark.parametrize("lens", [[1] * 5, [3, 0, 1], [2, 40]])
 @pytest.mark.parametrize("plain", [False, True])
 @pytest.mark.parametrize("heads,kvh,dim,vdim", [(4, 2, 128, 128), (3, 1, 48, 4), (2, 2, 64, 64), (6, 2, 100, 68), (2, 1, 127, 132)])
