@@ -301,55 +301,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const float cap_l2 = a.softcap * 1.4426950408889634f;
     const float twice_over_cap = a.softcap > 0.f ? 2.f * a.scale_log2 / a.softcap : 0.f;
     bool ok = true;
-    auto clear_values = [&](int j, int key_base) {
-      const bool ragged = key_base / BKEYS == p_last / BKEYS && (p_last + 1) % BKEYS != 0;
-      // pages smaller than a tile: the window's first tile and the last tile of kept tokens may hold pages that were given back
-      const int walked = a.newest_first ? nt - 1 - j : j;
-      const bool holes = a.page_size < BKEYS && (walked == kept_tiles || walked + 1 == kept_tiles);
-      if (ragged || holes) {
-        // Value rows of positions past the portion's end hold whatever the page held before, and those of pages that
-        // were given back are any page's (another request's numbers, possibly not finite): P is zero there, but
-        // 0 x NaN is NaN. Once the V tile has landed, the threads of those rows zero them.
-        if (!__all_sync(0xffffffffu, tc::mbar_wait(&v_full[j & 1], (j >> 1) & 1))) {
-          if (lane == 0) atomicExch(a.status, 22);
-          return false;
-        }
-        if (r < BKEYS && (key_base + r > p_last ||
-                          (holes && a.block_table[(size_t)seq * a.table_stride + (key_base + r) / a.page_size] < 0))) {
-          uint8_t* vrow = v_s + (j & 1) * KBYTES + (r / 8) * 1024 + (r % 8) * 128;
-#pragma unroll
-          for (int blk = 0; blk < DBLK; ++blk)
-#pragma unroll
-            for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(vrow + blk * KVBLOCK + q * 16) = make_uint4(0, 0, 0, 0);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA
-      }
-      return true;
-    };
-    // A warp none of whose rows is a token only hands the barriers on: whatever lies in its rows of P, a row of the
-    // products reaches its own row of O alone, and those rows are not written. (With its softmax, which would start over in
-    // every tile of a row without a token, a portion of 513 tokens took 265 us behind 7,000 where 512 took 159.)
-    const bool idle = warp_row >= n_valid;
-    if (idle) {
-      for (int j = 0; j < nt && ok; ++j) {
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(&s_full[j & 1], (j >> 1) & 1));
-        if (!ok) {
-          if (lane == 0) atomicExch(a.status, 16);
-          break;
-        }
-        if (lane == 0) tc::mbar_arrive(&s_free[j & 1]);
-        if (j > 0) ok = __all_sync(0xffffffffu, tc::mbar_wait(pv_done, (j - 1) & 1));
-        if (!ok) {
-          if (lane == 0) atomicExch(a.status, 17);
-          break;
-        }
-        tc::fence_after();
-        ok = clear_values(j, tile_key0(j));
-        tc::fence_before();
-        __syncwarp();
-        if (ok && lane == 0) tc::mbar_arrive(p_ready);
-      }
-    } else
     for (int j = 0; j < nt && ok; ++j) {
       const int sb = j & 1;
       if (!__all_sync(0xffffffffu, tc::mbar_wait(&s_full[sb], (j >> 1) & 1))) {
@@ -361,7 +312,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int key_base = tile_key0(j);
       // a tile every row of this warp sees whole needs no masks (most tiles of a long prompt)
       const int warp_first_pos = p_first + warp_row;
-      // (rows past the portion's end take what the tile gives them: they are not written)
+      // (rows past the portion's end take what the tile gives them: they are not written. Masked, they cost their warp 2,000
+      // tokens in one portion 78 us where 2,048 take 71; now 71.)
       const bool interior = (key_base + BKEYS - 1 <= warp_first_pos) &&
                             (key_base >= first_visible(warp_first_pos + 31) || key_base + BKEYS <= a.keep);
       float sv[BKEYS];
@@ -420,8 +372,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       // moves (and O and l are rescaled) only when some row of the warp has grown by more than
       // 2^8, so P stays below 256 and most tiles skip the pass over O. The result is the same
       // sum, scaled by a common factor that the final division removes.
-      // A row that has seen nothing yet (no token, or all masked so far) has nothing to move to.
-      const bool move = !sigmoid && __any_sync(0xffffffffu, mx > m + 8.f || (m == -INFINITY && mx > m));
+      // A row that has seen nothing yet, -inf on both sides, has nothing to move to. (While it did, the rows past a portion's
+      // end started over in every tile: a portion of 513 tokens behind 7,000, 16 heads, took 219 us where it takes 66.)
+      const bool move = !sigmoid && __any_sync(0xffffffffu, mx > m + 8.f);
       float corr = 1.f;
       if (move) {
         corr = (m == -INFINITY) ? 0.f : fast_exp2(m - mx);
@@ -494,7 +447,29 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tc::st32_nowait(tmem + lane_addr + sb * S_COLS, packed);
         tc::wait_st();
       }
-      if (!clear_values(j, key_base)) { ok = false; break; }
+      const bool ragged = key_base / BKEYS == p_last / BKEYS && (p_last + 1) % BKEYS != 0;
+      // pages smaller than a tile: the window's first tile and the last tile of kept tokens may hold pages that were given back
+      const int walked = a.newest_first ? nt - 1 - j : j;
+      const bool holes = a.page_size < BKEYS && (walked == kept_tiles || walked + 1 == kept_tiles);
+      if (ragged || holes) {
+        // Value rows of positions past the portion's end hold whatever the page held before, and those of pages that
+        // were given back are any page's (another request's numbers, possibly not finite): P is zero there, but
+        // 0 x NaN is NaN. Once the V tile has landed, the threads of those rows zero them.
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&v_full[sb], (j >> 1) & 1))) {
+          if (lane == 0) atomicExch(a.status, 22);
+          ok = false;
+          break;
+        }
+        if (r < BKEYS && (key_base + r > p_last ||
+                          (holes && a.block_table[(size_t)seq * a.table_stride + (key_base + r) / a.page_size] < 0))) {
+          uint8_t* vrow = v_s + sb * KBYTES + (r / 8) * 1024 + (r % 8) * 128;
+#pragma unroll
+          for (int blk = 0; blk < DBLK; ++blk)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(vrow + blk * KVBLOCK + q * 16) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA
+      }
       tc::fence_before();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(p_ready);
