@@ -292,7 +292,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const bool row_ok = row < n_valid;
     const int pos = p_first + row;
     const int lo = first_visible(pos);
-    float m = -INFINITY, l = 0.f;
+    // rows without a token start above every score, so they never move the maximum: a request's rounding does not depend on
+    // whose rows come after its own
+    float m = row_ok ? -INFINITY : INFINITY, l = 0.f;
     const float bias_log2 = (sigmoid && a.head_bias) ? a.head_bias[h] * 1.4426950408889634f : 0.f;
     // reshaped scores are brought to units of log 2 first and the code below then takes them with a scale of one
     const bool reshaped = a.softcap > 0.f || a.slopes != nullptr;
