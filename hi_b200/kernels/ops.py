@@ -620,15 +620,41 @@ def delta_conv_update(proj: torch.Tensor, chan_off: int, channels: int, taps_n: 
                                       _stream()), "delta_conv_update")
 
 
-CHUNKED_MIN_TOKENS = 80      # ... and 8 more for every request of the step
+CHUNKED_MIN_TOKENS = 80      # ... and 8 more for every request of the step, where its longest portion is not known
+# Microseconds of a step's recurrence one by one and by chunks, by key size: fixed, for a token (sixteen tokens) of the longest
+# portion, for 10^4 columns of all tokens' states (100 tiles of 32 columns of all chunks'). Fitted to 3,465 measurements: 1 to 64
+# requests of 4 to 512 tokens, even or all but one of one token, 4 to 64 heads of 16 x 16 to 128 x 128. What the sums choose is
+# 1 % from the faster form on average, and slower than one by one by more than 3 % in 122 of them, by half at most.
+_BY_TOKEN = {
+    "delta": {16: (4.1, 0.21, 0.14), 32: (4.2, 0.20, 0.09), 64: (4.8, 0.21, 0.26), 96: (10.9, 0.18, 0.71), 128: (10.8, 0.18, 0.76)},
+    "mlstm": {16: (2.9, 0.39, 0.31), 32: (3.5, 0.13, 0.24), 64: (4.8, 0.17, 0.39), 96: (7.5, 0.15, 0.68), 128: (6.6, 0.17, 0.67)}}
+_BY_TOKEN["plain"] = _BY_TOKEN["delta"]
+_BY_CHUNK = {
+    "delta": {16: (9.1, 1.22, 0.77), 32: (7.3, 2.10, 1.26), 64: (9.0, 1.31, 1.70), 96: (9.6, 1.62, 2.10), 128: (8.0, 1.57, 2.15)},
+    "plain": {16: (7.6, 0.95, 0.56), 32: (6.6, 1.42, 0.85), 64: (7.4, 0.93, 1.34), 96: (8.2, 1.07, 1.58), 128: (7.4, 1.01, 1.66)},
+    "mlstm": {16: (5.7, 2.13, 1.36), 32: (7.5, 1.68, 0.91), 64: (7.7, 0.97, 1.38), 96: (8.1, 0.88, 1.55), 128: (9.5, 0.87, 1.62)}}
 
 
-def _chunked_recurrence(n: int, n_seqs: int, dim: int) -> bool:
+def _chunked_recurrence(n: int, n_seqs: int, dim: int, rule: str = "delta", heads: int = 1, cols: int = 1, longest: int = 0) -> bool:
     """Whether a step's recurrence goes sixteen tokens at a time. A chunk costs about what a dozen tokens cost one by one,
-    however few tokens it holds, and there is a launch more. Measured, kernel times of 16 heads of 128 x 128, delta rule:
-    one request of 24 / 48 / 96 tokens 11.4 / 18.0 / 31.5 us one by one against 12.4 / 14.0 / 19.0; 64 requests of 3 tokens
-    132 against 157; 31 single tokens beside 512 214 against 162."""
-    return dim <= 128 and n >= CHUNKED_MIN_TOKENS + 8 * n_seqs
+    however few tokens it holds, and there is a launch more; where many requests fill the SMs the chain from token to token
+    is not what bounds the step, and with keys of up to 64 a chunk then costs more than its tokens. So the ``longest`` portion
+    decides, where the caller knows it, and the work of all (one by one / by chunks, us: delta rule, 16 heads of 128 x 128, one
+    request of 48 tokens 19 / 15, of 512 148 / 63; 32 heads of 64 x 128, 64 requests of 8 tokens 99 / 273, one of 449 beside 63
+    of one token 199 / 321). Where it is not known, the tokens in all decide: with 4 requests of 32 tokens, 16 heads of 64 x 64,
+    that is slower (12 / 15), with 125 tokens beside three of one faster (34 / 27)."""
+    if dim > 128:
+        return False
+    if not longest:
+        return n >= CHUNKED_MIN_TOKENS + 8 * n_seqs
+    if n < 48:                                          # (the least that was measured; 24 tokens are slower by chunks)
+        return False
+    of = lambda table: table[min(size for size in table if dim <= size)]
+    fixed, chain, work = of(_BY_TOKEN[rule])
+    by_token = fixed + chain * longest + work * n * heads * cols / 1e4
+    fixed, chain, work = of(_BY_CHUNK[rule])
+    chunks = (n - n_seqs) // 16 + n_seqs
+    return fixed + chain * longest / 16 + work * chunks * heads * -(-cols // 32) / 100 < by_token
 
 
 def _chunked_scratch(n: int, n_seqs: int, heads: int, device) -> torch.Tensor:
@@ -638,13 +664,14 @@ def _chunked_scratch(n: int, n_seqs: int, heads: int, device) -> torch.Tensor:
 def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Optional[torch.Tensor],
                      decay: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, heads: int,
                      kvh: int, dim: int, vdim: int, general: bool = False, rows: int = 0, single_tokens: bool = False,
-                     plain: bool = False) -> torch.Tensor:
+                     plain: bool = False, longest: int = 0) -> torch.Tensor:
     """Token after token per request and head, on ``state[slot, :heads*dim*vdim]`` ([heads, dim, vdim] float32):
     S <- decay * S (per row); u = beta (v - S^T k); S <- S + k u^T; o = S^T q. Returns o float32 [N, heads*vdim].
     ``general`` forces the kernel that keeps S in shared memory (any dim) instead of registers (dim <= 256);
     ``rows`` (16, 32) forces how many rows of a column a lane holds, else ``single_tokens`` (every request
     brings one token) decides: the order of the sums differs between the forms, by rounding only. Steps of enough tokens
-    go sixteen tokens at a time (``_chunked_recurrence``; dim <= 128).
+    go sixteen tokens at a time (``_chunked_recurrence``; dim <= 128); ``longest``, the longest portion where the caller
+    knows it, helps that choice.
     ``plain``: the rule without the correction, S <- decay * S + k v^T; o = S^T q (``beta`` is not read)."""
     for t, nm in ((q, "q"), (k, "k"), (v, "v"), (decay, "decay"), (state, "state")) + (() if plain else ((beta, "beta"),)):
         _need(t, nm, torch.float32)
@@ -656,7 +683,8 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Op
     if state.dim() != 2 or state.shape[1] < heads * dim * vdim or cu_seqlens.numel() != slots.numel() + 1:
         raise KernelError("the state or the request tables do not fit")
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
-    if not (general or rows or single_tokens) and _chunked_recurrence(n, slots.numel(), dim):
+    if not (general or rows or single_tokens) and _chunked_recurrence(
+            n, slots.numel(), dim, "plain" if plain else "delta", heads, vdim, longest):
         scratch = _chunked_scratch(n, slots.numel(), heads, q.device)
         _check(lib().hb_delta_recurrence_chunked(
             _ptr(q), _ptr(k), _ptr(v), None if plain else _ptr(beta), _ptr(decay), _ptr(state), state.shape[1],
@@ -878,7 +906,7 @@ def mlstm_gates(z: torch.Tensor, bias_i: Optional[torch.Tensor], bias_f: Optiona
 
 def mlstm_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_scale: float, keep: torch.Tensor,
                      take: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor,
-                     heads: int, dim: int, vdim: int, rows_per_lane: int = 0):
+                     heads: int, dim: int, vdim: int, rows_per_lane: int = 0, longest: int = 0):
     """S <- keep S + take k v^T and n <- keep n + take k token after token, from and into the requests' state
     rows; q, k [heads, dim] and v [heads, vdim] of a token are column runs of ``proj`` [N, ld] at the given
     offsets, q times ``q_scale``. Returns S^T q float32 [N, heads, vdim] and n . q float32 [N, heads]."""
@@ -892,7 +920,7 @@ def mlstm_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_s
         raise KernelError("the state row is too short for this memory")
     o = torch.empty((n, heads, vdim), dtype=torch.float32, device=proj.device)
     nq = torch.empty((n, heads), dtype=torch.float32, device=proj.device)
-    if not rows_per_lane and _chunked_recurrence(n, slots.numel(), dim):
+    if not rows_per_lane and _chunked_recurrence(n, slots.numel(), dim, "mlstm", heads, vdim + 1, longest):
         scratch = _chunked_scratch(n, slots.numel(), heads, proj.device)
         _check(lib().hb_mlstm_recurrence_chunked(
             _ptr(proj), _dt(proj), ld, q_off, k_off, v_off, float(q_scale), _ptr(keep), _ptr(take), _ptr(state),

@@ -75,7 +75,7 @@ class GatedLinearAttentionMixer(Part):
         q, k, v, decay = ops.gla_prep(proj, 0, self.off_k, self.off_v, z, self.b_a2, self.tau, self.dim ** -0.5, hd, hv)
         o = ops.delta_recurrence(q, k, v, None, decay, cache.state, ctx.cu_seqlens, ctx.slots, self.heads, self.heads,
                                  self.dim, self.vdim, general=self.GENERAL_KERNEL, single_tokens=ctx.max_new == 1,
-                                 plain=True)
+                                 plain=True, longest=ctx.max_new)
         y = ops.delta_out_norm(o, proj[:, self.off_g: self.off_g + hv], self.w_norm, self.eps, self.vdim, proj.dtype,
                                gate_silu=True)
         return linear(y, self.w_o)

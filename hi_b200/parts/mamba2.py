@@ -80,7 +80,8 @@ class Mamba2Mixer(Part):
         ops.delta_conv_update(proj, self.inner, self.channels, self.taps, cache.state, self.s_len, ctx.cu_seqlens,
                               ctx.slots)
         o = ops.delta_recurrence(q, k, v, None, decay, cache.state, ctx.cu_seqlens, ctx.slots, self.heads, self.groups,
-                                 self.n_state, self.vdim, single_tokens=ctx.max_new == 1, plain=True)
+                                 self.n_state, self.vdim, single_tokens=ctx.max_new == 1, plain=True,
+                                 longest=ctx.max_new)
         y = ops.mamba2_out(o, x, proj[:, : self.inner], self.d_skip, self.w_norm, self.eps, self.heads, self.vdim,
                            self.parts, proj.dtype)
         return linear(y, self.w_o)

@@ -78,6 +78,7 @@ class MLSTMMixer(Part):
         keep, take, floor = ops.mlstm_gates(z, self.b_i, self.b_f, self.cap, cache.state, ctx.cu_seqlens, ctx.slots,
                                             self.heads, self.dim, self.vdim)
         o, nq = ops.mlstm_recurrence(proj, 0, self.off_k, self.off_v, self.dim ** -0.5, keep, take, cache.state,
-                                     ctx.cu_seqlens, ctx.slots, self.heads, self.dim, self.vdim, self.ROWS_PER_LANE)
+                                     ctx.cu_seqlens, ctx.slots, self.heads, self.dim, self.vdim, self.ROWS_PER_LANE,
+                                     longest=ctx.max_new)
         y = ops.mlstm_out_norm(o, nq, floor, proj, self.off_g, self.w_norm, self.eps, proj.dtype)
         return linear(y, self.w_o)
