@@ -1139,6 +1139,31 @@ def portion_attention_splits(blocks: int, keys: int) -> int:
     return best[1]
 
 
+def portion_attention_pays(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, keep: int = 0) -> bool:
+    """Whether :func:`portion_attention` is faster than :func:`paged_attention` for a step of ``portions``, (cached, new)
+    tokens of every request. A tile of 64 rows by 32 keys takes 0.225 ns a number of its head size (0.38 with rows over 128: one
+    block an SM), whether all its rows are tokens or one; the general kernel takes 100 ns for 256 keys of one row, 140 where
+    contexts are short, and no less than two rounds of its blocks, 320 us, once there is work for them. So single tokens of
+    models with as many key heads as query heads are what the tiles lose by: 31 of them behind 4,000 keys, 16 heads of 128,
+    1,520 against 762 us, with 4 key heads 465 against 675; 24 heads of 64 1,106 against 964; 63 behind 1,000 keys, 16 heads of 128,
+    693 against 379, 24 heads of 64 478 against 631."""
+    group, tile = nh // nkv, hd * (0.225 if hd <= 128 else 0.38)
+    if tile <= 12.5 * group:                           # a tile of one token is no more than the rows of its heads
+        return True
+    tiles = rows = read = requests = 0
+    for cached, new in portions:
+        first = cached // chunk * chunk if chunk else 0
+        if window:
+            first = max(first, cached - window + 1)
+        keys = cached + new - first + min(keep, first)
+        tiles += -(-new * group // 64) * -(-keys // 32)
+        rows += new * ((keys - new / 2) / ATTENTION_SPLIT + 0.25)
+        read += keys
+        requests += 1
+    general = max(320.0, rows * nh * (0.1 if read >= 1024 * requests else 0.14))
+    return tiles * nkv * tile / 1000 <= general
+
+
 def portion_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
                       cu_seqlens: torch.Tensor, positions: torch.Tensor, n_new, chunk: int, window: int, scale: float,
                       max_context: int, sink: bool = False, softcap: float = 0.0, slopes: Optional[torch.Tensor] = None,

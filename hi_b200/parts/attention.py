@@ -80,7 +80,8 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
                         ctx.decode_max_context)
             o.index_copy_(0, rows, od)
         return o
-    if ctx.max_new > 1 and q.dtype == torch.float32:
+    if ctx.max_new > 1 and q.dtype == torch.float32 and \
+            ops.portion_attention_pays(zip(ctx.start_pos, ctx.n_new), nh, nkv, hd, chunk, sliding, keep):
         o = ops.portion_attention(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions, ctx.n_new, chunk, sliding, scale,
                                   ctx.max_context, sink=sink, softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep)
         if o is not None:

@@ -47,6 +47,18 @@ def test_recurrences_by_chunks_where_that_was_faster(heads, dim, vdim, lens, rul
     assert ops._chunked_recurrence(sum(lens), len(lens), dim, rule, heads, cols, max(lens)) == faster
 
 
+@pytest.mark.parametrize("nh,nkv,hd,portions,pays", [
+    (16, 16, 128, [(100, 2)] + [(3400, 1)] * 31, False), (16, 4, 128, [(100, 2)] + [(3400, 1)] * 31, True),
+    (24, 24, 64, [(100, 2)] + [(3400, 1)] * 31, False), (24, 24, 64, [(100, 2)] + [(760, 1)] * 63, True),
+    (16, 16, 128, [(0, 64)] + [(760, 1)] * 63, False), (16, 16, 128, [(100, 2)] + [(250, 1)] * 31, True),
+    (16, 16, 128, [(500, 300)] + [(3400, 1)] * 31, True), (8, 8, 64, [(500, 8), (3000, 1)], True), (40, 8, 128, [(0, 2048)], True),
+    (4, 4, 192, [(0, 600)], True), (16, 16, 128, [(100, 2)], True)])
+def test_float32_portions_by_tiles_where_that_was_faster(nh, nkv, hd, portions, pays):
+    """Measured both ways, single tokens behind long contexts above all."""
+    assert ops.portion_attention_pays(portions, nh, nkv, hd, 0, 0) == pays
+    assert ops.portion_attention_pays(portions, nh, nkv, hd, 0, 128)        # a window leaves a few tiles a token
+
+
 def test_products_of_a_few_rows_leave_foreign_operands_to_the_library(monkeypatch):
     """What is not on x's GPU, or x not on the current one, or wants gradients never reaches the kernel as a pointer."""
     class OnGpu(torch.Tensor):                # a host tensor that says it is on a GPU: no pointer of it may be used
