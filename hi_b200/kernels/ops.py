@@ -282,9 +282,12 @@ def skinny_linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
                   bias: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """``x @ weight.T (+ bias)`` for a few rows of bfloat16 ``x`` (its rows may be a column slice of a wider matrix), with
     float32 sums, in ``out_dtype``; None for what the kernel does not take (sizes, strides, alignment, operands on another GPU
-    or on the host beside ``x``, results that need gradients) or is not the faster one for."""
+    or on the host beside ``x``, results that need gradients or tangents, calls under a transform of ``torch.func``) or is not
+    the faster one for."""
     if not x.is_cuda:
         raise KernelError("x must be a CUDA tensor; this engine has no CPU path")
+    if torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None:
+        return None
     if weight.device != x.device or (bias is not None and bias.device != x.device) or x.device.index != torch.cuda.current_device() or \
             (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad))):
         return None

@@ -80,5 +80,7 @@ def test_products_of_a_few_rows_leave_foreign_operands_to_the_library(monkeypatc
     assert ops.skinny_linear(on(x), on(w, 1), bf16) is None
     assert ops.skinny_linear(on(x, 1), on(w, 1), bf16, on(b, 1)) is None
     assert ops.skinny_linear(on(x), on(w).requires_grad_(), bf16) is None
+    with torch.autograd.forward_ad.dual_level():
+        assert ops.skinny_linear(on(x), on(w), bf16) is None
     with pytest.raises(ops.KernelError):
         ops.skinny_linear(x, w, bf16)

@@ -59,3 +59,17 @@ def test_operands_on_the_host_are_refused_and_gradients_kept():
     linear(x, w).float().sum().backward()
     want = x.double().sum(0).expand_as(w)                # four terms in float32, rounded to bfloat16: 2^-9 of the value
     assert float((w.grad.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
+
+
+def test_tangents_and_transforms_go_through_the_library():
+    from hi_b200.parts.linear import linear
+
+    x, dx = (torch.randn(3, 4, 72, device=DEV).to(torch.bfloat16) for _ in range(2))
+    w = torch.randn(33, 72, device=DEV).to(torch.bfloat16)
+    close = lambda got, want: float((got.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
+    assert close(torch.func.vmap(lambda row: linear(row, w))(x), x.double() @ w.double().t())
+    y, dy = torch.func.jvp(lambda t: linear(t, w), (x[0],), (dx[0],))
+    assert close(y, x[0].double() @ w.double().t()) and close(dy, dx[0].double() @ w.double().t())
+    with torch.autograd.forward_ad.dual_level():
+        out = linear(torch.autograd.forward_ad.make_dual(x[1], dx[1]), w)
+        assert close(torch.autograd.forward_ad.unpack_dual(out).tangent, dx[1].double() @ w.double().t())
