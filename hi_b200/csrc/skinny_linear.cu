@@ -101,18 +101,35 @@ extern "C" int hb_skinny_linear(const void* x, long long x_ld, const void* w, co
   if (tokens == 0 || n_out == 0) return HB_OK;
   const int f = out_dtype == HB_DTYPE_F32;
   // As many warps a block as keep an SM's loads going with the blocks it gets; microseconds (w out of HBM, one launch after
-  // another in a graph), the library's first, for 5 tokens (1 and 8 are within 3 %) of n_out x K:
-  //   512 threads, up to a block an SM: 2048 x 8192 19.5 / 10.2, 1024 x 4096 10.7 / 5.6, 2048 x 2048 7.1 / 4.3, 64 x 2048 4.6 / 2.8
-  //   512 threads, up to two: 4096 x 14336 23.2 / 21.6, 4096 x 1024 5.3 / 4.0;  256 threads: 5120 x 8192 17.4 / 16.9,
-  //   6144 x 2048 7.1 / 6.6;  128 threads: 8192 x 2048 8.2 / 8.2, 7168 x 5120 14.5 / 14.9, 16384 x 5120 28.3 / 28.3,
-  //   32000 x 2048 25.5 / 22.0, 202048 x 5120 294.7 / 290.4
+  // another in a graph), the library's first, for 1 and 8 tokens of n_out x K:
+  //   512 threads, up to a block an SM: 2048 x 8192 20.6 / 9.9 and 20.1 / 9.9, 1024 x 4096 11.8 / 5.2 and 10.7 / 5.4, 2048 x 2048
+  //   8.1 / 4.3 and 7.1 / 4.4, 64 x 2048 4.5 / 3.4 and 4.5 / 3.5
+  //   512 threads, up to two: 4096 x 8192 22.2 / 15.4 and 21.9 / 15.4, 4096 x 1024 5.7 / 4.0 and 5.2 / 4.1, but 3072 x 14336 20.2 / 21.6
+  //   and 19.4 / 21.9: longer rows than 8,192 are the library's
+  //   256 threads: 5120 x 8192 (2 and 8 tokens) 18.0 / 17.6 and 17.9 / 17.8, 6144 x 2048 7.5 / 6.5 and 7.0 / 6.8
+  //   128 threads: 8192 x 2048 8.9 / 7.9 and 8.2 / 8.3, 8192 x 8192 (4 and 8) 24.3 / 23.7 and 23.6 / 24.3, 8192 x 1024 6.0 / 5.4 and 5.9 / 5.6: up to
+  //   four tokens, or short rows;
+  //   10240 x 2048 9.5 / 9.6 and 9.3 / 9.7, 14336 x 4096 (2 and 8) 21.2 / 22.5 and 21.4 / 23.0: the library's;
+  //   16384 x 5120 (2 and 8) 29.4 / 27.4 and 28.1 / 28.0, 32000 x 2048 23.7 / 20.9 and 23.4 / 21.5, 128256 x 5120 (2 and 8) 190.3 / 183.7
+  //   and 189.0 / 186.7, but 128256 x 512 22.4 / 27.9, 128256 x 4096 155.4 / 162.4 and 28672 x 14336 124.8 / 126.5: the lengths
+  //   between are the kernel's
   // For 9 to 16 tokens the library's wide kernels are the faster ones (8192 x 2048 8.4 / 9.9), its narrow ones are not
-  // (2048 x 8192 13.3 / 11.0, 2048 x 2048 5.6 / 4.7, 128 x 2048 4.7 / 3.2).
+  // (2048 x 8192 13.2 / 10.9, 2048 x 2048 5.6 / 4.6, 64 x 2048 4.6 / 3.7).
   // One token of wide rows of 4,096 and more: even alone, and beside the expert kernels of a step of one request the library
   // is the faster one (Scout-sized, eight layers: 1.451 ms a step against 1.459). With 8 tokens it is the other way (routed
-  // experts beside the shared one of 16384 x 5120 and 5120 x 8192: 304 us against 328 with the library).
+  // experts beside the shared one of 16384 x 5120 and 5120 x 8192: 304 us against 328 with the library). In decode steps of eight
+  // Scout-sized layers: 2 requests 1,098 tokens/s with the kernel, 1,093 with the library alone, 4 requests 1,691 and 1,682, 8 requests
+  // within what runs differ by (2,387 to 2,407 and 2,394).
   const bool narrow = n_out <= 148 * 16;
-  if (tokens > 16 || (tokens > 8 && !narrow) || (tokens == 1 && n_out > 296 * 16 && K >= 4096)) return HB_ERR_UNSUPPORTED;
+  auto faster = [&] {
+    if (narrow) return true;
+    if (tokens > 8 || (tokens == 1 && n_out > 296 * 16 && K >= 4096)) return false;
+    if (n_out <= 296 * 16) return K <= 8192;
+    if (n_out <= 6656) return true;
+    if (n_out <= 8192) return tokens <= 4 || K <= 1024;
+    return n_out >= 16384 && ((K >= 1024 && K <= 2048) || (K >= 5120 && K <= 8192));
+  };
+  if (tokens > 16 || !faster()) return HB_ERR_UNSUPPORTED;
   if (tokens > 8)
     return K >= 4096 ? launch_skinny<2, 4, 512>(x, x_ld, w, bias, out, f, tokens, n_out, K, stream)
                      : launch_skinny<2, 2, 512>(x, x_ld, w, bias, out, f, tokens, n_out, K, stream);

@@ -38,14 +38,32 @@ def test_what_is_left_to_the_library():
     x, w = torch.randn(4, 72, device=DEV).to(torch.bfloat16), torch.randn(33, 72, device=DEV).to(torch.bfloat16)
     flat = torch.randn(4 * 72 + 1, device=DEV).to(torch.bfloat16)
     for a, b in ((x[:, :68], w[:, :68].contiguous()), (x[:, 4:68], w[:, :64].contiguous()), (x, w.t().contiguous().t()),
-                 (torch.randn(17, 72, device=DEV).to(torch.bfloat16), w), (flat[1:].view(4, 72), w), (x[:0], w), (x.t()[:, :4].t(), w)):
-        if a.shape[0] and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and b.is_contiguous() and a.shape[1] % 8 == 0 and a.shape[0] <= 16:
-            continue
+                 (torch.randn(17, 72, device=DEV).to(torch.bfloat16), w), (flat[1:].view(4, 72), w), (x[:0], w),
+                 (x.t().contiguous().t(), w)):
         assert ops.skinny_linear(a, b, torch.bfloat16) is None
         got, want = linear(a, b), a.double() @ b.double().t()
         assert got.shape == want.shape and (not got.numel() or float((got.double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max()))
     with pytest.raises(Exception):
         linear(x, w[:, :64].contiguous())
+
+
+@pytest.mark.parametrize("n_out,k,tokens,taken", [
+    (4736, 8192, 8, True), (4736, 8200, 2, False), (4737, 4088, 1, True), (4737, 4096, 1, False), (4737, 4104, 2, True),
+    (4737, 2056, 8, True), (6657, 2056, 4, True), (6657, 2056, 5, False), (8192, 1024, 8, True), (8193, 1024, 2, False),
+    (16384, 1024, 3, True), (16384, 2056, 3, False), (16384, 5120, 8, True), (16383, 5120, 8, False), (16400, 8200, 2, False),
+    (2368, 8200, 16, True)])
+def test_where_the_kernel_is_the_faster_one(n_out, k, tokens, taken):
+    """The ends of the ranges that the kernel takes; rows long enough that its ring of loads goes round."""
+    from hi_b200.kernels import ops
+
+    g = torch.Generator(device=DEV).manual_seed(n_out + k)
+    x = torch.randn(tokens, k, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(n_out, k, device=DEV, generator=g) * k ** -0.5).to(torch.bfloat16)
+    got = ops.skinny_linear(x, w, torch.float32)
+    assert (got is not None) == taken
+    if taken:
+        want = x.double() @ w.double().t()
+        assert float((got.double() - want).abs().max()) <= 2e-6 * float(want.abs().max())
 
 
 def test_operands_on_the_host_are_refused_and_gradients_kept():
