@@ -100,19 +100,20 @@ extern "C" int hb_skinny_linear(const void* x, long long x_ld, const void* w, co
     return HB_ERR_UNSUPPORTED;
   if (tokens == 0 || n_out == 0) return HB_OK;
   const int f = out_dtype == HB_DTYPE_F32;
-  // As many warps a block as keep an SM's loads going with the blocks it gets; microseconds (w out of HBM, one launch after
-  // another in a graph), the library's first, for 1 and 8 tokens of n_out x K:
-  //   512 threads, up to a block an SM: 2048 x 8192 20.6 / 9.9 and 20.1 / 9.9, 1024 x 4096 11.8 / 5.2 and 10.7 / 5.4, 2048 x 2048
-  //   8.1 / 4.3 and 7.1 / 4.4, 64 x 2048 4.5 / 3.4 and 4.5 / 3.5
-  //   512 threads, up to two: 4096 x 8192 22.2 / 15.4 and 21.9 / 15.4, 4096 x 1024 5.7 / 4.0 and 5.2 / 4.1, but 3072 x 14336 20.2 / 21.6
-  //   and 19.4 / 21.9: longer rows than 8,192 are the library's
-  //   256 threads: 5120 x 8192 (2 and 8 tokens) 18.0 / 17.6 and 17.9 / 17.8, 6144 x 2048 7.5 / 6.5 and 7.0 / 6.8
-  //   128 threads: 8192 x 2048 8.9 / 7.9 and 8.2 / 8.3, 8192 x 8192 (4 and 8) 24.3 / 23.7 and 23.6 / 24.3, 8192 x 1024 6.0 / 5.4 and 5.9 / 5.6: up to
-  //   four tokens, or short rows;
-  //   10240 x 2048 9.5 / 9.6 and 9.3 / 9.7, 14336 x 4096 (2 and 8) 21.2 / 22.5 and 21.4 / 23.0: the library's;
-  //   16384 x 5120 (2 and 8) 29.4 / 27.4 and 28.1 / 28.0, 32000 x 2048 23.7 / 20.9 and 23.4 / 21.5, 128256 x 5120 (2 and 8) 190.3 / 183.7
-  //   and 189.0 / 186.7, but 128256 x 512 22.4 / 27.9, 128256 x 4096 155.4 / 162.4 and 28672 x 14336 124.8 / 126.5: the lengths
-  //   between are the kernel's
+  // As many warps a block as keep an SM's loads going with the blocks it gets; microseconds (w out of HBM, behind the norm that
+  // makes x, in a graph), the library's first, for 1 and 8 tokens of n_out x K (2 and 8 where one token is the library's):
+  //   512 threads, up to a block an SM: 2048 x 8192 22.0 / 9.7 and 19.7 / 9.7, 2048 x 2048 8.4 / 4.2 and 7.3 / 4.3, 2048 x 512 3.6 / 2.9
+  //   and 4.0 / 2.7
+  //   512 threads, up to two: 4096 x 8192 23.4 / 15.0 and 21.5 / 15.3, 4096 x 1024 6.1 / 4.0 and 5.8 / 4.1, but 3072 x 14336 19.6 / 21.2
+  //   and 19.7 / 21.5: longer rows than 8,192 are the library's
+  //   256 threads: 5120 x 8192 18.8 / 17.3 and 18.9 / 17.5, 6656 x 2048 7.1 / 6.1 and 6.8 / 6.3
+  //   128 threads: 8192 x 2048 8.2 / 7.6 and 8.2 / 8.0, 8192 x 8192 25.0 / 23.6 and 25.0 / 24.0, but 8192 x 14336 38.7 / 37.8 and 38.1 / 39.3;
+  //   14336 x 5120 27.0 / 24.7 and 25.7 / 25.1, 10240 x 4096 17.8 / 17.9 and 17.9 / 18.4, but 10240 x 8192 31.5 / 33.1 and 31.8 / 35.3,
+  //   14336 x 1024 6.9 / 7.4 and 6.9 / 7.5;
+  //   16384 x 5120 29.5 / 27.3 and 29.7 / 27.8, 32000 x 2048 24.3 / 20.6 and 25.1 / 21.4, 28672 x 4096 41.3 / 39.2 and 41.3 / 40.1, but
+  //   16384 x 512 5.5 / 5.9 and 5.6 / 6.1, 28672 x 14336 123.0 / 124.6 and 123.8 / 128.0;
+  //   128256 x 5120 192.0 / 184.9 and 191.2 / 187.6, but x 4096 156.2 / 164.3 and 158.9 / 167.2, x 8192 306.7 / 309.2 and 306.4 / 314.3
+  // In a whole step the library's kernels can cost more than that: three layers' 8192 x 2048 products for 5 tokens, 13 us a step.
   // For 9 to 16 tokens the library's wide kernels are the faster ones (8192 x 2048 8.4 / 9.9), its narrow ones are not
   // (2048 x 8192 13.2 / 10.9, 2048 x 2048 5.6 / 4.6, 64 x 2048 4.6 / 3.7).
   // One token of wide rows of 4,096 and more: even alone, and beside the expert kernels of a step of one request the library
@@ -126,8 +127,10 @@ extern "C" int hb_skinny_linear(const void* x, long long x_ld, const void* w, co
     if (tokens > 8 || (tokens == 1 && n_out > 296 * 16 && K >= 4096)) return false;
     if (n_out <= 296 * 16) return K <= 8192;
     if (n_out <= 6656) return true;
-    if (n_out <= 8192) return tokens <= 4 || K <= 1024;
-    return n_out >= 16384 && ((K >= 1024 && K <= 2048) || (K >= 5120 && K <= 8192));
+    if (n_out <= 8192) return K <= 8192;
+    if (n_out < 16384) return K > 1024 && K <= 5120;
+    if (n_out <= 65536) return K >= 1024 && K <= 8192;
+    return K >= 1024 && K < 8192 && (K <= 2048 || K >= 5120);
   };
   if (tokens > 16 || !faster()) return HB_ERR_UNSUPPORTED;
   if (tokens > 8)
