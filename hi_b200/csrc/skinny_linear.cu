@@ -114,20 +114,21 @@ extern "C" int hb_skinny_linear(const void* x, long long x_ld, const void* w, co
   //   16384 x 512 5.5 / 5.9 and 5.6 / 6.1, 28672 x 14336 123.0 / 124.6 and 123.8 / 128.0;
   //   128256 x 5120 192.0 / 184.9 and 191.2 / 187.6, but x 4096 156.2 / 164.3 and 158.9 / 167.2, x 8192 306.7 / 309.2 and 306.4 / 314.3
   // In a whole step the library's kernels can cost more than that: three layers' 8192 x 2048 products for 5 tokens, 13 us a step.
+  // (the other way for 8 tokens of 7168 x 5120: 0.3 % of a decode step of eight Scout-sized layers)
   // For 9 to 16 tokens the library's wide kernels are the faster ones (8192 x 2048 8.4 / 9.9), its narrow ones are not
   // (2048 x 8192 13.2 / 10.9, 2048 x 2048 5.6 / 4.6, 64 x 2048 4.6 / 3.7).
   // One token of wide rows of 4,096 and more: even alone, and beside the expert kernels of a step of one request the library
   // is the faster one (Scout-sized, eight layers: 1.451 ms a step against 1.459). With 8 tokens it is the other way (routed
   // experts beside the shared one of 16384 x 5120 and 5120 x 8192: 304 us against 328 with the library). In decode steps of eight
-  // Scout-sized layers: 2 requests 1,098 tokens/s with the kernel, 1,093 with the library alone, 4 requests 1,691 and 1,682, 8 requests
-  // within what runs differ by (2,387 to 2,407 and 2,394).
+  // Scout-sized layers: 2 requests 1,093 tokens/s with the kernel, 1,083 with the library alone, 4 requests 1,675 and 1,670; 8 requests
+  // 2,330 and 2,345 on a card at its power limit, the same on one below it.
   const bool narrow = n_out <= 148 * 16;
   auto faster = [&] {
     if (narrow) return true;
     if (tokens > 8 || (tokens == 1 && n_out > 296 * 16 && K >= 4096)) return false;
     if (n_out <= 296 * 16) return K <= 8192;
     if (n_out <= 6656) return true;
-    if (n_out <= 8192) return K <= 8192;
+    if (n_out <= 8192) return K <= 2048 || (tokens <= 4 && K <= 8192);
     if (n_out < 16384) return K > 1024 && K <= 5120;
     if (n_out <= 65536) return K >= 1024 && K <= 8192;
     return K >= 1024 && K < 8192 && (K <= 2048 || K >= 5120);

@@ -49,7 +49,8 @@ def test_what_is_left_to_the_library():
 
 @pytest.mark.parametrize("n_out,k,tokens,taken", [
     (4736, 8192, 8, True), (4736, 8200, 2, False), (4737, 4088, 1, True), (4737, 4096, 1, False), (4737, 4104, 2, True),
-    (4737, 2056, 8, True), (6657, 2056, 5, True), (6657, 8200, 2, False), (8193, 1024, 2, False), (8193, 1032, 8, True),
+    (4737, 2056, 8, True), (6657, 2048, 8, True), (6657, 2056, 5, False), (6657, 8192, 4, True),
+    (6657, 8200, 2, False), (8193, 1024, 2, False), (8193, 1032, 8, True),
     (16383, 5128, 8, False), (16384, 1016, 3, False), (16384, 5128, 8, True), (16400, 8200, 2, False), (65544, 2048, 1, True),
     (65544, 2056, 2, False), (2368, 8200, 16, True)])
 def test_where_the_kernel_is_the_faster_one(n_out, k, tokens, taken):
