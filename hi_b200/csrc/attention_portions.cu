@@ -11,10 +11,11 @@
 // What bounds it: mma.sync, at 2 cycles of an SM for [16, 16] x [16, 8], six of them a product (0.4 of the time), and the
 // chains between them: a block of four warps splits, multiplies and takes exponentials in turn, two blocks per SM (104 KB of
 // pieces each). The general kernel (a warp per row, uncoalesced rows of keys, every key read once per row) took 1,622 us for
-// 600 tokens behind 301, 16 heads / 4 kv heads of 128, and 18.1 ms for 2,048 tokens, 40 / 8 heads; this one 139 us and
-// 1.16 ms. Steps: keys and values loaded where they are needed, two key tiles of products side by side 187 us; four side by
-// side (the five small terms are a chain) 174; a tile's rows loaded into registers under the products before them 150; the
-// shares of a row tile's keys chosen by fractional rounds 139. Error against 64 bits 4.8e-7 -> 1.8e-7.
+// 600 tokens behind 301, 16 heads / 4 kv heads of 128, and 18.1 ms for 2,048 tokens, 40 / 8 heads; this one 112 us and
+// 1.19 ms. Steps (beside a merge of shares that took 27 us longer): keys and values loaded where they are needed, two key tiles
+// of products side by side 187 us; four side by side (the five small terms are a chain) 174; a tile's rows loaded into registers
+// under the products before them 150; the shares of a row tile's keys chosen by fractional rounds 139; the merge a warp a row 112.
+// Error against 64 bits 4.8e-7 -> 1.9e-7.
 #include "api.h"
 #include "common.cuh"
 #include "mma.cuh"

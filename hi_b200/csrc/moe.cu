@@ -706,7 +706,7 @@ int router_launch(const void* x, int x_dtype, const void* w, int w_dtype, const 
   if (n == 0) return HB_OK;
   if (x_dtype == HB_DTYPE_F32 && n >= 96 && hidden % 8 == 0 && (w_dtype == HB_DTYPE_F32 || w_dtype == HB_DTYPE_BF16)) {
     // many tokens (measured: faster than one block per token from about 100): register tiles of
-    // 4 tokens x 16 experts; with more than 16 experts the
+    // 4 tokens x 8 or 16 experts; with more than 16 experts the
     // selection needs the stored logits of all block columns
     const int columns = experts <= 8 ? 8 : 16;
     dim3 grid((n + ROUTER_TOK - 1) / ROUTER_TOK, (experts + columns - 1) / columns);

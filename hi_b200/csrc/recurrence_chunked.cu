@@ -14,8 +14,8 @@
 //     outputs, which nothing waits for.
 //
 // Measured (B200, one request of 2,048 tokens, 16 heads of 128 x 128; before: token after token, a chain of 2,048 steps):
-// delta rule 582 -> 230 us (24 of them the matrices), the rule without correction 573 -> 163, mLSTM 437 -> 184; 32 heads of
-// Mamba-2 709 -> 254. Error against 64 bits (2-norm, outputs / states): delta rule 9.1e-8 / 1.3e-7 -> 7.1e-8 / 7.0e-8, without
+// delta rule 582 -> 224 us (24 of them the matrices), the rule without correction 573 -> 155, mLSTM 437 -> 158; 32 heads of
+// Mamba-2 709 -> 249. Error against 64 bits (2-norm, outputs / states): delta rule 9.1e-8 / 1.3e-7 -> 7.1e-8 / 7.0e-8, without
 // correction 1.4e-7 / 1.1e-7 -> 8.7e-8 / 5.4e-8. A chunk is 1.6 us of a block: 6,000 warp instructions, of which the
 // preparation of its rows is 40 %, between three barriers. Tried: the products as float32 fma (the shared-memory reads of 4 x 4
 // tiles bound it: 293 us); two tf32 pieces a factor (error 1.1e-7, states of Mamba-2 1.9 times as far off: taken back).
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
     const T* qp = q + (size_t)t0 * a.q_ld;
     const float* gp = decay + (size_t)t0 * decay_ld;
     // (one decay a head: most chunks have nothing to ask about; 10 us of the mLSTM's 173 on ragged portions. With a decay a
-    // row the same made the delta rule slower, 244 us for 235.)
+    // row the same made the delta rule slower, by 9 us of 235.)
     if (SCALAR && count == C && d < a.dim && a.q_ld < (1 << 26)) {
       const int ql = (int)a.q_ld, gl = (int)decay_ld;
 #pragma unroll
