@@ -372,7 +372,7 @@ __global__ void delta_recurrence_smem_kernel(const RecurArgs a) {
 // A step of single tokens, rows of S in whole 16 bytes: a block holds up to 4 * LC columns of one head's S in registers, 16
 // bytes a load (LC lanes side by side, THREADS / LC groups of rows), so the state is read and written in full lines with
 // nothing staged first. The groups' sums meet in shared memory. What bounds it is moving the state: 32 requests of 32 heads
-// of 128 x 128 (134 MB both ways) 62 -> 37 us, 8 requests 17.4 -> 8.9, 64 requests of 16 heads of 64 x 64 13.8 -> 10.1 (before:
+// of 128 x 128 (134 MB both ways) 60 -> 30 us, 8 requests of 16 heads 10.9 -> 5.2, 8 requests of 32 heads of 64 x 64 5.6 -> 5.1 (before:
 // the kernel above, 8 columns of 4 bytes a warp behind a buffer for chunks of tokens).
 constexpr int kSingleThreads = 256;
 template <int LC, int ROWS>
@@ -564,8 +564,11 @@ extern "C" int hb_delta_recurrence(const float* q, const float* k, const float* 
   if (variant != 1 && variant != 0 && variant != 16 && variant != 32) return HB_ERR_BAD_ARG;
   const bool lines = vdim % 4 == 0 && state_stride % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  // (below 48 rows most of a block's groups are idle: 64 requests of 4 heads of 18 x 132 5.7 us in the other form, 12.9 here)
-  if (variant == 0 && single_tokens && dim >= 48 && dim <= 128 && lines && heads <= 65535 && n_seqs <= 65535) {
+  // (With up to 64 rows half of a block's groups are idle, with 48 and fewer most. States out of HBM, the other form / this one, us:
+  // 64 requests of 16 heads of 64 x 64 13.6 / 14.5, of 96 x 64 30.9 / 17.3; 8 requests of 32 heads of 64 x 64 5.6 / 5.1; 32 of 32 of
+  // 64 x 128 25.0 / 21.4, of 48 x 32 8.6 / 13.1; 64 of 8 of 64 x 16 5.3 / 7.0; 64 of 4 of 18 x 132 5.7 / 12.9.)
+  const bool rows_pay = dim > 64 || (dim > 48 && vdim >= 64 && (vdim > 64 || (long long)heads * n_seqs < 1024));
+  if (variant == 0 && single_tokens && rows_pay && dim <= 128 && lines && heads <= 65535 && n_seqs <= 65535) {
     if (vdim > 64)
       delta_single_kernel<32, 16><<<dim3((vdim + 127) / 128, heads, n_seqs), kSingleThreads, 0, stream>>>(a);
     else
