@@ -6,25 +6,35 @@
 //   S <- diag(P_16) S + sum_s (R_s k_s) u_s^T
 // Every factor is a product of decays, never a quotient: strong decays underflow to the zero they stand for.
 //
-//   chunk_matrices_kernel   T and B of all chunks and heads, side by side (they need no state)
-//   chunk_recurrence_kernel per (request, head, 16 or 32 columns of S): chunk after chunk. NW warps own 16 rows of S each,
-//     in registers as accumulator tiles; their products run on the tensor cores with every float32 factor as three
-//     bfloat16 pieces (see hb::split3), and the sums over all rows are brought together in shared memory in a fixed order.
-//     NW more warps, in two groups that take turns, prepare the next chunk's rows (decay products) and write the chunk's
-//     outputs, which nothing waits for.
+// T meets what does not need the state ahead of it: u = T v - (T P k) S, so that one product and one sum over the rows of S
+// lie between a chunk's state and its u.
 //
-// Measured (B200, one request of 2,048 tokens, 16 heads of 128 x 128; before: token after token, a chain of 2,048 steps):
-// delta rule 582 -> 224 us (24 of them the matrices), the rule without correction 573 -> 155, mLSTM 437 -> 158; 32 heads of
-// Mamba-2 709 -> 249. Error against 64 bits (2-norm, outputs / states): delta rule 9.1e-8 / 1.3e-7 -> 7.1e-8 / 7.0e-8, without
-// correction 1.4e-7 / 1.1e-7 -> 8.7e-8 / 5.4e-8. A chunk is 1.6 us of a block: 6,000 warp instructions, of which the
-// preparation of its rows is 40 %, between three barriers. Tried: the products as float32 fma (the shared-memory reads of 4 x 4
-// tiles bound it: 293 us); two tf32 pieces a factor (error 1.1e-7, states of Mamba-2 1.9 times as far off: taken back).
+//   chunk_prepare_kernel    everything that needs no state, of all chunks and heads side by side, once a head: T and B, and the
+//     rows T P k, P q, R k as three bfloat16 pieces a float (see hb::split3) in the order in which the tensor cores read them.
+//   chunk_recurrence_kernel per (request, head, 16 or 32 columns of S): chunk after chunk. NW warps own 16 rows of S each,
+//     in registers as accumulator tiles; the sums over all rows are brought together in shared memory in a fixed order.
+//     Two groups of four more warps take turns: they copy the prepared chunks in (bulk copies, three or four chunks ahead),
+//     make T v, and add up and write the outputs, which nothing waits for.
+// The prepared chunks (25 to 39 KB a head) are laid out for as many chunks as 128 MB hold; longer steps go in slices.
+//
+// Measured (B200, one request of 2,048 tokens, 16 heads of 128 x 128; token after token / sixteen at a time with the rows
+// prepared by every block for itself / now): delta rule 582 / 234 / 192 us (45 of them the preparation); mLSTM with 1,101 and
+// 467 tokens beside single ones 353 / 163 / 137; 1,100 tokens of the rule without correction, 16 heads of 128 x 128 85 -> 73,
+// of 64 x 128 67 -> 47. Over 1,800 steps of all three rules (4 to 40 heads of 16 x 16 to 128 x 128, 1 to 64 requests) 0.84 of the
+// time before; the delta rule's steps of many requests and 64 columns, which fill the SMs, pay for the preparation (40 heads, 16
+// requests of 100 tokens 221 -> 250). Error against 64 bits (2-norm) of the first: 7.0e-8 before and now.
+// What bounds it: the chain from chunk to chunk, 1.1 us; 4,200 warp instructions of 16 warps that wait for one another (an empty
+// chunk with its barriers takes 0.44 us; no part of it more than 0.1). Tried: twice the helpers (8 % slower: they share the
+// issue slots), half as many at keys of 64 and less (1.1 to 1.4 times as long); P q S by two helper warps from pieces of S kept
+// in shared memory (1.25 us a chunk); mbarriers in place of the named barriers (1.4); T v from memory a chunk ahead (1.4: the
+// loads arrive too late); the products as float32 fma; two tf32 pieces a factor (error 1.1e-7).
 //
 // What is not finite in a token's inputs reaches that token's and later outputs of the request, never an earlier one (an
 // infinite value or state comes out of the products as NaN, where token after token the sum could stay infinite).
 #include "api.h"
 #include "common.cuh"
 #include "mma.cuh"
+#include "tc.cuh"
 
 namespace {
 
@@ -57,6 +67,12 @@ struct Product {
     hi = h;
   }
   __device__ __forceinline__ float of(float x) const { return fmaf(hi, x, lo * x); }
+  // the product with x, and in `rest` what its rounding leaves
+  __device__ __forceinline__ float of(float x, float& rest) const {
+    const float y = hi * x;
+    rest = fmaf(lo, x, fmaf(hi, x, -y));
+    return y;
+  }
 };
 
 struct ChunkArgs {
@@ -73,24 +89,60 @@ struct ChunkArgs {
   int row_step, col_step;    // strides of S in the state
   const int* cu_seqlens;
   const int* slots;
-  float* matrices;           // [units, heads, 2, C, C]: T (not used by the plain rule), B
+  unsigned char* images;     // [units of the slice, heads]: ChunkImage
   float* out;                // [N, heads * vdim]
   float* nq;                 // [N, heads] (with take): outputs of column vdim
+  int* status;
   int n_seqs, heads, kvh, dim, vdim, cols;
+  int unit0, units;          // the slice's first unit and how many
 };
 
 // unit = a request's chunk: those of request s start at cu[s] / C + s (there is room for a partial one each)
 __device__ __forceinline__ int first_unit(const int* cu, int s) { return cu[s] / C + s; }
 
+// hb::split3 with the rests of the two floats in the last pieces
+__device__ __forceinline__ void split_more(float2 v, float2 rest, uint32_t (&p)[3]) {
+  p[0] = hb::pack_bf16_sat(v.x, v.y);
+  v.x -= __uint_as_float(p[0] << 16);
+  v.y -= __uint_as_float(p[0] & 0xffff0000u);
+  p[1] = hb::pack_bf16(v.x, v.y);
+  v.x -= __uint_as_float(p[1] << 16);
+  v.y -= __uint_as_float(p[1] & 0xffff0000u);
+  p[2] = hb::pack_bf16(v.x + rest.x, v.y + rest.y);
+}
+
+// What the recurrence reads of a chunk, as two blocks of memory that are copied into shared memory as they lie. The factors
+// that meet the tensor cores are there as three bfloat16 pieces (see hb::split3) in the order of the mma.sync fragments: lane l
+// of warp w has its 12 registers of 16 rows of S, [8-wide tile][piece][half], as three 16-byte words at [w][0 .. 2][l].
+template <int NW, bool PLAIN>
+struct ChunkImage {
+  struct Factors {
+    uint4 w[PLAIN ? 0 : NW][3][32];   // T P k (not with the plain rule)
+    uint4 pq[NW][3][32];              // P q
+    uint4 rk[NW][3][32];              // R k
+    float2 full[16 * NW];             // the whole chunk's decay and the rest of its rounding
+  } f;
+  struct Matrices {
+    float t[PLAIN ? 0 : C][20];       // T
+    float b[C][20];                   // B, zero above the diagonal
+  } m;
+};
+
 // grid (units, heads), 128 threads: warp w takes s = w, w + 4, w + 8, w + 12; a running row w_s = k_s g_(s+1) ... g_t
-// meets k_t and q_t, eight sums a token, brought together by a halving butterfly.
+// meets k_t and q_t, eight sums a token, brought together by a halving butterfly. Then a thread per row d of S: the products
+// of its decays with k and q, and its column of T P k.
 template <typename T, int NW, bool SCALAR, bool PLAIN>
-__global__ void __launch_bounds__(128) chunk_matrices_kernel(const ChunkArgs a) {
-  constexpr int DP = 16 * NW, DL = (DP + 31) / 32;
-  __shared__ __align__(16) float ks[C][DL * 32], qs[C][DL * 32], gs[SCALAR ? 1 : C][SCALAR ? C : DL * 32];
-  __shared__ float A[C][C + 1], B[C][C], bet[C];
+__global__ void __launch_bounds__(128) chunk_prepare_kernel(const ChunkArgs a) {
+  using Image = ChunkImage<NW, PLAIN>;
+  // row lengths that put a fragment's rows into different banks
+  constexpr int DP = 16 * NW, DL = (DP + 31) / 32, W = DL * 32, LD = W + 8;
+  __shared__ __align__(16) float ks[C][LD], qs[C][LD];
+  __shared__ __align__(16) float gr[SCALAR ? W * 20 : (C * LD > W * 20 ? C * LD : W * 20)];    // [token][row] decays, then [row][token] R k
+  __shared__ __align__(16) float A[C][C + 1], B[C][20], Ts[C][20], bet[C], g1[C];
+  // what the roundings of T P k, P q and R k leave: with the delta rule it goes into their third pieces
+  __shared__ __nv_bfloat16 kl[PLAIN ? 1 : C][LD], ql[PLAIN ? 1 : C][LD], rl[PLAIN ? 1 : W][C + 2];
   __shared__ int where[2];
-  const int unit = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int unit = a.unit0 + blockIdx.x, head = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) where[0] = -1;
   __syncthreads();
   for (int s = tid; s < a.n_seqs; s += 128) {
@@ -102,9 +154,10 @@ __global__ void __launch_bounds__(128) chunk_matrices_kernel(const ChunkArgs a) 
   if (t0 < 0) return;
   const int count = min(C, where[1] - t0);
   const int kvhead = head / (a.heads / a.kvh);
+  Image& img = reinterpret_cast<Image*>(a.images)[(size_t)blockIdx.x * a.heads + head];
   {
     // a column of the chunk a thread (or every STEP-th token of one)
-    constexpr int W = DL * 32, STEP = 128 / W > 0 ? 128 / W : 1;
+    constexpr int STEP = 128 / W > 0 ? 128 / W : 1;
     const int d = tid % W, from = tid / W;
     const T* q = reinterpret_cast<const T*>(a.q) + (size_t)(t0 + from) * a.q_ld + (size_t)kvhead * a.dim + d;
     const T* k = reinterpret_cast<const T*>(a.k) + (size_t)(t0 + from) * a.q_ld + (size_t)kvhead * a.dim + d;
@@ -115,12 +168,12 @@ __global__ void __launch_bounds__(128) chunk_matrices_kernel(const ChunkArgs a) 
         const bool in = t < count && d < a.dim;
         ks[t][d] = in ? hb::to_f32(*k) : 0.f;
         qs[t][d] = in ? hb::to_f32(*q) : 0.f;
-        if (!SCALAR) gs[t][d] = in ? *g : 1.f;
+        if (!SCALAR) gr[t * LD + d] = in ? *g : 1.f;
       }
     }
   }
   if (tid < C) {
-    if (SCALAR) gs[0][tid] = tid < count ? a.decay[(size_t)(t0 + tid) * a.heads + head] : 1.f;
+    if (SCALAR) g1[tid] = tid < count ? a.decay[(size_t)(t0 + tid) * a.heads + head] : 1.f;
     bet[tid] = (!PLAIN && tid < count) ? a.beta[(size_t)(t0 + tid) * a.heads + head] : 0.f;
   }
   __syncthreads();
@@ -137,7 +190,7 @@ __global__ void __launch_bounds__(128) chunk_matrices_kernel(const ChunkArgs a) 
       for (int i = 0; i < DL; ++i) {
         kt[i] = ks[t][lane * DL + i];
         qt[i] = qs[t][lane * DL + i];
-        gt[i] = SCALAR ? gs[0][t] : gs[SCALAR ? 0 : t][lane * DL + i];
+        gt[i] = SCALAR ? g1[t] : gr[SCALAR ? 0 : t * LD + lane * DL + i];
       }
       float v[8];
 #pragma unroll
@@ -182,9 +235,14 @@ __global__ void __launch_bounds__(128) chunk_matrices_kernel(const ChunkArgs a) 
       }
     }
   }
+  const int d = tid;
+  float gt[C], pk[C], pl[C];
+  if (d < W) {
+#pragma unroll
+    for (int t = 0; t < C; ++t) gt[t] = SCALAR ? g1[t] : gr[SCALAR ? 0 : t * LD + d];
+  }
   __syncthreads();
-  float* dst = a.matrices + ((size_t)unit * a.heads + head) * (2 * C * C);
-  for (int e = tid; e < C * C; e += 128) dst[C * C + e] = (e % C) <= e / C ? B[e / C][e % C] : 0.f;
+  for (int e = tid; e < C * C; e += 128) img.m.b[e / C][e % C] = (e % C) <= e / C ? B[e / C][e % C] : 0.f;
   if (!PLAIN && tid < C) {
     // column tid of T by forward substitution
     float x[C];
@@ -197,8 +255,90 @@ __global__ void __launch_bounds__(128) chunk_matrices_kernel(const ChunkArgs a) 
         else s0 = fmaf(-A[t][s], x[s], s0);
       }
       x[t] = t < tid ? 0.f : bet[t] * (s0 + s1);
-      dst[t * C + tid] = x[t];
+      Ts[t][tid] = x[t];
+      img.m.t[t][tid] = x[t];
     }
+  }
+  if (d < W) {
+    Product p;
+#pragma unroll
+    for (int t = 0; t < C; ++t) {
+      p.times(gt[t]);
+      if constexpr (PLAIN) {
+        qs[t][d] = p.of(qs[t][d]);
+      } else {
+        float rest;
+        pk[t] = p.of(ks[t][d], pl[t]);
+        qs[t][d] = p.of(qs[t][d], rest);
+        ql[t][d] = __float2bfloat16_rn(rest);
+      }
+    }
+    if (d < DP) img.f.full[d] = make_float2(p.hi, p.lo);
+    Product r;
+#pragma unroll
+    for (int t = C - 4; t >= 0; t -= 4) {
+      float x[4];
+#pragma unroll
+      for (int i = 3; i >= 0; --i) {
+        if constexpr (PLAIN) {
+          x[i] = r.of(ks[t + i][d]);
+        } else {
+          float rest;
+          x[i] = r.of(ks[t + i][d], rest);
+          rl[d][t + i] = __float2bfloat16_rn(rest);
+        }
+        r.times(gt[t + i]);
+      }
+      *reinterpret_cast<float4*>(&gr[d * 20 + t]) = make_float4(x[0], x[1], x[2], x[3]);
+    }
+  }
+  __syncthreads();
+  if (!PLAIN) {
+    if (d < W) {
+#pragma unroll
+      for (int t = 0; t < C; ++t) {
+        float tr[C], w0 = 0.f, w1 = 0.f;
+#pragma unroll
+        for (int s = 0; s <= t; s += 4) *reinterpret_cast<float4*>(&tr[s]) = *reinterpret_cast<const float4*>(&Ts[t][s]);
+        // a later token's rows never reach an earlier one, whatever they hold
+#pragma unroll
+        for (int s = 0; s < t; ++s) {
+          if (s & 1) w1 = fmaf(tr[s], pk[s], w1);
+          else w0 = fmaf(tr[s], pk[s], w0);
+        }
+        // the token's own row, the largest term, comes last
+        const float big = tr[t] * pk[t];
+        float rest = fmaf(tr[t], pl[t], fmaf(tr[t], pk[t], -big));
+        ks[t][d] = two_sum(big, w0 + w1, rest);
+        kl[t][d] = __float2bfloat16_rn(rest);
+      }
+    }
+    __syncthreads();
+  }
+  // the fragments: the mma's k is the row of S for T P k and P q (n the token), the token for R k (n the row)
+  for (int f = tid; f < NW * 32; f += 128) {
+    const int fw = f >> 5, g = (f & 31) >> 2, q4 = f & 3;
+    auto put = [&](uint4 (&to)[3][32], auto of, auto rest) {
+      uint32_t r[12];
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float2 v = *reinterpret_cast<const float2*>(of(n, h));
+          uint32_t p[3];
+          if constexpr (PLAIN) hb::split3(v.x, v.y, p);
+          else split_more(v, __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(rest(n, h))), p);
+#pragma unroll
+          for (int x = 0; x < 3; ++x) r[n * 6 + x * 2 + h] = p[x];
+        }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) to[j][f & 31] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+    };
+    auto token_row = [&](auto* rows) { return [=](int n, int h) { return &rows[8 * n + g][fw * 16 + 8 * h + 2 * q4]; }; };
+    auto row_token = [&](auto* rows, int ld) { return [=](int n, int h) { return &rows[(fw * 16 + 8 * n + g) * ld + 8 * h + 2 * q4]; }; };
+    if constexpr (!PLAIN) put(img.f.w[fw], token_row(ks), token_row(kl));
+    put(img.f.pq[fw], token_row(qs), token_row(ql));
+    put(img.f.rk[fw], row_token(gr, 20), row_token(&rl[0][0], C + 2));
   }
 }
 
@@ -246,40 +386,67 @@ __device__ __forceinline__ void mma3(float (&out)[2][4], const uint32_t (&a)[3][
     for (int e = 0; e < 4; ++e) out[n][e] = (out[n][e] + half[n][e]) + lo[n][e];
 }
 
+// the 12 registers of a fragment of 16 rows of S (ChunkImage)
+__device__ __forceinline__ void load_fragment(uint32_t (&r)[2][3][2], const uint4 (&from)[3][32], int lane) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const uint4 v = from[j][lane];
+    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[(4 * j + i) / 6][(4 * j + i) % 6 / 2][i & 1] = x[i];
+  }
+}
+
 template <int NW, int CT, bool PLAIN>
 struct ChunkSmem {
   // row lengths that put a fragment's rows into different banks
-  static constexpr int DP = 16 * NW, LD = DP + 8, ROWS = PLAIN ? C : 2 * C, LZ = ROWS + 8, CG = 16 * CT;
-  struct Stage {
-    float p[ROWS][LD];       // P k (not with the plain rule), then P q
-    float rk[DP][24];        // R k, [row][token]
-    float2 full[DP];         // the whole chunk's decay and the rest of its rounding
-    float t[C][20];          // T
-    float b[C][C];           // B
-    float v[C][CG + 4];      // values (0 past the end)
-  };
+  static constexpr int CG = 16 * CT, STAGES = CT == 1 ? 4 : 3, RING = 4, HELP = 128;
   struct All {
-    Stage stage[2];
-    float part[2][NW][CG][LZ];         // [column][token]: a warp's share of (P S)^T
-    float x[CG][20];                   // [column][token]
-    float u[2][CG][20];                // [column][token]
-    __nv_bfloat16 up[2][3][CG][24];    // the pieces of u
+    typename ChunkImage<NW, PLAIN>::Factors factors[STAGES];
+    typename ChunkImage<NW, PLAIN>::Matrices matrices[RING];
+    float part_w[PLAIN ? 0 : NW][CG][24];      // [column][token]: a warp's share of (T P k S)^T
+    float part_q[2][NW][C][CG + 4];            // [token][column]: a warp's share of P q S
+    float2 u0[PLAIN ? 0 : RING][CG][20];       // [column][token]: T v and the rest of its rounding
+    float v[PLAIN ? 0 : 2][CG][20];            // [column][token]
+    float u[PLAIN ? RING : 2][CG][20];         // [column][token]
+    __nv_bfloat16 up[PLAIN ? RING : 1][3][CG][24];    // the pieces of u
+    uint64_t full[STAGES], full_m[RING];
   };
 };
 
-template <typename T, int NW, int CT, bool SCALAR, bool PLAIN>
-__global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkArgs a) {
+template <typename T, int NW, int CT, bool PLAIN>
+__global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) chunk_recurrence_kernel(const ChunkArgs a) {
   using Smem = ChunkSmem<NW, CT, PLAIN>;
-  constexpr int CG = Smem::CG, COMP = 32 * NW, HELP = 16 * NW;
-  // barriers (+ the buffer's parity): chunk prepared; u and the shares of P S there; chunk used up; among the COMP threads
-  constexpr int FULL = 1, DONE = 3, EMPTY = 5, PEER = 7;
-  extern __shared__ __align__(16) unsigned char raw[];
+  using Image = ChunkImage<NW, PLAIN>;
+  constexpr int CG = Smem::CG, COMP = 32 * NW, HELP = Smem::HELP, STAGES = Smem::STAGES, RING = Smem::RING;
+  // barriers: (+ chunk & 3) T v or the pieces of v there; (+ chunk & 1) u and the shares of P q S there, the factors read;
+  // the outputs written; among a helper group; among the COMP threads
+  constexpr int FULL = 1, DONE = 5, FREED = 7, GROUP = 9, PEER = 11;
+  extern __shared__ __align__(128) unsigned char raw[];
   typename Smem::All& sm = *reinterpret_cast<typename Smem::All*>(raw);
   const int head = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CG;
-  const int first = a.cu_seqlens[seq], last = a.cu_seqlens[seq + 1];
-  if (first >= last) return;
-  const int chunks = (last - first + C - 1) / C;
+  const int last = a.cu_seqlens[seq + 1], unit0 = first_unit(a.cu_seqlens, seq);
+  const int skip = max(0, a.unit0 - unit0);                          // chunks of earlier slices
+  const int first = a.cu_seqlens[seq] + skip * C;
+  const int chunks = min((last - first + C - 1) / C, a.unit0 + a.units - (unit0 + skip));
+  if (first >= last || chunks <= 0) return;
   const int tid = threadIdx.x;
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < STAGES; ++i) tc::mbar_init(&sm.full[i], 1);
+#pragma unroll
+    for (int i = 0; i < RING; ++i) tc::mbar_init(&sm.full_m[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const Image* images = reinterpret_cast<const Image*>(a.images) + (size_t)(unit0 + skip - a.unit0) * a.heads + head;
+  bool ok = true;
+  auto there = [&](uint64_t* full, int use) {          // a copy has arrived
+    if (ok && !tc::mbar_wait(full, use & 1)) {
+      atomicExch(a.status, 41);
+      ok = false;                                     // go on without waiting: every barrier of the block is still met
+    }
+  };
 
   if (tid < COMP) {
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q4 = lane & 3;
@@ -302,10 +469,12 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
           const size_t i = at(m, n, e, in);
           s[m][n][e] = in ? S[i] : 0.f;
         }
+    // sums over all warps: token lane & 15 of one of two columns two apart (different banks)
+    constexpr int EN = (CG / 2 + NW - 1) / NW;
+    const int t = lane & 15;
+    auto pair_column = [&](int p) { return (p & 1) + 2 * (lane >> 4) + (p >> 1) * 4; };
     for (int i = 0; i < chunks; ++i) {
-      const int b = i & 1;
-      auto& st = sm.stage[b];
-      bar_sync(FULL + b, COMP + HELP);
+      const int b = i & 1, ring = i & 3;
       // the tiles of S^T are the A operand as they lie in the accumulators
       uint32_t sp[CT][3][4];
 #pragma unroll
@@ -317,98 +486,76 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
 #pragma unroll
           for (int x = 0; x < 3; ++x) sp[m][x][e] = p[x];
         }
-      // the warp's share of (P S)^T for sixteen rows of P
-      auto share = [&](int row) {
-        uint32_t pp[2][3][2];
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float2 v = *reinterpret_cast<const float2*>(&st.p[row + 8 * n + g][warp * 16 + 8 * h + 2 * q4]);
-            uint32_t p[3];
-            hb::split3(v.x, v.y, p);
-#pragma unroll
-            for (int x = 0; x < 3; ++x) pp[n][x][h] = p[x];
-          }
+      there(&sm.full[i % STAGES], i / STAGES);
+      const auto& img = sm.factors[i % STAGES];
+      uint32_t fr[2][3][2], qf[2][3][2];
+      if constexpr (!PLAIN) {
+        load_fragment(fr, img.w[warp], lane);
 #pragma unroll
         for (int m = 0; m < CT; ++m) {
           float z[2][4];
-          mma3(z, sp[m], pp);
+          mma3(z, sp[m], fr);
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
-            *reinterpret_cast<float2*>(&sm.part[b][warp][16 * m + g][row + 8 * n + 2 * q4]) = make_float2(z[n][0], z[n][1]);
-            *reinterpret_cast<float2*>(&sm.part[b][warp][16 * m + g + 8][row + 8 * n + 2 * q4]) = make_float2(z[n][2], z[n][3]);
+            *reinterpret_cast<float2*>(&sm.part_w[warp][16 * m + g][8 * n + 2 * q4]) = make_float2(z[n][0], z[n][1]);
+            *reinterpret_cast<float2*>(&sm.part_w[warp][16 * m + g + 8][8 * n + 2 * q4]) = make_float2(z[n][2], z[n][3]);
           }
+        }
+      }
+      load_fragment(qf, img.pq[warp], lane);
+      bar_sync(FULL + ring, COMP + HELP);
+      if (i >= 2) bar_sync(FREED + b, COMP + HELP);
+      auto outputs = [&]() {                     // the warp's share of P q S
+#pragma unroll
+        for (int m = 0; m < CT; ++m) {
+          float z[2][4];
+          mma3(z, sp[m], qf);
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sm.part_q[b][warp][8 * n + 2 * q4 + (e & 1)][16 * m + g + (e >> 1) * 8] = z[n][e];
         }
       };
-      share(0);
       if constexpr (!PLAIN) {
         const int count = min(C, last - first - i * C);
-        constexpr int EN = (C * CG + COMP - 1) / COMP;
-        const int t = tid % C;
-        float4 tr[C / 4];
-        float vv[EN], xx[EN];
-#pragma unroll
-        for (int r = 0; r < C / 4; ++r) tr[r] = *reinterpret_cast<const float4*>(&st.t[t][4 * r]);
-        const float own = st.t[t][t];
-#pragma unroll
-        for (int j = 0; j < EN; ++j) vv[j] = tid + j * COMP < C * CG ? st.v[t][(tid + j * COMP) / C] : 0.f;
         bar_sync(PEER, COMP);
+        float z[EN];
+        float2 u0[EN];
 #pragma unroll
         for (int j = 0; j < EN; ++j) {
-          const int c = (tid + j * COMP) / C;
-          if (tid + j * COMP >= C * CG) break;
-          xx[j] = vv[j] - tree_sum<NW>([&](int w) { return sm.part[b][w][c][t]; });
-          sm.x[c][t] = xx[j];
+          const int p = warp + j * NW, c = pair_column(p);
+          if (p >= CG / 2) break;
+          z[j] = tree_sum<NW>([&](int w) { return sm.part_w[w][c][t]; });
+          u0[j] = sm.u0[ring][c][t];
         }
-        share(C);                // (P q) S: nothing waits for it, it fills the time
-        __syncwarp();            // a warp reads back its own columns only
+        outputs();               // nothing waits for them, they fill the time
 #pragma unroll
         for (int j = 0; j < EN; ++j) {
-          const int c = (tid + j * COMP) / C;
-          if (tid + j * COMP >= C * CG) break;
-          float u0 = 0.f, u1 = 0.f;
-#pragma unroll
-          for (int r = 0; r < C; r += 4) {
-            const float4 xr = *reinterpret_cast<const float4*>(&sm.x[c][r]);
-            // a later token's rows never reach an earlier one, whatever they hold
-            if (r < t) u0 = fmaf(tr[r / 4].x, xr.x, u0);
-            if (r + 1 < t) u1 = fmaf(tr[r / 4].y, xr.y, u1);
-            if (r + 2 < t) u0 = fmaf(tr[r / 4].z, xr.z, u0);
-            if (r + 3 < t) u1 = fmaf(tr[r / 4].w, xr.w, u1);
-          }
-          // the token's own row, the largest term, comes last
-          const float u = t < count ? fmaf(own, xx[j], u0 + u1) : 0.f;
+          const int p = warp + j * NW, c = pair_column(p);
+          if (p >= CG / 2) break;
+          const float u = t < count ? (u0[j].x - z[j]) + u0[j].y : 0.f;
           sm.u[b][c][t] = u;
-          put_pieces(&sm.up[b][0][c][t], CG * 24, u);
+          put_pieces(&sm.up[0][0][c][t], CG * 24, u);
         }
         bar_sync(PEER, COMP);
+      } else {
+        outputs();
       }
-      bar_arrive(DONE + b, COMP + HELP);
-      uint32_t rp[2][3][2];
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float2 v = *reinterpret_cast<const float2*>(&st.rk[warp * 16 + 8 * n + g][8 * h + 2 * q4]);
-          uint32_t p[3];
-          hb::split3(v.x, v.y, p);
-#pragma unroll
-          for (int x = 0; x < 3; ++x) rp[n][x][h] = p[x];
-        }
+      load_fragment(fr, img.rk[warp], lane);
       float4 full[2];
 #pragma unroll
-      for (int n = 0; n < 2; ++n) full[n] = *reinterpret_cast<const float4*>(&st.full[warp * 16 + 8 * n + 2 * q4]);
+      for (int n = 0; n < 2; ++n) full[n] = *reinterpret_cast<const float4*>(&img.full[warp * 16 + 8 * n + 2 * q4]);
+      uint32_t up[CT][3][4];
 #pragma unroll
-      for (int m = 0; m < CT; ++m) {
-        uint32_t up[3][4];
+      for (int m = 0; m < CT; ++m)
 #pragma unroll
         for (int x = 0; x < 3; ++x)
+          hb::ldmatrix_x4(up[m][x], &sm.up[PLAIN ? ring : 0][x][16 * m + (lane & 15)][(lane >> 4) * 8]);
+      bar_arrive(DONE + b, COMP + HELP);
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            up[x][e] = *reinterpret_cast<const uint32_t*>(&sm.up[b][x][16 * m + g + (e & 1) * 8][2 * q4 + (e >> 1) * 8]);
+      for (int m = 0; m < CT; ++m) {
         float z[2][4];
-        mma3(z, up, rp);
+        mma3(z, up[m], fr);
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
@@ -416,7 +563,6 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
             s[m][n][e] = fmaf(s[m][n][e], (e & 1) ? full[n].z : full[n].x,
                               fmaf(s[m][n][e], (e & 1) ? full[n].w : full[n].y, z[n][e]));
       }
-      if (i + 2 < chunks) bar_arrive(EMPTY + b, COMP + HELP);
     }
 #pragma unroll
     for (int m = 0; m < CT; ++m)
@@ -431,146 +577,166 @@ __global__ void __launch_bounds__(64 * NW) chunk_recurrence_kernel(const ChunkAr
     return;
   }
 
-  // ---- two groups of helpers, a thread per row of S: group b prepares the chunks of parity b and writes their outputs,
-  // so the inputs of its next chunk, asked for as soon as the registers are free, have two chunks' time to arrive
-  const int b = (tid - COMP) / HELP, d = (tid - COMP) % HELP;
-  auto& st = sm.stage[b];
-  const int kvhead = head / (a.heads / a.kvh);
-  const T* q = reinterpret_cast<const T*>(a.q) + (size_t)kvhead * a.dim + d;
-  const T* k = reinterpret_cast<const T*>(a.k) + (size_t)kvhead * a.dim + d;
+  // ---- two groups of helpers that take turns: group b brings the images of the chunks of parity b in, makes T v of the
+  // next one while the other threads are at this one, and writes this one's outputs
+  const int b = (tid - COMP) / HELP, h = (tid - COMP) % HELP, hw = h >> 5, lane = h & 31;
   const T* v = reinterpret_cast<const T*>(a.v) + (size_t)head * a.vdim;
-  const float* decay = a.decay + (SCALAR ? (size_t)head : (size_t)head * a.dim + d);
-  const size_t decay_ld = SCALAR ? a.heads : (size_t)a.heads * a.dim;
-  constexpr int TB4 = (PLAIN ? 1 : 2) * C * C / 4, TBN = (TB4 + HELP - 1) / HELP, VN = (C * CG + HELP - 1) / HELP;
-  T kr[C], qr[C], vr[VN];
-  float gr[C], fr[VN];
-  float4 tbr[TBN];
-  const int unit0 = first_unit(a.cu_seqlens, seq);
+  constexpr int VN = (C * CG + HELP - 1) / HELP;
+  T vr[VN];
+  float fr[VN];
+  auto copy = [&](void* dst, const void* src, uint32_t bytes, uint64_t* full) {      // one thread
+    tc::mbar_expect_tx(full, bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(tc::smem_u32(dst)), "l"(src), "r"(bytes), "r"(tc::smem_u32(full)) : "memory");
+  };
+  auto bring_factors = [&](int i) {
+    copy(&sm.factors[i % STAGES], &images[(size_t)i * a.heads].f, sizeof(sm.factors[0]), &sm.full[i % STAGES]);
+  };
+  auto bring_matrices = [&](int i) {
+    copy(&sm.matrices[i % RING], &images[(size_t)i * a.heads].m, sizeof(sm.matrices[0]), &sm.full_m[i % RING]);
+  };
   auto load = [&](int i) {               // nothing is computed from the values here, so nothing waits for them
     const int t0 = first + i * C, count = min(C, last - t0);
-    const T* kp = k + (size_t)t0 * a.q_ld;
-    const T* qp = q + (size_t)t0 * a.q_ld;
-    const float* gp = decay + (size_t)t0 * decay_ld;
-    // (one decay a head: most chunks have nothing to ask about; 10 us of the mLSTM's 173 on ragged portions. With a decay a
-    // row the same made the delta rule slower, by 9 us of 235.)
-    if (SCALAR && count == C && d < a.dim && a.q_ld < (1 << 26)) {
-      const int ql = (int)a.q_ld, gl = (int)decay_ld;
-#pragma unroll
-      for (int t = 0; t < C; ++t) {
-        kr[t] = kp[t * ql];
-        qr[t] = qp[t * ql];
-        gr[t] = gp[t * gl];
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < C; ++t, kp += a.q_ld, qp += a.q_ld, gp += decay_ld) {
-        const bool in = t < count && d < a.dim;
-        kr[t] = in ? *kp : hb::from_f32<T>(0.f);
-        qr[t] = in ? *qp : hb::from_f32<T>(0.f);
-        gr[t] = in ? *gp : 1.f;
-      }
-    }
-    const float4* m = reinterpret_cast<const float4*>(a.matrices + ((size_t)(unit0 + i) * a.heads + head) * (2 * C * C) + (PLAIN ? C * C : 0));
-#pragma unroll
-    for (int j = 0; j < TBN; ++j)
-      if (d + j * HELP < TB4) tbr[j] = m[d + j * HELP];
 #pragma unroll
     for (int j = 0; j < VN; ++j) {
-      const int e = d + j * HELP, t = e / CG, col = col0 + e % CG;
+      const int e = h + j * HELP, t = e / CG, col = col0 + e % CG;
       const bool in = t < count && col < a.cols;
       vr[j] = in && col < a.vdim ? v[(size_t)(t0 + t) * a.v_ld + col] : hb::from_f32<T>(in ? 1.f : 0.f);
       fr[j] = in && a.take ? a.take[(size_t)(t0 + t) * a.heads + head] : 1.f;
     }
   };
-  if (b < chunks) load(b);
-  for (int i = b; i < chunks; i += 2) {
-    const int t0 = first + i * C, count = min(C, last - t0);
-    if (i >= 2) bar_sync(EMPTY + b, COMP + HELP);
-    Product p;
-#pragma unroll
-    for (int t = 0; t < C; ++t) {
-      p.times(gr[t]);
-      if constexpr (!PLAIN) st.p[t][d] = p.of(hb::to_f32(kr[t]));
-      st.p[(PLAIN ? 0 : C) + t][d] = p.of(hb::to_f32(qr[t]));
-    }
-    st.full[d] = make_float2(p.hi, p.lo);
-    Product r;
-#pragma unroll
-    for (int t = C - 4; t >= 0; t -= 4) {
-      float4 w;
-      w.w = r.of(hb::to_f32(kr[t + 3])); r.times(gr[t + 3]);
-      w.z = r.of(hb::to_f32(kr[t + 2])); r.times(gr[t + 2]);
-      w.y = r.of(hb::to_f32(kr[t + 1])); r.times(gr[t + 1]);
-      w.x = r.of(hb::to_f32(kr[t])); r.times(gr[t]);
-      *reinterpret_cast<float4*>(&st.rk[d][t]) = w;
-    }
-#pragma unroll
-    for (int j = 0; j < TBN; ++j) {
-      const int e = d + j * HELP;
-      if (e >= TB4) break;
-      if (!PLAIN && e < C * C / 4) *reinterpret_cast<float4*>(&st.t[e / (C / 4)][e % (C / 4) * 4]) = tbr[j];
-      else reinterpret_cast<float4*>(&st.b[0][0])[PLAIN ? e : e - C * C / 4] = tbr[j];
-    }
+  auto values = [&](int i) {             // of chunk i, from the registers
+    const int ring = i & 3;
 #pragma unroll
     for (int j = 0; j < VN; ++j) {
-      const int e = d + j * HELP;
+      const int e = h + j * HELP;
       if (e >= C * CG) break;
       const float x = hb::to_f32(vr[j]) * fr[j];
       if (PLAIN) {
-        sm.u[b][e % CG][e / CG] = x;
-        put_pieces(&sm.up[b][0][e % CG][e / CG], CG * 24, x);
+        sm.u[ring][e % CG][e / CG] = x;
+        put_pieces(&sm.up[ring][0][e % CG][e / CG], CG * 24, x);
       } else {
-        st.v[e / CG][e % CG] = x;
+        sm.v[b][e % CG][e / CG] = x;
       }
     }
-    bar_arrive(FULL + b, COMP + HELP);
-    if (i + 2 < chunks) load(i + 2);
+    if constexpr (!PLAIN) {
+      there(&sm.full_m[ring], i / RING);
+      const auto& img = sm.matrices[ring];
+      bar_sync(GROUP + b, HELP);
+      const int t = lane & 15;
+      float4 tr[C / 4];
+#pragma unroll
+      for (int r = 0; r < C / 4; ++r) tr[r] = *reinterpret_cast<const float4*>(&img.t[t][4 * r]);
+      const float own = img.t[t][t];
+#pragma unroll
+      for (int j = 0; j < VN; ++j) {
+        const int p = hw + j * (HELP / 32), c = (p & 1) + 2 * (lane >> 4) + (p >> 1) * 4;
+        if (p >= CG / 2) break;
+        float u0 = 0.f, u1 = 0.f;
+#pragma unroll
+        for (int r = 0; r < C; r += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(&sm.v[b][c][r]);
+          // a later token's rows never reach an earlier one, whatever they hold
+          if (r < t) u0 = fmaf(tr[r / 4].x, x.x, u0);
+          if (r + 1 < t) u1 = fmaf(tr[r / 4].y, x.y, u1);
+          if (r + 2 < t) u0 = fmaf(tr[r / 4].z, x.z, u0);
+          if (r + 3 < t) u1 = fmaf(tr[r / 4].w, x.w, u1);
+        }
+        // the token's own row, the largest term, comes last, and what is rounded off is kept: u rounds once
+        const float vt = sm.v[b][c][t], big = own * vt;
+        float lost = fmaf(own, vt, -big);
+        const float sum = two_sum(big, u0 + u1, lost);
+        sm.u0[ring][c][t] = make_float2(sum, lost);
+      }
+    }
+    bar_arrive(FULL + ring, COMP + HELP);
+  };
+  if (h == 0) {
+    for (int i = b; i < min(chunks, RING); i += 2) {
+      bring_matrices(i);
+      if (i < STAGES) bring_factors(i);
+    }
+  }
+  if (b < chunks) { load(b); values(b); }
+  bar_sync(GROUP + b, HELP);
+  if (b + 2 < chunks) load(b + 2);
+  for (int i = b; i < chunks; i += 2) {
+    const int t0 = first + i * C, count = min(C, last - t0), ring = i & 3;
+    if (i + 2 < chunks) values(i + 2);
+    if (i + 4 < chunks) load(i + 4);
     bar_sync(DONE + b, COMP + HELP);
+    if (PLAIN) there(&sm.full_m[ring], i / RING);
+    const auto& img = sm.matrices[ring];
 #pragma unroll
     for (int j = 0; j < VN; ++j) {
-      const int e = d + j * HELP, t = e / CG, c = e % CG, col = col0 + c;
+      const int e = h + j * HELP, t = e / CG, c = e % CG, col = col0 + c;
       if (e >= C * CG) break;
       float y0 = 0.f, y1 = 0.f;
 #pragma unroll
       for (int x = 0; x < C; x += 4) {
-        const float4 br = *reinterpret_cast<const float4*>(&st.b[t][x]);
-        const float4 u = *reinterpret_cast<const float4*>(&sm.u[b][c][x]);
+        const float4 br = *reinterpret_cast<const float4*>(&img.b[t][x]);
+        const float4 u = *reinterpret_cast<const float4*>(&sm.u[PLAIN ? ring : b][c][x]);
         if (x <= t) y0 = fmaf(br.x, u.x, y0);
         if (x + 1 <= t) y1 = fmaf(br.y, u.y, y1);
         if (x + 2 <= t) y0 = fmaf(br.z, u.z, y0);
         if (x + 3 <= t) y1 = fmaf(br.w, u.w, y1);
       }
       // the last three sums with what they round off, so that the output rounds once
-      auto z = [&](int w) { return sm.part[b][w][c][(PLAIN ? 0 : C) + t]; };
+      auto z = [&](int w) { return sm.part_q[b][w][t][c]; };
       float lost = 0.f;
       const float y = two_sum(y0, y1, lost);
       const float o = (two_sum(two_sum(tree_sum<NW - NW / 2>(z), tree_sum<NW / 2>(z, NW - NW / 2), lost), y, lost) + lost) * a.o_scale;
       if (t < count && col < a.vdim) a.out[(size_t)(t0 + t) * a.heads * a.vdim + (size_t)head * a.vdim + col] = o;
       else if (t < count && col < a.cols) a.nq[(size_t)(t0 + t) * a.heads + head] = o;
     }
+    bar_sync(GROUP + b, HELP);                        // the group has read the matrices and the values
+    if (h == 0) {
+      if (i + STAGES < chunks) bring_factors(i + STAGES);
+      if (i + RING < chunks) bring_matrices(i + RING);
+    }
+    if (i + 2 < chunks) bar_arrive(FREED + b, COMP + HELP);
   }
 }
 
-template <typename T, int NW, int CT, bool SCALAR, bool PLAIN>
+template <typename T, int NW, int CT, bool PLAIN>
 int launch_columns(const ChunkArgs& a, cudaStream_t stream) {
   const size_t smem = sizeof(typename ChunkSmem<NW, CT, PLAIN>::All);
-  cudaError_t e = cudaFuncSetAttribute(chunk_recurrence_kernel<T, NW, CT, SCALAR, PLAIN>,
+  cudaError_t e = cudaFuncSetAttribute(chunk_recurrence_kernel<T, NW, CT, PLAIN>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  chunk_recurrence_kernel<T, NW, CT, SCALAR, PLAIN>
-      <<<dim3((a.cols + 16 * CT - 1) / (16 * CT), a.heads, a.n_seqs), 64 * NW, smem, stream>>>(a);
+  chunk_recurrence_kernel<T, NW, CT, PLAIN>
+      <<<dim3((a.cols + 16 * CT - 1) / (16 * CT), a.heads, a.n_seqs), 32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP, smem, stream>>>(a);
   HB_LAUNCH_CHECK();
   return HB_OK;
 }
 
+// Units of a slice: as many images as 128 MB hold (the sequence of launches over the slices carries the states).
+inline int slice_units(int heads, size_t image_bytes, int units) {
+  const size_t fit = ((size_t)128 << 20) / (heads * image_bytes);
+  return fit < 1 ? 1 : fit < (size_t)units ? (int)fit : units;
+}
+
 template <typename T, int NW, bool SCALAR, bool PLAIN>
-int launch_chunked(const ChunkArgs& a, int units, cudaStream_t stream) {
-  chunk_matrices_kernel<T, NW, SCALAR, PLAIN><<<dim3(units, a.heads), 128, 0, stream>>>(a);
-  HB_LAUNCH_CHECK();
-  // 32 columns a block share the preparation of a chunk's rows, once 16 a block are more than a block per SM
-  const long long blocks = (long long)((a.cols + 15) / 16) * a.heads * a.n_seqs;
-  return blocks > 148 && a.cols > 16 ? launch_columns<T, NW, 2, SCALAR, PLAIN>(a, stream)
-                                     : launch_columns<T, NW, 1, SCALAR, PLAIN>(a, stream);
+int launch_chunked(ChunkArgs a, int units, cudaStream_t stream) {
+  const int step = slice_units(a.heads, sizeof(ChunkImage<NW, PLAIN>), units);
+  for (a.unit0 = 0; a.unit0 < units; a.unit0 += step) {
+    a.units = units - a.unit0 < step ? units - a.unit0 : step;
+    chunk_prepare_kernel<T, NW, SCALAR, PLAIN><<<dim3(a.units, a.heads), 128, 0, stream>>>(a);
+    HB_LAUNCH_CHECK();
+    // 32 columns a block share the images, once 16 a block are more than a block per SM
+    const long long blocks = (long long)((a.cols + 15) / 16) * a.heads * a.n_seqs;
+    const int rc = blocks > 148 && a.cols > 16 ? launch_columns<T, NW, 2, PLAIN>(a, stream)
+                                               : launch_columns<T, NW, 1, PLAIN>(a, stream);
+    if (rc != HB_OK) return rc;
+  }
+  return HB_OK;
+}
+
+size_t image_bytes(int dim, bool plain) {
+  if (dim <= 32) return plain ? sizeof(ChunkImage<2, true>) : sizeof(ChunkImage<2, false>);
+  if (dim <= 64) return plain ? sizeof(ChunkImage<4, true>) : sizeof(ChunkImage<4, false>);
+  if (dim <= 96) return plain ? sizeof(ChunkImage<6, true>) : sizeof(ChunkImage<6, false>);
+  return plain ? sizeof(ChunkImage<8, true>) : sizeof(ChunkImage<8, false>);
 }
 
 template <typename T, bool SCALAR, bool PLAIN>
@@ -584,23 +750,24 @@ int launch_by_dim(const ChunkArgs& a, int units, cudaStream_t stream) {
 }  // namespace
 
 // Floats of scratch that the chunked recurrences need for `n_tokens` tokens of `n_seqs` requests.
-extern "C" long long hb_recurrence_chunked_scratch_floats(int n_tokens, int n_seqs, int heads) {
-  return ((long long)n_tokens / C + n_seqs) * heads * (2 * C * C);
+extern "C" long long hb_recurrence_chunked_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int plain) {
+  const size_t bytes = image_bytes(dim, plain != 0);
+  return (long long)(slice_units(heads, bytes, n_tokens / C + n_seqs) * (heads * bytes) / 4);
 }
 
 extern "C" int hb_delta_recurrence_chunked(const float* q, const float* k, const float* v, const float* beta,
                                            const float* decay, float* state, long long state_stride,
                                            const int* cu_seqlens, const int* slots, float* scratch, float* out,
                                            int n_tokens, int n_seqs, int heads, int kvh, int dim, int vdim, int plain,
-                                           cudaStream_t stream) {
-  if (!q || !k || !v || (!beta && !plain) || !decay || !state || !cu_seqlens || !slots || !scratch || !out) return HB_ERR_BAD_ARG;
+                                           int* status, cudaStream_t stream) {
+  if (!q || !k || !v || (!beta && !plain) || !decay || !state || !cu_seqlens || !slots || !scratch || !out || !status) return HB_ERR_BAD_ARG;
   if (heads <= 0 || kvh <= 0 || heads % kvh || dim <= 0 || vdim <= 0 || n_seqs < 0 || n_tokens < 0) return HB_ERR_BAD_ARG;
   if (dim > 128 || heads > 65535 || n_seqs > 65535 || (reinterpret_cast<uintptr_t>(scratch) & 15)) return HB_ERR_UNSUPPORTED;
   if (n_seqs == 0 || n_tokens == 0) return HB_OK;
   ChunkArgs a = {};
   a.q = q; a.k = k; a.v = v; a.q_ld = (long long)kvh * dim; a.v_ld = (long long)heads * vdim; a.decay = decay; a.beta = beta;
   a.o_scale = 1.f; a.state = state; a.state_stride = state_stride; a.head_floats = (long long)dim * vdim;
-  a.row_step = vdim; a.col_step = 1; a.cu_seqlens = cu_seqlens; a.slots = slots; a.matrices = scratch; a.out = out;
+  a.row_step = vdim; a.col_step = 1; a.cu_seqlens = cu_seqlens; a.slots = slots; a.images = reinterpret_cast<unsigned char*>(scratch); a.out = out; a.status = status;
   a.n_seqs = n_seqs; a.heads = heads; a.kvh = kvh; a.dim = dim; a.vdim = vdim; a.cols = vdim;
   const int units = n_tokens / C + n_seqs;
   return plain ? launch_by_dim<float, false, true>(a, units, stream) : launch_by_dim<float, false, false>(a, units, stream);
@@ -610,8 +777,8 @@ extern "C" int hb_mlstm_recurrence_chunked(const void* proj, int proj_dtype, lon
                                            float q_scale, const float* keep, const float* take, float* state,
                                            long long state_stride, const int* cu_seqlens, const int* slots, float* scratch,
                                            float* o, float* nq, int n_tokens, int n_seqs, int heads, int dim, int vdim,
-                                           cudaStream_t stream) {
-  if (!proj || !keep || !take || !state || !cu_seqlens || !slots || !scratch || !o || !nq || n_seqs < 0 || n_tokens < 0 ||
+                                           int* status, cudaStream_t stream) {
+  if (!proj || !keep || !take || !state || !cu_seqlens || !slots || !scratch || !o || !nq || !status || n_seqs < 0 || n_tokens < 0 ||
       heads <= 0 || dim <= 0 || vdim <= 0)
     return HB_ERR_BAD_ARG;
   if (proj_dtype != HB_DTYPE_F32 && proj_dtype != HB_DTYPE_BF16) return HB_ERR_BAD_ARG;
@@ -623,7 +790,7 @@ extern "C" int hb_mlstm_recurrence_chunked(const void* proj, int proj_dtype, lon
   a.q = base + q_off * el; a.k = base + k_off * el; a.v = base + v_off * el; a.q_ld = ld; a.v_ld = ld; a.decay = keep;
   a.take = take; a.o_scale = q_scale; a.state = state; a.state_stride = state_stride;
   a.head_floats = (long long)(vdim + 1) * dim; a.row_step = 1; a.col_step = dim; a.cu_seqlens = cu_seqlens; a.slots = slots;
-  a.matrices = scratch; a.out = o; a.nq = nq; a.n_seqs = n_seqs; a.heads = heads; a.kvh = heads; a.dim = dim; a.vdim = vdim;
+  a.images = reinterpret_cast<unsigned char*>(scratch); a.out = o; a.status = status; a.nq = nq; a.n_seqs = n_seqs; a.heads = heads; a.kvh = heads; a.dim = dim; a.vdim = vdim;
   a.cols = vdim + 1;
   const int units = n_tokens / C + n_seqs;
   return proj_dtype == HB_DTYPE_F32 ? launch_by_dim<float, true, true>(a, units, stream)

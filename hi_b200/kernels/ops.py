@@ -78,8 +78,8 @@ _SIGNATURES = {
                       I, I, I, I, P],
     "hb_delta_conv_update": [P, I, c_longlong, I, P, c_longlong, c_longlong, P, P, I, I, I, P],
     "hb_delta_recurrence": [P, P, P, P, P, P, c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
-    "hb_delta_recurrence_chunked": [P, P, P, P, P, P, c_longlong, P, P, P, P, I, I, I, I, I, I, I, P],
-    "hb_mlstm_recurrence_chunked": [P, I, c_longlong, I, I, I, F, P, P, P, c_longlong, P, P, P, P, P, I, I, I, I, I, P],
+    "hb_delta_recurrence_chunked": [P, P, P, P, P, P, c_longlong, P, P, P, P, I, I, I, I, I, I, I, P, P],
+    "hb_mlstm_recurrence_chunked": [P, I, c_longlong, I, I, I, F, P, P, P, c_longlong, P, P, P, P, P, I, I, I, I, I, P, P],
     "hb_skinny_linear": [P, c_longlong, P, P, P, I, I, I, I, P],
     "hb_delta_out_norm": [P, P, I, P, F, P, I, c_longlong, I, I, c_longlong, I, P],
     "hb_hyper_step": [P, P, P, I, P, I, P, P, P, I, P, P, F, P, P, I, F, P, I, P, P, I, I, I, P],
@@ -111,7 +111,7 @@ def lib():
             fn = getattr(handle, name)
             fn.argtypes = sig
             fn.restype = c_int
-        handle.hb_recurrence_chunked_scratch_floats.argtypes = [I, I, I]
+        handle.hb_recurrence_chunked_scratch_floats.argtypes = [I, I, I, I, I]
         handle.hb_recurrence_chunked_scratch_floats.restype = c_longlong
         handle.hb_moe_down_tc_scratch_floats.argtypes = [I]
         handle.hb_moe_down_tc_scratch_floats.restype = c_longlong
@@ -660,8 +660,9 @@ def _chunked_recurrence(n: int, n_seqs: int, dim: int, rule: str = "delta", head
     return fixed + chain * longest / 16 + work * chunks * heads * -(-cols // 32) / 100 < by_token
 
 
-def _chunked_scratch(n: int, n_seqs: int, heads: int, device) -> torch.Tensor:
-    return torch.empty(lib().hb_recurrence_chunked_scratch_floats(n, n_seqs, heads), dtype=torch.float32, device=device)
+def _chunked_scratch(n: int, n_seqs: int, heads: int, dim: int, plain: bool, device) -> torch.Tensor:
+    return torch.empty(lib().hb_recurrence_chunked_scratch_floats(n, n_seqs, heads, dim, int(plain)), dtype=torch.float32,
+                       device=device)
 
 
 def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Optional[torch.Tensor],
@@ -688,11 +689,12 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Op
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     if not (general or rows or single_tokens) and _chunked_recurrence(
             n, slots.numel(), dim, "plain" if plain else "delta", heads, vdim, longest):
-        scratch = _chunked_scratch(n, slots.numel(), heads, q.device)
+        scratch = _chunked_scratch(n, slots.numel(), heads, dim, plain, q.device)
         _check(lib().hb_delta_recurrence_chunked(
             _ptr(q), _ptr(k), _ptr(v), None if plain else _ptr(beta), _ptr(decay), _ptr(state), state.shape[1],
             _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(out), n, slots.numel(), heads, kvh, dim, vdim, int(plain),
-            _stream()), "delta_recurrence")
+            _ptr(_tc_status(q.device)), _stream()), "delta_recurrence")
+        TC_USED[0] = True
         LAUNCHES[0] += 1
         return out
     _check(lib().hb_delta_recurrence(_ptr(q), _ptr(k), _ptr(v), None if plain else _ptr(beta), _ptr(decay), _ptr(state),
@@ -924,11 +926,12 @@ def mlstm_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_s
     o = torch.empty((n, heads, vdim), dtype=torch.float32, device=proj.device)
     nq = torch.empty((n, heads), dtype=torch.float32, device=proj.device)
     if not rows_per_lane and _chunked_recurrence(n, slots.numel(), dim, "mlstm", heads, vdim + 1, longest):
-        scratch = _chunked_scratch(n, slots.numel(), heads, proj.device)
+        scratch = _chunked_scratch(n, slots.numel(), heads, dim, True, proj.device)
         _check(lib().hb_mlstm_recurrence_chunked(
             _ptr(proj), _dt(proj), ld, q_off, k_off, v_off, float(q_scale), _ptr(keep), _ptr(take), _ptr(state),
             state.stride(0), _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(o), _ptr(nq), n, slots.numel(), heads, dim,
-            vdim, _stream()), "mlstm_recurrence")
+            vdim, _ptr(_tc_status(proj.device)), _stream()), "mlstm_recurrence")
+        TC_USED[0] = True
         LAUNCHES[0] += 1
         return o, nq
     _check(lib().hb_mlstm_recurrence(_ptr(proj), _dt(proj), ld, q_off, k_off, v_off, float(q_scale), _ptr(keep),
@@ -2065,7 +2068,8 @@ def check_tc_status(device=None) -> None:
                      2: "grouped product: the MMA issuer waiting for a loaded stage",
                      3: "grouped product: the epilogue waiting for the accumulator",
                      4: "grouped product: the MMA issuer waiting for a free accumulator",
-                     31: "decode attention: the warps waiting for a tile's TMA loads"}.get(
+                     31: "decode attention: the warps waiting for a tile's TMA loads",
+                     41: "recurrence by chunks: the warps waiting for a chunk's copies"}.get(
                 code, f"prefill attention, wait {code}" if code >= 11 else f"code {code}")
             raise KernelError(f"a kernel gave up a bounded wait ({where}); its output is invalid")
 

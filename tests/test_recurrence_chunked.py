@@ -183,3 +183,35 @@ def test_single_tokens_by_whole_lines(heads, kvh, dim, vdim, plain, lens):
         assert torch.equal(dev[slot, heads * dim * vdim:], state[slot, heads * dim * vdim:])
     for slot in set(range(len(lens) + 2)) - set(slots.tolist()):
         assert torch.equal(dev[slot], state[slot])
+
+
+@pytest.mark.parametrize("plain", [False, True])
+def test_steps_that_take_several_slices_of_scratch(plain):
+    """More prepared chunks than one slice of the scratch holds: the states go from launch to launch, wherever a request's
+    chunks are cut."""
+    from hi_b200.kernels import ops
+
+    heads, dim, vdim, lens = 64, 128, 8, [5, 1700, 600, 1, 33]
+    n, g = sum(lens), torch.Generator(device=DEV).manual_seed(3)
+    images = heads * (n // 16 + len(lens)) * (25 if plain else 38) * 1024          # (a little less than they take)
+    assert images > 128 << 20 and ops._chunked_recurrence(n, len(lens), dim)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, k = (F.normalize(rnd(n, heads, dim), dim=-1).reshape(n, -1) for _ in range(2))
+    v, beta = rnd(n, heads * vdim), torch.rand(n, heads, device=DEV, generator=g)
+    decay = torch.exp(-torch.exp(2.0 * rnd(n, heads * dim) - 2.0))
+    cu, slots = tables(lens)
+    state = rnd(len(lens) + 2, heads * dim * vdim)
+    after = state.clone()
+    o = ops.delta_recurrence(q, k, v, None if plain else beta, decay, after, cu.to(DEV), slots.to(DEV), heads, heads, dim, vdim,
+                             plain=plain)
+    row = lambda t, x, w: x[t].double().view(heads, w)
+    for s, slot in enumerate(slots.tolist()):
+        S, want = state[slot].double().view(heads, dim, vdim), []
+        for t in range(int(cu[s]), int(cu[s + 1])):
+            S = S * row(t, decay, dim)[:, :, None]
+            vt = row(t, v, vdim)
+            u = vt if plain else beta[t].double()[:, None] * (vt - torch.einsum("hdv,hd->hv", S, row(t, k, dim)))
+            S = S + row(t, k, dim)[:, :, None] * u[:, None, :]
+            want.append(torch.einsum("hdv,hd->hv", S, row(t, q, dim)).reshape(-1))
+        close(o[int(cu[s]): int(cu[s + 1])], torch.stack(want), f"request {s}")
+        close(after[slot], S.reshape(-1), f"state {s}")
