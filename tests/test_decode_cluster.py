@@ -1,0 +1,49 @@
+"""Decode attention whose splits meet inside a cluster of blocks, against the softmax in float64 and against the splits merged
+by a kernel of their own: 2 to 8 splits, tokens that have fewer of them than the batch's longest, every page size."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(40, 8, 128), (8, 2, 64), (3, 3, 128), (16, 1, 64)])
+@pytest.mark.parametrize("lens,page,chunk,sink", [([1000], 64, 0, False), ([65, 1, 64, 128, 63], 16, 0, True), ([513, 2], 32, 0, False),
+                                                  ([900, 300, 512, 513], 128, 512, True), ([2049], 64, 0, False), ([129, 700, 64], 64, 128, False)])
+def test_splits_meet_in_a_cluster(nh, nkv, hd, lens, page, chunk, sink, monkeypatch):
+    from hi_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(sum(lens) + nh)
+    n, pages = len(lens), sum(-(-k // page) for k in lens)
+    q = torch.randn(n, nh, hd, generator=g).to(torch.bfloat16)
+    kp, vp = (torch.randn(pages, nkv, page, hd, generator=g).to(torch.bfloat16) for _ in range(2))
+    order, at = torch.randperm(pages, generator=g).to(torch.int32), 0
+    table = torch.full((n, max(-(-k // page) for k in lens)), -1, dtype=torch.int32)
+    for i, k in enumerate(lens):
+        need = -(-k // page)
+        table[i, :need] = order[at: at + need]
+        at += need
+    pos = torch.tensor([k - 1 for k in lens], dtype=torch.int32)
+    args = [t.to(DEV) for t in (q, kp, vp, table, torch.arange(n, dtype=torch.int32), pos)]
+    call = lambda: ops.decode_attention(*args, chunk, 0, hd ** -0.5, max(lens), sink=sink)
+    splits = ops._decode_splits(min(max(lens), chunk or max(lens)), n * nkv)[1]
+    before = dict(ops.CALLS)
+    got = call()
+    if 1 < splits <= 8:
+        assert ops.CALLS.get("attention_merge", 0) == before.get("attention_merge", 0)
+    assert torch.equal(got, call())                        # the blocks of a cluster finish in any order: the sum has one
+    monkeypatch.setattr(ops, "DECODE_CLUSTER", 1)
+    apart = call()
+    for i, k in enumerate(lens):
+        lo = (k - 1) // chunk * chunk if chunk else 0
+        rows = lambda t: t[table[i, : -(-k // page)].long()].transpose(1, 2).reshape(-1, nkv, hd)[lo:k].double()
+        ks, vs = (rows(t).repeat_interleave(nh // nkv, dim=1) for t in (kp, vp))
+        scores = torch.einsum("hd,khd->hk", q[i].double(), ks) * hd ** -0.5
+        top = scores.max(dim=1, keepdim=True).values
+        e = torch.exp(scores - top)
+        want = torch.einsum("hk,khd->hd", e, vs) / (e.sum(1, keepdim=True) + (torch.exp(-top) if sink else 0.0))
+        # weights rounded to bfloat16 (2^-9 each, averaged over the keys) and the result rounded once more: 2^-8 of the largest
+        err = float((got[i].cpu().double() - want).abs().max() / want.abs().max())
+        assert err < 2 ** -7, (i, err)
+    # the same sums in the same order: at most the last place of bfloat16 where a product was contracted differently
+    assert float((got.float() - apart.float()).abs().max()) <= 2 ** -8 * float(apart.float().abs().max())
