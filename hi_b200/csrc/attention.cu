@@ -147,10 +147,12 @@ template <typename T, int W>
 __global__ void __launch_bounds__(32 * MERGE_ROWS) attention_merge_kernel(const float* __restrict__ part_acc,
                                                                           const float* __restrict__ part_ml, T* __restrict__ out,
                                                                           long long rows, int hd, int splits, int sink, int nh,
-                                                                          const float* __restrict__ sink_values) {
+                                                                          const float* __restrict__ sink_values,
+                                                                          const long long* __restrict__ token_rows) {
   const int lane = threadIdx.x & 31;
   const long long th = (long long)blockIdx.x * MERGE_ROWS + (threadIdx.x >> 5);
   if (th >= rows) return;
+  const long long to = token_rows ? token_rows[th / nh] * nh + th % nh : th;
   const float* acc = part_acc + (size_t)th * splits * hd;
   struct alignas(4 * W) Vec { float x[W]; };
   Vec ahead[MERGE_AHEAD];
@@ -202,20 +204,20 @@ __global__ void __launch_bounds__(32 * MERGE_ROWS) attention_merge_kernel(const 
       struct alignas(sizeof(T) * W) Out { T x[W]; } v;
 #pragma unroll
       for (int e = 0; e < W; ++e) v.x[e] = hb::from_f32<T>(o[e] * inv);
-      *reinterpret_cast<Out*>(out + (size_t)th * hd + d) = v;
+      *reinterpret_cast<Out*>(out + (size_t)to * hd + d) = v;
     }
   }
 }
 
 template <typename T>
 int launch_merge(const float* part_acc, const float* part_ml, void* out, long long rows, int hd, int splits, int sink, int nh,
-                 const float* sink_values, cudaStream_t stream) {
+                 const float* sink_values, const long long* token_rows, cudaStream_t stream) {
   const uintptr_t p = reinterpret_cast<uintptr_t>(part_acc), o = reinterpret_cast<uintptr_t>(out);
   const long long blocks = (rows + MERGE_ROWS - 1) / MERGE_ROWS;
   if (blocks > 0x7fffffffLL) return HB_ERR_UNSUPPORTED;
   auto fits = [&](int w) { return hd % w == 0 && p % (4 * w) == 0 && o % (sizeof(T) * w) == 0; };
 #define HB_MERGE(W) \
-  attention_merge_kernel<T, W><<<(int)blocks, 32 * MERGE_ROWS, 0, stream>>>(part_acc, part_ml, (T*)out, rows, hd, splits, sink, nh, sink_values)
+  attention_merge_kernel<T, W><<<(int)blocks, 32 * MERGE_ROWS, 0, stream>>>(part_acc, part_ml, (T*)out, rows, hd, splits, sink, nh, sink_values, token_rows)
   if (fits(4) && (hd % 128 == 0 || hd % 64 != 0)) HB_MERGE(4);
   else if (fits(2)) HB_MERGE(2);
   else HB_MERGE(1);
@@ -265,21 +267,28 @@ extern "C" int hb_paged_attention(const void* q, int dtype, const void* k_pages,
   HB_LAUNCH_CHECK();
   if (part_acc && out)
     return dtype == HB_DTYPE_F32
-               ? launch_merge<float>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, stream)
-               : launch_merge<__nv_bfloat16>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, stream);
+               ? launch_merge<float>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, nullptr, stream)
+               : launch_merge<__nv_bfloat16>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, nullptr, stream);
   return HB_OK;
 }
 
 // Merge of split partials alone (the decode kernel writes the same partial layout).
-extern "C" int hb_attention_merge(const float* part_acc, const float* part_ml, void* out, int dtype, int n_rows,
+// With `token_rows` (one a token of nh rows) the merged rows go to those tokens of `out`.
+extern "C" int hb_attention_merge_rows(const float* part_acc, const float* part_ml, void* out, int dtype, int n_rows,
                                   int hd, int max_splits, int sink, int nh, const float* sink_values,
-                                  cudaStream_t stream) {
-  if (!part_acc || !part_ml || !out || n_rows < 0 || hd <= 0 || max_splits < 1 || (sink_values && nh <= 0))
+                                  const long long* token_rows, cudaStream_t stream) {
+  if (!part_acc || !part_ml || !out || n_rows < 0 || hd <= 0 || max_splits < 1 || ((sink_values || token_rows) && nh <= 0))
     return HB_ERR_BAD_ARG;
   if (nh <= 0) nh = 1;
   if (n_rows == 0) return HB_OK;
-  if (dtype == HB_DTYPE_F32) return launch_merge<float>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, stream);
+  if (dtype == HB_DTYPE_F32) return launch_merge<float>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, token_rows, stream);
   if (dtype == HB_DTYPE_BF16)
-    return launch_merge<__nv_bfloat16>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, stream);
+    return launch_merge<__nv_bfloat16>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, token_rows, stream);
   return HB_ERR_BAD_ARG;
+}
+
+extern "C" int hb_attention_merge(const float* part_acc, const float* part_ml, void* out, int dtype, int n_rows,
+                                  int hd, int max_splits, int sink, int nh, const float* sink_values,
+                                  cudaStream_t stream) {
+  return hb_attention_merge_rows(part_acc, part_ml, out, dtype, n_rows, hd, max_splits, sink, nh, sink_values, nullptr, stream);
 }

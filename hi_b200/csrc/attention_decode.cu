@@ -60,7 +60,9 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
                    __nv_bfloat16* __restrict__ out, int nh, int nkv, int page_size, int chunk, int window, int keep,
                    float scale, int sink, const float* __restrict__ head_bias, float softcap,
                    const float* __restrict__ slopes, const float* __restrict__ sink_values, int split_size,
-                   int max_splits, float* __restrict__ part_acc, float* __restrict__ part_ml) {
+                   int max_splits, float* __restrict__ part_acc, float* __restrict__ part_ml,
+                   const long long* __restrict__ rows) {
+  // rows: the tokens this launch takes are those rows of q, out, seq_of_token and positions (null: all, in order)
   // softcap > 0: a scaled score s becomes softcap * tanh(s / softcap); slopes [nh]: slopes[head] * (distance to the
   // key) is taken off after the cap; sink_values [nh]: the sink's score is the head's own number instead of 0.
   // sink == 2: sigmoid weights. The weight of a key is sigmoid(score + head_bias[head]), nothing is normalised,
@@ -82,13 +84,15 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   const int G = min(ROWS, nh / nkv - row0);                   // heads of the row tile
   const int h0 = kvh * (nh / nkv) + row0;
   const bool parts = part_acc != nullptr;
-  const int pos = positions[t];
-  const int* table = block_table + (size_t)seq_of_token[t] * table_stride;
+  const int token = rows ? (int)rows[t] : t;
+  const int pos = positions[token];
+  const int* table = block_table + (size_t)seq_of_token[token] * table_stride;
   int lo = 0;
   if (chunk > 0) lo = (pos / chunk) * chunk;
   if (window > 0 && pos - window + 1 > lo) lo = pos - window + 1;
   const int first = lo + split * split_size;
-  const size_t th0 = (size_t)t * nh + h0;                     // (token, first head of the row tile)
+  const size_t th0 = (size_t)t * nh + h0;                     // (token, first head of the row tile), of the partial rows
+  const size_t qh0 = (size_t)token * nh + h0;                 // ... of q and out
   // kept tokens: tiles of the walk that lie before the window's first tile, this split's first tile, tiles in all
   const int kept_tiles = keep > 0 ? min((keep + TILE - 1) / TILE, lo / TILE) : 0;
   const int walk0 = split * (split_size / TILE);
@@ -116,7 +120,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   for (int c = tid; c < ROWS * CHUNKS; c += NWARPS * 32) {
     const int r = c / CHUNKS, ch = c % CHUNKS;
     const bool ok = r < G;
-    cp_async16(q_s + r * STRIDE + ch * 8, q + (th0 + (ok ? r : 0)) * HD + ch * 8, ok);
+    cp_async16(q_s + r * STRIDE + ch * 8, q + (qh0 + (ok ? r : 0)) * HD + ch * 8, ok);
   }
   // thread -> every 128th 16-byte chunk of a [TILE][CHUNKS] tile. When a tile never straddles a page (page_size
   // a multiple of TILE and the range starts on a TILE boundary) one table lookup serves the whole tile.
@@ -342,7 +346,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     } else {
       // a key without a value, of score 0 or of the head's own score
       if (sink && l > 0.f) l += expf((sink_values ? sink_values[h0 + row] : 0.f) - mx);
-      out[(th0 + row) * HD + d] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
+      out[(qh0 + row) * HD + d] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
     }
   }
   (void)m_all;
@@ -353,7 +357,7 @@ int launch_decode(const void* q, const void* k_pages, const void* v_pages, const
                   const int* seq_of_token, const int* positions, void* out, int n_tokens, int nh, int nkv,
                   int page_size, int chunk, int window, int keep, float scale, int sink, const float* head_bias, float softcap,
                   const float* slopes, const float* sink_values, int split_size,
-                  int max_splits, float* part_acc, float* part_ml, cudaStream_t stream) {
+                  int max_splits, float* part_acc, float* part_ml, const long long* rows, cudaStream_t stream) {
   constexpr int STRIDE = HD + 8;
   const size_t smem = (size_t)(ROWS * STRIDE + 4 * TILE * STRIDE) * sizeof(__nv_bfloat16) +
                       (size_t)(NWARPS * ROWS * 2) * sizeof(float);
@@ -364,7 +368,7 @@ int launch_decode(const void* q, const void* k_pages, const void* v_pages, const
   attn_decode_kernel<HD><<<grid, NWARPS * 32, smem, stream>>>(
       (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, table_stride,
       seq_of_token, positions, (__nv_bfloat16*)out, nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap,
-      slopes, sink_values, split_size, max_splits, part_acc, part_ml);
+      slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows);
   HB_LAUNCH_CHECK();
   return HB_OK;
 }
@@ -375,13 +379,15 @@ int launch_decode(const void* q, const void* k_pages, const void* v_pages, const
 // go to `out`; otherwise (max, sum, unnormalised row) of every split go to part_ml / part_acc and `out` is not used.
 // With `keep` > 0 (a sliding window only) `split_size * max_splits` has to cover the walk: at most
 // ceil((window + 63) / 64) + ceil(keep / 64) tiles of 64. Returns HB_ERR_UNSUPPORTED for other shapes (the caller then uses the
-// general kernel). The merge over splits is hb_attention_merge.
-extern "C" int hb_attention_decode(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
+// general kernel). The merge over splits is hb_attention_merge. With `rows` (n_tokens of them, each within q, out, seq_of_token
+// and positions) the launch takes those tokens of a larger step, where they are; their partial rows lie in the order of `rows`.
+// (Four single tokens beside three portions, 40 heads of 128: three gathers and a scatter around the kernel were 20 of 223 us.)
+extern "C" int hb_attention_decode_rows(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                    int table_stride, const int* seq_of_token, const int* positions, void* out,
                                    int n_tokens, int nh, int nkv, int hd, int page_size, int chunk, int window, int keep,
                                    float scale, int sink, const float* head_bias, float softcap, const float* slopes,
                                    const float* sink_values, int split_size, int max_splits,
-                                   float* part_acc, float* part_ml, cudaStream_t stream) {
+                                   float* part_acc, float* part_ml, const long long* rows, cudaStream_t stream) {
   if (sink == 2 && (softcap > 0.f || slopes || sink_values)) return HB_ERR_UNSUPPORTED;
   if (!q || !k_pages || !v_pages || !block_table || !seq_of_token || !positions || (!out && !part_acc)) return HB_ERR_BAD_ARG;
   if (n_tokens < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || table_stride <= 0 || chunk < 0 ||
@@ -392,14 +398,25 @@ extern "C" int hb_attention_decode(const void* q, const void* k_pages, const voi
   if (n_tokens == 0) return HB_OK;
   if (hd == 192)
     return launch_decode<192>(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
-                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, stream);
+                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, stream);
   if (hd == 128)
     return launch_decode<128>(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
-                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, stream);
+                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, stream);
   if (hd == 64)
     return launch_decode<64>(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
-                             nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, stream);
+                             nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, stream);
   return HB_ERR_UNSUPPORTED;
+}
+
+extern "C" int hb_attention_decode(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
+                                   int table_stride, const int* seq_of_token, const int* positions, void* out,
+                                   int n_tokens, int nh, int nkv, int hd, int page_size, int chunk, int window, int keep,
+                                   float scale, int sink, const float* head_bias, float softcap, const float* slopes,
+                                   const float* sink_values, int split_size, int max_splits,
+                                   float* part_acc, float* part_ml, cudaStream_t stream) {
+  return hb_attention_decode_rows(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens, nh,
+                                  nkv, hd, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values,
+                                  split_size, max_splits, part_acc, part_ml, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

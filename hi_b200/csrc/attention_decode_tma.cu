@@ -56,6 +56,7 @@ struct Args {
   int* status;
   int table_stride, nh, nkv, page_size, chunk, split_size, max_splits, box_rows;
   float scale;
+  const long long* rows;   // the tokens of the launch among those of q, out, seq_of_token and positions, or null
   int sink;      // the softmax's denominator has one more term, e^0: a key of score 0 without a value
 };
 
@@ -220,11 +221,13 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int split = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = a.nh / a.nkv;
-  const int pos = a.positions[t];
-  const int* table = a.block_table + (size_t)a.seq_of_token[t] * a.table_stride;
+  const int token = a.rows ? (int)a.rows[t] : t;
+  const int pos = a.positions[token];
+  const int* table = a.block_table + (size_t)a.seq_of_token[token] * a.table_stride;
   const int lo = a.chunk > 0 ? (pos / a.chunk) * a.chunk : 0;
   const int first = lo + split * a.split_size;
-  const size_t th0 = (size_t)t * a.nh + (size_t)kvh * G;      // (token, first head of the group)
+  const size_t th0 = (size_t)t * a.nh + (size_t)kvh * G;      // (token, first head of the group), of the partial rows
+  const size_t qh0 = (size_t)token * a.nh + (size_t)kvh * G;  // ... of q and out
   // with the merge inside (fused form with counters): this token's own splits; else all of them, and
   // the merge kernel is told which ones are empty
   const bool merge_inside = FUSED && f.counters != nullptr;
@@ -233,7 +236,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if (first > pos) {                                          // this token has fewer splits
     if (MERGE == CLUSTER) {                                   // (the barrier of a cluster counts the threads still there)
       if (split == 0)
-        for (int i = tid; i < G * HD; i += NWARPS * 32) a.out[th0 * HD + i] = __float2bfloat16_rn(0.f);
+        for (int i = tid; i < G * HD; i += NWARPS * 32) a.out[qh0 * HD + i] = __float2bfloat16_rn(0.f);
     } else if (!merge_inside && a.max_splits > 1 && tid < G) {
       float* ml = a.part_ml + ((th0 + tid) * a.max_splits + split) * 2;
       ml[0] = -INFINITY; ml[1] = 0.f;
@@ -320,7 +323,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     for (int c = tid; c < ROWS * CHUNKS; c += NWARPS * 32) {
       const int r = c / CHUNKS, ch = c % CHUNKS;
       const bool ok = r < G;
-      hb::cp_async16(q_s + r * STRIDE + ch * 8, a.q + (th0 + (ok ? r : 0)) * HD + ch * 8, ok);
+      hb::cp_async16(q_s + r * STRIDE + ch * 8, a.q + (qh0 + (ok ? r : 0)) * HD + ch * 8, ok);
     }
     hb::cp_async_commit();
     __syncthreads();                               // the barriers are initialised
@@ -535,7 +538,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             o.x = fmaf(v[sp].x, w[sp], o.x); o.y = fmaf(v[sp].y, w[sp], o.y);
             o.z = fmaf(v[sp].z, w[sp], o.z); o.w = fmaf(v[sp].w, w[sp], o.w);
           }
-        *reinterpret_cast<uint2*>(a.out + (th0 + row) * HD + d) =
+        *reinterpret_cast<uint2*>(a.out + (qh0 + row) * HD + d) =
             make_uint2(hb::pack_bf16(o.x * inv, o.y * inv), hb::pack_bf16(o.z * inv, o.w * inv));
       }
       cluster_sync();                                // nobody leaves while its rows are being read
@@ -561,7 +564,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
     } else {
       if (a.sink && l > 0.f) l += expf(-mx);
-      a.out[(th0 + row) * HD + d] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
+      a.out[(qh0 + row) * HD + d] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
     }
   }
   if (!counted || !arrive()) return;
@@ -618,7 +621,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     uint2 pack;
     pack.x = *reinterpret_cast<uint32_t*>(&lo);
     pack.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(a.out + (th0 + row) * HD + d) = pack;
+    *reinterpret_cast<uint2*>(a.out + (qh0 + row) * HD + d) = pack;
   }
   if (tid == 0) f.counters[t * a.nkv + kvh] = 0;     // zero again for the next launch
 }
@@ -663,13 +666,13 @@ int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, 
 // token one decode row; partials merged by hb_attention_merge), with TMA tile loads. Returns
 // HB_ERR_UNSUPPORTED for what those cannot take (a sliding window, a chunk size or page size
 // that breaks the 64-key tiles): the caller then uses hb_attention_decode. `status` is one int
-// on the device, zero before the call; nonzero afterwards = a wait on a load timed out.
-extern "C" int hb_attention_decode_tma(const void* q, const void* k_pages, const void* v_pages, int n_pages,
+// on the device, zero before the call; nonzero afterwards = a wait on a load timed out. `rows`: as hb_attention_decode_rows.
+extern "C" int hb_attention_decode_tma_rows(const void* q, const void* k_pages, const void* v_pages, int n_pages,
                                        const int* block_table, int table_stride, const int* seq_of_token,
                                        const int* positions, void* out, int n_tokens, int nh, int nkv, int hd,
                                        int page_size, int chunk, int window, float scale, int sink, int split_size,
                                        int max_splits, float* part_acc, float* part_ml, int* status,
-                                       cudaStream_t stream) {
+                                       const long long* rows, cudaStream_t stream) {
   if (!q || !k_pages || !v_pages || !block_table || !seq_of_token || !positions || !out || !status) return HB_ERR_BAD_ARG;
   if (n_tokens < 0 || n_pages <= 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || table_stride <= 0 ||
       chunk < 0 || window < 0 || max_splits < 1 || split_size <= 0 || split_size % TILE != 0)
@@ -683,13 +686,24 @@ extern "C" int hb_attention_decode_tma(const void* q, const void* k_pages, const
   if (cluster && reinterpret_cast<uintptr_t>(out) % 8) return HB_ERR_UNSUPPORTED;
   if (n_tokens == 0) return HB_OK;
   Args a{(const __nv_bfloat16*)q, block_table, seq_of_token, positions, (__nv_bfloat16*)out, part_acc, part_ml, status,
-         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, sink};
+         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, rows, sink};
   const Fuse none{};
   if (hd == 128) return cluster ? launch<128, CLUSTER>(k_pages, v_pages, n_pages, n_tokens, a, none, stream)
                                 : launch<128, APART>(k_pages, v_pages, n_pages, n_tokens, a, none, stream);
   if (hd == 64) return cluster ? launch<64, CLUSTER>(k_pages, v_pages, n_pages, n_tokens, a, none, stream)
                                : launch<64, APART>(k_pages, v_pages, n_pages, n_tokens, a, none, stream);
   return HB_ERR_UNSUPPORTED;
+}
+
+extern "C" int hb_attention_decode_tma(const void* q, const void* k_pages, const void* v_pages, int n_pages,
+                                       const int* block_table, int table_stride, const int* seq_of_token,
+                                       const int* positions, void* out, int n_tokens, int nh, int nkv, int hd,
+                                       int page_size, int chunk, int window, float scale, int sink, int split_size,
+                                       int max_splits, float* part_acc, float* part_ml, int* status,
+                                       cudaStream_t stream) {
+  return hb_attention_decode_tma_rows(q, k_pages, v_pages, n_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
+                                      nh, nkv, hd, page_size, chunk, window, scale, sink, split_size, max_splits, part_acc,
+                                      part_ml, status, nullptr, stream);
 }
 
 // The fused form: `qkv` [n_tokens, (nh + 2 nkv) * hd] is the q/k/v projection's output; the kernel
@@ -722,7 +736,7 @@ extern "C" int hb_attention_decode_fused(const void* qkv, const float* inv_freq,
   if ((long long)n_pages * nkv * page_size > 0x7fffffffLL) return HB_ERR_UNSUPPORTED;
   if (n_tokens == 0) return HB_OK;
   Args a{nullptr, block_table, seq_of_token, positions, (__nv_bfloat16*)out, part_acc, part_ml, status,
-         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, sink};
+         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, nullptr, sink};
   if (!norm_first && (q_norm_w || k_norm_w || rot_mul != 1.f)) return HB_ERR_UNSUPPORTED;   // as hb_qkv_post
   Fuse f{(const __nv_bfloat16*)qkv, inv_freq, rot_pairs, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, counters,
          interleaved, qk_norm, temp_on, qk_eps, floor_scale, attn_scale, q_norm_w, k_norm_w, norm_first, rot_mul, v_is_k};

@@ -39,6 +39,9 @@ _SIGNATURES = {
     "hb_paged_attention": [P, I, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, F, P, P, I, I, P, P, P],
     "hb_attention_portions": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, F, P, P, I, P, P, P],
     "hb_attention_merge": [P, P, P, I, I, I, I, I, I, P, P],
+    "hb_attention_merge_rows": [P, P, P, I, I, I, I, I, I, P, P, P],
+    "hb_attention_decode_rows": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P, P],
+    "hb_attention_decode_tma_rows": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P, P],
     "hb_attention_decode": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P],
     "hb_attention_decode_tma": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P],
     "hb_attention_decode_fused": [P, P, I, I, I, F, I, F, F, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P, P, P, P, P, I, F, I, I, P],
@@ -1402,15 +1405,24 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                      seq_of_token: torch.Tensor, positions: torch.Tensor, chunk: int, window: int, scale: float,
                      max_context: int, sink: bool = False, softcap: float = 0.0,
                      slopes: Optional[torch.Tensor] = None, sink_values: Optional[torch.Tensor] = None,
-                     keep: int = 0, parts: bool = False):
+                     keep: int = 0, parts: bool = False, rows: Optional[torch.Tensor] = None,
+                     out: Optional[torch.Tensor] = None):
     """Attention for a batch of single decoded tokens (every row of ``q`` is one request's
     token), bfloat16, split over runs of ``ATTENTION_SPLIT`` keys. Uses scratch memory for the
     partial results of the splits. ``softcap``, ``slopes``, ``sink_values``: as :func:`paged_attention`
-    (the kernel that loads its tiles by cp.async takes them)."""
+    (the kernel that loads its tiles by cp.async takes them). With ``rows`` (int64, distinct) only those tokens of the
+    step are decoded, from where they lie in ``q`` to where they lie in ``out`` [N, nh, hd] (not with ``parts``)."""
+    if rows is not None:
+        rows, seq_of_token, positions = rows.contiguous(), seq_of_token.contiguous(), positions.contiguous()
     _need(q, "q", torch.bfloat16); _need(k_pages, "k_pages", q.dtype); _need(v_pages, "v_pages", q.dtype)
     for t, nm in ((block_table, "block_table"), (seq_of_token, "seq_of_token"), (positions, "positions")):
         _need(t, nm, torch.int32)
     n, nh, hd = q.shape
+    if rows is not None:
+        _need(rows, "rows", torch.int64)
+        if parts or out is None or out.shape != q.shape or out.dtype != q.dtype or not out.is_contiguous():
+            raise KernelError("tokens decoded in place need an output of the queries' shape and type")
+        n = rows.numel()
     _, nkv, page_size, hd2 = k_pages.shape
     if hd2 != hd or k_pages.shape != v_pages.shape:
         raise KernelError("cache pages do not match the query's head_dim")
@@ -1424,7 +1436,8 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
     elif window > 0:
         longest = min(longest, window)
     split_size, splits = _decode_splits(longest, n * nkv * -(-(nh // nkv) // 16))
-    out = None if parts else torch.empty_like(q)
+    if rows is None:
+        out = None if parts else torch.empty_like(q)
     reshaped = bool(softcap) or slopes is not None or sink_values is not None or keep > 0 or parts
     part_acc = part_ml = None
 
@@ -1444,19 +1457,19 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                 raise KernelError(f"{nm} needs one number per query head")
     sink = bool(sink) or sink_values is not None
     # tile loads by TMA where the range and the pages allow it (the kernel says if not)
-    code = _UNSUPPORTED if reshaped else lib().hb_attention_decode_tma(
+    code = _UNSUPPORTED if reshaped else lib().hb_attention_decode_tma_rows(
         _ptr(q), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table), block_table.shape[1],
         _ptr(seq_of_token), _ptr(positions), _ptr(out), n, nh, nkv, hd, page_size, int(chunk), int(window), float(scale),
-        int(sink), split_size, splits, _ptr(part_acc), _ptr(part_ml), _ptr(_tc_status(q.device)), _stream())
+        int(sink), split_size, splits, _ptr(part_acc), _ptr(part_ml), _ptr(_tc_status(q.device)), _ptr(rows), _stream())
     if code == _UNSUPPORTED:
         if in_cluster:
             in_cluster = False
             part_acc, part_ml = scratch()
-        code = lib().hb_attention_decode(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.shape[1],
+        code = lib().hb_attention_decode_rows(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.shape[1],
                                          _ptr(seq_of_token), _ptr(positions), _ptr(out), n, nh, nkv, hd, page_size,
                                          int(chunk), int(window), int(keep), float(scale), int(sink), None, float(softcap),
                                          _ptr(slopes), _ptr(sink_values), split_size, splits,
-                                         _ptr(part_acc), _ptr(part_ml), _stream())
+                                         _ptr(part_acc), _ptr(part_ml), _ptr(rows), _stream())
         _check(code, "attention_decode")
     else:
         TC_USED[0] = True
@@ -1464,8 +1477,8 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
     if parts:
         return part_acc, part_ml
     if splits > 1 and not in_cluster:
-        _check(lib().hb_attention_merge(_ptr(part_acc), _ptr(part_ml), _ptr(out), _dt(out), n * nh, hd, splits,
-                                        int(sink), nh, _ptr(sink_values), _stream()), "attention_merge")
+        _check(lib().hb_attention_merge_rows(_ptr(part_acc), _ptr(part_ml), _ptr(out), _dt(out), n * nh, hd, splits,
+                                        int(sink), nh, _ptr(sink_values), _ptr(rows), _stream()), "attention_merge")
     return out
 
 

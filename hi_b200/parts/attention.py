@@ -52,13 +52,14 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
     positions = ctx.positions
     decode_ok = ops.decode_attention_supported(q.dtype, nh, nkv, hd)
 
-    def decode(rows_q, seq, pos, longest):
-        return ops.decode_attention(rows_q, k_pages, v_pages, block_table, seq, pos, chunk, sliding, scale, longest,
-                                    sink=sink, softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep)
+    def decode(longest, rows=None, out=None):
+        return ops.decode_attention(q, k_pages, v_pages, block_table, ctx.seq_of_token, positions, chunk, sliding, scale, longest,
+                                    sink=sink, softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep, rows=rows,
+                                    out=out)
 
     if ctx.max_new == 1 and decode_ok:
         # every token of the step is one request's decoded token: the tensor-core kernel
-        return decode(q, ctx.seq_of_token, positions, ctx.max_context)
+        return decode(ctx.max_context)
     # at least a tile of new tokens somewhere: the tcgen05 kernel; short portions: mma.sync
     tc = ctx.max_new >= ops.PREFILL_TC_MIN_TOKENS and ops.prefill_attention_tc_supported(q.dtype, nh, nkv, hd, ctx.page_size)
     if ctx.max_new > 1 and ops.prefill_attention_supported(q.dtype, nh, nkv, hd):
@@ -75,10 +76,7 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
                                       softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep)
         if single:
             # single tokens beside portions: their long key ranges go through the split decode kernel
-            rows = ctx.decode_rows
-            od = decode(q.index_select(0, rows), ctx.seq_of_token.index_select(0, rows), positions.index_select(0, rows),
-                        ctx.decode_max_context)
-            o.index_copy_(0, rows, od)
+            decode(ctx.decode_max_context, ctx.decode_rows, o)
         return o
     if ctx.max_new > 1 and q.dtype == torch.float32 and \
             ops.portion_attention_pays(zip(ctx.start_pos, ctx.n_new), nh, nkv, hd, chunk, sliding, keep):

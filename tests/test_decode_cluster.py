@@ -47,3 +47,35 @@ def test_splits_meet_in_a_cluster(nh, nkv, hd, lens, page, chunk, sink, monkeypa
         assert err < 2 ** -7, (i, err)
     # the same sums in the same order: at most the last place of bfloat16 where a product was contracted differently
     assert float((got.float() - apart.float()).abs().max()) <= 2 ** -8 * float(apart.float().abs().max())
+
+
+# by a cluster, by the merge of several rounds' splits, of more than eight splits, by the cp.async kernel (rows of 192, a window)
+@pytest.mark.parametrize("nh,nkv,hd,lens,window", [(8, 2, 128, [900, 1, 300], 0), (24, 24, 128, [700] * 30, 0), (4, 1, 64, [9000, 64], 0),
+                                                   (8, 4, 192, [300, 77, 1000], 0), (8, 2, 64, [1500, 3], 1024)])
+def test_tokens_decoded_where_they_lie_in_a_step(nh, nkv, hd, lens, window):
+    from hi_b200.kernels import ops
+
+    g = torch.Generator(device=DEV).manual_seed(hd + len(lens))
+    page, n = 64, len(lens)
+    need = [-(-k // page) for k in lens]
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16)
+    kp, vp = rnd(sum(need), nkv, page, hd), rnd(sum(need), nkv, page, hd)
+    table, at = torch.zeros(n, max(need), dtype=torch.int32, device=DEV), 0
+    for i, k in enumerate(need):
+        table[i, :k] = torch.arange(at, at + k)
+        at += k
+    total = 3 * n + 5                                       # tokens of the step; every third or so is a decoded one
+    rows = (torch.randperm(total, device=DEV, generator=g)[:n]).sort().values
+    q, out = rnd(total, nh, hd), rnd(total, nh, hd)
+    i32 = lambda: torch.zeros(total, dtype=torch.int32, device=DEV)
+    seq, pos = i32(), i32()
+    seq[rows] = torch.arange(n, dtype=torch.int32, device=DEV)
+    pos[rows] = torch.tensor([k - 1 for k in lens], dtype=torch.int32, device=DEV)
+    rest = (hd ** -0.5, max(lens))
+    want = ops.decode_attention(q[rows], kp, vp, table, seq[rows], pos[rows], 0, window, *rest)
+    before = out.clone()
+    assert ops.decode_attention(q, kp, vp, table, seq, pos, 0, window, *rest, rows=rows, out=out) is out
+    assert torch.equal(out[rows], want)                     # the same kernels and cuts, other addresses
+    others = torch.ones(total, dtype=torch.bool, device=DEV)
+    others[rows] = False
+    assert torch.equal(out[others], before[others])
