@@ -43,6 +43,17 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// The largest of a row's scores in four chains of pairs (a maximum takes three operands): 64 steps that waited for one another cost
+// 2,048 tokens of 40 heads of 128 74.7 us where they take 73.0, 513 tokens behind 7,000 and others beside them 202 where 197.
+__device__ __forceinline__ float row_max(const float (&v)[BKEYS]) {
+  float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int i = 0; i < BKEYS; i += 8)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) top[c] = fmaxf(fmaxf(top[c], v[i + 2 * c]), v[i + 2 * c + 1]);
+  return fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+}
+
 // What the epilogue does with the two maps a1, a2 of a head (float32, normalised by their softmax):
 //   o = a1 - lambda a2;  o <- o rsqrt(mean over vdim of o^2 + eps) mul;  out = o * sigmoid(gate)   (gate null: no gate)
 // `out` is [rows, nh / 2, vdim]; gate row t starts at gate + t * gate_stride and is laid out as a row of `out`.
@@ -352,19 +363,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (interior && sigmoid) {
         // nothing to mask and no maximum to follow
       } else if (interior) {
-        float top = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < BKEYS; ++i) top = fmaxf(top, sv[i]);
-        mx = fmaxf(mx, top * scale_l2);     // the scale is positive
+        mx = fmaxf(mx, row_max(sv) * scale_l2);     // the scale is positive
       } else {
 #pragma unroll
         for (int i = 0; i < BKEYS; ++i) {
           const int key = key_base + i;
           // masked scores become -inf BEFORE scaling, so the same exponential code serves both paths
-          const float s = (row_ok && key <= pos && (key >= lo || key < a.keep)) ? sv[i] : -INFINITY;
-          sv[i] = s;
-          mx = fmaxf(mx, s * scale_l2);
+          sv[i] = (row_ok && key <= pos && (key >= lo || key < a.keep)) ? sv[i] : -INFINITY;
         }
+        mx = fmaxf(mx, row_max(sv) * scale_l2);
       }
       // the S buffer may be overwritten by the MMA two tiles on
       tc::fence_before();
