@@ -40,11 +40,22 @@ mlstm_gates_kernel(const float* __restrict__ z, const float* __restrict__ bias_i
   float m_before_block = *m_state;          // every thread carries the maximum that enters the block of tokens
   // A token maps the maximum m to max(m + f, i); two tokens in turn map it to max(m + f1 + f2, max(i1 + f2, i2)):
   // the pairs (F, I) combine associatively, so a block of tokens is scanned in a few steps instead of one by one.
+  // The next block's pre-activations are asked for ahead of this one's scan: the blocks come in turn, and the trip to memory was
+  // half of each one's time.
+  float next_i = 0.f, next_f = 0.f;
+  auto ask = [&](int t) {
+    if (t < end) {
+      next_i = z[(size_t)t * 2 * heads + h];
+      next_f = z[(size_t)t * 2 * heads + heads + h];
+    }
+  };
+  ask(begin + threadIdx.x);
   for (int t0 = begin; t0 < end; t0 += GATE_THREADS) {
     const int t = t0 + threadIdx.x;
     float gi = -INFINITY, gf = 0.f;          // past the end: the identity map
+    const float zi = next_i + bi, zf = next_f + bf;
+    ask(t + GATE_THREADS);
     if (t < end) {
-      const float zi = z[(size_t)t * 2 * heads + h] + bi, zf = z[(size_t)t * 2 * heads + heads + h] + bf;
       const float cf = cap * tanhf(zf * inv_cap);
       gi = cap * tanhf(zi * inv_cap);
       gf = fminf(cf, 0.f) - log1pf(expf(-fabsf(cf)));      // log sigmoid

@@ -632,6 +632,8 @@ CHUNKED_MIN_TOKENS = 80      # ... and 8 more for every request of the step, whe
 # portion, for 10^4 columns of all tokens' states (100 tiles of 32 columns of all chunks'). Fitted to 3,465 measurements: 1 to 64
 # requests of 4 to 512 tokens, even or all but one of one token, 4 to 64 heads of 16 x 16 to 128 x 128. What the sums choose is
 # 1 % from the faster form on average, and slower than one by one by more than 3 % in 122 of them, by half at most.
+# (Chunks have become 0.84 of these times on average since, their rows being prepared once a head; over 1,800 further steps the
+# choice is 3 % from the faster form, and tables fitted anew moved as many steps the wrong way as the right one.)
 _BY_TOKEN = {
     "delta": {16: (4.1, 0.21, 0.14), 32: (4.2, 0.20, 0.09), 64: (4.8, 0.21, 0.26), 96: (10.9, 0.18, 0.71), 128: (10.8, 0.18, 0.76)},
     "mlstm": {16: (2.9, 0.39, 0.31), 32: (3.5, 0.13, 0.24), 64: (4.8, 0.17, 0.39), 96: (7.5, 0.15, 0.68), 128: (6.6, 0.17, 0.67)}}
