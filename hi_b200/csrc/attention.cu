@@ -143,7 +143,9 @@ __global__ void paged_attention_kernel(const T* __restrict__ q, const T* __restr
 // splits of 128 dims, 11.6 us for 2,560 rows of five, 32 us for 9,600 rows of two in float32; this one 2.1, 3.5 and 5.8 us.)
 constexpr int MERGE_AHEAD = 8, MERGE_ROWS = 8;
 
-template <typename T, int W>
+// PLACED: the rows of a token go to that of `token_rows`. (A form of its own: the division that finds the token cost the other one
+// 0.7 us where all blocks look.)
+template <typename T, int W, bool PLACED>
 __global__ void __launch_bounds__(32 * MERGE_ROWS) attention_merge_kernel(const float* __restrict__ part_acc,
                                                                           const float* __restrict__ part_ml, T* __restrict__ out,
                                                                           long long rows, int hd, int splits, int sink, int nh,
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(32 * MERGE_ROWS) attention_merge_kernel(const 
   const int lane = threadIdx.x & 31;
   const long long th = (long long)blockIdx.x * MERGE_ROWS + (threadIdx.x >> 5);
   if (th >= rows) return;
-  const long long to = token_rows ? token_rows[th / nh] * nh + th % nh : th;
+  const long long to = PLACED ? token_rows[th / nh] * nh + th % nh : th;
   const float* acc = part_acc + (size_t)th * splits * hd;
   struct alignas(4 * W) Vec { float x[W]; };
   Vec ahead[MERGE_AHEAD];
@@ -216,8 +218,9 @@ int launch_merge(const float* part_acc, const float* part_ml, void* out, long lo
   const long long blocks = (rows + MERGE_ROWS - 1) / MERGE_ROWS;
   if (blocks > 0x7fffffffLL) return HB_ERR_UNSUPPORTED;
   auto fits = [&](int w) { return hd % w == 0 && p % (4 * w) == 0 && o % (sizeof(T) * w) == 0; };
-#define HB_MERGE(W) \
-  attention_merge_kernel<T, W><<<(int)blocks, 32 * MERGE_ROWS, 0, stream>>>(part_acc, part_ml, (T*)out, rows, hd, splits, sink, nh, sink_values, token_rows)
+#define HB_MERGE(W)                                                                                                                \
+  (token_rows ? attention_merge_kernel<T, W, true> : attention_merge_kernel<T, W, false>)<<<(int)blocks, 32 * MERGE_ROWS, 0, stream>>>( \
+      part_acc, part_ml, (T*)out, rows, hd, splits, sink, nh, sink_values, token_rows)
   if (fits(4) && (hd % 128 == 0 || hd % 64 != 0)) HB_MERGE(4);
   else if (fits(2)) HB_MERGE(2);
   else HB_MERGE(1);
