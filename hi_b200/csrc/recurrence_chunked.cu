@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(const ChunkArgs a) {
   __shared__ __align__(16) float gr[SCALAR ? W * 20 : (C * LD > W * 20 ? C * LD : W * 20)];    // [token][row] decays, then [row][token] R k
   __shared__ __align__(16) float A[C][C + 1], B[C][20], Ts[C][20], bet[C], g1[C];
   // what the roundings of T P k, P q and R k leave: with the delta rule it goes into their third pieces
-  __shared__ __nv_bfloat16 kl[PLAIN ? 1 : C][LD], ql[PLAIN ? 1 : C][LD], rl[PLAIN ? 1 : W][C + 2];
+  __shared__ __align__(4) __nv_bfloat16 kl[PLAIN ? 1 : C][LD], ql[PLAIN ? 1 : C][LD], rl[PLAIN ? 1 : W][C + 2];     // (read in pairs)
   __shared__ int where[2];
   const int unit = a.unit0 + blockIdx.x, head = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) where[0] = -1;
