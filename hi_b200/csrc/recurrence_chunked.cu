@@ -15,7 +15,7 @@
 //     in registers as accumulator tiles; the sums over all rows are brought together in shared memory in a fixed order.
 //     Two groups of four more warps take turns: they copy the prepared chunks in (bulk copies, three or four chunks ahead),
 //     make T v, and add up and write the outputs, which nothing waits for.
-// The prepared chunks (25 to 39 KB a head) are laid out for as many chunks as 128 MB hold; longer steps go in slices.
+// The prepared chunks (7.5 to 39.5 KB a head, by key size and rule) go through a scratch of bounded size: see slices_of.
 //
 // Measured (B200, one request of 2,048 tokens, 16 heads of 128 x 128; token after token / sixteen at a time with the rows
 // prepared by every block for itself / now): delta rule 582 / 234 / 192 us (45 of them the preparation); mLSTM with 1,101 and
@@ -31,6 +31,8 @@
 //
 // What is not finite in a token's inputs reaches that token's and later outputs of the request, never an earlier one (an
 // infinite value or state comes out of the products as NaN, where token after token the sum could stay infinite).
+#include <algorithm>
+
 #include "api.h"
 #include "common.cuh"
 #include "mma.cuh"
@@ -39,6 +41,7 @@
 namespace {
 
 constexpr int C = 16;       // tokens of a chunk
+constexpr int SMS = 148;
 
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
@@ -89,16 +92,29 @@ struct ChunkArgs {
   int row_step, col_step;    // strides of S in the state
   const int* cu_seqlens;
   const int* slots;
-  unsigned char* images;     // [units of the slice, heads]: ChunkImage
+  unsigned char* images;     // [units of the launch, heads]: ChunkImage
   float* out;                // [N, heads * vdim]
   float* nq;                 // [N, heads] (with take): outputs of column vdim
   int* status;
   int n_seqs, heads, kvh, dim, vdim, cols;
-  int unit0, units;          // the slice's first unit and how many
+  int share, shares;         // which share of every request's chunks, and how many there are
+  int unit0, units;          // the launch's first unit of the share and how many
 };
 
-// unit = a request's chunk: those of request s start at cu[s] / C + s (there is room for a partial one each)
-__device__ __forceinline__ int first_unit(const int* cu, int s) { return cu[s] / C + s; }
+// A request's chunks in a launch: the first of them, how many, and the first one's place among the launch's units.
+struct Span {
+  int chunk, count, unit;
+};
+
+// Share i of a request of c chunks is the i-th run of ceil(c / shares) of them. A unit is a chunk of the share; those of request s
+// start at cu[s] / (C shares) + s, which leaves every request room for ceil(its tokens / (C shares)).
+__host__ __device__ inline Span span_of(const int* cu, int s, int share, int shares, int unit0, int units) {
+  const int chunks = (cu[s + 1] - cu[s] + C - 1) / C, run = shares == 1 ? chunks : (chunks + shares - 1) / shares;
+  const int at = (shares == 1 ? cu[s] / C : cu[s] / (C * shares)) + s - unit0, from = at < 0 ? -at : 0;
+  int to = run < chunks - share * run ? run : chunks - share * run;
+  if (to > units - at) to = units - at;
+  return {share * run + from, to - from, at + from};
+}
 
 // hb::split3 with the rests of the two floats in the last pieces
 __device__ __forceinline__ void split_more(float2 v, float2 rest, uint32_t (&p)[3]) {
@@ -142,19 +158,20 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(const ChunkArgs a) {
   // what the roundings of T P k, P q and R k leave: with the delta rule it goes into their third pieces
   __shared__ __align__(4) __nv_bfloat16 kl[PLAIN ? 1 : C][LD], ql[PLAIN ? 1 : C][LD], rl[PLAIN ? 1 : W][C + 2];     // (read in pairs)
   __shared__ int where[2];
-  const int unit = a.unit0 + blockIdx.x, head = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int unit = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) where[0] = -1;
   __syncthreads();
   for (int s = tid; s < a.n_seqs; s += 128) {
-    const int c = unit - first_unit(a.cu_seqlens, s), n = a.cu_seqlens[s + 1] - a.cu_seqlens[s];
-    if (c >= 0 && c * C < n) { where[0] = a.cu_seqlens[s] + c * C; where[1] = a.cu_seqlens[s + 1]; }
+    const Span span = span_of(a.cu_seqlens, s, a.share, a.shares, a.unit0, a.units);
+    const int c = unit - span.unit;
+    if (c >= 0 && c < span.count) { where[0] = a.cu_seqlens[s] + (span.chunk + c) * C; where[1] = a.cu_seqlens[s + 1]; }
   }
   __syncthreads();
   const int t0 = where[0];
   if (t0 < 0) return;
   const int count = min(C, where[1] - t0);
   const int kvhead = head / (a.heads / a.kvh);
-  Image& img = reinterpret_cast<Image*>(a.images)[(size_t)blockIdx.x * a.heads + head];
+  Image& img = reinterpret_cast<Image*>(a.images)[(size_t)unit * a.heads + head];
   {
     // a column of the chunk a thread (or every STEP-th token of one)
     constexpr int STEP = 128 / W > 0 ? 128 / W : 1;
@@ -425,11 +442,9 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
   extern __shared__ __align__(128) unsigned char raw[];
   typename Smem::All& sm = *reinterpret_cast<typename Smem::All*>(raw);
   const int head = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CG;
-  const int last = a.cu_seqlens[seq + 1], unit0 = first_unit(a.cu_seqlens, seq);
-  const int skip = max(0, a.unit0 - unit0);                          // chunks of earlier slices
-  const int first = a.cu_seqlens[seq] + skip * C;
-  const int chunks = min((last - first + C - 1) / C, a.unit0 + a.units - (unit0 + skip));
-  if (first >= last || chunks <= 0) return;
+  const Span span = span_of(a.cu_seqlens, seq, a.share, a.shares, a.unit0, a.units);
+  const int first = a.cu_seqlens[seq] + span.chunk * C, last = a.cu_seqlens[seq + 1], chunks = span.count;
+  if (chunks <= 0) return;
   const int tid = threadIdx.x;
   if (tid == 0) {
 #pragma unroll
@@ -439,7 +454,7 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  const Image* images = reinterpret_cast<const Image*>(a.images) + (size_t)(unit0 + skip - a.unit0) * a.heads + head;
+  const Image* images = reinterpret_cast<const Image*>(a.images) + (size_t)span.unit * a.heads + head;
   bool ok = true;
   auto there = [&](uint64_t* full, int use) {          // a copy has arrived
     if (ok && !tc::mbar_wait(full, use & 1)) {
@@ -710,25 +725,59 @@ int launch_columns(const ChunkArgs& a, cudaStream_t stream) {
   return HB_OK;
 }
 
-// Units of a slice: as many images as 128 MB hold (the sequence of launches over the slices carries the states).
-inline int slice_units(int heads, size_t image_bytes, int units) {
-  const size_t fit = ((size_t)128 << 20) / (heads * image_bytes);
-  return fit < 1 ? 1 : fit < (size_t)units ? (int)fit : units;
+// How a step's chunks go through `most_bytes` of scratch: every request's in `shares` runs, and the units of a share `units` at a
+// time, launch after launch (the states go through memory).
+// Shares keep the requests side by side, so the chain is the longest request's however many launches there are. Slices of
+// 128 MB that took the chunks in order ran the requests one after another: two of 4,096 tokens (delta rule, 16 heads of
+// 128 x 128) 1,037 us, 660 by shares; four of 2,048, 8 heads, 524 and 335. A launch more costs about 25 us, so the scratch is not
+// small (those in 256 / 64 / 32 MB: 654 / 687 / 761 and 327 / 343 / 362).
+// In order is the better way where a slice's blocks keep the SMs busy four times as long as the longest chain (64 requests of 100
+// tokens, 64 heads: 2,550 us, by shares of 128 MB 2,896; with "once as long" instead of four times, four requests of 2,048 and
+// 16 heads are 841 instead of 659), and where the requests' room for a partial chunk each would fill most of the scratch.
+struct Slices {
+  int shares, units;
+};
+inline Slices slices_of(int n_tokens, int n_seqs, int longest, int heads, int cols, size_t image_bytes, long long most_bytes) {
+  const long long images = most_bytes / (long long)image_bytes;
+  const int all = n_tokens / C + n_seqs, fit = (int)std::min<long long>(std::max(images / heads, 1LL), all), room = fit - n_seqs;
+  if (all == fit) return {1, all};
+  if (longest <= 0 || longest > n_tokens) longest = n_tokens;
+  const bool full = 4LL * ((longest + C - 1) / C) * SMS <= images * ((cols + 31) / 32);
+  if (full || 4 * (long long)room < fit) return {1, fit};
+  const int shares = (n_tokens / C + room - 1) / room;
+  return {shares, n_tokens / (C * shares) + n_seqs};
+}
+
+// Whether blocks of 32 columns take less time than blocks of 16: a chunk of theirs takes 1.6 times as long (with 1.4 or 1.9 in its
+// place 300 steps took 1.006 or 1.001 of the time, single ones up to 1.1 or 1.3). A step's time is that of all blocks' chunks over
+// all SMs or, if that is more, the rounds of the long requests' blocks, each a chain of the longest; a block's start and end count
+// as four chunks. (mLSTM, 16 heads, two requests of 4,096 tokens: 129 columns are 160 blocks of 32 and two rounds, 723 us, or 288
+// of 16 and two rounds, 498; 40 heads without correction, one of 304 tokens and 70 of one: 500 us in blocks of 16, 362 of 32.)
+inline bool wide_blocks(int n_tokens, int n_seqs, int longest, int heads, int cols) {
+  if (longest <= 0 || longest > n_tokens) longest = (n_tokens + n_seqs - 1) / n_seqs;
+  const long long chain = (longest + C - 1) / C + 4, work = n_tokens / C + 5LL * n_seqs;
+  const int requests = std::min(n_seqs, (2 * n_tokens + longest) / (2 * longest));
+  auto steps = [&](int width) {
+    const long long blocks = (long long)heads * ((cols + width - 1) / width);
+    return std::max(work * blocks / SMS, (requests * blocks + SMS - 1) / SMS * chain);
+  };
+  return 10 * steps(16) > 16 * steps(32);
 }
 
 template <typename T, int NW, bool SCALAR, bool PLAIN>
-int launch_chunked(ChunkArgs a, int units, cudaStream_t stream) {
-  const int step = slice_units(a.heads, sizeof(ChunkImage<NW, PLAIN>), units);
-  for (a.unit0 = 0; a.unit0 < units; a.unit0 += step) {
-    a.units = units - a.unit0 < step ? units - a.unit0 : step;
-    chunk_prepare_kernel<T, NW, SCALAR, PLAIN><<<dim3(a.units, a.heads), 128, 0, stream>>>(a);
-    HB_LAUNCH_CHECK();
-    // 32 columns a block share the images, once 16 a block are more than a block per SM
-    const long long blocks = (long long)((a.cols + 15) / 16) * a.heads * a.n_seqs;
-    const int rc = blocks > 148 && a.cols > 16 ? launch_columns<T, NW, 2, PLAIN>(a, stream)
-                                               : launch_columns<T, NW, 1, PLAIN>(a, stream);
-    if (rc != HB_OK) return rc;
-  }
+int launch_chunked(ChunkArgs a, int n_tokens, int longest, long long most_bytes, cudaStream_t stream) {
+  const Slices slices = slices_of(n_tokens, a.n_seqs, longest, a.heads, a.cols, sizeof(ChunkImage<NW, PLAIN>), most_bytes);
+  a.shares = slices.shares;
+  const bool wide = wide_blocks(n_tokens, a.n_seqs, longest, a.heads, a.cols);
+  const int units = n_tokens / (C * a.shares) + a.n_seqs;
+  for (a.share = 0; a.share < a.shares; ++a.share)
+    for (a.unit0 = 0; a.unit0 < units; a.unit0 += slices.units) {
+      a.units = units - a.unit0 < slices.units ? units - a.unit0 : slices.units;
+      chunk_prepare_kernel<T, NW, SCALAR, PLAIN><<<dim3(a.units, a.heads), 128, 0, stream>>>(a);
+      HB_LAUNCH_CHECK();
+      const int rc = wide ? launch_columns<T, NW, 2, PLAIN>(a, stream) : launch_columns<T, NW, 1, PLAIN>(a, stream);
+      if (rc != HB_OK) return rc;
+    }
   return HB_OK;
 }
 
@@ -740,26 +789,41 @@ size_t image_bytes(int dim, bool plain) {
 }
 
 template <typename T, bool SCALAR, bool PLAIN>
-int launch_by_dim(const ChunkArgs& a, int units, cudaStream_t stream) {
-  if (a.dim <= 32) return launch_chunked<T, 2, SCALAR, PLAIN>(a, units, stream);
-  if (a.dim <= 64) return launch_chunked<T, 4, SCALAR, PLAIN>(a, units, stream);
-  if (a.dim <= 96) return launch_chunked<T, 6, SCALAR, PLAIN>(a, units, stream);
-  return launch_chunked<T, 8, SCALAR, PLAIN>(a, units, stream);
+int launch_by_dim(const ChunkArgs& a, int n_tokens, int longest, long long most_bytes, cudaStream_t stream) {
+  if (a.dim <= 32) return launch_chunked<T, 2, SCALAR, PLAIN>(a, n_tokens, longest, most_bytes, stream);
+  if (a.dim <= 64) return launch_chunked<T, 4, SCALAR, PLAIN>(a, n_tokens, longest, most_bytes, stream);
+  if (a.dim <= 96) return launch_chunked<T, 6, SCALAR, PLAIN>(a, n_tokens, longest, most_bytes, stream);
+  return launch_chunked<T, 8, SCALAR, PLAIN>(a, n_tokens, longest, most_bytes, stream);
 }
 
 }  // namespace
 
-// Floats of scratch that the chunked recurrences need for `n_tokens` tokens of `n_seqs` requests.
-extern "C" long long hb_recurrence_chunked_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int plain) {
+// Floats of scratch that the chunked recurrences need for `n_tokens` tokens of `n_seqs` requests, `cols` columns a head (vdim; the
+// mLSTM vdim + 1), where `most_bytes` are to be enough or a single chunk of all heads needs more; `longest`: the longest portion,
+// 0 where it is not known. The recurrence is called with the same numbers.
+extern "C" long long hb_recurrence_chunked_scratch_floats(int n_tokens, int n_seqs, int longest, int heads, int dim, int cols, int plain,
+                                                          long long most_bytes) {
   const size_t bytes = image_bytes(dim, plain != 0);
-  return (long long)(slice_units(heads, bytes, n_tokens / C + n_seqs) * (heads * bytes) / 4);
+  return (long long)(slices_of(n_tokens, n_seqs, longest, heads, cols, bytes, most_bytes).units * (heads * bytes) / 4);
+}
+
+// What the launches of such a step take, for a look without a GPU: `out` = shares, units a launch; with `cu_seqlens` (of the host)
+// also request `seq`'s first chunk, number of chunks (<= 0: none) and first unit in the launch of `share` that starts at `unit0`.
+extern "C" void hb_recurrence_chunked_slices(int n_tokens, int n_seqs, int longest, int heads, int dim, int cols, int plain,
+                                             long long most_bytes, const int* cu_seqlens, int seq, int share, int unit0, int* out) {
+  const Slices slices = slices_of(n_tokens, n_seqs, longest, heads, cols, image_bytes(dim, plain != 0), most_bytes);
+  out[0] = slices.shares;
+  out[1] = slices.units;
+  if (!cu_seqlens) return;
+  const Span span = span_of(cu_seqlens, seq, share, slices.shares, unit0, slices.units);
+  out[2] = span.chunk; out[3] = span.count; out[4] = span.unit;
 }
 
 extern "C" int hb_delta_recurrence_chunked(const float* q, const float* k, const float* v, const float* beta,
                                            const float* decay, float* state, long long state_stride,
                                            const int* cu_seqlens, const int* slots, float* scratch, float* out,
-                                           int n_tokens, int n_seqs, int heads, int kvh, int dim, int vdim, int plain,
-                                           int* status, cudaStream_t stream) {
+                                           int n_tokens, int n_seqs, int longest, int heads, int kvh, int dim,
+                                           int vdim, int plain, long long most_bytes, int* status, cudaStream_t stream) {
   if (!q || !k || !v || (!beta && !plain) || !decay || !state || !cu_seqlens || !slots || !scratch || !out || !status) return HB_ERR_BAD_ARG;
   if (heads <= 0 || kvh <= 0 || heads % kvh || dim <= 0 || vdim <= 0 || n_seqs < 0 || n_tokens < 0) return HB_ERR_BAD_ARG;
   if (dim > 128 || heads > 65535 || n_seqs > 65535 || (reinterpret_cast<uintptr_t>(scratch) & 15)) return HB_ERR_UNSUPPORTED;
@@ -769,15 +833,14 @@ extern "C" int hb_delta_recurrence_chunked(const float* q, const float* k, const
   a.o_scale = 1.f; a.state = state; a.state_stride = state_stride; a.head_floats = (long long)dim * vdim;
   a.row_step = vdim; a.col_step = 1; a.cu_seqlens = cu_seqlens; a.slots = slots; a.images = reinterpret_cast<unsigned char*>(scratch); a.out = out; a.status = status;
   a.n_seqs = n_seqs; a.heads = heads; a.kvh = kvh; a.dim = dim; a.vdim = vdim; a.cols = vdim;
-  const int units = n_tokens / C + n_seqs;
-  return plain ? launch_by_dim<float, false, true>(a, units, stream) : launch_by_dim<float, false, false>(a, units, stream);
+  return plain ? launch_by_dim<float, false, true>(a, n_tokens, longest, most_bytes, stream) : launch_by_dim<float, false, false>(a, n_tokens, longest, most_bytes, stream);
 }
 
 extern "C" int hb_mlstm_recurrence_chunked(const void* proj, int proj_dtype, long long ld, int q_off, int k_off, int v_off,
                                            float q_scale, const float* keep, const float* take, float* state,
                                            long long state_stride, const int* cu_seqlens, const int* slots, float* scratch,
-                                           float* o, float* nq, int n_tokens, int n_seqs, int heads, int dim, int vdim,
-                                           int* status, cudaStream_t stream) {
+                                           float* o, float* nq, int n_tokens, int n_seqs, int longest, int heads, int dim, int vdim,
+                                           long long most_bytes, int* status, cudaStream_t stream) {
   if (!proj || !keep || !take || !state || !cu_seqlens || !slots || !scratch || !o || !nq || !status || n_seqs < 0 || n_tokens < 0 ||
       heads <= 0 || dim <= 0 || vdim <= 0)
     return HB_ERR_BAD_ARG;
@@ -792,7 +855,6 @@ extern "C" int hb_mlstm_recurrence_chunked(const void* proj, int proj_dtype, lon
   a.head_floats = (long long)(vdim + 1) * dim; a.row_step = 1; a.col_step = dim; a.cu_seqlens = cu_seqlens; a.slots = slots;
   a.images = reinterpret_cast<unsigned char*>(scratch); a.out = o; a.status = status; a.nq = nq; a.n_seqs = n_seqs; a.heads = heads; a.kvh = heads; a.dim = dim; a.vdim = vdim;
   a.cols = vdim + 1;
-  const int units = n_tokens / C + n_seqs;
-  return proj_dtype == HB_DTYPE_F32 ? launch_by_dim<float, true, true>(a, units, stream)
-                                    : launch_by_dim<__nv_bfloat16, true, true>(a, units, stream);
+  return proj_dtype == HB_DTYPE_F32 ? launch_by_dim<float, true, true>(a, n_tokens, longest, most_bytes, stream)
+                                    : launch_by_dim<__nv_bfloat16, true, true>(a, n_tokens, longest, most_bytes, stream);
 }

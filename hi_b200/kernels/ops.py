@@ -81,8 +81,8 @@ _SIGNATURES = {
                       I, I, I, I, P],
     "hb_delta_conv_update": [P, I, c_longlong, I, P, c_longlong, c_longlong, P, P, I, I, I, P],
     "hb_delta_recurrence": [P, P, P, P, P, P, c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
-    "hb_delta_recurrence_chunked": [P, P, P, P, P, P, c_longlong, P, P, P, P, I, I, I, I, I, I, I, P, P],
-    "hb_mlstm_recurrence_chunked": [P, I, c_longlong, I, I, I, F, P, P, P, c_longlong, P, P, P, P, P, I, I, I, I, I, P, P],
+    "hb_delta_recurrence_chunked": [P, P, P, P, P, P, c_longlong, P, P, P, P, I, I, I, I, I, I, I, I, c_longlong, P, P],
+    "hb_mlstm_recurrence_chunked": [P, I, c_longlong, I, I, I, F, P, P, P, c_longlong, P, P, P, P, P, I, I, I, I, I, I, c_longlong, P, P],
     "hb_skinny_linear": [P, c_longlong, P, P, P, I, I, I, I, P],
     "hb_delta_out_norm": [P, P, I, P, F, P, I, c_longlong, I, I, c_longlong, I, P],
     "hb_hyper_step": [P, P, P, I, P, I, P, P, P, I, P, P, F, P, P, I, F, P, I, P, P, I, I, I, P],
@@ -114,7 +114,7 @@ def lib():
             fn = getattr(handle, name)
             fn.argtypes = sig
             fn.restype = c_int
-        handle.hb_recurrence_chunked_scratch_floats.argtypes = [I, I, I, I, I]
+        handle.hb_recurrence_chunked_scratch_floats.argtypes = [I, I, I, I, I, I, I, c_longlong]
         handle.hb_recurrence_chunked_scratch_floats.restype = c_longlong
         handle.hb_moe_down_tc_scratch_floats.argtypes = [I]
         handle.hb_moe_down_tc_scratch_floats.restype = c_longlong
@@ -666,9 +666,12 @@ def _chunked_recurrence(n: int, n_seqs: int, dim: int, rule: str = "delta", head
     return fixed + chain * longest / 16 + work * chunks * heads * -(-cols // 32) / 100 < by_token
 
 
-def _chunked_scratch(n: int, n_seqs: int, heads: int, dim: int, plain: bool, device) -> torch.Tensor:
-    return torch.empty(lib().hb_recurrence_chunked_scratch_floats(n, n_seqs, heads, dim, int(plain)), dtype=torch.float32,
-                       device=device)
+CHUNKED_SCRATCH_BYTES = 256 << 20        # prepared chunks that a launch of a recurrence may hold (longer steps are several launches)
+
+
+def _chunked_scratch(n: int, n_seqs: int, longest: int, heads: int, dim: int, cols: int, plain: bool, device) -> torch.Tensor:
+    return torch.empty(lib().hb_recurrence_chunked_scratch_floats(n, n_seqs, int(longest), heads, dim, cols, int(plain),
+                                                                  CHUNKED_SCRATCH_BYTES), dtype=torch.float32, device=device)
 
 
 def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Optional[torch.Tensor],
@@ -695,11 +698,11 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Op
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     if not (general or rows or single_tokens) and _chunked_recurrence(
             n, slots.numel(), dim, "plain" if plain else "delta", heads, vdim, longest):
-        scratch = _chunked_scratch(n, slots.numel(), heads, dim, plain, q.device)
+        scratch = _chunked_scratch(n, slots.numel(), longest, heads, dim, vdim, plain, q.device)
         _check(lib().hb_delta_recurrence_chunked(
             _ptr(q), _ptr(k), _ptr(v), None if plain else _ptr(beta), _ptr(decay), _ptr(state), state.shape[1],
-            _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(out), n, slots.numel(), heads, kvh, dim, vdim, int(plain),
-            _ptr(_tc_status(q.device)), _stream()), "delta_recurrence")
+            _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(out), n, slots.numel(), int(longest), heads, kvh, dim, vdim,
+            int(plain), CHUNKED_SCRATCH_BYTES, _ptr(_tc_status(q.device)), _stream()), "delta_recurrence")
         TC_USED[0] = True
         LAUNCHES[0] += 1
         return out
@@ -932,11 +935,11 @@ def mlstm_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_s
     o = torch.empty((n, heads, vdim), dtype=torch.float32, device=proj.device)
     nq = torch.empty((n, heads), dtype=torch.float32, device=proj.device)
     if not rows_per_lane and _chunked_recurrence(n, slots.numel(), dim, "mlstm", heads, vdim + 1, longest):
-        scratch = _chunked_scratch(n, slots.numel(), heads, dim, True, proj.device)
+        scratch = _chunked_scratch(n, slots.numel(), longest, heads, dim, vdim + 1, True, proj.device)
         _check(lib().hb_mlstm_recurrence_chunked(
             _ptr(proj), _dt(proj), ld, q_off, k_off, v_off, float(q_scale), _ptr(keep), _ptr(take), _ptr(state),
-            state.stride(0), _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(o), _ptr(nq), n, slots.numel(), heads, dim,
-            vdim, _ptr(_tc_status(proj.device)), _stream()), "mlstm_recurrence")
+            state.stride(0), _ptr(cu_seqlens), _ptr(slots), _ptr(scratch), _ptr(o), _ptr(nq), n, slots.numel(), int(longest),
+            heads, dim, vdim, CHUNKED_SCRATCH_BYTES, _ptr(_tc_status(proj.device)), _stream()), "mlstm_recurrence")
         TC_USED[0] = True
         LAUNCHES[0] += 1
         return o, nq

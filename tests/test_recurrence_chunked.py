@@ -185,33 +185,56 @@ def test_single_tokens_by_whole_lines(heads, kvh, dim, vdim, plain, lens):
         assert torch.equal(dev[slot], state[slot])
 
 
-@pytest.mark.parametrize("plain", [False, True])
-def test_steps_that_take_several_slices_of_scratch(plain):
-    """More prepared chunks than one slice of the scratch holds: the states go from launch to launch, wherever a request's
-    chunks are cut."""
+# by shares (the first: of the scratch as it is) with blocks of 16 and of 32 columns, and in order, where most requests' first chunks
+# fill the scratch: launches that hold different requests
+@pytest.mark.parametrize("heads,dim,vdim,lens,scratch", [(64, 128, 8, [5, 2300, 600, 1, 33], 0), (3, 96, 80, [130, 1, 17, 260, 40], 1 << 20),
+                                                         (16, 64, 128, [200, 0, 150, 40, 1], 5 << 20), (8, 33, 70, [20] * 30, 4 << 20),
+                                                         (16, 128, 100, [100, 3, 40, 70], 1 << 19)])
+@pytest.mark.parametrize("rule", ["delta", "plain", "mlstm"])
+def test_steps_that_take_several_slices_of_scratch(rule, heads, dim, vdim, lens, scratch, monkeypatch):
+    """More prepared chunks than the scratch holds: the states go from launch to launch, wherever a request's chunks are cut."""
     from hi_b200.kernels import ops
 
-    heads, dim, vdim, lens = 64, 128, 8, [5, 1700, 600, 1, 33]
-    n, g = sum(lens), torch.Generator(device=DEV).manual_seed(3)
-    images = heads * (n // 16 + len(lens)) * (25 if plain else 38) * 1024          # (a little less than they take)
-    assert images > 128 << 20 and ops._chunked_recurrence(n, len(lens), dim)
+    n, g, cols = sum(lens), torch.Generator(device=DEV).manual_seed(3), vdim + (rule == "mlstm")
+    if scratch:
+        monkeypatch.setattr(ops, "CHUNKED_SCRATCH_BYTES", scratch)
+    size = lambda *a: ops._chunked_scratch(*a, dim, cols, rule != "delta", "cpu").numel()
+    assert size(n, len(lens), max(lens), heads) < (n // 16 + len(lens)) * heads * size(1, 1, 1, 1)
     rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
-    q, k = (F.normalize(rnd(n, heads, dim), dim=-1).reshape(n, -1) for _ in range(2))
-    v, beta = rnd(n, heads * vdim), torch.rand(n, heads, device=DEV, generator=g)
-    decay = torch.exp(-torch.exp(2.0 * rnd(n, heads * dim) - 2.0))
     cu, slots = tables(lens)
-    state = rnd(len(lens) + 2, heads * dim * vdim)
-    after = state.clone()
-    o = ops.delta_recurrence(q, k, v, None if plain else beta, decay, after, cu.to(DEV), slots.to(DEV), heads, heads, dim, vdim,
-                             plain=plain)
-    row = lambda t, x, w: x[t].double().view(heads, w)
+    kw = dict(longest=max(lens))
+    monkeypatch.setattr(ops, "_chunked_recurrence", lambda *a, **k: True)
+    if rule == "mlstm":
+        proj = 0.5 * rnd(n, heads * (2 * dim + vdim))
+        q, k, v = (t.reshape(n, heads, -1).double() for t in proj.split([heads * dim, heads * dim, heads * vdim], dim=1))
+        v = torch.cat([v, torch.ones(n, heads, 1, dtype=torch.float64, device=DEV)], dim=2)
+        keep, take = torch.rand(n, heads, device=DEV, generator=g), torch.rand(n, heads, device=DEV, generator=g)
+        state = 0.3 * rnd(len(lens) + 2, ops.mlstm_state_floats(heads, dim, vdim))
+        after = state.clone()
+        o, nq = ops.mlstm_recurrence(proj, 0, heads * dim, 2 * heads * dim, dim ** -0.5, keep, take, after, cu.to(DEV), slots.to(DEV), heads,
+                                     dim, vdim, **kw)
+        o = torch.cat([o.view(n, heads, vdim), nq.view(n, heads, 1)], dim=2).reshape(n, -1)
+        q, v, decay = q * dim ** -0.5, v * take.double()[:, :, None], keep.double()[:, :, None].expand(n, heads, dim)
+        shape, order = (heads, cols, dim), lambda S: S.permute(0, 2, 1)
+    else:
+        q, k = (F.normalize(rnd(n, heads, dim), dim=-1) for _ in range(2))
+        v, beta = rnd(n, heads, vdim), torch.rand(n, heads, device=DEV, generator=g)
+        decay = torch.exp(-torch.exp(2.0 * rnd(n, heads, dim) - 2.0))
+        state = rnd(len(lens) + 2, heads * dim * vdim)
+        after = state.clone()
+        o = ops.delta_recurrence(q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1), None if rule == "plain" else beta, decay.reshape(n, -1),
+                                 after, cu.to(DEV), slots.to(DEV), heads, heads, dim, vdim, plain=rule == "plain", **kw)
+        q, k, v, decay = q.double(), k.double(), v.double(), decay.double()
+        shape, order = (heads, dim, cols), lambda S: S
     for s, slot in enumerate(slots.tolist()):
-        S, want = state[slot].double().view(heads, dim, vdim), []
+        if lens[s] == 0:
+            assert torch.equal(after[slot], state[slot])
+            continue
+        S, want = order(state[slot, : heads * dim * cols].double().view(shape)), []
         for t in range(int(cu[s]), int(cu[s + 1])):
-            S = S * row(t, decay, dim)[:, :, None]
-            vt = row(t, v, vdim)
-            u = vt if plain else beta[t].double()[:, None] * (vt - torch.einsum("hdv,hd->hv", S, row(t, k, dim)))
-            S = S + row(t, k, dim)[:, :, None] * u[:, None, :]
-            want.append(torch.einsum("hdv,hd->hv", S, row(t, q, dim)).reshape(-1))
+            S = S * decay[t][:, :, None]
+            u = v[t] if rule != "delta" else beta[t].double()[:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None, :]
+            want.append(torch.einsum("hdv,hd->hv", S, q[t]).reshape(-1))
         close(o[int(cu[s]): int(cu[s + 1])], torch.stack(want), f"request {s}")
-        close(after[slot], S.reshape(-1), f"state {s}")
+        close(order(after[slot, : heads * dim * cols].view(shape)), S, f"state {s}")
