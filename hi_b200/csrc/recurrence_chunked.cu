@@ -711,6 +711,13 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
     }
     if (i + 2 < chunks) bar_arrive(FREED + b, COMP + HELP);
   }
+  // No copy is under way when the block leaves, also where a wait was given up: the last ones into each place, again with the limit
+  // (the others were waited for before their place was used again; where all went well these return at once).
+  if (h == 0)
+    for (int i = max(0, chunks - RING); i < chunks; ++i) {
+      if (i >= chunks - STAGES) tc::mbar_wait(&sm.full[i % STAGES], (i / STAGES) & 1);
+      tc::mbar_wait(&sm.full_m[i % RING], (i / RING) & 1);
+    }
 }
 
 template <typename T, int NW, int CT, bool PLAIN>
