@@ -628,20 +628,27 @@ def delta_conv_update(proj: torch.Tensor, chan_off: int, channels: int, taps_n: 
 
 
 CHUNKED_MIN_TOKENS = 80      # ... and 8 more for every request of the step, where its longest portion is not known
-# Microseconds of a step's recurrence one by one and by chunks, by key size: fixed, for a token (sixteen tokens) of the longest
-# portion, for 10^4 columns of all tokens' states (100 tiles of 32 columns of all chunks'). Fitted to 3,465 measurements: 1 to 64
-# requests of 4 to 512 tokens, even or all but one of one token, 4 to 64 heads of 16 x 16 to 128 x 128. What the sums choose is
-# 1 % from the faster form on average, and slower than one by one by more than 3 % in 122 of them, by half at most.
-# (Chunks have become 0.84 of these times on average since, their rows being prepared once a head; over 1,800 further steps the
-# choice is 3 % from the faster form, and tables fitted anew moved as many steps the wrong way as the right one.)
+# Microseconds of a step's recurrence one by one and by chunks, by key size: fixed; for a token (sixteen tokens) of the longest
+# portion; by chunks, for 100 chunks' preparation (a head each, whatever its columns); for 10^4 columns of all tokens' states, in
+# whole sixteens (100 tiles of 32 columns of all chunks'); for 10^4 columns of the requests' states, in and out. Fitted to 2,900
+# measurements of both forms: 1 to 97 requests of up to 2,900 tokens, even, uneven or one or two beside single tokens, 4 to 64 heads
+# of 16 x 16 to 128 x 128. What the sums choose is 0.5 % from the faster form on average and slower than one by one by more than 3 %
+# in 56 of them, by 0.29 at most (2.1 %, 102 and 0.83 with the tables before, without the preparation and the states, from when every
+# block prepared its chunks for itself). In 270 they choose another form than those: 0.84 of the time on average, by a tenth and more
+# the slower form in 17, most of them of 30 and more requests of few tokens.
 _BY_TOKEN = {
-    "delta": {16: (4.1, 0.21, 0.14), 32: (4.2, 0.20, 0.09), 64: (4.8, 0.21, 0.26), 96: (10.9, 0.18, 0.71), 128: (10.8, 0.18, 0.76)},
-    "mlstm": {16: (2.9, 0.39, 0.31), 32: (3.5, 0.13, 0.24), 64: (4.8, 0.17, 0.39), 96: (7.5, 0.15, 0.68), 128: (6.6, 0.17, 0.67)}}
+    "delta": {16: (3.2, 0.20, 0.07, 0.70), 32: (3.2, 0.20, 0.08, 0.41), 64: (3.3, 0.21, 0.18, 1.42),
+              96: (4.7, 0.21, 0.43, 6.15), 128: (3.9, 0.22, 0.46, 6.51)},
+    "mlstm": {16: (6.0, 0.12, 0.09, 0.16), 32: (3.4, 0.13, 0.17, 0.31), 64: (4.9, 0.16, 0.22, 1.72),
+              96: (3.6, 0.15, 0.38, 3.63), 128: (3.0, 0.16, 0.39, 3.72)}}
 _BY_TOKEN["plain"] = _BY_TOKEN["delta"]
 _BY_CHUNK = {
-    "delta": {16: (9.1, 1.22, 0.77), 32: (7.3, 2.10, 1.26), 64: (9.0, 1.31, 1.70), 96: (9.6, 1.62, 2.10), 128: (8.0, 1.57, 2.15)},
-    "plain": {16: (7.6, 0.95, 0.56), 32: (6.6, 1.42, 0.85), 64: (7.4, 0.93, 1.34), 96: (8.2, 1.07, 1.58), 128: (7.4, 1.01, 1.66)},
-    "mlstm": {16: (5.7, 2.13, 1.36), 32: (7.5, 1.68, 0.91), 64: (7.7, 0.97, 1.38), 96: (8.1, 0.88, 1.55), 128: (9.5, 0.87, 1.62)}}
+    "delta": {16: (9.5, 0.58, 0.54, 0.62, 1.03), 32: (9.7, 0.59, 0.51, 0.64, 0.68), 64: (9.1, 0.54, 0.90, 0.86, 3.72),
+              96: (9.4, 0.79, 1.43, 1.04, 4.25), 128: (8.9, 0.75, 1.45, 1.19, 4.46)},
+    "plain": {16: (7.5, 0.38, 0.16, 0.43, 1.36), 32: (7.3, 0.36, 0.26, 0.40, 1.41), 64: (7.5, 0.44, 0.40, 0.50, 2.10),
+              96: (7.1, 0.55, 0.66, 0.68, 4.55), 128: (6.9, 0.57, 0.90, 0.83, 4.97)},
+    "mlstm": {16: (7.6, 0.32, 0.13, 0.41, 1.68), 32: (7.8, 0.36, 0.36, 0.35, 1.54), 64: (7.8, 0.43, 0.66, 0.41, 2.76),
+              96: (8.1, 0.47, 0.86, 0.54, 6.74), 128: (7.7, 0.52, 1.06, 0.68, 7.03)}}
 
 
 def _chunked_recurrence(n: int, n_seqs: int, dim: int, rule: str = "delta", heads: int = 1, cols: int = 1, longest: int = 0) -> bool:
@@ -649,9 +656,9 @@ def _chunked_recurrence(n: int, n_seqs: int, dim: int, rule: str = "delta", head
     however few tokens it holds, and there is a launch more; where many requests fill the SMs the chain from token to token
     is not what bounds the step, and with keys of up to 64 a chunk then costs more than its tokens. So the ``longest`` portion
     decides, where the caller knows it, and the work of all (one by one / by chunks, us: delta rule, 16 heads of 128 x 128, one
-    request of 48 tokens 19 / 15, of 512 148 / 63; 32 heads of 64 x 128, 64 requests of 8 tokens 99 / 273, one of 449 beside 63
-    of one token 199 / 321). Where it is not known, the tokens in all decide: with 4 requests of 32 tokens, 16 heads of 64 x 64,
-    that is slower (12 / 15), with 125 tokens beside three of one faster (34 / 27)."""
+    request of 48 tokens 18 / 15, of 512 147 / 52; 32 heads of 64 x 128, 64 requests of 8 tokens 98 / 230, one of 449 beside 63
+    of one token 160 / 270). Where it is not known, the tokens in all decide: with 4 requests of 32 tokens, 16 heads of 64 x 64,
+    that is slower (11 / 15), with 125 tokens beside three of one faster (33 / 18)."""
     if dim > 128:
         return False
     if not longest:
@@ -659,11 +666,15 @@ def _chunked_recurrence(n: int, n_seqs: int, dim: int, rule: str = "delta", head
     if n < 48:                                          # (the least that was measured; 24 tokens are slower by chunks)
         return False
     of = lambda table: table[min(size for size in table if dim <= size)]
-    fixed, chain, work = of(_BY_TOKEN[rule])
-    by_token = fixed + chain * longest + work * n * heads * cols / 1e4
-    fixed, chain, work = of(_BY_CHUNK[rule])
-    chunks = (n - n_seqs) // 16 + n_seqs
-    return fixed + chain * longest / 16 + work * chunks * heads * -(-cols // 32) / 100 < by_token
+    columns, chunks = -(-cols // 16) * 16 * heads / 1e4, (n - n_seqs) // 16 + n_seqs
+    fixed, chain, work, states = of(_BY_TOKEN[rule])
+    by_token = fixed + chain * longest + (work * n + states * n_seqs) * columns
+    fixed, chain, prepare, work, states = of(_BY_CHUNK[rule])
+    by_chunk = fixed + chain * longest / 16 + (prepare + work * -(-cols // 32)) * chunks * heads / 100
+    by_chunk += states * n_seqs * heads * cols / 1e4
+    # where most requests bring a token or a few and their states are more than L2 keeps beside the rest, the sums favour chunks
+    large = chunks < 2 * n_seqs and 4 * n_seqs * heads * dim * cols >= 32 << 20
+    return by_chunk < (0.84 if large else 1.0) * by_token
 
 
 CHUNKED_SCRATCH_BYTES = 256 << 20        # prepared chunks that a launch of a recurrence may hold (longer steps are several launches)

@@ -40,7 +40,10 @@ def test_key_shares_of_any_mix_of_portions():
     (16, 128, 128, [48], "delta", True), (16, 128, 128, [24], "delta", False), (16, 128, 128, [512], "mlstm", True),
     (32, 64, 128, [8] * 64, "delta", False), (32, 64, 128, [449] + [1] * 63, "plain", False), (16, 16, 16, [512], "mlstm", True),
     (64, 64, 64, [128] * 8, "delta", False), (16, 128, 128, [16] * 64, "plain", True), (4, 64, 64, [24] * 32, "mlstm", False),
-    (16, 129, 128, [2048], "delta", False), (16, 128, 128, [1] * 256, "mlstm", False), (16, 64, 64, [2048], "delta", True)])
+    (16, 129, 128, [2048], "delta", False), (16, 128, 128, [1] * 256, "mlstm", False), (16, 64, 64, [2048], "delta", True),
+    # where chunks are prepared once a head, whatever its columns (us one by one / by chunks: 44 / 70, 175 / 208, 33 / 20, 397 / 289, 125 / 94)
+    (32, 128, 16, [108] * 9, "delta", False), (20, 96, 32, [100] * 40, "delta", False), (10, 64, 80, [40] * 13, "mlstm", True),
+    (40, 64, 80, [351] * 14, "plain", True), (16, 64, 128, [46] * 48, "plain", True)])
 def test_recurrences_by_chunks_where_that_was_faster(heads, dim, vdim, lens, rule, faster):
     """Measured both ways (the rule before counted tokens and requests only and was up to 3.2 times slower)."""
     cols = vdim + (rule == "mlstm")
