@@ -225,8 +225,8 @@ int hb_head_gate(const void* in, const void* gate, long long gate_stride, void* 
 int hb_delta_prep(const void* proj, int proj_dtype, long long ld, int chan_off, int beta_off, const float* taps,
                   float* state, long long state_stride, long long conv_off, const void* a_pre, int a_dtype,
                   const float* dt_bias, const float* a_log, const int* cu_seqlens, const int* seq_of_token,
-                  const int* slots, float* q, float* k, float* v, float* beta, float* decay, int n_tokens, int heads,
-                  int kvh, int dim, int vdim, int taps_n, int head_decay, cudaStream_t stream);
+                  const int* slots, float* q, float* k, float* v, float* beta, float* decay, int n_tokens, int n_seqs,
+                  int heads, int kvh, int dim, int vdim, int taps_n, int head_decay, cudaStream_t stream);
 int hb_gla_prep(const void* proj, int proj_dtype, long long ld, int q_off, int k_off, int v_off, const float* z,
                 const float* bias, float tau, float q_scale, float* q, float* k, float* v, float* decay, int n_tokens,
                 int qk_cols, int v_cols, cudaStream_t stream);

@@ -124,8 +124,8 @@ __global__ void delta_prep_kernel(const PrepArgs a, int longest) {
 // tokens a warp, whose rows are all asked for before the first product; the taps and the rows of the tokens before stay in
 // registers from token to token. What bounds it: the trips to memory of a few tokens (TT = 1); of a prompt's the exponentials,
 // logarithms and divisions (about 20 million warp instructions, 20 us if nothing waited) beside rows of 32 KB a token. 48 units
-// of 128 channels (16 heads), bfloat16: 5 tokens 10.6 -> 5.2 us; 1,966 tokens 112 -> 77 us with one token a warp (the taps, 2 KB a
-// unit, came again for every token), 71 with eight.
+// of 128 channels (16 heads), bfloat16: 5 tokens 10.6 -> 5.2 us; 2,000 tokens 119 -> 80 us with one token a warp (the taps, 2 KB a
+// unit, came again for every token), 71 with two or eight.
 template <int NG, int TT>
 __global__ void __launch_bounds__(128) delta_prep_vec_kernel(const PrepArgs a, int n_tokens) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -674,12 +674,12 @@ extern "C" int hb_delta_prep(const void* proj, int proj_dtype, long long ld, int
                              const float* taps, float* state, long long state_stride, long long conv_off,
                              const void* a_pre, int a_dtype, const float* dt_bias, const float* a_log,
                              const int* cu_seqlens, const int* seq_of_token, const int* slots, float* q, float* k,
-                             float* v, float* beta, float* decay, int n_tokens, int heads, int kvh, int dim, int vdim,
-                             int taps_n, int head_decay, cudaStream_t stream) {
+                             float* v, float* beta, float* decay, int n_tokens, int n_seqs, int heads, int kvh, int dim,
+                             int vdim, int taps_n, int head_decay, cudaStream_t stream) {
   if (!proj || !taps || !state || !a_pre || !dt_bias || !a_log || !cu_seqlens || !seq_of_token || !slots || !q || !k ||
       !v || !beta || !decay)
     return HB_ERR_BAD_ARG;
-  if (heads <= 0 || kvh <= 0 || heads % kvh || dim <= 0 || vdim <= 0 || taps_n < 1 || n_tokens < 0) return HB_ERR_BAD_ARG;
+  if (heads <= 0 || kvh <= 0 || heads % kvh || dim <= 0 || vdim <= 0 || taps_n < 1 || n_tokens < 0 || n_seqs < 0) return HB_ERR_BAD_ARG;
   if (n_tokens == 0) return HB_OK;
   const int longest = dim > vdim ? dim : vdim;
   const int warps = 4;
@@ -695,20 +695,30 @@ extern "C" int hb_delta_prep(const void* proj, int proj_dtype, long long ld, int
   const int units = 2 * kvh + heads;
   int per_token = (units + warps - 1) / warps;
   if (per_token > 64) per_token = 64;
-  // four channels a lane where every row of four starts on its bytes
+  // Four channels a lane where every row of four starts on its bytes and keeps more than a quarter of a warp busy, one, two or eight
+  // tokens a warp: where most of them start a request, the three rows before each are loaded in turn, and few tokens leave the SMs
+  // idle. us of 256 / 1,024 single tokens: the general kernel 16.4 / 63.1, one a warp 11.2 / 43.8, eight 16.9 / 51.9 (16 heads of
+  // 128); 17.7 / 69.8, 16.9 / 75.6, 26.1 / 95.0 (32 of 64). Prompts of 400 / 1,000 / 4,000 tokens by one, two, eight a warp: 17.4,
+  // 16.0, 23.5 / 37.9, 31.9, 32.8 / 156.8, 136.7, 134.5 (16 of 128); 62.2, 52.8, 55.7 / 155, 136, 133 / 607, 527, 496 (64 of 128).
+  // Rows of more than 128: 34, 32, 46 / 90, 89, 104 / 352, 342, 397. Rows of 32, the general kernel and two a warp: 14.9, 19.5 /
+  // 31.8, 43.5 / 122, 173.
   auto on = [](const void* p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
   const int pb = proj_dtype == HB_DTYPE_F32 ? 16 : 8, ab = a_dtype == HB_DTYPE_F32 ? 16 : 8;
-  if (taps_n == 4 && longest <= 256 && !((dim | vdim | ld | chan_off | state_stride | conv_off) & 3) && on(proj, pb) && on(taps, 16) &&
+  const long long load = (long long)n_tokens * units;
+  const bool few = load < 12000 || 2LL * n_tokens < 5LL * n_seqs;
+  const bool wide = longest > 64 || (longest > 32 && !(few && load > 64000));
+  if (wide && taps_n == 4 && longest <= 256 && !((dim | vdim | ld | chan_off | state_stride | conv_off) & 3) && on(proj, pb) && on(taps, 16) &&
       on(state, 16) && (head_decay || (on(a_pre, ab) && on(dt_bias, 16))) && on(q, 16) && on(k, 16) && on(v, 16) && on(decay, 16)) {
-    constexpr int MANY = 8;
-    const bool many = n_tokens >= 256;               // enough warps for the SMs with eight tokens each
-    const dim3 grid(many ? (n_tokens + MANY - 1) / MANY : n_tokens, per_token);
-    if (longest <= 128) {
-      if (many) delta_prep_vec_kernel<1, MANY><<<grid, warps * 32, 0, stream>>>(a, n_tokens);
-      else delta_prep_vec_kernel<1, 1><<<grid, warps * 32, 0, stream>>>(a, n_tokens);
+    const dim3 one(n_tokens, per_token), two((n_tokens + 1) / 2, per_token), eight((n_tokens + 7) / 8, per_token);
+    if (longest > 128) {
+      if (few) delta_prep_vec_kernel<2, 1><<<one, warps * 32, 0, stream>>>(a, n_tokens);
+      else delta_prep_vec_kernel<2, 2><<<two, warps * 32, 0, stream>>>(a, n_tokens);
+    } else if (few) {
+      delta_prep_vec_kernel<1, 1><<<one, warps * 32, 0, stream>>>(a, n_tokens);
+    } else if (load < 128000 || n_tokens < 16LL * n_seqs) {
+      delta_prep_vec_kernel<1, 2><<<two, warps * 32, 0, stream>>>(a, n_tokens);
     } else {
-      if (many) delta_prep_vec_kernel<2, MANY><<<grid, warps * 32, 0, stream>>>(a, n_tokens);
-      else delta_prep_vec_kernel<2, 1><<<grid, warps * 32, 0, stream>>>(a, n_tokens);
+      delta_prep_vec_kernel<1, 8><<<eight, warps * 32, 0, stream>>>(a, n_tokens);
     }
     HB_LAUNCH_CHECK();
     return HB_OK;

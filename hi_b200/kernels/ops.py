@@ -77,7 +77,7 @@ _SIGNATURES = {
     "hb_sigmoid_attention": [P, I, P, P, P, I, P, P, P, P, I, I, P, I, I, I, I, I, I, I, F, I, I, P, P],
     "hb_gla_prep": [P, I, c_longlong, I, I, I, P, P, F, F, P, P, P, P, I, I, I, P],
     "hb_head_gate": [P, P, c_longlong, P, I, I, I, I, P],
-    "hb_delta_prep": [P, I, c_longlong, I, I, P, P, c_longlong, c_longlong, P, I, P, P, P, P, P, P, P, P, P, P, I, I, I,
+    "hb_delta_prep": [P, I, c_longlong, I, I, P, P, c_longlong, c_longlong, P, I, P, P, P, P, P, P, P, P, P, P, I, I, I, I,
                       I, I, I, I, P],
     "hb_delta_conv_update": [P, I, c_longlong, I, P, c_longlong, c_longlong, P, P, I, I, I, P],
     "hb_delta_recurrence": [P, P, P, P, P, P, c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
@@ -611,7 +611,7 @@ def delta_prep(proj: torch.Tensor, chan_off: int, beta_off: int, taps: torch.Ten
     _check(lib().hb_delta_prep(_ptr(proj), _dt(proj), ld, int(chan_off), int(beta_off), _ptr(taps), _ptr(state),
                                state.shape[1], int(conv_off), _ptr(a_pre), _dt(a_pre), _ptr(dt_bias), _ptr(a_log),
                                _ptr(cu_seqlens), _ptr(seq_of_token), _ptr(slots), _ptr(q), _ptr(k), _ptr(v), _ptr(beta),
-                               _ptr(decay), n, heads, kvh, dim, vdim, k_taps, int(head_decay), _stream()), "delta_prep")
+                               _ptr(decay), n, slots.numel(), heads, kvh, dim, vdim, k_taps, int(head_decay), _stream()), "delta_prep")
     return q, k, v, beta, decay
 
 

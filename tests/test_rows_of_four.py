@@ -16,12 +16,12 @@ def test_delta_prep(heads, kvh, dim, vdim, taps, shift, head_decay, dt, lens):
     from hi_b200.kernels import ops
 
     g = torch.Generator().manual_seed(dim + vdim + taps)
-    slots = [2, 0, 3, 1][: len(lens)]
+    slots = ([2, 0, 3, 1] if len(lens) <= 4 else list(range(len(lens)))[::-1])[: len(lens)]
     n, c = sum(lens), 2 * kvh * dim + heads * vdim
     rnd = lambda *s: torch.randn(*s, generator=g)
     off = taps + (4 if taps == 4 else 1)                             # where the convolution's rows start in the state
     proj = rnd(n, shift + c + heads + (-(shift + c + heads)) % 4).to(dt)
-    w, state, per = rnd(c, taps), rnd(4, off + (taps - 1) * c + (-(off + (taps - 1) * c)) % 4), heads if head_decay else heads * dim
+    w, state, per = rnd(c, taps), rnd(max(4, len(lens)), off + (taps - 1) * c + (-(off + (taps - 1) * c)) % 4), heads if head_decay else heads * dim
     pre, bias, a_log = rnd(n, per).to(dt), rnd(per), 0.3 * rnd(heads)
     cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32)
     seq = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).to(torch.int32)
@@ -43,6 +43,13 @@ def test_delta_prep(heads, kvh, dim, vdim, taps, shift, head_decay, dt, lens):
     for a, b, name in zip(got, want, ("q", "k", "v", "beta", "decay")):
         # a few float32 roundings of 6e-8 in sums of four products, and of the length's sum over at most 260 squares
         assert float((a.cpu().double() - b).abs().max() / b.abs().max()) < 2e-6, name
+
+
+# two tokens a warp (rows of up to 128 and of more, borders of requests inside a warp's), eight, and one where the step is of single tokens
+@pytest.mark.parametrize("heads,kvh,dim,vdim,lens", [(16, 16, 128, 128, [3, 250, 13, 1]), (8, 8, 132, 40, [1, 700, 3]), (16, 4, 40, 36, [300, 215]),
+                                                     (16, 16, 64, 96, [5, 2000, 703]), (32, 16, 128, 100, [2001]), (16, 16, 128, 128, [1] * 260)])
+def test_delta_prep_of_many_tokens(heads, kvh, dim, vdim, lens):
+    test_delta_prep(heads, kvh, dim, vdim, 4, 0, False, torch.bfloat16, lens)
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
