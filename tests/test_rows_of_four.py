@@ -54,13 +54,15 @@ def test_delta_prep_of_many_tokens(heads, kvh, dim, vdim, lens):
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("silu", [False, True])
-@pytest.mark.parametrize("n,heads,vdim,shift", [(5, 4, 128, 0), (3, 2, 4, 4), (2, 3, 200, 0), (2, 1, 256, 8), (3, 2, 130, 0), (2, 2, 64, 1), (1, 2, 260, 0)])
-def test_delta_out_norm(n, heads, vdim, shift, silu, dt):
+@pytest.mark.parametrize("n,heads,vdim,shift,pad", [(5, 4, 128, 0, 0), (3, 2, 36, 4, 4), (2, 3, 200, 0, 8), (2, 1, 256, 8, 0), (3, 2, 132, 4, 0), (9, 3, 64, 0, 4),
+                                                    # the general kernel: an odd stride, rows not of whole fours, off their bytes, too long, too short
+                                                    (5, 4, 128, 0, 3), (3, 2, 130, 0, 0), (2, 2, 64, 1, 3), (1, 2, 260, 0, 0), (3, 2, 4, 4, 0), (3, 5, 32, 0, 0)])
+def test_delta_out_norm(n, heads, vdim, shift, pad, silu, dt):
     from hi_b200.kernels import ops
 
     g = torch.Generator().manual_seed(vdim + n)
     rnd = lambda *s: torch.randn(*s, generator=g)
-    o, wide, w = rnd(n, heads * vdim), rnd(n, shift + heads * vdim + 3).to(dt), rnd(vdim).to(dt)
+    o, wide, w = rnd(n, heads * vdim), rnd(n, shift + heads * vdim + pad).to(dt), rnd(vdim).to(dt)
     gate = wide[:, shift: shift + heads * vdim]
     got = ops.delta_out_norm(o.to(DEV), wide.to(DEV)[:, shift: shift + heads * vdim], w.to(DEV), 1e-5, vdim, dt, gate_silu=silu)
     x, z = o.double().view(n, heads, vdim), gate.double().reshape(n, heads, vdim)
