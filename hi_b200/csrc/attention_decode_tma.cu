@@ -14,11 +14,11 @@
 // memory, so whatever the pool holds there cannot reach the sum. Every mbarrier wait is bounded;
 // on a time-out the kernel records it in `status` and stops.
 //
-// Where a token has 2 to 8 splits and all blocks run at once, its splits are a cluster: every block keeps its rows in shared
+// Where a token has 2 to 8 splits and all clusters run at once, its splits are a cluster: every block keeps its rows in shared
 // memory and the blocks of the cluster share out the merge among themselves, reading one another's (the caller gives no
 // part_acc / part_ml then). What that saves is a launch, its gap and the partial rows' way through memory: one token of 1,000
-// keys, 40 heads of 128: 12.7 -> 11.5 us, of 300 keys 12.1 -> 9.6 us; with several rounds of blocks it loses (clusters wait for
-// their slowest block and for slots that lie together; ops.decode_attention has the rule and both sides).
+// keys, 40 heads of 128: 12.7 -> 11.5 us, of 300 keys 12.1 -> 9.6 us; with one cluster more than run at once it takes 1.2 to 1.5
+// times as long as with the merge (ops.decode_attention has the rule and both sides).
 //
 // The fused form (hb_attention_decode_fused) takes the q/k/v projection's output as it is and
 // does in the same launch what hb_qkv_post and hb_attention_merge do around the plain form: every
@@ -626,6 +626,36 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if (tid == 0) f.counters[t * a.nkv + kvh] = 0;     // zero again for the next launch
 }
 
+template <int HD>
+constexpr size_t smem_bytes() {
+  return 1024 + 2 * (size_t)STAGES * (HD / 64) * HALF_BYTES + (size_t)ROWS * (HD + 8) * 2 + (size_t)NWARPS * ROWS * 2 * sizeof(float) +
+         STAGES * sizeof(uint64_t) + HD * sizeof(float);
+}
+
+// A launch whose token's splits are a cluster.
+inline void cluster_of(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, dim3 grid, size_t smem, cudaStream_t stream) {
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = grid.x;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.gridDim = grid; cfg.blockDim = dim3(NWARPS * 32); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+}
+
+template <int HD>
+int clusters_at_once(int splits) {
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = {};
+  cluster_of(cfg, attr, dim3(splits, 1, 1), smem_bytes<HD>(), nullptr);
+  int n = 0;
+  if (cudaFuncSetAttribute(attn_decode_tma_kernel<HD, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<HD>()) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<HD, CLUSTER>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 template <int HD, Merge MERGE>
 int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, const Args& a, const Fuse& f,
            cudaStream_t stream) {
@@ -634,10 +664,8 @@ int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, 
   if (!tc::make_map_bf16(&mk, k_pages, pool_rows, HD, a.box_rows) || !tc::make_map_bf16(&mv, v_pages, pool_rows, HD, a.box_rows))
     return HB_ERR_UNSUPPORTED;
   constexpr bool FUSED = MERGE == FUSED_FORM;
-  constexpr int STRIDE = HD + 8;
   constexpr int KV_BYTES = (HD / 64) * HALF_BYTES;
-  const size_t smem = 1024 + 2 * (size_t)STAGES * KV_BYTES + (size_t)ROWS * STRIDE * 2 +
-                      (size_t)NWARPS * ROWS * 2 * sizeof(float) + STAGES * sizeof(uint64_t) + HD * sizeof(float);
+  constexpr size_t smem = smem_bytes<HD>();
   static_assert((size_t)STAGES * KV_BYTES >= (size_t)ROWS * HD * sizeof(float), "o_s aliases the K tiles");
   // the fused merge keeps [G][splits] weights and [G] sums where the V tiles were
   if (FUSED && (size_t)(a.nh / a.nkv) * (2 * a.max_splits + 1) * sizeof(float) > (size_t)STAGES * KV_BYTES) return HB_ERR_UNSUPPORTED;
@@ -645,15 +673,12 @@ int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, 
   if (e != cudaSuccess) return (int)e;
   dim3 grid(a.max_splits, a.nkv, n_tokens);
   if (MERGE == CLUSTER) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.max_splits;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = dim3(NWARPS * 32); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, attn_decode_tma_kernel<HD, MERGE>, mk, mv, a, f);
-    return e == cudaSuccess ? HB_OK : (int)e;
+    cluster_of(cfg, attr, grid, smem, stream);
+    cudaLaunchKernelEx(&cfg, attn_decode_tma_kernel<HD, MERGE>, mk, mv, a, f);
+    HB_LAUNCH_CHECK();
+    return HB_OK;
   }
   attn_decode_tma_kernel<HD, MERGE><<<grid, NWARPS * 32, smem, stream>>>(mk, mv, a, f);
   HB_LAUNCH_CHECK();
@@ -661,6 +686,13 @@ int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, 
 }
 
 }  // namespace
+
+// How many (token, kv head) pairs of `splits` splits run at a time as clusters on the current device: a cluster's blocks lie in one
+// GPC, so that is less than the blocks that fit alone (0: none, or no such form).
+extern "C" int hb_attention_decode_clusters(int hd, int splits) {
+  if (splits < 2 || splits > MAX_CLUSTER) return 0;
+  return hd == 128 ? clusters_at_once<128>(splits) : hd == 64 ? clusters_at_once<64>(splits) : 0;
+}
 
 // As hb_attention_decode (bfloat16; head_dim 64 or 128; at most 16 query heads per kv head; every
 // token one decode row; partials merged by hb_attention_merge), with TMA tile loads. Returns

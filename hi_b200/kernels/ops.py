@@ -41,6 +41,7 @@ _SIGNATURES = {
     "hb_attention_merge": [P, P, P, I, I, I, I, I, I, P, P],
     "hb_attention_merge_rows": [P, P, P, I, I, I, I, I, I, P, P, P],
     "hb_attention_decode_rows": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P, P],
+    "hb_attention_decode_clusters": [I, I],
     "hb_attention_decode_tma_rows": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P, P],
     "hb_attention_decode": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P],
     "hb_attention_decode_tma": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P],
@@ -1405,10 +1406,19 @@ def _decode_splits(longest: int, groups: int) -> Tuple[int, int]:
 TC_ROW_LENGTHS = (64, 128, 192)
 
 
-# Splits of a token that one cluster of blocks can be. In one round of blocks a launch and its gap are saved: 167 batches of 1
-# to 64 tokens take 0.88 of the time with the merge kernel (one token of 300 keys 12.1 -> 9.6 us), none longer; in several
-# rounds 1.10 of it (32 tokens of up to 4,000 keys of 24 heads 167 -> 205).
+# Splits of a token that one cluster of blocks can be. Where all clusters run at once a launch and its gap are saved: 0.80 to 0.97 of
+# the time with the merge kernel (2 to 8 splits of 128 and 768 keys, 8 pairs to as many as fit, heads of 64 and 128; one token of
+# 300 keys, 40 heads of 128, 12.1 -> 9.6 us); with one cluster more than that 1.2 to 1.5 of it (6 splits of 768 keys, heads of
+# 128: 71 pairs 33.4 / 35.8, 72 pairs 50.6 / 36.5), also where their blocks would fit alone.
 DECODE_CLUSTER = 8
+
+
+@functools.lru_cache(maxsize=None)
+def _decode_clusters(device: int, hd: int, splits: int) -> int:
+    """How many clusters of ``splits`` blocks of the decode kernel run at a time on the device. A cluster's blocks lie in one group
+    of SMs: 444 blocks of heads of 128 fit, but 71 clusters of 6 and not 74."""
+    with torch.cuda.device(device):
+        return int(lib().hb_attention_decode_clusters(hd, splits))
 
 
 def decode_attention_supported(q_dtype: torch.dtype, nh: int, nkv: int, hd: int) -> bool:
@@ -1461,9 +1471,8 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         return (torch.empty((n, nh, splits, hd), dtype=torch.float32, device=q.device),
                 torch.empty((n, nh, splits, 2), dtype=torch.float32, device=q.device))
 
-    # the splits meet in a cluster's shared memory; where the blocks come in several rounds, clusters that wait for their
-    # slowest block and for slots that lie together cost more than the merge
-    in_cluster = not reshaped and 1 < splits <= DECODE_CLUSTER and n * nkv * splits <= DECODE_RESIDENT_BLOCKS
+    # the splits meet in a cluster's shared memory where all clusters run at once
+    in_cluster = not reshaped and 1 < splits <= DECODE_CLUSTER and n * nkv <= _decode_clusters(q.device.index, hd, splits)
     if (splits > 1 or parts) and not in_cluster:
         part_acc, part_ml = scratch()
     for t, nm in ((slopes, "slopes"), (sink_values, "sink_values")):

@@ -49,6 +49,28 @@ def test_splits_meet_in_a_cluster(nh, nkv, hd, lens, page, chunk, sink, monkeypa
     assert float((got.float() - apart.float()).abs().max()) <= 2 ** -8 * float(apart.float().abs().max())
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("splits", [2, 5, 6, 8, 9])
+def test_clusters_only_where_all_run_at_once(splits, hd, monkeypatch):
+    from hi_b200.kernels import ops
+
+    fit = ops._decode_clusters(0, hd, splits)
+    assert (fit == 0) == (splits > 8) and fit * splits <= 148 * 8
+    monkeypatch.setattr(ops, "_decode_splits", lambda *a: (64, splits))
+    g = torch.Generator(device=DEV).manual_seed(splits)
+    for n in (max(1, fit), fit + 1):
+        q, kp, vp = (torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16) for s in ((n, 4, hd), (n * splits, 1, 64, hd), (n * splits, 1, 64, hd)))
+        table = torch.arange(n * splits, dtype=torch.int32, device=DEV).view(n, splits)
+        pos = torch.randint(0, 64 * splits, (n,), device=DEV, generator=g).to(torch.int32)
+        call = lambda: ops.decode_attention(q, kp, vp, table, torch.arange(n, dtype=torch.int32, device=DEV), pos, 0, 0, hd ** -0.5, 64 * splits)
+        before = ops.CALLS.get("attention_merge", 0)
+        got = call()
+        assert ops.CALLS.get("attention_merge", 0) - before == (n > fit)
+        with monkeypatch.context() as m:
+            m.setattr(ops, "DECODE_CLUSTER", 1)
+            assert float((got.float() - call().float()).abs().max()) <= 2 ** -8 * float(got.float().abs().max())      # one bfloat16 place
+
+
 # by a cluster, by the merge of several rounds' splits, of more than eight splits, by the cp.async kernel (rows of 192, a window)
 @pytest.mark.parametrize("nh,nkv,hd,lens,window", [(8, 2, 128, [900, 1, 300], 0), (24, 24, 128, [700] * 30, 0), (4, 1, 64, [9000, 64], 0),
                                                    (8, 4, 192, [300, 77, 1000], 0), (8, 2, 64, [1500, 3], 1024)])
