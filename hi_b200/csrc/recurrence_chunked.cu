@@ -109,11 +109,17 @@ struct Span {
 // Share i of a request of c chunks is the i-th run of ceil(c / shares) of them. A unit is a chunk of the share; those of request s
 // start at cu[s] / (C shares) + s, which leaves every request room for ceil(its tokens / (C shares)).
 __host__ __device__ inline Span span_of(const int* cu, int s, int share, int shares, int unit0, int units) {
-  const int chunks = (cu[s + 1] - cu[s] + C - 1) / C, run = shares == 1 ? chunks : (chunks + shares - 1) / shares;
-  const int at = (shares == 1 ? cu[s] / C : cu[s] / (C * shares)) + s - unit0, from = at < 0 ? -at : 0;
-  int to = run < chunks - share * run ? run : chunks - share * run;
+  const int begin = cu[s], chunks = (cu[s + 1] - begin + C - 1) / C;
+  int at = begin / C + s - unit0, chunk = 0, to = chunks;
+  if (shares > 1) {                  // (the divisions and what hangs on them are 0.2 us of a short step)
+    const int run = (chunks + shares - 1) / shares;
+    at = begin / (C * shares) + s - unit0;
+    chunk = share * run;
+    to = run < chunks - chunk ? run : chunks - chunk;
+  }
+  const int from = at < 0 ? -at : 0;
   if (to > units - at) to = units - at;
-  return {share * run + from, to - from, at + from};
+  return {chunk + from, to - from, at + from};
 }
 
 // hb::split3 with the rests of the two floats in the last pieces
@@ -463,6 +469,15 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
     }
   };
 
+  // A thread that gave up waits for the last copies into each place before it leaves, again with the limit, so that none is under
+  // way when the block ends.
+  auto see_copies_land = [&]() {
+    for (int i = max(0, chunks - RING); i < chunks; ++i) {
+      if (i >= chunks - STAGES) tc::mbar_wait(&sm.full[i % STAGES], (i / STAGES) & 1);
+      tc::mbar_wait(&sm.full_m[i % RING], (i / RING) & 1);
+    }
+  };
+
   if (tid < COMP) {
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q4 = lane & 3;
     // S^T as accumulator tiles [16 columns][8 rows]: s[m][n][0, 1] = column 16 m + g, rows 8 n + 2 q4 and the next;
@@ -589,6 +604,7 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
           const size_t i = at(m, n, e, in);
           if (in) S[i] = s[m][n][e];
         }
+    if (!ok) see_copies_land();
     return;
   }
 
@@ -711,13 +727,7 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
     }
     if (i + 2 < chunks) bar_arrive(FREED + b, COMP + HELP);
   }
-  // No copy is under way when the block leaves, also where a wait was given up: the last ones into each place, again with the limit
-  // (the others were waited for before their place was used again; where all went well these return at once).
-  if (h == 0)
-    for (int i = max(0, chunks - RING); i < chunks; ++i) {
-      if (i >= chunks - STAGES) tc::mbar_wait(&sm.full[i % STAGES], (i / STAGES) & 1);
-      tc::mbar_wait(&sm.full_m[i % RING], (i / RING) & 1);
-    }
+  if (!ok) see_copies_land();
 }
 
 template <typename T, int NW, int CT, bool PLAIN>
