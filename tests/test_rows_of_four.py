@@ -55,8 +55,9 @@ def test_delta_prep_of_many_tokens(heads, kvh, dim, vdim, lens):
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("silu", [False, True])
 @pytest.mark.parametrize("n,heads,vdim,shift,pad", [(5, 4, 128, 0, 0), (3, 2, 36, 4, 4), (2, 3, 200, 0, 8), (2, 1, 256, 8, 0), (3, 2, 132, 4, 0), (9, 3, 64, 0, 4),
-                                                    # the general kernel: an odd stride, rows not of whole fours, off their bytes, too long, too short
-                                                    (5, 4, 128, 0, 3), (3, 2, 130, 0, 0), (2, 2, 64, 1, 3), (1, 2, 260, 0, 0), (3, 2, 4, 4, 0), (3, 5, 32, 0, 0)])
+                                                    # the general kernel: an odd stride, rows not of whole fours, off their bytes, too long, many short ones
+                                                    (5, 4, 128, 0, 3), (3, 2, 130, 0, 0), (2, 2, 64, 1, 3), (1, 2, 260, 0, 0), (2501, 4, 32, 0, 0),
+                                                    (3, 2, 4, 4, 0), (3, 5, 32, 0, 0)])
 def test_delta_out_norm(n, heads, vdim, shift, pad, silu, dt):
     from hi_b200.kernels import ops
 
