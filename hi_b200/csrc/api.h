@@ -60,10 +60,10 @@ int hb_paged_attention(const void* q, int dtype, const void* k_pages, const void
 
 int hb_attention_merge(const float* part_acc, const float* part_ml, void* out, int dtype, int n_rows, int hd,
                        int max_splits, int sink, int nh, const float* sink_values, cudaStream_t stream);
-// the same into the tokens `token_rows` of `out` (one a token of nh rows)
+// the same into the tokens `token_rows` of the `step_tokens` of `out` (one a token of nh rows)
 int hb_attention_merge_rows(const float* part_acc, const float* part_ml, void* out, int dtype, int n_rows, int hd,
                             int max_splits, int sink, int nh, const float* sink_values, const long long* token_rows,
-                            cudaStream_t stream);
+                            int step_tokens, cudaStream_t stream);
 int hb_attention_decode(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                         int table_stride, const int* seq_of_token, const int* positions, void* out, int n_tokens,
                         int nh, int nkv, int hd, int page_size, int chunk, int window, int keep, float scale, int sink,
@@ -72,19 +72,19 @@ int hb_attention_decode(const void* q, const void* k_pages, const void* v_pages,
                         cudaStream_t stream);   // sink == 2: sigmoid weights with head_bias; plain sums go to part_acc
                                                 // softcap, slopes, sink_values: as hb_paged_attention
 
-// the same for the tokens `rows` of a larger step: rows of q, out, seq_of_token and positions
+// the same for the tokens `rows` of a step of `step_tokens`: rows of q, out, seq_of_token and positions
 int hb_attention_decode_rows(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                              int table_stride, const int* seq_of_token, const int* positions, void* out, int n_tokens,
                              int nh, int nkv, int hd, int page_size, int chunk, int window, int keep, float scale, int sink,
                              const float* head_bias, float softcap, const float* slopes, const float* sink_values,
                              int split_size, int max_splits, float* part_acc, float* part_ml, const long long* rows,
-                             cudaStream_t stream);
+                             int step_tokens, int* status, cudaStream_t stream);
 
 int hb_attention_decode_tma_rows(const void* q, const void* k_pages, const void* v_pages, int n_pages, const int* block_table,
                                  int table_stride, const int* seq_of_token, const int* positions, void* out, int n_tokens,
                                  int nh, int nkv, int hd, int page_size, int chunk, int window, float scale, int sink,
                                  int split_size, int max_splits, float* part_acc, float* part_ml, int* status,
-                                 const long long* rows, cudaStream_t stream);
+                                 const long long* rows, int step_tokens, cudaStream_t stream);
 int hb_attention_decode_tma(const void* q, const void* k_pages, const void* v_pages, int n_pages, const int* block_table,
                             int table_stride, const int* seq_of_token, const int* positions, void* out, int n_tokens,
                             int nh, int nkv, int hd, int page_size, int chunk, int window, float scale, int sink,

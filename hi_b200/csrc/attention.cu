@@ -150,11 +150,16 @@ __global__ void __launch_bounds__(32 * MERGE_ROWS) attention_merge_kernel(const 
                                                                           const float* __restrict__ part_ml, T* __restrict__ out,
                                                                           long long rows, int hd, int splits, int sink, int nh,
                                                                           const float* __restrict__ sink_values,
-                                                                          const long long* __restrict__ token_rows) {
+                                                                          const long long* __restrict__ token_rows, int step_tokens) {
   const int lane = threadIdx.x & 31;
   const long long th = (long long)blockIdx.x * MERGE_ROWS + (threadIdx.x >> 5);
   if (th >= rows) return;
-  const long long to = PLACED ? token_rows[th / nh] * nh + th % nh : th;
+  long long to = th;
+  if constexpr (PLACED) {
+    const long long token = token_rows[th / nh];
+    if (token < 0 || token >= step_tokens) return;              // (the decode kernel has said so)
+    to = token * nh + th % nh;
+  }
   const float* acc = part_acc + (size_t)th * splits * hd;
   struct alignas(4 * W) Vec { float x[W]; };
   Vec ahead[MERGE_AHEAD];
@@ -213,14 +218,14 @@ __global__ void __launch_bounds__(32 * MERGE_ROWS) attention_merge_kernel(const 
 
 template <typename T>
 int launch_merge(const float* part_acc, const float* part_ml, void* out, long long rows, int hd, int splits, int sink, int nh,
-                 const float* sink_values, const long long* token_rows, cudaStream_t stream) {
+                 const float* sink_values, const long long* token_rows, int step_tokens, cudaStream_t stream) {
   const uintptr_t p = reinterpret_cast<uintptr_t>(part_acc), o = reinterpret_cast<uintptr_t>(out);
   const long long blocks = (rows + MERGE_ROWS - 1) / MERGE_ROWS;
   if (blocks > 0x7fffffffLL) return HB_ERR_UNSUPPORTED;
   auto fits = [&](int w) { return hd % w == 0 && p % (4 * w) == 0 && o % (sizeof(T) * w) == 0; };
 #define HB_MERGE(W)                                                                                                                \
   (token_rows ? attention_merge_kernel<T, W, true> : attention_merge_kernel<T, W, false>)<<<(int)blocks, 32 * MERGE_ROWS, 0, stream>>>( \
-      part_acc, part_ml, (T*)out, rows, hd, splits, sink, nh, sink_values, token_rows)
+      part_acc, part_ml, (T*)out, rows, hd, splits, sink, nh, sink_values, token_rows, step_tokens)
   if (fits(4) && (hd % 128 == 0 || hd % 64 != 0)) HB_MERGE(4);
   else if (fits(2)) HB_MERGE(2);
   else HB_MERGE(1);
@@ -270,28 +275,28 @@ extern "C" int hb_paged_attention(const void* q, int dtype, const void* k_pages,
   HB_LAUNCH_CHECK();
   if (part_acc && out)
     return dtype == HB_DTYPE_F32
-               ? launch_merge<float>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, nullptr, stream)
-               : launch_merge<__nv_bfloat16>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, nullptr, stream);
+               ? launch_merge<float>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, nullptr, 0, stream)
+               : launch_merge<__nv_bfloat16>(part_acc, part_ml, out, (long long)n_tokens * nh, hd, max_splits, sink, nh, sink_values, nullptr, 0, stream);
   return HB_OK;
 }
 
 // Merge of split partials alone (the decode kernel writes the same partial layout).
-// With `token_rows` (one a token of nh rows) the merged rows go to those tokens of `out`.
+// With `token_rows` (one a token of nh rows) the merged rows go to those of the `step_tokens` tokens of `out`; one outside is left out.
 extern "C" int hb_attention_merge_rows(const float* part_acc, const float* part_ml, void* out, int dtype, int n_rows,
                                   int hd, int max_splits, int sink, int nh, const float* sink_values,
-                                  const long long* token_rows, cudaStream_t stream) {
+                                  const long long* token_rows, int step_tokens, cudaStream_t stream) {
   if (!part_acc || !part_ml || !out || n_rows < 0 || hd <= 0 || max_splits < 1 || ((sink_values || token_rows) && nh <= 0))
     return HB_ERR_BAD_ARG;
   if (nh <= 0) nh = 1;
   if (n_rows == 0) return HB_OK;
-  if (dtype == HB_DTYPE_F32) return launch_merge<float>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, token_rows, stream);
+  if (dtype == HB_DTYPE_F32) return launch_merge<float>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, token_rows, step_tokens, stream);
   if (dtype == HB_DTYPE_BF16)
-    return launch_merge<__nv_bfloat16>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, token_rows, stream);
+    return launch_merge<__nv_bfloat16>(part_acc, part_ml, out, n_rows, hd, max_splits, sink, nh, sink_values, token_rows, step_tokens, stream);
   return HB_ERR_BAD_ARG;
 }
 
 extern "C" int hb_attention_merge(const float* part_acc, const float* part_ml, void* out, int dtype, int n_rows,
                                   int hd, int max_splits, int sink, int nh, const float* sink_values,
                                   cudaStream_t stream) {
-  return hb_attention_merge_rows(part_acc, part_ml, out, dtype, n_rows, hd, max_splits, sink, nh, sink_values, nullptr, stream);
+  return hb_attention_merge_rows(part_acc, part_ml, out, dtype, n_rows, hd, max_splits, sink, nh, sink_values, nullptr, 0, stream);
 }

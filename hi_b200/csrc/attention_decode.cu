@@ -61,8 +61,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
                    float scale, int sink, const float* __restrict__ head_bias, float softcap,
                    const float* __restrict__ slopes, const float* __restrict__ sink_values, int split_size,
                    int max_splits, float* __restrict__ part_acc, float* __restrict__ part_ml,
-                   const long long* __restrict__ rows) {
-  // rows: the tokens this launch takes are those rows of q, out, seq_of_token and positions (null: all, in order)
+                   const long long* __restrict__ rows, int step_tokens, int* __restrict__ status) {
+  // rows: the tokens this launch takes are those rows of q, out, seq_of_token and positions, of step_tokens each (null: all, in order)
   // softcap > 0: a scaled score s becomes softcap * tanh(s / softcap); slopes [nh]: slopes[head] * (distance to the
   // key) is taken off after the cap; sink_values [nh]: the sink's score is the head's own number instead of 0.
   // sink == 2: sigmoid weights. The weight of a key is sigmoid(score + head_bias[head]), nothing is normalised,
@@ -84,7 +84,12 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   const int G = min(ROWS, nh / nkv - row0);                   // heads of the row tile
   const int h0 = kvh * (nh / nkv) + row0;
   const bool parts = part_acc != nullptr;
-  const int token = rows ? (int)rows[t] : t;
+  const long long row = rows ? rows[t] : t;
+  if (rows && (row < 0 || row >= step_tokens)) {
+    if (tid == 0) atomicExch(status, 32);
+    return;
+  }
+  const int token = (int)row;
   const int pos = positions[token];
   const int* table = block_table + (size_t)seq_of_token[token] * table_stride;
   int lo = 0;
@@ -357,7 +362,7 @@ int launch_decode(const void* q, const void* k_pages, const void* v_pages, const
                   const int* seq_of_token, const int* positions, void* out, int n_tokens, int nh, int nkv,
                   int page_size, int chunk, int window, int keep, float scale, int sink, const float* head_bias, float softcap,
                   const float* slopes, const float* sink_values, int split_size,
-                  int max_splits, float* part_acc, float* part_ml, const long long* rows, cudaStream_t stream) {
+                  int max_splits, float* part_acc, float* part_ml, const long long* rows, int step_tokens, int* status, cudaStream_t stream) {
   constexpr int STRIDE = HD + 8;
   const size_t smem = (size_t)(ROWS * STRIDE + 4 * TILE * STRIDE) * sizeof(__nv_bfloat16) +
                       (size_t)(NWARPS * ROWS * 2) * sizeof(float);
@@ -368,7 +373,7 @@ int launch_decode(const void* q, const void* k_pages, const void* v_pages, const
   attn_decode_kernel<HD><<<grid, NWARPS * 32, smem, stream>>>(
       (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, table_stride,
       seq_of_token, positions, (__nv_bfloat16*)out, nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap,
-      slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows);
+      slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, step_tokens, status);
   HB_LAUNCH_CHECK();
   return HB_OK;
 }
@@ -379,15 +384,18 @@ int launch_decode(const void* q, const void* k_pages, const void* v_pages, const
 // go to `out`; otherwise (max, sum, unnormalised row) of every split go to part_ml / part_acc and `out` is not used.
 // With `keep` > 0 (a sliding window only) `split_size * max_splits` has to cover the walk: at most
 // ceil((window + 63) / 64) + ceil(keep / 64) tiles of 64. Returns HB_ERR_UNSUPPORTED for other shapes (the caller then uses the
-// general kernel). The merge over splits is hb_attention_merge. With `rows` (n_tokens of them, each within q, out, seq_of_token
-// and positions) the launch takes those tokens of a larger step, where they are; their partial rows lie in the order of `rows`.
+// general kernel). The merge over splits is hb_attention_merge. With `rows` (n_tokens of them) the launch takes those tokens of a
+// larger step of `step_tokens`, where they lie in q, out, seq_of_token and positions; their partial rows lie in the order of `rows`.
+// A row outside the step is left out and 32 goes to `status` (one int on the device, not null with `rows`).
 // (Four single tokens beside three portions, 40 heads of 128: three gathers and a scatter around the kernel were 20 of 223 us.)
 extern "C" int hb_attention_decode_rows(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                    int table_stride, const int* seq_of_token, const int* positions, void* out,
                                    int n_tokens, int nh, int nkv, int hd, int page_size, int chunk, int window, int keep,
                                    float scale, int sink, const float* head_bias, float softcap, const float* slopes,
                                    const float* sink_values, int split_size, int max_splits,
-                                   float* part_acc, float* part_ml, const long long* rows, cudaStream_t stream) {
+                                   float* part_acc, float* part_ml, const long long* rows, int step_tokens, int* status,
+                                   cudaStream_t stream) {
+  if (rows && (!status || step_tokens < 0)) return HB_ERR_BAD_ARG;
   if (sink == 2 && (softcap > 0.f || slopes || sink_values)) return HB_ERR_UNSUPPORTED;
   if (!q || !k_pages || !v_pages || !block_table || !seq_of_token || !positions || (!out && !part_acc)) return HB_ERR_BAD_ARG;
   if (n_tokens < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || table_stride <= 0 || chunk < 0 ||
@@ -398,13 +406,13 @@ extern "C" int hb_attention_decode_rows(const void* q, const void* k_pages, cons
   if (n_tokens == 0) return HB_OK;
   if (hd == 192)
     return launch_decode<192>(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
-                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, stream);
+                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, step_tokens, status, stream);
   if (hd == 128)
     return launch_decode<128>(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
-                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, stream);
+                              nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, step_tokens, status, stream);
   if (hd == 64)
     return launch_decode<64>(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
-                             nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, stream);
+                             nh, nkv, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values, split_size, max_splits, part_acc, part_ml, rows, step_tokens, status, stream);
   return HB_ERR_UNSUPPORTED;
 }
 
@@ -416,7 +424,7 @@ extern "C" int hb_attention_decode(const void* q, const void* k_pages, const voi
                                    float* part_acc, float* part_ml, cudaStream_t stream) {
   return hb_attention_decode_rows(q, k_pages, v_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens, nh,
                                   nkv, hd, page_size, chunk, window, keep, scale, sink, head_bias, softcap, slopes, sink_values,
-                                  split_size, max_splits, part_acc, part_ml, nullptr, stream);
+                                  split_size, max_splits, part_acc, part_ml, nullptr, 0, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

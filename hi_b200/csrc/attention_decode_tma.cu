@@ -56,7 +56,8 @@ struct Args {
   int* status;
   int table_stride, nh, nkv, page_size, chunk, split_size, max_splits, box_rows;
   float scale;
-  const long long* rows;   // the tokens of the launch among those of q, out, seq_of_token and positions, or null
+  const long long* rows;   // the tokens of the launch among the step's, of q, out, seq_of_token and positions, or null
+  int step_tokens;
   int sink;      // the softmax's denominator has one more term, e^0: a key of score 0 without a value
 };
 
@@ -221,7 +222,12 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int split = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = a.nh / a.nkv;
-  const int token = a.rows ? (int)a.rows[t] : t;
+  const long long row = a.rows ? a.rows[t] : t;
+  if (a.rows && (row < 0 || row >= a.step_tokens)) {          // (all blocks of a cluster are of one token)
+    if (tid == 0) atomicExch(a.status, 32);
+    return;
+  }
+  const int token = (int)row;
   const int pos = a.positions[token];
   const int* table = a.block_table + (size_t)a.seq_of_token[token] * a.table_stride;
   const int lo = a.chunk > 0 ? (pos / a.chunk) * a.chunk : 0;
@@ -704,7 +710,8 @@ extern "C" int hb_attention_decode_tma_rows(const void* q, const void* k_pages, 
                                        const int* positions, void* out, int n_tokens, int nh, int nkv, int hd,
                                        int page_size, int chunk, int window, float scale, int sink, int split_size,
                                        int max_splits, float* part_acc, float* part_ml, int* status,
-                                       const long long* rows, cudaStream_t stream) {
+                                       const long long* rows, int step_tokens, cudaStream_t stream) {
+  if (rows && step_tokens < 0) return HB_ERR_BAD_ARG;
   if (!q || !k_pages || !v_pages || !block_table || !seq_of_token || !positions || !out || !status) return HB_ERR_BAD_ARG;
   if (n_tokens < 0 || n_pages <= 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || table_stride <= 0 ||
       chunk < 0 || window < 0 || max_splits < 1 || split_size <= 0 || split_size % TILE != 0)
@@ -718,7 +725,7 @@ extern "C" int hb_attention_decode_tma_rows(const void* q, const void* k_pages, 
   if (cluster && reinterpret_cast<uintptr_t>(out) % 8) return HB_ERR_UNSUPPORTED;
   if (n_tokens == 0) return HB_OK;
   Args a{(const __nv_bfloat16*)q, block_table, seq_of_token, positions, (__nv_bfloat16*)out, part_acc, part_ml, status,
-         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, rows, sink};
+         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, rows, step_tokens, sink};
   const Fuse none{};
   if (hd == 128) return cluster ? launch<128, CLUSTER>(k_pages, v_pages, n_pages, n_tokens, a, none, stream)
                                 : launch<128, APART>(k_pages, v_pages, n_pages, n_tokens, a, none, stream);
@@ -735,7 +742,7 @@ extern "C" int hb_attention_decode_tma(const void* q, const void* k_pages, const
                                        cudaStream_t stream) {
   return hb_attention_decode_tma_rows(q, k_pages, v_pages, n_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
                                       nh, nkv, hd, page_size, chunk, window, scale, sink, split_size, max_splits, part_acc,
-                                      part_ml, status, nullptr, stream);
+                                      part_ml, status, nullptr, 0, stream);
 }
 
 // The fused form: `qkv` [n_tokens, (nh + 2 nkv) * hd] is the q/k/v projection's output; the kernel
@@ -768,7 +775,7 @@ extern "C" int hb_attention_decode_fused(const void* qkv, const float* inv_freq,
   if ((long long)n_pages * nkv * page_size > 0x7fffffffLL) return HB_ERR_UNSUPPORTED;
   if (n_tokens == 0) return HB_OK;
   Args a{nullptr, block_table, seq_of_token, positions, (__nv_bfloat16*)out, part_acc, part_ml, status,
-         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, nullptr, sink};
+         table_stride, nh, nkv, page_size, chunk, split_size, max_splits, page_size < TILE ? page_size : TILE, scale, nullptr, 0, sink};
   if (!norm_first && (q_norm_w || k_norm_w || rot_mul != 1.f)) return HB_ERR_UNSUPPORTED;   // as hb_qkv_post
   Fuse f{(const __nv_bfloat16*)qkv, inv_freq, rot_pairs, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, counters,
          interleaved, qk_norm, temp_on, qk_eps, floor_scale, attn_scale, q_norm_w, k_norm_w, norm_first, rot_mul, v_is_k};

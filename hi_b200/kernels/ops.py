@@ -39,10 +39,10 @@ _SIGNATURES = {
     "hb_paged_attention": [P, I, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, F, P, P, I, I, P, P, P],
     "hb_attention_portions": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, F, P, P, I, P, P, P],
     "hb_attention_merge": [P, P, P, I, I, I, I, I, I, P, P],
-    "hb_attention_merge_rows": [P, P, P, I, I, I, I, I, I, P, P, P],
-    "hb_attention_decode_rows": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P, P],
+    "hb_attention_merge_rows": [P, P, P, I, I, I, I, I, I, P, P, I, P],
+    "hb_attention_decode_rows": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P, I, P, P],
     "hb_attention_decode_clusters": [I, I],
-    "hb_attention_decode_tma_rows": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P, P],
+    "hb_attention_decode_tma_rows": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P, I, P],
     "hb_attention_decode": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P],
     "hb_attention_decode_tma": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P],
     "hb_attention_decode_fused": [P, P, I, I, I, F, I, F, F, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P, P, P, P, P, I, F, I, I, P],
@@ -1434,21 +1434,27 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                      keep: int = 0, parts: bool = False, rows: Optional[torch.Tensor] = None,
                      out: Optional[torch.Tensor] = None):
     """Attention for a batch of single decoded tokens (every row of ``q`` is one request's
-    token), bfloat16, split over runs of ``ATTENTION_SPLIT`` keys. Uses scratch memory for the
-    partial results of the splits. ``softcap``, ``slopes``, ``sink_values``: as :func:`paged_attention`
+    token), bfloat16, split over runs of ``ATTENTION_SPLIT`` keys. The splits' partial results meet in
+    a cluster's shared memory or in scratch memory. ``softcap``, ``slopes``, ``sink_values``: as :func:`paged_attention`
     (the kernel that loads its tiles by cp.async takes them). With ``rows`` (int64, distinct) only those tokens of the
-    step are decoded, from where they lie in ``q`` to where they lie in ``out`` [N, nh, hd] (not with ``parts``)."""
+    step are decoded, from where they lie in ``q`` to where they lie in ``out`` [N, nh, hd] (not with ``parts``); a row outside
+    the step is left out and found by :func:`check_tc_status`."""
     if rows is not None:
         rows, seq_of_token, positions = rows.contiguous(), seq_of_token.contiguous(), positions.contiguous()
     _need(q, "q", torch.bfloat16); _need(k_pages, "k_pages", q.dtype); _need(v_pages, "v_pages", q.dtype)
     for t, nm in ((block_table, "block_table"), (seq_of_token, "seq_of_token"), (positions, "positions")):
         _need(t, nm, torch.int32)
     n, nh, hd = q.shape
+    step_tokens = n
     if rows is not None:
         _need(rows, "rows", torch.int64)
         if parts or out is None or out.shape != q.shape or out.dtype != q.dtype or not out.is_contiguous():
             raise KernelError("tokens decoded in place need an output of the queries' shape and type")
+        if seq_of_token.numel() < n or positions.numel() < n:
+            raise KernelError("seq_of_token / positions do not hold every token of the step")
         n = rows.numel()
+    elif out is not None:
+        raise KernelError("an output is given with the rows that are decoded into it")
     _, nkv, page_size, hd2 = k_pages.shape
     if hd2 != hd or k_pages.shape != v_pages.shape:
         raise KernelError("cache pages do not match the query's head_dim")
@@ -1485,7 +1491,8 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
     code = _UNSUPPORTED if reshaped else lib().hb_attention_decode_tma_rows(
         _ptr(q), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table), block_table.shape[1],
         _ptr(seq_of_token), _ptr(positions), _ptr(out), n, nh, nkv, hd, page_size, int(chunk), int(window), float(scale),
-        int(sink), split_size, splits, _ptr(part_acc), _ptr(part_ml), _ptr(_tc_status(q.device)), _ptr(rows), _stream())
+        int(sink), split_size, splits, _ptr(part_acc), _ptr(part_ml), _ptr(_tc_status(q.device)), _ptr(rows),
+        step_tokens, _stream())
     if code == _UNSUPPORTED:
         if in_cluster:
             in_cluster = False
@@ -1494,8 +1501,10 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                                          _ptr(seq_of_token), _ptr(positions), _ptr(out), n, nh, nkv, hd, page_size,
                                          int(chunk), int(window), int(keep), float(scale), int(sink), None, float(softcap),
                                          _ptr(slopes), _ptr(sink_values), split_size, splits,
-                                         _ptr(part_acc), _ptr(part_ml), _ptr(rows), _stream())
+                                         _ptr(part_acc), _ptr(part_ml), _ptr(rows), step_tokens, _ptr(_tc_status(q.device)), _stream())
         _check(code, "attention_decode")
+        if rows is not None:
+            TC_USED[0] = True
     else:
         TC_USED[0] = True
         _check(code, "attention_decode_tma")
@@ -1503,7 +1512,8 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         return part_acc, part_ml
     if splits > 1 and not in_cluster:
         _check(lib().hb_attention_merge_rows(_ptr(part_acc), _ptr(part_ml), _ptr(out), _dt(out), n * nh, hd, splits,
-                                        int(sink), nh, _ptr(sink_values), _ptr(rows), _stream()), "attention_merge")
+                                        int(sink), nh, _ptr(sink_values), _ptr(rows), step_tokens, _stream()),
+               "attention_merge")
     return out
 
 
@@ -2107,7 +2117,8 @@ def _tc_status(device: torch.device) -> torch.Tensor:
 
 def check_tc_status(device=None) -> None:
     """Raise if a kernel with bounded mbarrier waits (the tcgen05 products and attention, the TMA
-    decode attention) timed out on one of its barriers since the last check
+    decode attention, the recurrences by chunks) timed out on one of its barriers since the last check, or the decode
+    attention was given a row that its step does not have
     (synchronises; skipped while a stream is being captured)."""
     TC_USED[0] = False
     if torch.cuda.is_current_stream_capturing():
@@ -2119,6 +2130,8 @@ def check_tc_status(device=None) -> None:
             for buffers in (_down_scratch_buffers.get(key),):       # a kernel that gave up may have left a count behind
                 if buffers is not None:
                     buffers[1].zero_()
+            if code == 32:
+                raise KernelError("decode attention was given a row outside the step; its output is invalid")
             where = {1: "grouped product: the TMA producer waiting for a free stage",
                      2: "grouped product: the MMA issuer waiting for a loaded stage",
                      3: "grouped product: the epilogue waiting for the accumulator",

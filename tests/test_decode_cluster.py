@@ -71,10 +71,14 @@ def test_clusters_only_where_all_run_at_once(splits, hd, monkeypatch):
             assert float((got.float() - call().float()).abs().max()) <= 2 ** -8 * float(got.float().abs().max())      # one bfloat16 place
 
 
-# by a cluster, by the merge of several rounds' splits, of more than eight splits, by the cp.async kernel (rows of 192, a window)
-@pytest.mark.parametrize("nh,nkv,hd,lens,window", [(8, 2, 128, [900, 1, 300], 0), (24, 24, 128, [700] * 30, 0), (4, 1, 64, [9000, 64], 0),
-                                                   (8, 4, 192, [300, 77, 1000], 0), (8, 2, 64, [1500, 3], 1024)])
-def test_tokens_decoded_where_they_lie_in_a_step(nh, nkv, hd, lens, window):
+# by a cluster, by the merge of several rounds' splits, of more than eight splits, by the cp.async kernel (rows of 192, a window, kept
+# tokens, a cap, a bias and a learned sink), the sink of all of them
+@pytest.mark.parametrize("nh,nkv,hd,lens,window,merged,more", [
+    (8, 2, 128, [900, 1, 300], 0, False, {}), (8, 2, 64, [900, 1, 300], 0, False, {"sink": True}), (8, 8, 64, [600, 480] * 15, 0, True, {}),
+    (4, 1, 64, [9000, 64], 0, True, {"sink": True}), (8, 4, 192, [300, 77, 1000], 0, True, {}), (8, 2, 64, [1500, 3], 1024, True, {}),
+    (8, 2, 128, [1500, 3, 700], 512, True, {"keep": 100}), (6, 2, 64, [700, 20], 0, True, {"softcap": 5.0, "slopes": 1}),
+    (6, 2, 128, [700, 20], 0, True, {"sink_values": 1})])
+def test_tokens_decoded_where_they_lie_in_a_step(nh, nkv, hd, lens, window, merged, more):
     from hi_b200.kernels import ops
 
     g = torch.Generator(device=DEV).manual_seed(hd + len(lens))
@@ -93,11 +97,37 @@ def test_tokens_decoded_where_they_lie_in_a_step(nh, nkv, hd, lens, window):
     seq, pos = i32(), i32()
     seq[rows] = torch.arange(n, dtype=torch.int32, device=DEV)
     pos[rows] = torch.tensor([k - 1 for k in lens], dtype=torch.int32, device=DEV)
+    more = {k: torch.rand(nh, device=DEV, generator=g) if k in ("slopes", "sink_values") else v for k, v in more.items()}
     rest = (hd ** -0.5, max(lens))
-    want = ops.decode_attention(q[rows], kp, vp, table, seq[rows], pos[rows], 0, window, *rest)
+    called = ops.CALLS.get("attention_merge", 0)
+    want = ops.decode_attention(q[rows], kp, vp, table, seq[rows], pos[rows], 0, window, *rest, **more)
+    assert ops.CALLS.get("attention_merge", 0) - called == merged
     before = out.clone()
-    assert ops.decode_attention(q, kp, vp, table, seq, pos, 0, window, *rest, rows=rows, out=out) is out
+    assert ops.decode_attention(q, kp, vp, table, seq, pos, 0, window, *rest, rows=rows, out=out, **more) is out
     assert torch.equal(out[rows], want)                     # the same kernels and cuts, other addresses
     others = torch.ones(total, dtype=torch.bool, device=DEV)
     others[rows] = False
     assert torch.equal(out[others], before[others])
+    ops.check_tc_status()
+    # rows that the step does not have are left out and found
+    wrong, out = rows.clone(), before.clone()
+    wrong[0], wrong[-1] = -1, total
+    ops.decode_attention(q, kp, vp, table, seq, pos, 0, window, *rest, rows=wrong, out=out, **more)
+    with pytest.raises(ops.KernelError, match="row outside the step"):
+        ops.check_tc_status()
+    ops.check_tc_status()
+    assert torch.equal(out[rows[1:-1]], want[1:-1])
+    others[rows[0]] = others[rows[-1]] = True
+    assert torch.equal(out[others], before[others])
+
+
+def test_an_output_is_given_with_its_rows():
+    from hi_b200.kernels import ops
+
+    q, pages = torch.zeros(2, 4, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(2, 1, 64, 64, dtype=torch.bfloat16, device=DEV)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    rows = torch.tensor([1], device=DEV)
+    for seq, pos, more in ((i32(0, 1), i32(3, 3), {"out": q.clone()}), (i32(0, 1), i32(3, 3), {"rows": rows}),
+                           (i32(0), i32(3, 3), {"rows": rows, "out": q.clone()}), (i32(0, 1), i32(3), {"rows": rows, "out": q.clone()})):
+        with pytest.raises(ops.KernelError):
+            ops.decode_attention(q, pages, pages, i32(0, 1).view(2, 1), seq, pos, 0, 0, 0.125, 4, **more)
