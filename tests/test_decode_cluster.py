@@ -8,9 +8,12 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("nh,nkv,hd", [(40, 8, 128), (8, 2, 64), (3, 3, 128), (16, 1, 64)])
-@pytest.mark.parametrize("lens,page,chunk,sink", [([1000], 64, 0, False), ([65, 1, 64, 128, 63], 16, 0, True), ([513, 2], 32, 0, False),
-                                                  ([900, 300, 512, 513], 128, 512, True), ([2049], 64, 0, False), ([129, 700, 64], 64, 128, False)])
-def test_splits_meet_in_a_cluster(nh, nkv, hd, lens, page, chunk, sink, monkeypatch):
+@pytest.mark.parametrize("lens,page,chunk,sink,splits", [([300, 1, 64, 128, 63], 16, 0, True, 2), ([900, 300, 512, 513], 128, 512, True, 2),
+                                                         ([513, 2], 32, 0, False, 3), ([1000], 64, 0, False, 4), ([1100, 40, 257], 16, 0, True, 5),
+                                                         ([1500, 1], 32, 0, False, 6), ([1791, 700, 256], 16, 0, True, 7), ([1900, 3, 257], 64, 0, True, 8),
+                                                         # one split, and more than a cluster has: the same kernels either way
+                                                         ([65, 1, 64, 128, 63], 16, 0, True, 1), ([129, 700, 64], 64, 128, False, 1), ([2100], 64, 0, False, 9)])
+def test_splits_meet_in_a_cluster(nh, nkv, hd, lens, page, chunk, sink, splits, monkeypatch):
     from hi_b200.kernels import ops
 
     g = torch.Generator().manual_seed(sum(lens) + nh)
@@ -26,14 +29,14 @@ def test_splits_meet_in_a_cluster(nh, nkv, hd, lens, page, chunk, sink, monkeypa
     pos = torch.tensor([k - 1 for k in lens], dtype=torch.int32)
     args = [t.to(DEV) for t in (q, kp, vp, table, torch.arange(n, dtype=torch.int32), pos)]
     call = lambda: ops.decode_attention(*args, chunk, 0, hd ** -0.5, max(lens), sink=sink)
-    splits = ops._decode_splits(min(max(lens), chunk or max(lens)), n * nkv)[1]
-    before = dict(ops.CALLS)
+    assert ops._decode_splits(min(max(lens), chunk or max(lens)), n * nkv)[1] == splits
+    before = ops.CALLS.get("attention_merge", 0)
     got = call()
-    if 1 < splits <= 8:
-        assert ops.CALLS.get("attention_merge", 0) == before.get("attention_merge", 0)
+    assert ops.CALLS.get("attention_merge", 0) - before == (splits > 8)
     assert torch.equal(got, call())                        # the blocks of a cluster finish in any order: the sum has one
     monkeypatch.setattr(ops, "DECODE_CLUSTER", 1)
     apart = call()
+    assert ops.CALLS.get("attention_merge", 0) - before == (1 < splits <= 8) + 3 * (splits > 8)
     for i, k in enumerate(lens):
         lo = (k - 1) // chunk * chunk if chunk else 0
         rows = lambda t: t[table[i, : -(-k // page)].long()].transpose(1, 2).reshape(-1, nkv, hd)[lo:k].double()
