@@ -85,13 +85,10 @@ int hb_attention_decode_tma_rows(const void* q, const void* k_pages, const void*
                                  int nh, int nkv, int hd, int page_size, int chunk, int window, float scale, int sink,
                                  int split_size, int max_splits, float* part_acc, float* part_ml, int* status,
                                  const long long* rows, int step_tokens, cudaStream_t stream);
-int hb_attention_decode_tma(const void* q, const void* k_pages, const void* v_pages, int n_pages, const int* block_table,
-                            int table_stride, const int* seq_of_token, const int* positions, void* out, int n_tokens,
-                            int nh, int nkv, int hd, int page_size, int chunk, int window, float scale, int sink,
-                            int split_size, int max_splits, float* part_acc, float* part_ml, int* status,
-                            cudaStream_t stream);
+// clusters of `splits` blocks that run at a time
+int hb_attention_decode_clusters(int hd, int splits);
 
-// hb_qkv_post, hb_attention_decode_tma and hb_attention_merge in one launch (attention_decode_tma.cu)
+// hb_qkv_post, hb_attention_decode_tma_rows and hb_attention_merge in one launch (attention_decode_tma.cu)
 int hb_attention_decode_fused(const void* qkv, const float* inv_freq, int rot_pairs, int interleaved, int qk_norm,
                               float qk_eps, int temp_on, float floor_scale, float attn_scale, void* k_pages,
                               void* v_pages, int n_pages, const int* block_table, int table_stride,

@@ -704,7 +704,8 @@ extern "C" int hb_attention_decode_clusters(int hd, int splits) {
 // token one decode row; partials merged by hb_attention_merge), with TMA tile loads. Returns
 // HB_ERR_UNSUPPORTED for what those cannot take (a sliding window, a chunk size or page size
 // that breaks the 64-key tiles): the caller then uses hb_attention_decode. `status` is one int
-// on the device, zero before the call; nonzero afterwards = a wait on a load timed out. `rows`: as hb_attention_decode_rows.
+// on the device, zero before the call; nonzero afterwards = a wait on a load timed out or a row lies outside the step. `rows`: as
+// hb_attention_decode_rows.
 extern "C" int hb_attention_decode_tma_rows(const void* q, const void* k_pages, const void* v_pages, int n_pages,
                                        const int* block_table, int table_stride, const int* seq_of_token,
                                        const int* positions, void* out, int n_tokens, int nh, int nkv, int hd,
@@ -734,24 +735,13 @@ extern "C" int hb_attention_decode_tma_rows(const void* q, const void* k_pages, 
   return HB_ERR_UNSUPPORTED;
 }
 
-extern "C" int hb_attention_decode_tma(const void* q, const void* k_pages, const void* v_pages, int n_pages,
-                                       const int* block_table, int table_stride, const int* seq_of_token,
-                                       const int* positions, void* out, int n_tokens, int nh, int nkv, int hd,
-                                       int page_size, int chunk, int window, float scale, int sink, int split_size,
-                                       int max_splits, float* part_acc, float* part_ml, int* status,
-                                       cudaStream_t stream) {
-  return hb_attention_decode_tma_rows(q, k_pages, v_pages, n_pages, block_table, table_stride, seq_of_token, positions, out, n_tokens,
-                                      nh, nkv, hd, page_size, chunk, window, scale, sink, split_size, max_splits, part_acc,
-                                      part_ml, status, nullptr, 0, stream);
-}
-
 // The fused form: `qkv` [n_tokens, (nh + 2 nkv) * hd] is the q/k/v projection's output; the kernel
 // encodes q, k and v as hb_qkv_post does (inv_freq [rot_pairs] or null; pairs (j, j + rot_pairs) or
 // (2j, 2j + 1); weightless norm after the rotation, or with norm_first the weighted RMS norm before it; rot_mul on
 // cos and sin; temperature on q; v_is_k as in hb_qkv_post; sink: one more term of score 0 in the softmax's denominator), appends the token's key and value to its page,
 // attends, and combines its own splits: `counters` holds n_tokens * nkv ints that are zero before
 // the call and zero after it. With `counters` null the splits are left in part_acc / part_ml for
-// hb_attention_merge, as hb_attention_decode_tma leaves them. Same shapes and refusals as hb_attention_decode_tma; every token is
+// hb_attention_merge, as hb_attention_decode_tma_rows leaves them. Same shapes and refusals as there; every token is
 // one decode row whose page the host has reserved.
 extern "C" int hb_attention_decode_fused(const void* qkv, const float* inv_freq, int rot_pairs, int interleaved, int qk_norm,
                                          float qk_eps, int temp_on, float floor_scale, float attn_scale, void* k_pages,
