@@ -41,6 +41,11 @@ def bytes_per_token(cache_specs: Dict[int, Optional[CacheSpec]], element_size: i
     return out
 
 
+def pool_budget(free_bytes: int, fraction: float, scratch_bytes: int) -> int:
+    """Bytes for the pools: ``fraction`` of what is free, but never the workspace that a step's kernels will ask for."""
+    return max(0, min(int(free_bytes * fraction), free_bytes - scratch_bytes))
+
+
 def pool_tokens_for_budget(cache_specs: Dict[int, Optional[CacheSpec]], element_size: int, budget_bytes: int,
                            page_size: int, max_requests: int, most_tokens: Optional[int] = None,
                            portion_tokens: int = 8192) -> List[int]:

@@ -18,7 +18,7 @@ from typing import Dict, Hashable, List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
-from ..cache.device import DeviceCache, plan_groups, pool_tokens_for_budget
+from ..cache.device import DeviceCache, plan_groups, pool_budget, pool_tokens_for_budget
 from ..cache.pages import CacheManager, OutOfPages
 from ..config.registry import load_architecture, lookup
 from ..parts.context import StepContext
@@ -86,7 +86,7 @@ class Engine:
     ``kv_cache_tokens`` sizes every page pool (tokens, rounded up to pages);
     ``windowed_cache_tokens`` optionally gives the windowed groups (chunked layers) a smaller
     pool. Without ``kv_cache_tokens`` the pools are sized from the device memory that is free once
-    the weights are loaded: ``cache_memory_fraction`` of it, windowed groups at what
+    the weights are loaded: ``cache_memory_fraction`` of it (less where the parts' workspaces need the rest), windowed groups at what
     ``max_active_requests`` windows need, the rest to the groups that keep every key.
     ``max_active_requests`` is the number of state slots / block-table rows.
     """
@@ -109,7 +109,7 @@ class Engine:
             free, _total = torch.cuda.mem_get_info(self.device)
             longest = model.spec.max_position_embeddings
             auto = pool_tokens_for_budget(model.cache_specs, torch.empty((), dtype=model.dtype).element_size(),
-                                          int(free * cache_memory_fraction), self.page_size, max_active_requests,
+                                          pool_budget(free, cache_memory_fraction, model.scratch_bytes), self.page_size, max_active_requests,
                                           most_tokens=None if longest is None else longest * max_active_requests)
         pages = []
         for g, spec in enumerate(groups):

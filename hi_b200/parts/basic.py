@@ -19,9 +19,11 @@ class Part:
 
     ``graph_safe``: the part's forward only enqueues work whose shape depends on the number of
     tokens and reads the step's device tensors, never its host-side lists; a decode step made of
-    such parts may be captured in a CUDA graph. A part that does not say so is never captured."""
+    such parts may be captured in a CUDA graph. A part that does not say so is never captured.
+    ``scratch_bytes``: a workspace of a step's size that its kernels take at a time, at most (beside activations)."""
 
     graph_safe = False
+    scratch_bytes = 0
 
     def __init__(self, params: dict, prefix: str, env: BuildEnv):
         self.params, self.prefix, self.env = params, prefix, env

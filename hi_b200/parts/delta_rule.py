@@ -41,6 +41,7 @@ class ChannelDeltaMixer(Part):
     ``<prefix>.o`` [H, heads*vdim]."""
 
     graph_safe = True
+    scratch_bytes = ops.CHUNKED_SCRATCH_BYTES
     GENERAL_KERNEL = False       # tests: force the recurrence kernel that keeps S in shared memory
 
     def __init__(self, params, prefix, env):

@@ -30,6 +30,7 @@ class GatedLinearAttentionMixer(Part):
     ``<prefix>.a2`` [heads*dim, r], ``<prefix>.a2.b`` [heads*dim], ``<prefix>.norm`` [vdim], ``<prefix>.o`` [H, heads*vdim]."""
 
     graph_safe = True
+    scratch_bytes = ops.CHUNKED_SCRATCH_BYTES
     GENERAL_KERNEL = False       # tests: force the recurrence kernel that keeps S in shared memory
 
     def __init__(self, params, prefix, env):

@@ -31,6 +31,7 @@ class Mamba2Mixer(Part):
     ``<prefix>.norm`` [inner], ``<prefix>.o`` [H, inner]."""
 
     graph_safe = True
+    scratch_bytes = ops.CHUNKED_SCRATCH_BYTES
 
     def __init__(self, params, prefix, env):
         super().__init__(params, prefix, env)

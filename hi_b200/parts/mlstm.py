@@ -31,6 +31,7 @@ class MLSTMMixer(Part):
     with ``.b`` [heads], ``<prefix>.norm`` [heads*vdim], ``<prefix>.o`` [H, heads*vdim]."""
 
     graph_safe = True
+    scratch_bytes = ops.CHUNKED_SCRATCH_BYTES
     ROWS_PER_LANE = 0            # tests: force a layout of the recurrence kernel (0: chosen by dim)
 
     def __init__(self, params, prefix, env):

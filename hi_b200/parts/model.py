@@ -82,6 +82,7 @@ class Model:
                 raise ValueError(f"cache slot {slot} is read but no schedule entry writes it")
         self.loaded = False
         self.graph_safe = all(getattr(p, "graph_safe", False) for p in self.all_parts())
+        self.scratch_bytes = max(getattr(p, "scratch_bytes", 0) for p in self.all_parts())       # one part at a time
 
     # ---- weights
     def all_parts(self):

@@ -24,6 +24,7 @@ class MixerPair(Part):
         self.sides = [build("mixer", PartSpec(params[s]["kind"], dict(params[s]["params"])), env, f"{prefix}.{s}")
                       for s in ("left", "right")]
         self.graph_safe = all(getattr(m, "graph_safe", False) for m in self.sides)
+        self.scratch_bytes = max(getattr(m, "scratch_bytes", 0) for m in self.sides)
         self.w = [None, None]
         specs = [m.cache_spec() for m in self.sides]
         paged = [s for s in specs if s is not None and s.paged]

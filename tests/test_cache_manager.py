@@ -2,6 +2,7 @@
 import random
 
 import pytest
+import torch
 
 from hi_b200.cache import FREED, CacheManager, OutOfPages, OutOfSlots, PagePool
 from hi_b200.parts.spec import CacheSpec
@@ -193,3 +194,21 @@ def test_pool_sizes_from_a_byte_budget():
     small = pool_tokens_for_budget(specs, 2, 1 << 20, 64, 8)
     assert all(t >= 2 * 64 for t in small)
     assert pool_tokens_for_budget({0: None}, 2, budget, 64, 8) == []
+
+
+def test_the_pools_leave_a_step_its_workspace():
+    """The recurrences' prepared chunks are asked for in the middle of a step: a fraction near one must not give them to the pools."""
+    from hi_b200.cache.device import pool_budget
+    from hi_b200.config.registry import lookup
+    from hi_b200.kernels import ops
+    from hi_b200.parts.model import Model
+    from tiny_configs import TINY_A
+    from vinurax_configs import VX_A
+
+    scratch = ops.CHUNKED_SCRATCH_BYTES
+    assert pool_budget(80 << 30, 0.9, scratch) == int((80 << 30) * 0.9)
+    assert pool_budget(80 << 30, 1.0, scratch) == (80 << 30) - scratch and pool_budget(80 << 30, 1.0, 0) == 80 << 30
+    assert pool_budget(scratch // 2, 1.0, scratch) == 0
+    for config, want in ((VX_A, scratch), (TINY_A, 0)):
+        arch = lookup(config)
+        assert Model(arch.build_spec(arch.parse_config(config, None)), torch.float32, "cpu").scratch_bytes == want
