@@ -18,11 +18,12 @@
 // The prepared chunks (7.5 to 39.5 KB a head, by key size and rule) go through a scratch of bounded size: see slices_of.
 //
 // Measured (B200, one request of 2,048 tokens, 16 heads of 128 x 128; token after token / sixteen at a time with the rows
-// prepared by every block for itself / now): delta rule 582 / 234 / 192 us (45 of them the preparation); mLSTM with 1,101 and
-// 467 tokens beside single ones 353 / 163 / 137; 1,100 tokens of the rule without correction, 16 heads of 128 x 128 85 -> 73,
-// of 64 x 128 67 -> 47. Over 1,800 steps of all three rules (4 to 40 heads of 16 x 16 to 128 x 128, 1 to 64 requests) 0.84 of the
-// time before; the delta rule's steps of many requests and 64 columns, which fill the SMs, pay for the preparation (40 heads, 16
-// requests of 100 tokens 221 -> 250). Error against 64 bits (2-norm) of the first: 7.0e-8 before and now.
+// prepared by every block for itself / now): delta rule 576 / 224 / 182 us (45 of them the preparation); mLSTM with 1,101 and
+// 467 tokens beside single ones 328 / 133 / 107; 1,100 tokens of the rule without correction, 16 heads of 128 x 128 307 / 85 / 74,
+// of 64 x 128 263 / 66 / 52. Over 900 steps of all three rules (4 to 40 heads of 16 x 16 to 128 x 128, 1 to 73 requests) 0.80 of
+// the second. The preparation costs the same whatever the columns are, so steps of many requests and few columns pay for it: delta
+// rule, 40 heads of 96 x 64, 16 requests of 100 tokens 222 -> 227; 20 heads of 128 x 16, 19 uneven ones of 8,084 in all 262 -> 351
+// (ops._chunked_recurrence gives most of them to the other form). Error against 64 bits (2-norm) of the first: 7.0e-8 before and now.
 // What bounds it: the chain from chunk to chunk, 1.1 us; 4,200 warp instructions of 16 warps that wait for one another (an empty
 // chunk with its barriers takes 0.44 us; no part of it more than 0.1). Tried: twice the helpers (8 % slower: they share the
 // issue slots), half as many at keys of 64 and less (1.1 to 1.4 times as long); P q S by two helper warps from pieces of S kept
@@ -434,6 +435,7 @@ struct ChunkSmem {
     float u[PLAIN ? RING : 2][CG][20];         // [column][token]
     __nv_bfloat16 up[PLAIN ? RING : 1][3][CG][24];    // the pieces of u
     uint64_t full[STAGES], full_m[RING];
+    int gave_up;                               // a wait for a copy
   };
 };
 
@@ -457,6 +459,7 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
     for (int i = 0; i < STAGES; ++i) tc::mbar_init(&sm.full[i], 1);
 #pragma unroll
     for (int i = 0; i < RING; ++i) tc::mbar_init(&sm.full_m[i], 1);
+    sm.gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -465,16 +468,9 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
   auto there = [&](uint64_t* full, int use) {          // a copy has arrived
     if (ok && !tc::mbar_wait(full, use & 1)) {
       atomicExch(a.status, 41);
+      sm.gave_up = 1;
+      tc::mbar_wait(full, use & 1);                   // once more, so that the copy does not outlive the block
       ok = false;                                     // go on without waiting: every barrier of the block is still met
-    }
-  };
-
-  // A thread that gave up waits for the last copies into each place before it leaves, again with the limit, so that none is under
-  // way when the block ends.
-  auto see_copies_land = [&]() {
-    for (int i = max(0, chunks - RING); i < chunks; ++i) {
-      if (i >= chunks - STAGES) tc::mbar_wait(&sm.full[i % STAGES], (i / STAGES) & 1);
-      tc::mbar_wait(&sm.full_m[i % RING], (i / RING) & 1);
     }
   };
 
@@ -594,6 +590,13 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
                               fmaf(s[m][n][e], (e & 1) ? full[n].w : full[n].y, z[n][e]));
       }
     }
+    // Where a wait was given up, no copy is under way when the block ends: the last ones into each place are waited for, again with
+    // the limit. (Behind the helpers' loop, or behind the states below, the same lines cost the delta rule 2 to 4 %.)
+    if (*reinterpret_cast<volatile int*>(&sm.gave_up))
+      for (int i = max(0, chunks - RING); i < chunks; ++i) {
+        if (i >= chunks - STAGES) tc::mbar_wait(&sm.full[i % STAGES], (i / STAGES) & 1);
+        tc::mbar_wait(&sm.full_m[i % RING], (i / RING) & 1);
+      }
 #pragma unroll
     for (int m = 0; m < CT; ++m)
 #pragma unroll
@@ -604,7 +607,6 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
           const size_t i = at(m, n, e, in);
           if (in) S[i] = s[m][n][e];
         }
-    if (!ok) see_copies_land();
     return;
   }
 
@@ -727,7 +729,6 @@ __global__ void __launch_bounds__(32 * NW + 2 * ChunkSmem<NW, CT, PLAIN>::HELP) 
     }
     if (i + 2 < chunks) bar_arrive(FREED + b, COMP + HELP);
   }
-  if (!ok) see_copies_land();
 }
 
 template <typename T, int NW, int CT, bool PLAIN>
