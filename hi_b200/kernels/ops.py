@@ -1477,17 +1477,18 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                 torch.empty((n, nh, splits, 2), dtype=torch.float32, device=q.device))
 
     # the splits meet in a cluster's shared memory where all clusters run at once
-    in_cluster = not reshaped and 1 < splits <= DECODE_CLUSTER and n * nkv <= _decode_clusters(q.device.index, hd, splits)
+    in_cluster = not reshaped and 1 < splits <= DECODE_CLUSTER and n * nkv <= _decode_clusters(q.get_device(), hd, splits)
     if (splits > 1 or parts) and not in_cluster:
         part_acc, part_ml = scratch()
-    for t, nm in ((slopes, "slopes"), (sink_values, "sink_values")):
-        if t is not None:
-            _need(t, nm, torch.float32)
-            if t.numel() != nh:
-                raise KernelError(f"{nm} needs one number per query head")
+    if slopes is not None or sink_values is not None:
+        for t, nm in ((slopes, "slopes"), (sink_values, "sink_values")):
+            if t is not None:
+                _need(t, nm, torch.float32)
+                if t.numel() != nh:
+                    raise KernelError(f"{nm} needs one number per query head")
     sink = bool(sink) or sink_values is not None
     # tile loads by TMA where the range and the pages allow it (the kernel says if not)
-    code = _UNSUPPORTED if reshaped else lib().hb_attention_decode_tma_rows(
+    code = _UNSUPPORTED if reshaped or hd == 192 else lib().hb_attention_decode_tma_rows(
         _ptr(q), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table), block_table.shape[1],
         _ptr(seq_of_token), _ptr(positions), _ptr(out), n, nh, nkv, hd, page_size, int(chunk), int(window), float(scale),
         int(sink), split_size, splits, _ptr(part_acc), _ptr(part_ml), _ptr(_tc_status(q.device)), _ptr(rows),
@@ -1500,7 +1501,8 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                                          _ptr(seq_of_token), _ptr(positions), _ptr(out), n, nh, nkv, hd, page_size,
                                          int(chunk), int(window), int(keep), float(scale), int(sink), None, float(softcap),
                                          _ptr(slopes), _ptr(sink_values), split_size, splits,
-                                         _ptr(part_acc), _ptr(part_ml), _ptr(rows), step_tokens, _ptr(_tc_status(q.device)), _stream())
+                                         _ptr(part_acc), _ptr(part_ml), _ptr(rows), step_tokens,
+                                         None if rows is None else _ptr(_tc_status(q.device)), _stream())
         _check(code, "attention_decode")
         if rows is not None:
             TC_USED[0] = True
