@@ -17,24 +17,28 @@ DIFF_TC_MIN_TOKENS = 64      # new tokens of a request from which differential a
                              # tile is 64 tokens by two maps)
 
 
-def _key_splits(ctx, nh: int, hd: int, chunk: int, sliding: int, keep: int, single: bool, device) -> int:
+def _key_splits(ctx, nh: int, nkv: int, hd: int, chunk: int, sliding: int, keep: int, single: bool, pairs: bool, device) -> int:
     """Portions far into long contexts on a layer that sees every key: all blocks of the
     tensor-core prefill kernel then have about the same many key tiles, and a partly filled
     last round of blocks is worth splitting the keys for (ops.prefill_key_splits). Everything else: what a model of
-    the kernel's time says (ops.prefill_shares)."""
+    the kernel's time says (ops.prefill_shares; for the kernel of two query tiles a block ops.prefill_pair_shares, which then
+    also says into how many)."""
     if keep:
         return 1
     portions = [(s, n) for s, n in zip(ctx.start_pos, ctx.n_new) if n > 1 or not single]
     if not portions:
         return 1
-    sms = ops.sm_count(device)
+    sms, least = ops.sm_count(device), 1
     if not chunk and not sliding:
         shortest, longest_new = min(s for s, _n in portions), max(n for _s, n in portions)
         if shortest >= 2 * longest_new:
             blocks = nh * sum(-(-n // ops.PREFILL_TC_MIN_TOKENS) for _s, n in portions)
             shares = ops.prefill_key_splits(blocks, shortest // 64, sms)
-            if shares > 1:
+            if shares > 1 and not pairs:
                 return shares
+            least = min(shares, 2)
+    if pairs:
+        return ops.prefill_pair_shares(portions, nh, nkv, hd, chunk, sliding, ctx.n_tokens, sms, least)
     return ops.prefill_shares(portions, nh, hd, chunk, sliding, ctx.n_tokens, sms)
 
 
@@ -68,7 +72,8 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
         if tc:
             o = ops.prefill_attention_tc(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions,
                                          ctx.n_seqs, ctx.max_new, chunk, sliding, scale, skip_single=single,
-                                         key_splits=_key_splits(ctx, nh, hd, chunk, sliding, keep, single, q.device), sink=sink,
+                                         key_splits=_key_splits(ctx, nh, nkv, hd, chunk, sliding, keep, single,
+                                                                ops.prefill_pairs(hd, softcap, slopes, keep), q.device), sink=sink,
                                          softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep)
         else:
             o = ops.prefill_attention(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions,
