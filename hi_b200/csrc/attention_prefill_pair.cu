@@ -7,7 +7,20 @@
 //   warp 8            TMA loads: both Q tiles, then K and V tiles of 128 keys in turn through one ring, a box per page.
 //   warp 9            issues the products, tile after tile: O0 += P0 V, S0 = Q0 K^T of the next tile, then the same of item 1. While
 //                     one item's softmax runs, the tensor cores have the other's two products.
-// S and O of both items take all of tensor memory, so one block lives on an SM.
+// S and O of both items take all of tensor memory, so one block lives on an SM; when a work's loads are under way, the block takes the
+// next one that has not started (cluster launch control), and its Q and first K arrive while the last tiles of this one are worked at.
+//
+// Measured (B200, one tile a block and two blocks an SM / this, us): 2,048 tokens of 40 heads of 128 on 8 69.3 / 44.7, 4,096 207 / 153,
+// 1,024 behind 16,384 424 / 336, 600 beside 700 behind 300 and 400 behind 100 49 / 35, 2,048 behind 8,192 in a window of 1,024 92 / 61,
+// 24 heads on 24 49 / 37; prompts of 160 to 300 tokens, which are a block's latency, 9.2 to 11.1 / 10.6 to 12.1 (an eager call
+// takes the host 17).
+// What bounds it: a pair of 128-key tiles takes 3,000 cycles where its products take 2,048 and its exponentials, 16 a cycle, as many:
+// a chain of softmax (1,550), the last 32 keys' P V and Q K^T (640) and the hand-overs between them (about 350 from the last
+// product to the softmax's first load, 200 back). What mattered on the way there, in us for 256 tokens behind 16,384: one lane that
+// walked the products' loop alone 285, the warp together 231; waits that vote over each lane's own loop 235, over one try 230; P V
+// begun before the last 32 keys of P are there 215 (64 keys: the same). Two warps that issue the products, one an item, 284: both
+// items then wait for their products at the same time. Rows stored by the lane that holds them, 32 lines an instruction: 2.5 us a
+// pair, by fours of lanes 1.4.
 // Every mbarrier wait is bounded; on a time-out a code goes to `status` and the block leaves through the common exit.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -59,9 +72,10 @@ __device__ __forceinline__ void trade_rows(uint4 (&v)[4], int lane) {
   }
 }
 
-// An item: its first token, how many there are, the head, the first and last position, its key tiles [begin, end).
+// An item: its first token, how many there are, the head, the first and last position, the first key that any row reads, its key tiles
+// [begin, end).
 struct Item {
-  int tok0, n_valid, head, p_first, p_last, begin, end;
+  int tok0, n_valid, head, p_first, p_last, first, begin, end;
 };
 
 // What a block works at: two items (the second may have no tokens), their key tiles in one run, the last position.
@@ -109,7 +123,8 @@ __device__ __forceinline__ bool work_of(const PrefillPairArgs& a, int bx, int by
     x.n_valid = in ? min(BQ, n_new - t * BQ) : 0;
     x.p_first = p0 + t * BQ;
     x.p_last = x.p_first + x.n_valid - 1;
-    x.begin = first_visible(a, x.p_first) / BK;
+    x.first = first_visible(a, x.p_first);
+    x.begin = x.first / BK;
     x.end = in ? x.p_last / BK + 1 : x.begin;
   }
   // neighbours in tokens, so what they read is one run
@@ -145,7 +160,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   uint8_t* other = ring + STAGES * L::KBYTES;
   uint4* answer = reinterpret_cast<uint4*>(other);
   Work* works = reinterpret_cast<Work*>(other + 16);           // 2
-  uint64_t* bars = reinterpret_cast<uint64_t*>(other + 16 + 2 * sizeof(Work) + 8);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(other + 16 + 2 * sizeof(Work));
   uint64_t* full = bars;                                       // STAGES
   uint64_t* empty = full + STAGES;                             // STAGES
   uint64_t* q_full = empty + STAGES;                           // 1: both Q tiles
@@ -159,7 +174,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   uint64_t* work_read = work_full + 2;                         // 2
   uint64_t* answered = work_read + 2;                          // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(answered + 1);
-  static_assert(sizeof(Work) % 8 == 4 && 16 + 2 * sizeof(Work) + 8 + (2 * STAGES + 16) * 8 + 4 <= L::OTHER, "barriers and works fit");
+  static_assert(sizeof(Work) % 4 == 0 && 16 + 2 * sizeof(Work) + (2 * STAGES + 16) * 8 + 4 <= L::OTHER, "barriers and works fit");
 
   const int warp = tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   // What a block does first hangs together in a chain of memory latencies: the barriers, the tensor memory, the maps and the first
@@ -176,9 +191,20 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   } else if (warp == 10 && lane < 3) {
     tc::prefetch_map(lane == 0 ? &map_q : lane == 1 ? &map_k : &map_v);
   }
-  Work job;                                                    // of the loads' warp
+  Work job = {};                                               // of the loads' warp
   bool some = true;
-  if (warp == 8 && !work_of(a, blockIdx.x, blockIdx.y, blockIdx.z, job)) job.there = 0;
+  int page = -1;                                               // this lane's of the tile that is loaded next
+  // a lane a box of K or V: 64 elements of a page's rows (or of 64 of them)
+  const int box = lane / DBLK, box_col = lane % DBLK * 64;
+  const bool boxes = box < BK / a.box_rows;
+  auto page_of = [&](int j) {
+    const int key0 = j * BK + box * a.box_rows;
+    return boxes && key0 <= job.p_end ? a.block_table[(size_t)job.seq * a.table_stride + key0 / a.page_size] : -1;
+  };
+  if (warp == 8) {
+    if (!work_of(a, blockIdx.x, blockIdx.y, blockIdx.z, job)) job.there = 0;
+    else if (job.begin < job.end) page = page_of(job.begin);
+  }
   if (warp == 9) tc::alloc(tmem_slot, 512);
   tc::fence_before();
   __syncthreads();
@@ -217,23 +243,14 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         __syncwarp();
         some = got != 0;
         if (!some || !work_of(a, bx, by, bz, job)) job.there = 0;
+        else if (job.begin < job.end) page = page_of(job.begin);
       };
       for (int w = 0; ok; ) {
         if (!job.there && some) {               // nothing in this block of the grid
           bid();
           continue;
         }
-        // a lane a box: 64 elements of a page's rows (or of 64 of them)
-        const int* table = a.block_table + (size_t)job.seq * a.table_stride;
-        const int box = lane / DBLK, c = lane % DBLK;
-        const bool mine = box < BK / a.box_rows, loads = job.there && job.begin < job.end;
-        auto page_row = [&](int j) {
-          const int key0 = j * BK + box * a.box_rows;
-          const int page = mine && key0 <= job.p_end ? table[key0 / a.page_size] : -1;
-          // keys past the last position, or on pages given back, are read by no row: any row will do
-          return page >= 0 ? (page * a.nkv + job.kvh) * a.page_size + key0 % a.page_size : 0;
-        };
-        int row = loads ? page_row(job.begin) : 0;
+        const bool loads = job.there && job.begin < job.end;
         // (every work's Q phase is waited for, also of those without keys: the barrier is never two phases on)
         if ((w >= 2 && !tc::mbar_wait_warp(&work_read[w & 1], ((w >> 1) - 1) & 1)) ||
             (w >= 1 && !tc::mbar_wait_warp(q_empty, (w - 1) & 1))) {
@@ -241,26 +258,31 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           ok = false;
           break;
         }
-        if (lane == 0) {
-          if (loads) {
-            const bool two = job.x[1].n_valid > 0;
-            tc::mbar_expect_tx(q_full, (two ? 2 : 1) * L::QBYTES);
-            for (int d = 0; d < DBLK; ++d) {
-              tc::tma_load_2d(q_s + d * L::BLOCK, &map_q, job.x[0].head * HD + d * 64, job.x[0].tok0, q_full);
-              if (two) tc::tma_load_2d(q_s + L::QBYTES + d * L::BLOCK, &map_q, job.x[1].head * HD + d * 64, job.x[1].tok0, q_full);
-            }
+        if (lane == 0 && loads) {
+          const bool two = job.x[1].n_valid > 0;
+          tc::mbar_expect_tx(q_full, (two ? 2 : 1) * L::QBYTES);
+          for (int d = 0; d < DBLK; ++d) {
+            tc::tma_load_2d(q_s + d * L::BLOCK, &map_q, job.x[0].head * HD + d * 64, job.x[0].tok0, q_full);
+            if (two) tc::tma_load_2d(q_s + L::QBYTES + d * L::BLOCK, &map_q, job.x[1].head * HD + d * 64, job.x[1].tok0, q_full);
           }
-          works[w & 1] = job;
-          tc::mbar_arrive(&work_full[w & 1]);
         }
         queries += loads;
-        ++w;
+        auto publish = [&]() {                  // to the products' and the softmax's warps
+          if (lane == 0) {
+            works[w & 1] = job;
+            tc::mbar_arrive(&work_full[w & 1]);
+          }
+          ++w;
+        };
+        if (!loads) publish();
         if (!some) break;
         if (loads) {
           // Rows of V past the last position meet weights of zero in their step of 16 keys, and may hold anything: they are cleared.
           const int clear = (job.p_end + 1) % 16 != 0 && job.p_end / BK == job.end - 1 ? job.p_end % BK + 1 : 0;
           for (int j = job.begin; j < job.end && ok; ++j) {
-            const int next = j + 1 < job.end ? page_row(j + 1) : 0;
+            const int next = j + 1 < job.end ? page_of(j + 1) : -1;
+            // keys past the last position, or on pages given back, are read by no row: any row will do
+            const int row = page >= 0 ? (page * a.nkv + job.kvh) * a.page_size + (j * BK + box * a.box_rows) % a.page_size : 0;
             for (int v = 0; v < 2 && ok; ++v, ++n) {
               const int s = n % STAGES, use = n / STAGES;
               uint8_t* dst = ring + s * L::KBYTES;
@@ -273,7 +295,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               uint64_t* bar = last ? tail : &full[s];
               if (lane == 0) tc::mbar_expect_tx(bar, L::KBYTES);
               __syncwarp();
-              if (mine) tc::tma_load_2d(dst + c * L::BLOCK + box * a.box_rows * 128, v ? &map_v : &map_k, c * 64, row, bar);
+              if (boxes) tc::tma_load_2d(dst + box_col / 64 * L::BLOCK + box * a.box_rows * 128, v ? &map_v : &map_k, box_col, row, bar);
+              if (v == 0 && j == job.begin) publish();       // the first K is under way
               if (last) {
                 if (!tc::mbar_wait_warp(tail, tails & 1)) {
                   if (lane == 0) atomicExch(a.status, 53);
@@ -290,7 +313,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 if (lane == 0) tc::mbar_arrive(&full[s]);
               }
             }
-            row = next;
+            page = next;
           }
         }
         if (ok) bid();
@@ -324,7 +347,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         for (int i = 0; i < 2; ++i) {
           x_begin[i] = tc::uniform(job.x[i].begin);
           x_end[i] = tc::uniform(job.x[i].end);
-          x_first[i] = tc::uniform(first_visible(a, job.x[i].p_first));
+          x_first[i] = tc::uniform(job.x[i].first);
           x_last[i] = tc::uniform(job.x[i].p_last);
         }
         __syncwarp();
@@ -512,10 +535,6 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         break;
       }
       tc::fence_after();
-      uint32_t o[HD / 32][32];
-#pragma unroll
-      for (int c = 0; c < HD / 32; ++c) tc::ld32_nowait(o_addr + 32 * c, o[c]);
-      tc::wait_ld();
       if (a.key_splits > 1) {
         // this share of the keys only: the row as it is, with its maximum and sum, for the merge
         const size_t at = ((size_t)(x.tok0 + r) * a.nh + x.head) * a.key_splits + piece;
@@ -523,34 +542,41 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           a.part_ml[at * 2] = m == -INFINITY ? -INFINITY : m * 0.6931471805599453f;
           a.part_ml[at * 2 + 1] = l;
         }
+#pragma unroll 1
+        for (int c = 0; c < HD; c += 32) {
+          uint32_t o[32];
+          tc::ld32_nowait(o_addr + c, o);
+          tc::wait_ld();
 #pragma unroll
-        for (int c = 0; c < HD / 16; ++c) {
-          uint4 v[4];
+          for (int h = 0; h < 32; h += 16) {
+            uint4 v[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            v[e] = make_uint4(o[c / 2][c % 2 * 16 + 4 * e], o[c / 2][c % 2 * 16 + 4 * e + 1], o[c / 2][c % 2 * 16 + 4 * e + 2],
-                              o[c / 2][c % 2 * 16 + 4 * e + 3]);
-          trade_rows(v, lane);
+            for (int e = 0; e < 4; ++e) v[e] = make_uint4(o[h + 4 * e], o[h + 4 * e + 1], o[h + 4 * e + 2], o[h + 4 * e + 3]);
+            trade_rows(v, lane);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int row = (r & ~3) + e;
-            if (row < x.n_valid)
-              *reinterpret_cast<uint4*>(a.part_acc + (((size_t)(x.tok0 + row) * a.nh + x.head) * a.key_splits + piece) * HD + 16 * c +
-                                        4 * (lane & 3)) = v[e];
+            for (int e = 0; e < 4; ++e) {
+              const int to = (r & ~3) + e;
+              if (to < x.n_valid)
+                *reinterpret_cast<uint4*>(a.part_acc + (((size_t)(x.tok0 + to) * a.nh + x.head) * a.key_splits + piece) * HD + c + h +
+                                          4 * (lane & 3)) = v[e];
+            }
           }
         }
       } else {
         if (a.sink && l > 0.f) l += exp2f((a.sink_values ? a.sink_values[x.head] * 1.4426950408889634f : 0.f) - m);
         const float inv = l > 0.f ? 1.f / l : 0.f;
-#pragma unroll
-        for (int c = 0; c < HD / 32; ++c) {
+#pragma unroll 1
+        for (int c = 0; c < HD; c += 32) {
+          uint32_t o[32];
+          tc::ld32_nowait(o_addr + c, o);
+          tc::wait_ld();
           uint4 v[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             uint32_t u[4];
 #pragma unroll
             for (int f = 0; f < 4; ++f) {
-              __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(o[c][8 * e + 2 * f]) * inv, __uint_as_float(o[c][8 * e + 2 * f + 1]) * inv);
+              __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(o[8 * e + 2 * f]) * inv, __uint_as_float(o[8 * e + 2 * f + 1]) * inv);
               u[f] = *reinterpret_cast<uint32_t*>(&hh);
             }
             v[e] = make_uint4(u[0], u[1], u[2], u[3]);
@@ -558,9 +584,9 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           trade_rows(v, lane);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int row = (r & ~3) + e;
-            if (row < x.n_valid)
-              *reinterpret_cast<uint4*>(a.out + ((size_t)(x.tok0 + row) * a.nh + x.head) * HD + 32 * c + 8 * (lane & 3)) = v[e];
+            const int to = (r & ~3) + e;
+            if (to < x.n_valid)
+              *reinterpret_cast<uint4*>(a.out + ((size_t)(x.tok0 + to) * a.nh + x.head) * HD + c + 8 * (lane & 3)) = v[e];
           }
         }
       }

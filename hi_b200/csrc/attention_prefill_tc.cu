@@ -1,6 +1,7 @@
 // Prefill attention on the 5th-generation tensor cores (tcgen05), bfloat16: portions of prompts of
-// at least a tile of new tokens against the paged cache. One block = 128 consecutive new tokens
-// of one request and one query head:
+// at least a tile of new tokens against the paged cache. Plain softmax rows of 64 and 128 values go two query tiles a block
+// (attention_prefill_pair.cu); here are rows of 192, reshaped scores, kept first tokens, sigmoid weights and differential
+// attention. One block = 128 consecutive new tokens of one request and one query head:
 //   warp 0      one lane issues TMA loads: the Q tile once, then K and V tiles of 64 key positions
 //               (one box per page, 128-byte swizzle): K into a ring of three and a tile ahead of V,
 //               V into a ring of two (a load takes about as long as a tile's work, so with two

@@ -1974,10 +1974,16 @@ def prefill_pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window
     takes the next pair when it is done). A key tile of 128 takes 1.73 us (rows of 64: 1.52), a pair half a tile more. The heaviest start
     first, so a launch takes the most of: all tiles over all SMs, the longest block, and for every n the n + 1 that some SM has to
     take of the first n * SMs + 1 blocks. Shared rows are written and read in float32 and merged in a launch of its own; shares must
-    save 7 %. Fitted to 3,745 launches (1 to 3 portions of 64 to 2,048 tokens behind up to 65,000) in 1 to 8 shares: 5 % off on
+    save 7 % and 8 us, for the launch and two tensors more cost the host about 12 (eager calls, 128 tokens behind 500, 8 heads: 17
+    and 30 us). Fitted to 3,745 launches (1 to 3 portions of 64 to 2,048 tokens behind up to 65,000) in 1 to 8 shares: 5 % off on
     average; what it chooses takes 0.856 of the time of one share and 1.006 of the best. 40 heads of 128, us in one share and as
     chosen: 128 tokens behind 7,000 101 -> 33, 1,024 behind 16,384 438 -> 336, 150 behind 9,000 beside 700 behind 300 127 -> 85;
     2,048 alone stay in one (50, in two 99)."""
+    return _pair_shares(tuple(portions), nh, nkv, hd, chunk, window, rows, sms, least)
+
+
+@functools.lru_cache(maxsize=256)                  # a step's layers ask the same
+def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, rows: int, sms: int, least: int) -> int:
     runs = []                           # (key tiles, blocks), eight runs a portion at most
 
     def visible(first):
@@ -1993,11 +1999,9 @@ def prefill_pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window
             first, last = (a + b - 1) // group, min(a + b, items - 1) // group
             end = min(cached + 128 * (last + 1), cached + new) - 1
             runs.append((end // 128 - visible(cached + 128 * first) // 128 + 1, (b - a) * nkv))
-    return _fewest_pair_us(tuple(runs), rows * nh * hd, hd, sms, least) if runs else 1
-
-
-@functools.lru_cache(maxsize=256)                  # a step's layers ask the same
-def _fewest_pair_us(runs, numbers: int, hd: int, sms: int, least: int) -> int:
+    if not runs:
+        return 1
+    numbers = rows * nh * hd
     fixed, tile, merge, share, whole = (7.75, 1.515, 1.46, 0.6, 6.2) if hd <= 64 else (8.4, 1.73, 1.27, 0.63, 4.05)
 
     def cost(k):
@@ -2011,7 +2015,7 @@ def _fewest_pair_us(runs, numbers: int, hd: int, sms: int, least: int) -> int:
         return fixed + tile * most + (merge + (share * k + whole) * numbers / 1e6 if k > 1 else 0.0)
 
     best = min((k for k in (1, 2, 3, 4, 6, 8) if k >= least), key=cost)
-    return best if least > 1 or cost(best) < 0.93 * cost(1) else 1
+    return best if least > 1 or cost(best) < min(0.93 * cost(1), cost(1) - 8.0) else 1
 
 
 # --------------------------------------------------------------------------- experts

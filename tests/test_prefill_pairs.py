@@ -1,0 +1,93 @@
+"""The tcgen05 prefill attention of two query tiles a block: where pairs, tiles, steps of 16 keys and shares of the keys end."""
+import pytest
+import torch
+
+from hi_b200.kernels import ops
+
+DEV = "cuda:0"
+
+
+def reference(q, k, v, starts, lens, chunk, window, scale, sinks):
+    out, at = torch.zeros(q.shape, dtype=torch.float64), 0
+    group = q.shape[1] // k[0].shape[1]
+    for s, (c, n) in enumerate(zip(starts, lens)):
+        pos, key = torch.arange(c, c + n).view(-1, 1), torch.arange(c + n).view(1, -1)
+        hidden = key > pos
+        if chunk:
+            hidden |= key < pos // chunk * chunk
+        if window:
+            hidden |= key <= pos - window
+        for h in range(q.shape[1]):
+            kk, vv = (x[s][:, h // group].double() for x in (k, v))
+            scores = (q[at: at + n, h].double() @ kk.t() * scale).masked_fill(hidden, float("-inf"))
+            if sinks is not None:
+                scores = torch.cat([scores, sinks[h].double().expand(n, 1)], dim=1)
+                vv = torch.cat([vv, torch.zeros(1, vv.shape[1], dtype=torch.float64)])
+            out[at: at + n, h] = torch.softmax(scores, 1) @ vv
+        at += n
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nh,nkv,hd,page,chunk,window,lens,starts,sink", [
+    (5, 1, 128, 64, 0, 0, [300, 128, 1, 129], [0, 37, 500, 127], False),        # odd groups: a pair of two tiles; single items
+    (3, 3, 128, 16, 0, 0, [257, 1], [128, 3], True),                            # a group of one: pairs of tiles of one head
+    (2, 1, 64, 64, 0, 0, [128], [0], False),                                    # one block
+    (10, 2, 64, 32, 300, 0, [385, 140, 17], [250, 299, 300], False),            # chunks that start inside tiles and steps
+    (4, 2, 128, 64, 0, 100, [260, 131], [700, 0], False),                       # windows: pages before them were given back
+    (40, 8, 64, 128, 0, 0, [700, 400, 513, 2], [0, 260, 5, 900], False),        # more pairs than SMs: blocks take another
+])
+def test_pairs_of_query_tiles(nh, nkv, hd, page, chunk, window, lens, starts, sink):
+    g = torch.Generator().manual_seed(nh * hd + page)
+    total, S = [c + n for c, n in zip(starts, lens)], len(lens)
+    k, v = ([torch.randn(t, nkv, hd, generator=g).bfloat16() for t in total] for _ in range(2))
+    q = torch.randn(sum(lens), nh, hd, generator=g).bfloat16()
+    need = [-(-t // page) for t in total]
+    pages = torch.randperm(sum(need), generator=g).int()
+    # whatever no token may read holds NaN: the rows behind a request's end, and page 0's stand-in for pages given back
+    kp, vp = (torch.full((sum(need) + 1, nkv, page, hd), float("nan"), dtype=torch.bfloat16) for _ in range(2))
+    table, at = torch.full((S, max(need)), -1, dtype=torch.int32), 0
+    for s in range(S):
+        first = starts[s] // chunk * chunk if chunk else max(0, starts[s] - window + 1) if window else 0
+        for b in range(need[s]):
+            slot = int(pages[at + b]) + 1
+            here = slice(b * page, min((b + 1) * page, total[s]))
+            kp[slot, :, : here.stop - here.start], vp[slot, :, : here.stop - here.start] = (x[s][here].transpose(0, 1) for x in (k, v))
+            if (b + 1) * page > first:
+                table[s, b] = slot
+        at += need[s]
+    cu = torch.tensor([0] + lens).cumsum(0).int()
+    pos = torch.cat([torch.arange(c, c + n) for c, n in zip(starts, lens)]).int()
+    sinks = torch.randn(nh, generator=g) if sink else None
+    want = reference(q, k, v, starts, lens, chunk, window, hd ** -0.5, sinks)
+    dev = lambda x: None if x is None else x.to(DEV)
+    assert ops.prefill_pairs(hd)
+    for splits in (1, 2, 5):
+        got = ops.prefill_attention_tc(dev(q), dev(kp), dev(vp), dev(table), dev(cu), dev(pos), S, max(lens), chunk, window, hd ** -0.5,
+                                       key_splits=splits, sink_values=dev(sinks))
+        ops.check_tc_status()
+        # P in bfloat16 (2^-9 of each weight, weights that sum to one) and the output's own rounding, on values of a few units
+        err = float((got.double().cpu() - want).abs().max())
+        assert err <= 2e-2, (splits, err)
+        if 1 not in lens:
+            continue
+        out = torch.full_like(dev(q), 7.0)
+        ops.prefill_attention_tc(dev(q), dev(kp), dev(vp), dev(table), dev(cu), dev(pos), S, max(lens), chunk, window, hd ** -0.5,
+                                 key_splits=splits, sink_values=dev(sinks), skip_single=True, out=out)
+        ops.check_tc_status()
+        alone = int(cu[lens.index(1)])
+        rest = [i for i in range(q.shape[0]) if i != alone]
+        assert torch.equal(out[rest], got[rest])
+        if splits == 1:
+            assert bool((out[alone] == 7.0).all()), "a single token is left to the decode kernel"
+
+
+@pytest.mark.parametrize("portions,nh,nkv,hd,chunk,window,least,want", [
+    ([(0, 2048)], 40, 8, 128, 0, 0, 1, {1}), ([(7000, 128)], 40, 8, 128, 8192, 0, 1, {4, 6, 8}), ([(0, 128)], 8, 2, 64, 0, 0, 1, {1}),
+    ([(0, 2048)], 40, 8, 128, 0, 0, 2, {2, 3, 4, 6, 8}), ([(9000, 150), (300, 700)], 40, 8, 128, 0, 0, 1, {2, 3, 4}),
+    ([(100000, 128)], 16, 4, 128, 0, 64, 1, {1}), ([], 40, 8, 128, 0, 0, 1, {1}), ([(500, 128)], 8, 2, 128, 0, 0, 1, {1}),
+    ([(20000, 4096)], 24, 24, 64, 0, 0, 1, {1}), ([(65000, 200)], 1, 1, 64, 0, 0, 1, {6, 8})])
+def test_shares_of_pairs(portions, nh, nkv, hd, chunk, window, least, want):
+    """Prompts from the start, short launches and those that fill the GPU stay in one share; few long pairs are shared out."""
+    rows = sum(n for _c, n in portions)
+    assert ops.prefill_pair_shares(portions, nh, nkv, hd, chunk, window, rows, 148, least) in want
