@@ -11,10 +11,10 @@
 // decode-sized steps a tile holds at most 64 tokens (8 KB) and the ring is five / eight stages
 // deep (measured at 64 tokens over 16 experts: 427 -> 415 us and 235 -> 222 us).
 // Persistent blocks (one per SM) walk the tiles (expert, 128 features, up to 192 tokens):
-//   warp 0      one lane issues the TMA loads (W tile 128x64, twice when DUAL; X tile of 32, 64,
+//   warp 0      issues the TMA loads (W tile 128x64, twice when DUAL; X tile of 32, 64,
 //               128 or 192 rows x 64; 128-byte swizzle) into a ring of stages, signalled by
 //               mbarrier transaction counts;
-//   warp 1      allocates tensor memory; one lane issues tcgen05.mma (M 128, N tokens, K 16, four
+//   warp 1      allocates tensor memory; issues tcgen05.mma (M 128, N tokens, K 16, four
 //               per stage and weight stack) and tcgen05.commit, which frees the stage / publishes
 //               the accumulator;
 //   warps 2..9  read the accumulator back with tcgen05.ld (each warp 32 lanes = 32 features, the
@@ -25,6 +25,9 @@
 //            scales the expert input, which is the same by linearity), or with `limit` > 0 the clamped
 //            unit min(g, limit) sigmoid(1.702 .) (clamp(u) + 1);
 //     else   the float32 product (down projection).
+// Both of these warps walk their loops together and one lane of them issues: alone in its loop, the lane moved every product's
+// descriptors to the uniform registers first, some 40 cycles a product of 96 (2,048 tokens, 2 of 8 experts of 2,048 x 4,096, gather
+// included: 150 -> 134 us, down 80 -> 73; 4 of 16 of 1,024 x 2,048: 105 -> 90, 51 -> 47; 64 tokens, 16 of 5,120 x 8,192: 390 -> 386).
 // Tensor memory is two slots of 256 columns. A tile takes one slot, and the next tile
 // accumulates into the other while this one is written out; only a DUAL tile of more than 128
 // tokens needs both (gate in one, up in the other), and its epilogue gives them back as soon as
@@ -183,7 +186,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
   int* s_last = reinterpret_cast<int*>(tmem_slot + 2);      // whether this block's piece arrived last
   int* s_offsets = s_last + 1;                              // [experts + 1]: the tile search never waits on global memory
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   for (int e = threadIdx.x; e <= p.experts; e += THREADS) s_offsets[e] = p.offsets[e];
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
@@ -203,64 +206,74 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
   const int num_kb = (p.K + BK - 1) / BK;
   const WorkList<BT> list(s_offsets, p.experts, f_tiles, num_kb, !DUAL && p.scratch != nullptr);
 
-  if (warp == 0) {
-    if (lane == 0) {                            // ---- TMA producer
-      uint32_t it = 0;                          // stages filled so far, over all tiles
-      bool ok = true;
-      Work work;
-      for (int i = 0; ok && list.get(i, work); ++i) {
-        const Tile& tile = work.tile;
-        const int box = tile.tokens <= 32 ? 0 : (tile.tokens <= 64 ? 1 : (tile.tokens <= 128 ? 2 : 3));
-        const uint32_t bytes = NW * W_BYTES + (uint32_t)x_box_rows(box, BT) * BK * 2;
-        const int w_row = tile.expert * p.n_out + tile.f0;
-        for (int kb = work.kb0; kb < work.kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          if (it >= STAGES && !tc::mbar_wait(&empty[s], ((it / STAGES) - 1) & 1)) { atomicExch(p.status, 1); ok = false; break; }
+  if (warp == 0) {                              // ---- TMA producer: the whole warp waits, one lane issues
+    int s = 0, turn = 1;                        // (the first wait on a fresh barrier for the phase before it returns at once)
+    bool ok = true;
+    Work work;
+    for (int i = 0; ok && list.get(i, work); ++i) {
+      const Tile& tile = work.tile;
+      const int box = tile.tokens <= 32 ? 0 : (tile.tokens <= 64 ? 1 : (tile.tokens <= 128 ? 2 : 3));
+      const uint32_t bytes = NW * W_BYTES + (uint32_t)x_box_rows(box, BT) * BK * 2;
+      const int w_row = tile.expert * p.n_out + tile.f0;
+      for (int kb = work.kb0; kb < work.kb1; ++kb) {
+        if (!tc::mbar_wait_warp(&empty[s], turn)) {
+          if (lane == 0) atomicExch(p.status, 1);
+          ok = false;
+          break;
+        }
+        if (lane == 0) {
           uint8_t* st = smem + s * STAGE_BYTES;
           tc::mbar_expect_tx(&full[s], bytes);
           tc::tma_load_2d(st, &maps.w0, kb * BK, w_row, &full[s]);
           if (DUAL) tc::tma_load_2d(st + W_BYTES, &maps.w1, kb * BK, w_row, &full[s]);
           tc::tma_load_2d(st + NW * W_BYTES, &maps.x[box], kb * BK, tile.row0, &full[s]);
         }
+        __syncwarp();
+        if (++s == STAGES) { s = 0; turn ^= 1; }
       }
     }
-  } else if (warp == 1) {
-    if (lane == 0) {                            // ---- MMA issuer
-      uint32_t it = 0;
-      SlotWalk walk;
-      bool ok = true;
-      Work work;
-      for (int i = 0; ok && list.get(i, work); ++i) {
-        const Tile& tile = work.tile;
-        bool both;
-        const int b = walk.take(DUAL, tile.tokens, both);
-        for (int q = b; ok && q <= (both ? 1 : b); ++q)      // the slot(s) must have been written out
-          if (walk.use[q] > 0 && !tc::mbar_wait(&acc_empty[q], (walk.use[q] - 1) & 1)) { atomicExch(p.status, 4); ok = false; }
-        if (!ok) break;
-        tc::fence_after();
-        const uint32_t idesc = tc::idesc_bf16(BF, (tile.tokens + 15) & ~15, false);
-        const uint32_t acc = tmem + b * SLOT_COLS;
-        const uint32_t up_off = both ? SLOT_COLS : DUAL_SLOT_T;  // where the second accumulator starts
-        const int kb0 = work.kb0;
-        for (int kb = kb0; kb < work.kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          if (!tc::mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(p.status, 2); ok = false; break; }
-          tc::fence_after();
-          const uint32_t w_addr = tc::smem_u32(smem + s * STAGE_BYTES);
-          const uint32_t x_addr = w_addr + NW * W_BYTES;
-#pragma unroll
-          for (int k = 0; k < BK / UK; ++k) {
-            const uint64_t xd = tc::desc_kmajor(x_addr + k * UK * 2);
-            tc::mma(acc, tc::desc_kmajor(w_addr + k * UK * 2), xd, idesc, (kb - kb0) | k);
-            if (DUAL) tc::mma(acc + up_off, tc::desc_kmajor(w_addr + W_BYTES + k * UK * 2), xd, idesc, (kb - kb0) | k);
-          }
-          tc::commit(&empty[s]);                 // the stage is free once these MMAs have read it
+  } else if (warp == 1) {                       // ---- MMA issuer: the whole warp walks, one lane issues
+    const uint32_t mine = tc::elect_one();
+    const uint64_t ring = tc::desc_kmajor(tc::smem_u32(smem));
+    int s = 0, turn = 0;
+    SlotWalk walk;
+    bool ok = true;
+    Work work;
+    for (int i = 0; ok && list.get(i, work); ++i) {
+      const int tokens = tc::uniform(work.tile.tokens), kbs = tc::uniform(work.kb1 - work.kb0);
+      bool both;
+      const int b = walk.take(DUAL, tokens, both);
+      for (int q = b; ok && q <= (both ? 1 : b); ++q)      // the slot(s) must have been written out
+        if (walk.use[q] > 0 && !tc::mbar_wait_warp(&acc_empty[q], (walk.use[q] - 1) & 1)) {
+          if (lane == 0) atomicExch(p.status, 4);
+          ok = false;
         }
-        // this tile's accumulator is complete (also on the error path)
-        tc::commit(&acc_full[b]);
-        ++walk.use[b];
-        if (both) { tc::commit(&acc_full[1]); ++walk.use[1]; }
+      if (!ok) break;
+      tc::fence_after();
+      const uint32_t idesc = tc::idesc_bf16(BF, (tokens + 15) & ~15, false);
+      const uint32_t acc = tmem + b * SLOT_COLS;
+      const uint32_t up = acc + (both ? SLOT_COLS : DUAL_SLOT_T);  // where the second accumulator starts
+      for (int kb = 0; kb < kbs; ++kb) {
+        if (!tc::mbar_wait_warp(&full[s], turn)) {
+          if (lane == 0) atomicExch(p.status, 2);
+          ok = false;
+          break;
+        }
+        tc::fence_after();
+        const uint64_t w = ring + s * (STAGE_BYTES >> 4), x = w + (NW * W_BYTES >> 4);
+#pragma unroll
+        for (int k = 0; k < BK / UK; ++k) {
+          const uint32_t more = kb | k;
+          tc::mma_if(mine, acc, w + (k * UK * 2 >> 4), x + (k * UK * 2 >> 4), idesc, more);
+          if (DUAL) tc::mma_if(mine, up, w + ((W_BYTES + k * UK * 2) >> 4), x + (k * UK * 2 >> 4), idesc, more);
+        }
+        tc::commit_if(mine, &empty[s]);          // the stage is free once these MMAs have read it
+        if (++s == STAGES) { s = 0; turn ^= 1; }
       }
+      // this tile's accumulator is complete (also on the error path)
+      tc::commit_if(mine, &acc_full[b]);
+      ++walk.use[b];
+      if (both) { tc::commit_if(mine, &acc_full[1]); ++walk.use[1]; }
     }
   } else {                                      // ---- epilogue: warps 2..9
     const int quarter = warp & 3;               // the lanes of tensor memory this warp may read
@@ -283,9 +296,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
         const int tk = half * 32 + q * 64 + lane;
         my_score[q] = (DUAL && tk < tile.tokens) ? p.scores[p.sorted_entry[tile.row0 + tk]] : 1.f;
       }
-      bool waited = tc::mbar_wait(&acc_full[b], walk.use[b] & 1);
-      if (both) waited = tc::mbar_wait(&acc_full[1], walk.use[1] & 1) && waited;
-      if (!__all_sync(0xffffffffu, waited)) {
+      if (!tc::mbar_wait_warp(&acc_full[b], walk.use[b] & 1) || (both && !tc::mbar_wait_warp(&acc_full[1], walk.use[1] & 1))) {
         if (lane == 0) atomicExch(p.status, 3);
         ok = false;
         break;
