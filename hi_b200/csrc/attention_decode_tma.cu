@@ -2,10 +2,13 @@
 // the same flash-decoding as attention_decode.cu (grid (split, kv head, token); the query heads
 // of a kv head are the rows of one 16-row tile; mma.sync m16n8k16 with float32 accumulation and
 // softmax; four warps of 16 keys each per 64-key tile; partials merged by attention_merge), but
-// one thread issues a tile's loads as a few tensor-map copies (a page's 64 rows x 64 dims per
-// copy, 128-byte swizzle) that an mbarrier counts, instead of every thread issuing sixteen
+// a fifth warp brings a tile in as a few tensor-map copies (a page's 64 rows x 64 dims per
+// copy and lane, 128-byte swizzle) that an mbarrier counts, instead of every thread issuing sixteen
 // 16-byte cp.async with their address arithmetic. ldmatrix reads the swizzled tiles (16-byte
-// chunk c of row r sits at chunk c ^ (r % 8)).
+// chunk c of row r sits at chunk c ^ (r % 8)). A computing warp reads its own 16 keys of a tile only, so the warps meet
+// at the tiles' barriers and not at one another: with a thread of theirs that looked up the pages and issued the loads, and two
+// block barriers a tile, a tile of a block alone took 1.05 us, now 0.65 (one token of 16,064 keys in one split 291 -> 178 us, of
+// 1,000 in four 11.1 -> 9.9; 64 uneven ones of up to 4,000, 40 heads on 8, 102.5 -> 97.3 with the splits chosen for it).
 //
 // Takes what the tile loads need: pages of 16, 32 or a multiple of 64 positions, and ranges that
 // start on a multiple of 64 (no sliding window; a chunk size that is a multiple of 64). Rows of a
@@ -17,7 +20,7 @@
 // Where a token has 2 to 8 splits and all clusters run at once, its splits are a cluster: every block keeps its rows in shared
 // memory and the blocks of the cluster share out the merge among themselves, reading one another's (the caller gives no
 // part_acc / part_ml then). What that saves is a launch, its gap and the partial rows' way through memory: one token of 1,000
-// keys, 40 heads of 128: 12.7 -> 11.5 us, of 300 keys 12.1 -> 9.6 us; with one cluster more than run at once it takes 1.2 to 1.5
+// keys, 40 heads of 128: 12.7 -> 11.5 us, of 300 keys 12.1 -> 9.6 us (before the tiles had a warp of their own); with one cluster more than run at once it takes 1.2 to 1.5
 // times as long as with the merge (ops.decode_attention has the rule and both sides).
 //
 // The fused form (hb_attention_decode_fused) takes the q/k/v projection's output as it is and
@@ -40,9 +43,14 @@
 namespace {
 
 constexpr int TILE = 64;     // keys per shared-memory tile
-constexpr int NWARPS = 4;
+constexpr int NWARPS = 4;    // that compute; one more warp brings the tiles in
+constexpr int COMP = NWARPS * 32;
 constexpr int ROWS = 16;     // query rows of the tile (heads of one kv group, padded)
-constexpr int STAGES = 2;     // measured: three stages (two blocks per SM instead of three) are no faster
+// Tiles in flight and blocks an SM: rows of 128 two and three (three and two blocks are as fast where each has its best split), rows of
+// 64 three and four, or two and five where a split has no more than two tiles (us, two and five / three and four: 16 tokens of 4,000
+// keys, 40 heads on 8, 26.0 / 22.8; 10 of 10,000, 8 on 2, 15.7 / 13.9, 32 on 8 31.8 / 36.3; 30 of 108, 24 on 24, 8.6 / 10.8).
+template <int HD> constexpr int STAGES_OF = HD == 128 ? 2 : 3;
+template <int HD, int STAGES> constexpr int BLOCKS_OF = HD == 128 ? 3 : STAGES == 2 ? 5 : 4;
 constexpr int HALF_BYTES = TILE * 128;   // a tile's 64 rows x 64 dims (128 bytes a row)
 
 struct Args {
@@ -178,6 +186,17 @@ __device__ __forceinline__ uint32_t tile_offset(int r, int d) {
 enum Merge { APART, FUSED_FORM, CLUSTER };
 constexpr int MAX_CLUSTER = 8;
 
+// a barrier of the computing warps; and one over which they agree
+__device__ __forceinline__ void comp_sync() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(COMP) : "memory"); }
+__device__ __forceinline__ bool comp_and(bool x) {
+  uint32_t all;
+  asm volatile(
+      "{\n.reg .pred p, q;\n"
+      "setp.ne.u32 q, %1, 0;\n"
+      "barrier.cta.red.and.pred p, 1, %2, q;\n"
+      "selp.u32 %0, 1, 0, p;\n}" : "=r"(all) : "r"((uint32_t)x), "n"(COMP) : "memory");
+  return all != 0;
+}
 __device__ __forceinline__ void cluster_sync() {      // of the blocks that have not left
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -197,8 +216,8 @@ __device__ __forceinline__ float4 load4_cluster(uint32_t at) {
   return v;
 }
 
-template <int HD, Merge MERGE>
-__global__ void __launch_bounds__(NWARPS * 32)
+template <int HD, int STAGES, Merge MERGE>
+__global__ void __launch_bounds__(COMP + 32, (BLOCKS_OF<HD, STAGES>))
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Args a,
                        const Fuse f) {
   constexpr bool FUSED = MERGE == FUSED_FORM;
@@ -213,14 +232,15 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(v_s + STAGES * KV_BYTES);   // [ROWS][STRIDE]
   float* ml_s = reinterpret_cast<float*>(q_s + ROWS * STRIDE);  // [NWARPS][ROWS][2]
   uint64_t* full = reinterpret_cast<uint64_t*>(ml_s + NWARPS * ROWS * 2);           // [STAGES]
-  float* cs_s = reinterpret_cast<float*>(full + STAGES);        // [HD / 2] cosines, [HD / 2] sines (fused form)
+  uint64_t* empty = full + STAGES;                              // [STAGES]
+  float* cs_s = reinterpret_cast<float*>(empty + STAGES);       // [HD / 2] cosines, [HD / 2] sines (fused form)
   float* sn_s = cs_s + HD / 2;
   float* o_s = reinterpret_cast<float*>(k_s);    // [ROWS][HD], reuses the K tiles once the key loop is over
   __shared__ int last_block;
   __shared__ float2 block_ml[MERGE == CLUSTER ? ROWS : 1];      // cluster form: the block's maxima and sums
 
   const int split = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tc::uniform(tid >> 5);
   const int G = a.nh / a.nkv;
   const long long row = a.rows ? a.rows[t] : t;
   if (a.rows && (row < 0 || row >= a.step_tokens)) {          // (all blocks of a cluster are of one token)
@@ -242,7 +262,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if (first > pos) {                                          // this token has fewer splits
     if (MERGE == CLUSTER) {                                   // (the barrier of a cluster counts the threads still there)
       if (split == 0)
-        for (int i = tid; i < G * HD; i += NWARPS * 32) a.out[qh0 * HD + i] = __float2bfloat16_rn(0.f);
+        for (int i = tid; i < G * HD; i += COMP + 32) a.out[qh0 * HD + i] = __float2bfloat16_rn(0.f);
     } else if (!merge_inside && a.max_splits > 1 && tid < G) {
       float* ml = a.part_ml + ((th0 + tid) * a.max_splits + split) * 2;
       ml[0] = -INFINITY; ml[1] = 0.f;
@@ -252,36 +272,46 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int last = min(pos, first + a.split_size - 1);
   const int n_tiles = (last - first + TILE) / TILE;
 
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) tc::mbar_init(&full[s], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  // One thread issues a tile: for every page under the tile (one, or 64 / page_size of them) that
-  // holds a key of the range, the page's rows of K and of V, 64 dims per copy.
-  auto issue = [&](int tile, int stage) {
-    const int base = first + tile * TILE;
-    const int rows_per_box = a.box_rows;           // min(page_size, 64)
-    uint32_t bytes = 0;
-    for (int r0 = 0; r0 < TILE; r0 += rows_per_box)
-      if (base + r0 <= last && table[(base + r0) / a.page_size] >= 0) bytes += 2u * HALVES * rows_per_box * 128;
-    tc::mbar_expect_tx(&full[stage], bytes);
-    for (int r0 = 0; r0 < TILE; r0 += rows_per_box) {
-      const int key = base + r0;
-      if (key > last) break;
-      const int page = table[key / a.page_size];
-      if (page < 0) continue;
-      const int row = (page * a.nkv + kvh) * a.page_size + key % a.page_size;
-#pragma unroll
-      for (int h = 0; h < HALVES; ++h) {
-        tc::tma_load_2d(k_s + stage * KV_BYTES + h * HALF_BYTES + r0 * 128, &map_k, h * 64, row, &full[stage]);
-        tc::tma_load_2d(v_s + stage * KV_BYTES + h * HALF_BYTES + r0 * 128, &map_v, h * 64, row, &full[stage]);
-      }
+  // The last warp brings the tiles in: for every page under a tile (one, or 64 / page_size of them) that holds a key of the range,
+  // the page's rows of K and of V, 64 dims per copy and lane. The ids of 32 pages are asked for at a time.
+  if (warp == NWARPS) {
+    if (lane == 0) {
+      for (int s = 0; s < STAGES; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], NWARPS); }
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-  };
-  // the first tiles are on their way while the query rows are made ready (the thread that
-  // initialised the barriers issues them, so it needs no one else to have seen the barriers yet)
-  if (tid == 0)
-    for (int i = 0; i < STAGES - 1 && i < n_tiles; ++i) issue(i, i);
+    const int boxes = TILE / a.box_rows;           // box_rows: min(page_size, 64)
+    const int box = lane / (2 * HALVES), half = lane % HALVES, is_v = lane / HALVES % 2;    // of this lane's copy
+    auto page_of = [&](int n) {                    // of box n of the range
+      const int key = first + n * a.box_rows;
+      return key <= last ? table[key / a.page_size] : -1;
+    };
+    int pages = page_of(lane);
+    bool ok = true;
+    __syncwarp();
+    for (int tile = 0; tile < n_tiles; ++tile) {
+      const int s = tile % STAGES, n = tile * boxes;
+      if (n % 32 == 0 && n > 0) pages = page_of(n + lane);
+      const int page = __shfl_sync(0xffffffffu, pages, (n + box) % 32);
+      if (tile >= STAGES && !tc::mbar_wait_warp(&empty[s], (tile / STAGES - 1) & 1)) {
+        if (lane == 0) atomicExch(a.status, 31);
+        ok = false;
+        break;
+      }
+      const bool mine = box < boxes && page >= 0;
+      const uint32_t copies = __popc(__ballot_sync(0xffffffffu, mine));
+      if (lane == 0) tc::mbar_expect_tx(&full[s], copies * a.box_rows * 128);
+      __syncwarp();
+      if (mine) {
+        const int at = first + tile * TILE + box * a.box_rows;
+        tc::tma_load_2d((is_v ? v_s : k_s) + s * KV_BYTES + half * HALF_BYTES + box * a.box_rows * 128, is_v ? &map_v : &map_k,
+                        half * 64, (page * a.nkv + kvh) * a.page_size + at % a.page_size, &full[s]);
+      }
+      if (tile == min(n_tiles, STAGES) - 1) __syncthreads();         // the others may wait on the barriers
+    }
+    // no copy is under way when the block ends, whoever gave up
+    for (int tile = max(0, n_tiles - STAGES); ok && tile < n_tiles; ++tile) tc::mbar_wait_warp(&full[tile % STAGES], (tile / STAGES) & 1);
+    return;
+  }
 
   // the query rows of this kv group
   uint4 own_c0 = make_uint4(0u, 0u, 0u, 0u), own_c1 = own_c0;   // fused: this lane's part of the token's own key or value
@@ -290,15 +320,15 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if constexpr (FUSED) {
     constexpr int LPH = HD / 16, HPW = 32 / LPH;
     if (f.inv_freq != nullptr)
-      for (int j = tid; j < f.rot_pairs; j += NWARPS * 32) {
+      for (int j = tid; j < f.rot_pairs; j += COMP) {
         float sn, cs;
         sincosf((float)pos * f.inv_freq[j], &sn, &cs);
         sn_s[j] = sn * f.rot_mul;
         cs_s[j] = cs * f.rot_mul;
       }
-    for (int c = tid; c < (ROWS - G) * CHUNKS; c += NWARPS * 32)      // the tile's rows past the group are zeros
+    for (int c = tid; c < (ROWS - G) * CHUNKS; c += COMP)      // the tile's rows past the group are zeros
       *reinterpret_cast<uint4*>(q_s + (G + c / CHUNKS) * STRIDE + (c % CHUNKS) * 8) = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();                               // sines and cosines; the barriers are initialised
+    comp_sync();                                   // sines and cosines
     const __nv_bfloat16* row = f.qkv + (size_t)t * (a.nh + (f.v_is_k ? 1 : 2) * a.nkv) * HD;
     const int sub = lane % LPH, slot = warp * HPW + lane / LPH;     // NWARPS * HPW = 16 head slots
     {
@@ -311,9 +341,9 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         *reinterpret_cast<uint4*>(q_s + slot * STRIDE + d1) = c1;
       }
     }
-    if (last == pos && warp == 0) {                // this block's range ends at the token itself: its key and value
-      const bool active = slot < 2;
-      const int kind = 1 + (slot & 1);
+    if (last == pos && warp == ((pos - first) % TILE) / 16) {     // the range ends at the token itself: its key and value, by the warp that reads them
+      const bool active = lane / LPH < 2;
+      const int kind = 1 + (lane / LPH & 1);
       const __nv_bfloat16* src = row + (size_t)(a.nh + (kind == 2 && !f.v_is_k ? a.nkv : 0) + kvh) * HD;
       encode_head<HD>(src, kind, active, sub, f, cs_s, sn_s, pos, own_c0, own_c1, own_d0, own_d1);
       own_kv = active;
@@ -326,14 +356,15 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
     }
   } else {
-    for (int c = tid; c < ROWS * CHUNKS; c += NWARPS * 32) {
+    for (int c = tid; c < ROWS * CHUNKS; c += COMP) {
       const int r = c / CHUNKS, ch = c % CHUNKS;
       const bool ok = r < G;
       hb::cp_async16(q_s + r * STRIDE + ch * 8, a.q + (qh0 + (ok ? r : 0)) * HD + ch * 8, ok);
     }
     hb::cp_async_commit();
-    __syncthreads();                               // the barriers are initialised
+    hb::cp_async_wait<0>();
   }
+  __syncthreads();                                 // the query rows; the barriers are initialised
 
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   float o_acc[HD / 8][4];
@@ -346,12 +377,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
   for (int tile = 0; tile < n_tiles; ++tile) {
     const int buf = tile % STAGES;
-    if (tid == 0 && tile + STAGES - 1 < n_tiles)                              // its stage was freed by the last sync
-      issue(tile + STAGES - 1, (tile + STAGES - 1) % STAGES);
-    if (!FUSED && tile == 0) hb::cp_async_wait<0>();                           // the query rows
-    if (!tc::mbar_wait(&full[buf], (tile / STAGES) & 1)) {
-      if (tid == 0) atomicExch(a.status, 31);
+    if (!tc::mbar_wait_warp(&full[buf], (tile / STAGES) & 1)) {
+      if (lane == 0) atomicExch(a.status, 31);
       ok = false;
+      break;
     }
     const int base = first + tile * TILE;
     uint8_t* kt = k_s + buf * KV_BYTES;
@@ -362,17 +391,14 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       *reinterpret_cast<uint4*>(own + tile_offset<HD>(pos - base, own_d0)) = own_c0;
       *reinterpret_cast<uint4*>(own + tile_offset<HD>(pos - base, own_d1)) = own_c1;
     }
-    if (base + TILE - 1 > last) {                  // the last tile: V rows past the range must not reach the sum
-      for (int c = tid; c < TILE * HALVES * 8; c += NWARPS * 32) {
-        const int r = c / (HALVES * 8), rest = c % (HALVES * 8);
+    if (base + TILE - 1 > last) {                  // the last tile: V rows past the range must not reach the sum (a warp reads its own 16)
+      for (int c = lane; c < 16 * HALVES * 8; c += 32) {
+        const int r = warp * 16 + c / (HALVES * 8), rest = c % (HALVES * 8);
         if (base + r > last)
           *reinterpret_cast<uint4*>(vt + (rest / 8) * HALF_BYTES + r * 128 + (rest % 8) * 16) = make_uint4(0u, 0u, 0u, 0u);
       }
     }
-    // q rows and zeroed rows are visible to every warp; and the block agrees on whether the tile
-    // arrived (a wait that ran out in some threads only must not split the block at a barrier)
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
+    __syncwarp();
     if (tile == 0) {
 #pragma unroll
       for (int ks = 0; ks < HD / 16; ++ks)
@@ -451,18 +477,20 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       hb::mma_bf16(o_acc[j], p_frag, b[0], b[1]);
       hb::mma_bf16(o_acc[j + 1], p_frag, b[2], b[3]);
     }
-    __syncthreads();      // everyone is done with this buffer before it is refilled
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&empty[buf]);   // this warp is done with the buffer
   }
+  ok = comp_and(ok);        // every warp is done with the tiles; and they agree on whether all of them arrived
   // fused form: the blocks of a (token, kv head) count themselves in; the last one combines the splits
   const bool counted = merge_inside && n_splits > 1;
   auto arrive = [&]() {
-    __syncthreads();                                 // this block's partial results are written; one thread
+    comp_sync();                                 // this block's partial results are written; one thread
     if (tid == 0) {                                  // publishes them (the fence is cumulative over the barrier)
       __threadfence();
       last_block = atomicAdd(&f.counters[t * a.nkv + kvh], 1) == n_splits - 1;
       __threadfence();
     }
-    __syncthreads();
+    comp_sync();
     return last_block != 0;
   };
   if (MERGE == CLUSTER ? !ok && n_splits == 1 : !ok) {      // a load never arrived (recorded in status): nothing sensible to write
@@ -476,7 +504,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     ml_s[(warp * ROWS + r0) * 2] = m_run[0];     ml_s[(warp * ROWS + r0) * 2 + 1] = l_run[0];
     ml_s[(warp * ROWS + r0 + 8) * 2] = m_run[1]; ml_s[(warp * ROWS + r0 + 8) * 2 + 1] = l_run[1];
   }
-  __syncthreads();
+  comp_sync();
   float fr[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -501,7 +529,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         }
       }
     }
-    __syncthreads();
+    comp_sync();
   }
   if constexpr (MERGE == CLUSTER) {
     if (n_splits > 1) {
@@ -517,7 +545,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       cluster_sync();
       // o = sum_s o_s e^{m_s - m} / sum_s l_s e^{m_s - m} in split order, the sums as attention_merge_kernel takes them; the
       // blocks share the group's rows
-      for (int i = split * NWARPS * 32 + tid; i < G * (HD / 4); i += n_splits * NWARPS * 32) {
+      for (int i = split * COMP + tid; i < G * (HD / 4); i += n_splits * COMP) {
         const int row = i / (HD / 4), d = (i % (HD / 4)) * 4;
         float2 ml[MAX_CLUSTER];
         float4 v[MAX_CLUSTER];
@@ -552,7 +580,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
   }
   // rows < G are real heads; thread `tid` finishes (row, dims) pairs
-  for (int i = tid; i < G * HD; i += NWARPS * 32) {
+  for (int i = tid; i < G * HD; i += COMP) {
     const int row = i / HD, d = i % HD;
     float mx = -INFINITY;
     for (int w = 0; w < NWARPS; ++w) mx = fmaxf(mx, ml_s[(w * ROWS + row) * 2]);
@@ -581,13 +609,13 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   // weights: thread (row, split) pairs; the maxima and sums of a row go through shared memory
   float* m_s = o_s;                                  // [G][n_splits] maxima, then the same for the sums (o_s is done with
   float* l_s = m_s + G * n_splits;                   // where G * splits fit; the launcher checks the room)
-  for (int i = tid; i < G * n_splits; i += NWARPS * 32) {
+  for (int i = tid; i < G * n_splits; i += COMP) {
     const int row = i / n_splits, sp = i % n_splits;
     const float2 ml = __ldcg(reinterpret_cast<const float2*>(a.part_ml + ((th0 + row) * a.max_splits + sp) * 2));
     m_s[i] = ml.x;
     l_s[i] = ml.y;
   }
-  __syncthreads();
+  comp_sync();
   for (int row = warp; row < G; row += NWARPS) {
     float mx = -INFINITY;
     for (int sp = lane; sp < n_splits; sp += 32) mx = fmaxf(mx, m_s[row * n_splits + sp]);
@@ -602,11 +630,11 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     if (a.sink && l > 0.f) l += expf(-mx);
     if (lane == 0) inv_s[row] = l > 0.f ? 1.f / l : 0.f;
   }
-  __syncthreads();
+  comp_sync();
   // outputs: a thread takes four dims of a row; up to 16 splits' loads are in flight at a time, and the
   // sum runs over the splits in their order
   constexpr int AHEAD = 16;
-  for (int i = tid; i < G * (HD / 4); i += NWARPS * 32) {
+  for (int i = tid; i < G * (HD / 4); i += COMP) {
     const int row = i / (HD / 4), d = (i % (HD / 4)) * 4;
     const float* acc = a.part_acc + (th0 + row) * a.max_splits * HD + d;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -632,10 +660,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if (tid == 0) f.counters[t * a.nkv + kvh] = 0;     // zero again for the next launch
 }
 
-template <int HD>
+template <int HD, int STAGES>
 constexpr size_t smem_bytes() {
   return 1024 + 2 * (size_t)STAGES * (HD / 64) * HALF_BYTES + (size_t)ROWS * (HD + 8) * 2 + (size_t)NWARPS * ROWS * 2 * sizeof(float) +
-         STAGES * sizeof(uint64_t) + HD * sizeof(float);
+         2 * STAGES * sizeof(uint64_t) + HD * sizeof(float);
 }
 
 // A launch whose token's splits are a cluster.
@@ -643,50 +671,54 @@ inline void cluster_of(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, dim3 
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = grid.x;
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.gridDim = grid; cfg.blockDim = dim3(NWARPS * 32); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.gridDim = grid; cfg.blockDim = dim3(COMP + 32); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cfg.attrs = &attr; cfg.numAttrs = 1;
 }
 
 template <int HD>
 int clusters_at_once(int splits) {
+  constexpr int STAGES = STAGES_OF<HD>;
+  constexpr size_t smem = smem_bytes<HD, STAGES>();
   cudaLaunchAttribute attr;
   cudaLaunchConfig_t cfg = {};
-  cluster_of(cfg, attr, dim3(splits, 1, 1), smem_bytes<HD>(), nullptr);
+  cluster_of(cfg, attr, dim3(splits, 1, 1), smem, nullptr);
   int n = 0;
-  if (cudaFuncSetAttribute(attn_decode_tma_kernel<HD, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<HD>()) !=
+  if (cudaFuncSetAttribute(attn_decode_tma_kernel<HD, STAGES, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<HD, CLUSTER>, &cfg) != cudaSuccess) {
+      cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<HD, STAGES, CLUSTER>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return n;
 }
 
-template <int HD, Merge MERGE>
+template <int HD, Merge MERGE, int STAGES = STAGES_OF<HD>>
 int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, const Args& a, const Fuse& f,
            cudaStream_t stream) {
+  if constexpr (HD == 64 && STAGES == STAGES_OF<HD>)
+    if (a.split_size <= 2 * TILE) return launch<HD, MERGE, 2>(k_pages, v_pages, n_pages, n_tokens, a, f, stream);
   const uint64_t pool_rows = (uint64_t)n_pages * a.nkv * a.page_size;
   CUtensorMap mk, mv;
   if (!tc::make_map_bf16(&mk, k_pages, pool_rows, HD, a.box_rows) || !tc::make_map_bf16(&mv, v_pages, pool_rows, HD, a.box_rows))
     return HB_ERR_UNSUPPORTED;
   constexpr bool FUSED = MERGE == FUSED_FORM;
   constexpr int KV_BYTES = (HD / 64) * HALF_BYTES;
-  constexpr size_t smem = smem_bytes<HD>();
+  constexpr size_t smem = smem_bytes<HD, STAGES>();
   static_assert((size_t)STAGES * KV_BYTES >= (size_t)ROWS * HD * sizeof(float), "o_s aliases the K tiles");
   // the fused merge keeps [G][splits] weights and [G] sums where the V tiles were
   if (FUSED && (size_t)(a.nh / a.nkv) * (2 * a.max_splits + 1) * sizeof(float) > (size_t)STAGES * KV_BYTES) return HB_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<HD, MERGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<HD, STAGES, MERGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   dim3 grid(a.max_splits, a.nkv, n_tokens);
   if (MERGE == CLUSTER) {
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = {};
     cluster_of(cfg, attr, grid, smem, stream);
-    cudaLaunchKernelEx(&cfg, attn_decode_tma_kernel<HD, MERGE>, mk, mv, a, f);
+    cudaLaunchKernelEx(&cfg, attn_decode_tma_kernel<HD, STAGES, MERGE>, mk, mv, a, f);
     HB_LAUNCH_CHECK();
     return HB_OK;
   }
-  attn_decode_tma_kernel<HD, MERGE><<<grid, NWARPS * 32, smem, stream>>>(mk, mv, a, f);
+  attn_decode_tma_kernel<HD, STAGES, MERGE><<<grid, COMP + 32, smem, stream>>>(mk, mv, a, f);
   HB_LAUNCH_CHECK();
   return HB_OK;
 }

@@ -1381,13 +1381,17 @@ def sigmoid_prefill_attention_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages
 
 
 @functools.lru_cache(maxsize=1024)           # a step's layers ask the same (a search over every number of splits)
-def _decode_splits(longest: int, groups: int) -> Tuple[int, int]:
+@functools.lru_cache(maxsize=4096)                 # a step's layers ask the same
+def _decode_splits(longest: int, groups: int, hd: int = 0, device: int = -1) -> Tuple[int, int]:
     """How to cut ``longest`` keys for ``groups`` (token, kv head) pairs: the number of splits
     that minimises waves x (tiles per block + a block's fixed cost) + a cost per split (the
     merge) on 148 SMs x 3 resident blocks, none shorter than ATTENTION_SPLIT keys. Measured at
     8 requests x 8,192 keys: 6 splits (one wave of 384 blocks) 57 us, 13 splits (two waves) 63 us;
     one request x 32,768 keys: 32 splits 33 us, 47 splits 36 us.
-    The cut moves results by rounding only."""
+    The cut moves results by rounding only. With ``hd`` and ``device``: for the kernel whose tiles come by TMA; rows
+    of 128 have a model of their own there (:func:`_tma_splits`)."""
+    if hd == 128:
+        return _tma_splits(-(-longest // 64), groups, device, DECODE_CLUSTER + 1 if _decode_splits(longest, groups)[1] > DECODE_CLUSTER else 1)
     best = (None, 1, longest)
     for s in range(1, max(1, -(-longest // ATTENTION_SPLIT)) + 1):
         size = -(-(-(-longest // s)) // 64) * 64
@@ -1397,6 +1401,28 @@ def _decode_splits(longest: int, groups: int) -> Tuple[int, int]:
         if best[0] is None or cost < best[0]:
             best = (cost, real, size)
     return best[2], best[1]
+
+
+def _tma_splits(tiles: int, groups: int, device: int, least: int) -> Tuple[int, int]:
+    """The cut of ``tiles`` tiles of 64 keys for the decode kernel whose tiles come by TMA, rows of 128: the least by a model of its
+    time in us: waves of blocks (4.1 each and 0.65 a tile) or the bytes of all tiles (0.00263 a tile; 0.092 for a tile of the blocks
+    that run last, 0.44 a wave), whichever is more, plus what brings the splits together (0.023 for each in a cluster,
+    else the merge kernel's 3.4 and 0.215 for 1,000 splits); ``least`` splits and more, none shorter than 128 keys.
+    Fitted to 1,174 steps of 1 to 64 tokens, even and uneven contexts, up to 280,000 keys, in up to 14 cuts each: what it takes is
+    1.014 of the best cut's time on average, :func:`_decode_splits`'s own was 1.053. One token of 1,000 keys, 40 heads, 4 splits / 8
+    of 128 keys: 9.9 / 8.6 us; 64 of 1,000, 32 heads on 8 kv heads, 4 / 2: 68 / 61."""
+    best = (None, 64 * tiles, 1)
+    for s in range(least, max(least, min(tiles // 2, 48)) + 1):
+        size = -(-tiles // s)
+        real = -(-tiles // size)
+        waves = -(-(real * groups) // DECODE_RESIDENT_BLOCKS)
+        cost = max(waves * (4.1 + 0.65 * size), 0.00263 * groups * tiles + 0.092 * size + 0.44 * waves)
+        if real > 1:
+            met = real <= DECODE_CLUSTER and groups <= _decode_clusters(device, 128, real)
+            cost += 0.023 * real if met else 3.4 + 0.000215 * real * groups
+        if best[0] is None or cost < best[0]:
+            best = (cost, 64 * size, real)
+    return best[1], best[2]
 
 
 # Row lengths (head dims) of the tensor-core attention kernels. 192 is a latent of 128 with a rotated key part of 64;
@@ -1466,10 +1492,13 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         longest = min(-(-longest // 64), -(-(window + 63) // 64) + -(-keep // 64)) * 64
     elif window > 0:
         longest = min(longest, window)
-    split_size, splits = _decode_splits(longest, n * nkv * -(-(nh // nkv) // 16))
+    reshaped = bool(softcap) or slopes is not None or sink_values is not None or keep > 0 or parts
+    tma = not reshaped and hd <= 128 and window == 0 and chunk % 64 == 0 and nh // nkv <= 16 and \
+        (page_size % 64 == 0 or page_size in (16, 32))
+    split_size, splits = _decode_splits(longest, n * nkv, hd, q.get_device()) if tma else \
+        _decode_splits(longest, n * nkv * -(-(nh // nkv) // 16))
     if rows is None:
         out = None if parts else torch.empty_like(q)
-    reshaped = bool(softcap) or slopes is not None or sink_values is not None or keep > 0 or parts
     part_acc = part_ml = None
 
     def scratch():
@@ -1573,6 +1602,8 @@ def decode_attention_fused(qkv: torch.Tensor, nh: int, nkv: int, hd: int, positi
     if window > 0:
         longest = min(longest, window)
     split_size, splits = _decode_splits(longest, n * nkv)
+    if splits <= DECODE_CLUSTER:       # (of more the last block combines them all: 4 requests of 65,536 keys 13 splits 165 us, 32 187)
+        split_size, splits = _decode_splits(longest, n * nkv, hd, qkv.get_device())
     out = torch.empty((n, nh, hd), dtype=qkv.dtype, device=qkv.device)
     part_acc = part_ml = None
     if splits > 1:
