@@ -54,24 +54,6 @@ __device__ __forceinline__ float row_max(const float (&v)[BK]) {
   return fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
 }
 
-// Four lanes that each hold four 16-byte words of a row of their own trade them: lane q then holds word q of the four rows, and the
-// four store 64 bytes of a row together. (Every lane its own row is 32 lines a store; 2.5 us for two items of 128 rows.)
-__device__ __forceinline__ void trade_rows(uint4 (&v)[4], int lane) {
-#pragma unroll
-  for (int bit = 1; bit <= 2; bit <<= 1) {
-    const bool up = lane & bit;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k & bit) continue;
-      const uint4 give = up ? v[k] : v[k | bit];
-      const uint4 got = make_uint4(__shfl_xor_sync(0xffffffffu, give.x, bit), __shfl_xor_sync(0xffffffffu, give.y, bit),
-                                   __shfl_xor_sync(0xffffffffu, give.z, bit), __shfl_xor_sync(0xffffffffu, give.w, bit));
-      if (up) v[k] = got;
-      else v[k | bit] = got;
-    }
-  }
-}
-
 // An item: its first token, how many there are, the head, the first and last position, the first key that any row reads, its key tiles
 // [begin, end).
 struct Item {
@@ -552,7 +534,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             uint4 v[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = make_uint4(o[h + 4 * e], o[h + 4 * e + 1], o[h + 4 * e + 2], o[h + 4 * e + 3]);
-            trade_rows(v, lane);
+            tc::trade_rows(v, lane);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int to = (r & ~3) + e;
@@ -581,7 +563,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             }
             v[e] = make_uint4(u[0], u[1], u[2], u[3]);
           }
-          trade_rows(v, lane);
+          tc::trade_rows(v, lane);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int to = (r & ~3) + e;

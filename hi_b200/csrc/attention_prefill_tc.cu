@@ -7,7 +7,7 @@
 //               V into a ring of two (a load takes about as long as a tile's work, so with two
 //               stages and K and V in turn the products waited for their K: measured 5.76 -> 5.16 ms
 //               for 4,096 new tokens behind 61,440);
-//   warp 1      allocates tensor memory; one lane issues S = Q K^T (tcgen05.mma, M 128, N 64) into
+//   warp 1      allocates tensor memory; issues S = Q K^T (tcgen05.mma, M 128, N 64) into
 //               one of two S buffers and, a tile behind, O += P V (P read from tensor memory, where
 //               it lies over its own S; V from shared memory as the MN-major operand), so the next
 //               S is computed while the softmax works on this one;
@@ -21,6 +21,9 @@
 // and BOTH maps of a head. Row r of the tile is token r % 64 of map r / 64, so the two maps share every key and value
 // tile, and the epilogue subtracts them, norms the head's row and gates it before it leaves (see Pair).
 // A window that keeps the first tokens of a request (keep > 0) walks the tiles of the kept tokens first.
+// The products' warp walks its loop together and one lane of it issues (alone in the loop it moved each product's descriptors to the
+// uniform registers first), and rows leave 64 bytes a quad: 2,048 tokens, 40 heads of 192, 111 -> 102 us; 513 behind 7,000, 16 heads of
+// 192, 115 -> 99; with a distance bias, 40 heads of 128, 75 -> 67, with a cap 112 -> 107.
 // Every mbarrier wait is bounded; on a time-out a code goes to `status` and the block leaves
 // through the common exit, where tensor memory is freed.
 #include <cuda.h>
@@ -148,7 +151,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int heads = kPair ? a.nh / 2 : a.nh;
   const int seq = blockIdx.z, h = blockIdx.x % heads, piece = blockIdx.x / heads;
   const int qt = gridDim.y - 1 - blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int seq_begin = a.cu_seqlens[seq], seq_end = a.cu_seqlens[seq + 1];
   const int tok0 = seq_begin + qt * TOKENS;
   const int n_valid = min(TOKENS, seq_end - tok0);
@@ -254,46 +257,55 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {                            // ---- MMA issuer: S_j = Q K_j^T, then O += P_{j-1} V_{j-1}
-      constexpr uint32_t idesc_qk = tc::idesc_bf16(BQ, BKEYS, false);
-      constexpr uint32_t idesc_pv = tc::idesc_bf16(BQ, HD, true);
-      bool ok = tc::mbar_wait(q_full, 0);
-      if (!ok) atomicExch(a.status, 12);
-      tc::fence_after();
-      const uint32_t q_addr = tc::smem_u32(q_s);
-      for (int j = 0; j <= nt && ok; ++j) {
-        if (j < nt) {
-          const int s = j & 1;
-          const int ks = j % kst;
-          if (!tc::mbar_wait(&k_full[ks], (j / kst) & 1)) { atomicExch(a.status, 13); ok = false; break; }
-          if (j >= 2 && !tc::mbar_wait(&s_free[s], ((j >> 1) - 1) & 1)) { atomicExch(a.status, 14); ok = false; break; }
-          // S_j goes where P_{j-2} lies: the product that reads that P must be through (it is the last one
-          // committed to this barrier so far, so the parity is its own)
-          if (j >= 2 && !tc::mbar_wait(pv_done, (j - 2) & 1)) { atomicExch(a.status, 24); ok = false; break; }
-          tc::fence_after();
-          const uint32_t k_addr = tc::smem_u32(k_s + ks * KBYTES);
+    // ---- MMA issuer: S_j = Q K_j^T, then O += P_{j-1} V_{j-1}; the whole warp walks, one lane issues
+    constexpr uint32_t idesc_qk = tc::idesc_bf16(BQ, BKEYS, false);
+    constexpr uint32_t idesc_pv = tc::idesc_bf16(BQ, HD, true);
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, int parity, int code) {
+      if (ok && !tc::mbar_wait_warp(bar, parity)) {
+        if (lane == 0) atomicExch(a.status, code);
+        ok = false;
+      }
+    };
+    const uint32_t mine = tc::elect_one();
+    wait(q_full, 0, 12);
+    const uint64_t q_desc = tc::desc_kmajor(tc::smem_u32(q_s));
+    const uint32_t k_addr = tc::smem_u32(k_s), v_addr = tc::smem_u32(v_s);
+    const int tiles = tc::uniform(nt);
+    int ks = 0, kturn = 0;
+    for (int j = 0; j <= tiles && ok; ++j) {
+      if (j < tiles) {
+        const int s = j & 1;
+        wait(&k_full[ks], kturn, 13);
+        if (j >= 2) wait(&s_free[s], ((j >> 1) - 1) & 1, 14);
+        // S_j goes where P_{j-2} lies: the product that reads that P must be through (it is the last one
+        // committed to this barrier so far, so the parity is its own)
+        if (j >= 2) wait(pv_done, (j - 2) & 1, 24);
+        if (!ok) break;
+        tc::fence_after();
+        const uint64_t k_desc = tc::desc_kmajor(k_addr + ks * KBYTES);
 #pragma unroll
-          for (int k = 0; k < HD / 16; ++k) {
-            tc::mma(tmem + s * S_COLS, tc::desc_kmajor(q_addr + (k / 4) * QBLOCK + (k % 4) * 32),
-                   tc::desc_kmajor(k_addr + (k / 4) * KVBLOCK + (k % 4) * 32), idesc_qk, k != 0);
-          }
-          tc::commit(&s_full[s]);
-          tc::commit(&k_empty[ks]);             // the K buffer is free once these MMAs have read it
-        }
-        if (j >= 1) {
-          const int i = j - 1, s = i & 1;
-          if (!tc::mbar_wait(&v_full[s], (i >> 1) & 1)) { atomicExch(a.status, 21); ok = false; break; }
-          if (!tc::mbar_wait(p_ready, i & 1)) { atomicExch(a.status, 15); ok = false; break; }
-          tc::fence_after();
-          const uint32_t v_addr = tc::smem_u32(v_s + s * KBYTES);
-          const uint32_t p_tmem = tmem + s * S_COLS;     // P_i lies over the first half of S_i's columns
+        for (int k = 0; k < HD / 16; ++k)
+          tc::mma_if(mine, tmem + s * S_COLS, q_desc + (((k / 4) * QBLOCK + (k % 4) * 32) >> 4),
+                     k_desc + (((k / 4) * KVBLOCK + (k % 4) * 32) >> 4), idesc_qk, k != 0);
+        tc::commit_if(mine, &s_full[s]);
+        tc::commit_if(mine, &k_empty[ks]);      // the K buffer is free once these MMAs have read it
+        if (++ks == kst) { ks = 0; kturn ^= 1; }
+      }
+      if (j >= 1) {
+        const int i = j - 1, s = i & 1;
+        wait(&v_full[s], (i >> 1) & 1, 21);
+        wait(p_ready, i & 1, 15);
+        if (!ok) break;
+        tc::fence_after();
+        const uint64_t v_desc = tc::desc_mnmajor(v_addr + s * KBYTES, KVBLOCK);
+        const uint32_t p_tmem = tmem + s * S_COLS;     // P_i lies over the first half of S_i's columns
+        const uint32_t more = i != 0;
 #pragma unroll
-          for (int k = 0; k < BKEYS / 16; ++k) {
-            tc::mma_a_tmem(tmem_o, p_tmem + k * 8, tc::desc_mnmajor(v_addr + k * 2048, KVBLOCK), idesc_pv, (i | k) != 0);
-          }
-          tc::commit(&v_empty[s]);
-          tc::commit(pv_done);
-        }
+        for (int k = 0; k < BKEYS / 16; ++k)
+          tc::mma_a_tmem_if(mine, tmem_o, p_tmem + k * 8, v_desc + k * (2048 >> 4), idesc_pv, k == 0 ? more : 1u);
+        tc::commit_if(mine, &v_empty[s]);
+        tc::commit_if(mine, pv_done);
       }
     }
   } else {                                      // ---- softmax: thread = row = tensor-memory lane
@@ -318,7 +330,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     bool ok = true;
     for (int j = 0; j < nt && ok; ++j) {
       const int sb = j & 1;
-      if (!__all_sync(0xffffffffu, tc::mbar_wait(&s_full[sb], (j >> 1) & 1))) {
+      if (!tc::mbar_wait_warp(&s_full[sb], (j >> 1) & 1)) {
         if (lane == 0) atomicExch(a.status, 16);
         ok = false;
         break;
@@ -427,7 +439,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // and the MMA issuer within a tile of one another: that product started only after every
         // warp had handed over its P of the tile before and the issuer had seen it, so the one
         // barrier that counts the hand-overs tile after tile never runs a phase ahead of anyone.
-        if (!__all_sync(0xffffffffu, tc::mbar_wait(pv_done, (j - 1) & 1))) {
+        if (!tc::mbar_wait_warp(pv_done, (j - 1) & 1)) {
           if (lane == 0) atomicExch(a.status, 17);
           ok = false;
           break;
@@ -466,7 +478,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // Value rows of positions past the portion's end hold whatever the page held before, and those of pages that
         // were given back are any page's (another request's numbers, possibly not finite): P is zero there, but
         // 0 x NaN is NaN. Once the V tile has landed, the threads of those rows zero them.
-        if (!__all_sync(0xffffffffu, tc::mbar_wait(&v_full[sb], (j >> 1) & 1))) {
+        if (!tc::mbar_wait_warp(&v_full[sb], (j >> 1) & 1)) {
           if (lane == 0) atomicExch(a.status, 22);
           ok = false;
           break;
@@ -486,7 +498,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (lane == 0) tc::mbar_arrive(p_ready);
     }
     if (ok) {
-      if (!__all_sync(0xffffffffu, tc::mbar_wait(pv_done, (nt - 1) & 1))) {
+      if (!tc::mbar_wait_warp(pv_done, (nt - 1) & 1)) {
         if (lane == 0) atomicExch(a.status, 18);
       } else {
         tc::fence_after();
@@ -508,7 +520,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           }
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(ex_ready);
-          bool met = __all_sync(0xffffffffu, tc::mbar_wait(ex_ready, 0));
+          bool met = tc::mbar_wait_warp(ex_ready, 0);
           float v[HALF];
           float ss = 0.f;
           if (met) {
@@ -527,7 +539,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             ex_ss[mp * TOKENS + row] = ss;
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(ex_ready);
-            met = __all_sync(0xffffffffu, tc::mbar_wait(ex_ready, 1));
+            met = tc::mbar_wait_warp(ex_ready, 1);
           }
           if (!met) {
             if (lane == 0) atomicExch(a.status, 23);
@@ -635,34 +647,47 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           }
 #pragma unroll 1
           for (int c = 0; c < HD; c += 32) {
-            float o[32];
-            tc::ld32(tmem_o + lane_addr + c, o);
-            if (row_ok) {
-              float4* dst4 = reinterpret_cast<float4*>(a.part_acc + at * HD + c);
+            uint32_t o[32];
+            tc::ld32_nowait(tmem_o + lane_addr + c, o);
+            tc::wait_ld();
 #pragma unroll
-              for (int i = 0; i < 8; ++i) dst4[i] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+            for (int i = 0; i < 32; i += 16) {
+              uint4 v[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) v[e] = make_uint4(o[i + 4 * e], o[i + 4 * e + 1], o[i + 4 * e + 2], o[i + 4 * e + 3]);
+              tc::trade_rows(v, lane);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int to = (r & ~3) + e;
+                if (to < n_valid)
+                  *reinterpret_cast<uint4*>(a.part_acc + (((size_t)(tok0 + to) * a.nh + h) * a.key_splits + piece) * HD + c + i +
+                                            4 * (lane & 3)) = v[e];
+              }
             }
           }
         } else {
         if (a.sink && l > 0.f) l += exp2f((a.sink_values ? a.sink_values[h] * 1.4426950408889634f : 0.f) - m);   // m is in units of log 2
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        __nv_bfloat16* dst = a.out + ((size_t)(tok0 + r) * a.nh + h) * HD;
 #pragma unroll 1
         for (int c = 0; c < HD; c += 32) {
           float o[32];
           tc::ld32(tmem_o + lane_addr + c, o);
-          if (row_ok) {
+          uint4 v[4];
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 pack;
-              uint32_t* w = reinterpret_cast<uint32_t*>(&pack);
+          for (int e = 0; e < 4; ++e) {
+            uint32_t u[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                __nv_bfloat162 hh = __floats2bfloat162_rn(o[i + 2 * e] * inv, o[i + 2 * e + 1] * inv);
-                w[e] = *reinterpret_cast<uint32_t*>(&hh);
-              }
-              *reinterpret_cast<uint4*>(dst + c + i) = pack;
+            for (int i = 0; i < 4; ++i) {
+              __nv_bfloat162 hh = __floats2bfloat162_rn(o[8 * e + 2 * i] * inv, o[8 * e + 2 * i + 1] * inv);
+              u[i] = *reinterpret_cast<uint32_t*>(&hh);
             }
+            v[e] = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+          tc::trade_rows(v, lane);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int to = (r & ~3) + e;
+            if (to < n_valid) *reinterpret_cast<uint4*>(a.out + ((size_t)(tok0 + to) * a.nh + h) * HD + c + 8 * (lane & 3)) = v[e];
           }
         }
         }
