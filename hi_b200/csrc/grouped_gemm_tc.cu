@@ -92,11 +92,10 @@ struct Maps {                // X boxes of 32, 64, 128 and 192 rows; the weight 
 // share a weight tile are neighbours, so they run at the same time and the weight tile comes from
 // HBM once. Returns false past the last tile. `f_tiles` = feature tiles.
 struct Tile { int expert, row0, tokens, f0; };
-template <int BT>
-__device__ __forceinline__ bool find_tile(const int* offsets, int experts, int t, int f_tiles, Tile& out) {
+__device__ __forceinline__ bool find_tile(const int* offsets, int experts, int t, int f_tiles, int most, Tile& out) {
   for (int e = 0; e < experts; ++e) {
     const int begin = offsets[e], cnt = offsets[e + 1] - begin;
-    const int t_tiles = (cnt + BT - 1) / BT;
+    const int t_tiles = (cnt + most - 1) / most;
     const int here = t_tiles * f_tiles;
     if (t < here) {
       const int ft = t / t_tiles, tt = t - ft * t_tiles;
@@ -112,18 +111,38 @@ __device__ __forceinline__ bool find_tile(const int* offsets, int experts, int t
   return false;
 }
 
+// The most tokens of a tile in a long DUAL launch: 192, or 128 where that takes less time. A tile of up to 128 leaves its slot to the
+// next one's accumulators, a larger one has both and the next waits until it is in registers; a stage brings less with it, but the
+// weights come once more. By the rounds over the SMs times what a stage brings (32 KB of weights, the box of tokens) and, for the
+// larger tiles, 480 KB a tile for that wait (us, 192 / 128: 2,048 tokens, 2 of 8 experts of 2,048 x 4,096, up product with gather, 136
+// / 128; 4 of 16 of 1,024 x 2,048 91 / 78; 1 of 16 of 2,048 x 8,192, where weights come from HBM, 196 / 208). One warp asks.
+__device__ __forceinline__ int dual_tokens(const int* offsets, int experts, int f_tiles, int num_kb, int blocks) {
+  int few = 0, many = 0, large = 0;
+  for (int e = threadIdx.x & 31; e < experts; e += 32) {
+    const int cnt = offsets[e + 1] - offsets[e], tiles = (cnt + BT_LONG - 1) / BT_LONG;
+    many += (cnt + DUAL_SLOT_T - 1) / DUAL_SLOT_T;
+    few += tiles;
+    if (cnt > tiles * DUAL_SLOT_T) large = 1;
+  }
+  few = __reduce_add_sync(0xffffffffu, few);
+  many = __reduce_add_sync(0xffffffffu, many);
+  if (__reduce_max_sync(0xffffffffu, large) == 0) return BT_LONG;
+  const long long at_192 = (long long)((few * f_tiles + blocks - 1) / blocks) * ((32 + 24) * num_kb + 480);
+  const long long at_128 = (long long)((many * f_tiles + blocks - 1) / blocks) * (32 + 16) * num_kb;
+  return at_128 < at_192 ? DUAL_SLOT_T : BT_LONG;
+}
+
 // The work of a block, in order: its tiles of the full rounds (blockIdx.x, blockIdx.x + gridDim.x,
 // ...), then its share of the last, partly filled round: a whole tile, or piece `piece` of `pieces`
 // of cut tile number `cut` (k blocks kb0 .. kb1). Every role of the block walks the same list.
 struct Work { Tile tile; int kb0, kb1, cut, piece, pieces; };
-template <int BT>
 struct WorkList {
   const int* offsets;
-  int experts, f_tiles, num_kb, rounds, rest, pieces, per;
-  __device__ WorkList(const int* offsets_, int experts_, int f_tiles_, int num_kb_, bool may_cut)
-      : offsets(offsets_), experts(experts_), f_tiles(f_tiles_), num_kb(num_kb_) {
+  int experts, f_tiles, num_kb, most, rounds, rest, pieces, per;
+  __device__ WorkList(const int* offsets_, int experts_, int f_tiles_, int num_kb_, int most_, bool may_cut)
+      : offsets(offsets_), experts(experts_), f_tiles(f_tiles_), num_kb(num_kb_), most(most_) {
     int tiles = 0;
-    for (int e = 0; e < experts; ++e) tiles += (offsets[e + 1] - offsets[e] + BT - 1) / BT * f_tiles;
+    for (int e = 0; e < experts; ++e) tiles += (offsets[e + 1] - offsets[e] + most - 1) / most * f_tiles;
     rounds = tiles / (int)gridDim.x;
     rest = tiles - rounds * (int)gridDim.x;
     pieces = 1;
@@ -138,17 +157,17 @@ struct WorkList {
   }
   __device__ __forceinline__ bool get(int i, Work& w) const {
     w.kb0 = 0; w.kb1 = num_kb; w.cut = -1; w.piece = 0; w.pieces = 1;
-    if (i < rounds) return find_tile<BT>(offsets, experts, (int)blockIdx.x + i * (int)gridDim.x, f_tiles, w.tile);
+    if (i < rounds) return find_tile(offsets, experts, (int)blockIdx.x + i * (int)gridDim.x, f_tiles, most, w.tile);
     if (i > rounds) return false;
     const int b = (int)blockIdx.x;
-    if (pieces == 1) return b < rest && find_tile<BT>(offsets, experts, rounds * (int)gridDim.x + b, f_tiles, w.tile);
+    if (pieces == 1) return b < rest && find_tile(offsets, experts, rounds * (int)gridDim.x + b, f_tiles, most, w.tile);
     if (b >= rest * pieces) return false;
     w.cut = b / pieces;                              // the pieces of one tile are neighbours: they share its tokens
     w.piece = b - w.cut * pieces;
     w.pieces = pieces;
     w.kb0 = w.piece * per;
     w.kb1 = min(num_kb, w.kb0 + per);
-    return find_tile<BT>(offsets, experts, rounds * (int)gridDim.x + w.cut, f_tiles, w.tile);
+    return find_tile(offsets, experts, rounds * (int)gridDim.x + w.cut, f_tiles, most, w.tile);
   }
 };
 
@@ -204,7 +223,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
   const uint32_t tmem = *tmem_slot;
   const int f_tiles = (p.n_out + BF - 1) / BF;
   const int num_kb = (p.K + BK - 1) / BK;
-  const WorkList<BT> list(s_offsets, p.experts, f_tiles, num_kb, !DUAL && p.scratch != nullptr);
+  const int most = DUAL && BT == BT_LONG ? dual_tokens(s_offsets, p.experts, f_tiles, num_kb, gridDim.x) : BT;
+  const WorkList list(s_offsets, p.experts, f_tiles, num_kb, most, !DUAL && p.scratch != nullptr);
 
   if (warp == 0) {                              // ---- TMA producer: the whole warp waits, one lane issues
     int s = 0, turn = 1;                        // (the first wait on a fresh barrier for the phase before it returns at once)
@@ -509,7 +529,7 @@ extern "C" int hb_moe_gate_up_tc(const void* xs, const int* sorted_entry, const 
   if (hidden % 8 != 0 || inter % 8 != 0 || hidden <= 0 || inter <= 0) return HB_ERR_UNSUPPORTED;
   if (rows == 0) return HB_OK;
   const bool few = rows <= SHORT_STEP_ROWS;
-  const int bt = few ? BT_SHORT : BT_LONG;
+  const int bt = few ? BT_SHORT : DUAL_SLOT_T;      // (or more: dual_tokens)
   const int max_tiles = (rows + bt - 1) / bt + (experts < rows ? experts : rows);
   if (max_tiles > 65535) return HB_ERR_UNSUPPORTED;
   Params p{offsets, sorted_entry, scores, act, status, experts, inter, hidden, rows, nullptr, nullptr, limit, 0};
