@@ -28,6 +28,9 @@
 // Both of these warps walk their loops together and one lane of them issues: alone in its loop, the lane moved every product's
 // descriptors to the uniform registers first, some 40 cycles a product of 96 (2,048 tokens, 2 of 8 experts of 2,048 x 4,096, gather
 // included: 150 -> 134 us, down 80 -> 73; 4 of 16 of 1,024 x 2,048: 105 -> 90, 51 -> 47; 64 tokens, 16 of 5,120 x 8,192: 390 -> 386).
+// Launches with many rows an expert run as pairs of blocks, 256 weight rows a tile (see pairs): the even block issues the products of
+// both (cta_group::2), every block's loads count on the even one's barriers, commits reach both, and each block writes out its 128
+// features from its own tensor memory.
 // Tensor memory is two slots of 256 columns. A tile takes one slot, and the next tile
 // accumulates into the other while this one is written out; only a DUAL tile of more than 128
 // tokens needs both (gate in one, up in the other), and its epilogue gives them back as soon as
@@ -54,6 +57,7 @@ namespace {
 constexpr int BF = 128;          // features (weight rows) of a tile: UMMA M
 constexpr int BT_LONG = 192;     // most tokens of a tile (UMMA N; the X tile of a stage is BT x 64) in steps of many
 constexpr int SHORT_STEP_ROWS = 256;   // steps of up to this many routed rows use BT_SHORT
+constexpr int PAIR_ROWS = 256;   // rows an expert on average from which two blocks share a tile
 constexpr int BT_SHORT = 64;     // tokens, and in decode-sized steps: less room for tokens, more stages of weights
 constexpr int SLOT_COLS = 256;   // tensor memory is two slots of 256 columns
 constexpr int TMEM_COLS = 2 * SLOT_COLS;
@@ -92,7 +96,7 @@ struct Maps {                // X boxes of 32, 64, 128 and 192 rows; the weight 
 // share a weight tile are neighbours, so they run at the same time and the weight tile comes from
 // HBM once. Returns false past the last tile. `f_tiles` = feature tiles.
 struct Tile { int expert, row0, tokens, f0; };
-__device__ __forceinline__ bool find_tile(const int* offsets, int experts, int t, int f_tiles, int most, Tile& out) {
+__device__ __forceinline__ bool find_tile(const int* offsets, int experts, int t, int f_tiles, int most, int features, Tile& out) {
   for (int e = 0; e < experts; ++e) {
     const int begin = offsets[e], cnt = offsets[e + 1] - begin;
     const int t_tiles = (cnt + most - 1) / most;
@@ -103,7 +107,7 @@ __device__ __forceinline__ bool find_tile(const int* offsets, int experts, int t
       out.expert = e;
       out.row0 = begin + tt * per;
       out.tokens = min(per, cnt - tt * per);
-      out.f0 = ft * BF;
+      out.f0 = ft * features;
       return true;
     }
     t -= here;
@@ -138,17 +142,17 @@ __device__ __forceinline__ int dual_tokens(const int* offsets, int experts, int 
 struct Work { Tile tile; int kb0, kb1, cut, piece, pieces; };
 struct WorkList {
   const int* offsets;
-  int experts, f_tiles, num_kb, most, rounds, rest, pieces, per;
-  __device__ WorkList(const int* offsets_, int experts_, int f_tiles_, int num_kb_, int most_, bool may_cut)
-      : offsets(offsets_), experts(experts_), f_tiles(f_tiles_), num_kb(num_kb_), most(most_) {
+  int experts, f_tiles, num_kb, most, features, unit, units, rounds, rest, pieces, per;
+  __device__ WorkList(const int* offsets_, int experts_, int f_tiles_, int num_kb_, int most_, int features_, int unit_, int units_, bool may_cut)
+      : offsets(offsets_), experts(experts_), f_tiles(f_tiles_), num_kb(num_kb_), most(most_), features(features_), unit(unit_), units(units_) {
     int tiles = 0;
     for (int e = 0; e < experts; ++e) tiles += (offsets[e + 1] - offsets[e] + most - 1) / most * f_tiles;
-    rounds = tiles / (int)gridDim.x;
-    rest = tiles - rounds * (int)gridDim.x;
+    rounds = tiles / units;
+    rest = tiles - rounds * units;
     pieces = 1;
     per = num_kb;
     if (may_cut && rest > 0) {
-      int want = min(min(MAX_PIECES, (int)gridDim.x / rest), num_kb / MIN_PIECE_KB);
+      int want = min(min(MAX_PIECES, units / rest), num_kb / MIN_PIECE_KB);
       if (want > 1) {
         per = (num_kb + want - 1) / want;
         pieces = (num_kb + per - 1) / per;          // no piece is empty
@@ -157,17 +161,17 @@ struct WorkList {
   }
   __device__ __forceinline__ bool get(int i, Work& w) const {
     w.kb0 = 0; w.kb1 = num_kb; w.cut = -1; w.piece = 0; w.pieces = 1;
-    if (i < rounds) return find_tile(offsets, experts, (int)blockIdx.x + i * (int)gridDim.x, f_tiles, most, w.tile);
+    if (i < rounds) return find_tile(offsets, experts, unit + i * units, f_tiles, most, features, w.tile);
     if (i > rounds) return false;
-    const int b = (int)blockIdx.x;
-    if (pieces == 1) return b < rest && find_tile(offsets, experts, rounds * (int)gridDim.x + b, f_tiles, most, w.tile);
+    const int b = unit;
+    if (pieces == 1) return b < rest && find_tile(offsets, experts, rounds * units + b, f_tiles, most, features, w.tile);
     if (b >= rest * pieces) return false;
     w.cut = b / pieces;                              // the pieces of one tile are neighbours: they share its tokens
     w.piece = b - w.cut * pieces;
     w.pieces = pieces;
     w.kb0 = w.piece * per;
     w.kb1 = min(num_kb, w.kb0 + per);
-    return find_tile(offsets, experts, rounds * (int)gridDim.x + w.cut, f_tiles, most, w.tile);
+    return find_tile(offsets, experts, rounds * units + w.cut, f_tiles, most, features, w.tile);
   }
 };
 
@@ -187,10 +191,11 @@ struct SlotWalk {
 };
 
 // Persistent: each block walks its work list. The shared-memory ring runs on across tiles.
-template <bool DUAL, int STAGES, int BT>
+template <bool DUAL, int STAGES, int BT, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
-  constexpr int W_BYTES = BF * BK * 2, X_BYTES = BT * BK * 2;
+  constexpr int XR = PAIR ? BT / 2 : BT;             // token rows of a stage
+  constexpr int W_BYTES = BF * BK * 2, X_BYTES = XR * BK * 2;
   constexpr int NW = DUAL ? 2 : 1;
   constexpr int STAGE_BYTES = NW * W_BYTES + X_BYTES;
   static_assert(BT <= SLOT_COLS && 2 * DUAL_SLOT_T <= SLOT_COLS, "a slot holds one accumulator of any tile");
@@ -207,59 +212,81 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
 
   const int warp = tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   for (int e = threadIdx.x; e <= p.experts; e += THREADS) s_offsets[e] = p.offsets[e];
+  const int rank = PAIR ? (int)tc::cluster_rank() : 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], EPI_WARPS); }
+    for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], PAIR ? 2 * EPI_WARPS : EPI_WARPS); }
     tc::mbar_init(&cut_bar[0], EPI_WARPS);
     tc::mbar_init(&cut_bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {                              // tensor memory for the two slots
-    tc::alloc(tmem_slot, TMEM_COLS);
+    if constexpr (PAIR) tc::alloc_pair(tmem_slot, TMEM_COLS);
+    else tc::alloc(tmem_slot, TMEM_COLS);
   }
   tc::fence_before();
+  if constexpr (PAIR) tc::cluster_meet();       // (the other block's barriers are ready too)
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = *tmem_slot;
-  const int f_tiles = (p.n_out + BF - 1) / BF;
+  constexpr int FEATURES = PAIR ? 2 * BF : BF;       // of a tile
+  const int f_tiles = (p.n_out + FEATURES - 1) / FEATURES;
   const int num_kb = (p.K + BK - 1) / BK;
-  const int most = DUAL && BT == BT_LONG ? dual_tokens(s_offsets, p.experts, f_tiles, num_kb, gridDim.x) : BT;
-  const WorkList list(s_offsets, p.experts, f_tiles, num_kb, most, !DUAL && p.scratch != nullptr);
+  const int units = PAIR ? gridDim.x / 2 : gridDim.x, unit = PAIR ? blockIdx.x / 2 : blockIdx.x;
+  const int most = DUAL && BT == BT_LONG ? dual_tokens(s_offsets, p.experts, f_tiles, num_kb, units) : BT;
+  const WorkList list(s_offsets, p.experts, f_tiles, num_kb, most, FEATURES, unit, units, !DUAL && p.scratch != nullptr);
 
   if (warp == 0) {                              // ---- TMA producer: the whole warp waits, one lane issues
     int s = 0, turn = 1;                        // (the first wait on a fresh barrier for the phase before it returns at once)
     bool ok = true;
+    const uint32_t mine = tc::elect_one(), ring = tc::smem_u32(smem);
+    const uint32_t bars = PAIR ? tc::even_block(full) : tc::smem_u32(full);
     Work work;
     for (int i = 0; ok && list.get(i, work); ++i) {
       const Tile& tile = work.tile;
-      const int box = tile.tokens <= 32 ? 0 : (tile.tokens <= 64 ? 1 : (tile.tokens <= 128 ? 2 : 3));
-      const uint32_t bytes = NW * W_BYTES + (uint32_t)x_box_rows(box, BT) * BK * 2;
-      const int w_row = tile.expert * p.n_out + tile.f0;
-      for (int kb = work.kb0; kb < work.kb1; ++kb) {
+      // a pair's tokens, as many as its product has, are half in one block and half in the other
+      const int x_rows = PAIR ? ((tile.tokens + 15) & ~15) / 2 : tile.tokens, x_row = tc::uniform(tile.row0 + rank * x_rows);
+      const int box = tc::uniform(x_rows <= 32 ? 0 : (x_rows <= 64 ? 1 : (x_rows <= 128 ? 2 : 3)));
+      const uint32_t bytes = (PAIR ? 2 : 1) * (NW * W_BYTES + (uint32_t)x_box_rows(box, XR) * BK * 2);
+      const int w_row = tc::uniform(tile.expert * p.n_out + tile.f0 + rank * BF);
+      const int kb1 = tc::uniform(work.kb1);
+      const CUtensorMap* x_map = &maps.x[box];
+      for (int kb = tc::uniform(work.kb0); kb < kb1; ++kb) {
         if (!tc::mbar_wait_warp(&empty[s], turn)) {
           if (lane == 0) atomicExch(p.status, 1);
           ok = false;
           break;
         }
-        if (lane == 0) {
-          uint8_t* st = smem + s * STAGE_BYTES;
-          tc::mbar_expect_tx(&full[s], bytes);
-          tc::tma_load_2d(st, &maps.w0, kb * BK, w_row, &full[s]);
-          if (DUAL) tc::tma_load_2d(st + W_BYTES, &maps.w1, kb * BK, w_row, &full[s]);
-          tc::tma_load_2d(st + NW * W_BYTES, &maps.x[box], kb * BK, tile.row0, &full[s]);
+        const uint32_t st = ring + s * STAGE_BYTES, bar = bars + s * 8;
+        if (mine && rank == 0) tc::mbar_expect_tx(&full[s], bytes);
+        if constexpr (PAIR) {
+          tc::tma_load_2d_pair_if(mine, st, &maps.w0, kb * BK, w_row, bar);
+          if (DUAL) tc::tma_load_2d_pair_if(mine, st + W_BYTES, &maps.w1, kb * BK, w_row, bar);
+          tc::tma_load_2d_pair_if(mine, st + NW * W_BYTES, x_map, kb * BK, x_row, bar);
+        } else {
+          tc::tma_load_2d_if(mine, st, &maps.w0, kb * BK, w_row, bar);
+          if (DUAL) tc::tma_load_2d_if(mine, st + W_BYTES, &maps.w1, kb * BK, w_row, bar);
+          tc::tma_load_2d_if(mine, st + NW * W_BYTES, x_map, kb * BK, x_row, bar);
         }
-        __syncwarp();
         if (++s == STAGES) { s = 0; turn ^= 1; }
       }
     }
   } else if (warp == 1) {                       // ---- MMA issuer: the whole warp walks, one lane issues
     const uint32_t mine = tc::elect_one();
     const uint64_t ring = tc::desc_kmajor(tc::smem_u32(smem));
+    auto product = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t more) {
+      if constexpr (PAIR) tc::mma_pair_if(mine, d, a, b, idesc, more);
+      else tc::mma_if(mine, d, a, b, idesc, more);
+    };
+    auto commit = [&](uint64_t* bar) {
+      if constexpr (PAIR) tc::commit_pair_if(mine, bar);
+      else tc::commit_if(mine, bar);
+    };
     int s = 0, turn = 0;
     SlotWalk walk;
     bool ok = true;
     Work work;
-    for (int i = 0; ok && list.get(i, work); ++i) {
+    for (int i = 0; rank == 0 && ok && list.get(i, work); ++i) {      // (the odd block of a pair leaves it to the even one)
       const int tokens = tc::uniform(work.tile.tokens), kbs = tc::uniform(work.kb1 - work.kb0);
       bool both;
       const int b = walk.take(DUAL, tokens, both);
@@ -270,7 +297,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
         }
       if (!ok) break;
       tc::fence_after();
-      const uint32_t idesc = tc::idesc_bf16(BF, (tokens + 15) & ~15, false);
+      const uint32_t idesc = tc::idesc_bf16(FEATURES, (tokens + 15) & ~15, false);
       const uint32_t acc = tmem + b * SLOT_COLS;
       const uint32_t up = acc + (both ? SLOT_COLS : DUAL_SLOT_T);  // where the second accumulator starts
       for (int kb = 0; kb < kbs; ++kb) {
@@ -284,20 +311,24 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
 #pragma unroll
         for (int k = 0; k < BK / UK; ++k) {
           const uint32_t more = kb | k;
-          tc::mma_if(mine, acc, w + (k * UK * 2 >> 4), x + (k * UK * 2 >> 4), idesc, more);
-          if (DUAL) tc::mma_if(mine, up, w + ((W_BYTES + k * UK * 2) >> 4), x + (k * UK * 2 >> 4), idesc, more);
+          product(acc, w + (k * UK * 2 >> 4), x + (k * UK * 2 >> 4), idesc, more);
+          if (DUAL) product(up, w + ((W_BYTES + k * UK * 2) >> 4), x + (k * UK * 2 >> 4), idesc, more);
         }
-        tc::commit_if(mine, &empty[s]);          // the stage is free once these MMAs have read it
+        commit(&empty[s]);                       // the stage is free once these MMAs have read it
         if (++s == STAGES) { s = 0; turn ^= 1; }
       }
       // this tile's accumulator is complete (also on the error path)
-      tc::commit_if(mine, &acc_full[b]);
+      commit(&acc_full[b]);
       ++walk.use[b];
-      if (both) { tc::commit_if(mine, &acc_full[1]); ++walk.use[1]; }
+      if (both) { commit(&acc_full[1]); ++walk.use[1]; }
     }
   } else {                                      // ---- epilogue: warps 2..9
     const int quarter = warp & 3;               // the lanes of tensor memory this warp may read
     const int half = (warp - 2) >> 2;           // which runs of 32 tokens it takes
+    auto written = [&](int b) {                 // one lane: this warp has read the slot
+      if constexpr (PAIR) tc::arrive_even(tc::even_block(&acc_empty[b]));
+      else tc::mbar_arrive(&acc_empty[b]);
+    };
     SlotWalk walk;
     bool ok = true;
     Work work;
@@ -305,7 +336,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
       const Tile& tile = work.tile;
       bool both;
       const int b = walk.take(DUAL, tile.tokens, both);
-      const int f = tile.f0 + quarter * 32 + lane;        // this thread's feature = its lane of tensor memory
+      const int f = tile.f0 + rank * BF + quarter * 32 + lane;        // this thread's feature = its lane of tensor memory
       const bool f_ok = f < p.n_out;
       // lane j fetches the scores of tokens c + j for this warp's runs c (at most BT / 64 of
       // them) while the tile still accumulates; the loops below take them by shuffle
@@ -362,8 +393,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
         tc::fence_before();
         __syncwarp();
         if (lane == 0) {
-          tc::mbar_arrive(&acc_empty[b]);
-          if (both) tc::mbar_arrive(&acc_empty[1]);
+          written(b);
+          if (both) written(1);
         }
 #pragma unroll
         for (int q = 0; q < RUNS; ++q) {
@@ -378,7 +409,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
       } else {
         // a whole tile goes to `out`; a piece to its place in the scratch memory, [token][feature of the tile]
         const bool cut = work.cut >= 0;
-        float* part = p.scratch + ((size_t)(work.cut * work.pieces + work.piece) * BT) * BF + quarter * 32 + lane;
+        const int tile_cut = PAIR ? 2 * work.cut + rank : work.cut;        // the blocks of a pair bring their halves together apart
+        float* part = p.scratch + ((size_t)(tile_cut * work.pieces + work.piece) * BT) * BF + quarter * 32 + lane;
 #pragma unroll
         for (int q = 0; q < RUNS; ++q) {
           const int c = half * 32 + q * 64;
@@ -409,7 +441,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
         }
         tc::fence_before();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&acc_empty[b]);
+        if (lane == 0) written(b);
         if (cut) {
           // Count this piece in once all eight epilogue warps have written theirs; the last piece of the
           // tile to arrive adds them all, in the order of the pieces. A block has at most one piece (its
@@ -420,10 +452,10 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
           if (warp == 2 && lane == 0) {
             if (tc::mbar_wait(&cut_bar[0], 0)) {
               __threadfence();
-              const int before = atomicAdd(p.counters + work.cut, 1);
+              const int before = atomicAdd(p.counters + tile_cut, 1);
               __threadfence();
               *s_last = before == work.pieces - 1;
-              if (*s_last) p.counters[work.cut] = 0;     // every piece has arrived: ready for the next launch
+              if (*s_last) p.counters[tile_cut] = 0;     // every piece has arrived: ready for the next launch
             } else {
               atomicExch(p.status, 5);
               *s_last = 0;
@@ -436,7 +468,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
             break;
           }
           if (*s_last) {
-            const float* first = p.scratch + ((size_t)(work.cut * work.pieces) * BT) * BF + quarter * 32 + lane;
+            const float* first = p.scratch + ((size_t)(tile_cut * work.pieces) * BT) * BF + quarter * 32 + lane;
 #pragma unroll
             for (int q = 0; q < RUNS; ++q) {
               const int c = half * 32 + q * 64;
@@ -466,9 +498,11 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
   }
   tc::fence_before();
   __syncthreads();
+  if constexpr (PAIR) tc::cluster_meet();       // neither block's barriers or tensor memory are reached for any more
   if (warp == 1) {
     tc::fence_after();
-    tc::dealloc(tmem, TMEM_COLS);
+    if constexpr (PAIR) tc::dealloc_pair(tmem, TMEM_COLS);
+    else tc::dealloc(tmem, TMEM_COLS);
   }
 }
 
@@ -482,19 +516,20 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const in
   for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) d[i] = s[i];
 }
 
-template <bool DUAL, int STAGES, int BT>
+template <bool DUAL, int STAGES, int BT, bool PAIR = false>
 int launch(const void* x, const void* w0, const void* w1, const Params& p, int max_tiles, cudaStream_t stream) {
+  constexpr int XR = PAIR ? BT / 2 : BT;
   Maps maps;
   for (int b = 0; b < 4; ++b)
-    if (!tc::make_map_bf16(&maps.x[b], x, (uint64_t)p.rows, (uint64_t)p.K, (uint32_t)x_box_rows(b, BT))) return HB_ERR_UNSUPPORTED;
+    if (!tc::make_map_bf16(&maps.x[b], x, (uint64_t)p.rows, (uint64_t)p.K, (uint32_t)x_box_rows(b, XR))) return HB_ERR_UNSUPPORTED;
   if (!tc::make_map_bf16(&maps.w0, w0, (uint64_t)p.experts * p.n_out, (uint64_t)p.K, BF) ||
       !tc::make_map_bf16(&maps.w1, DUAL ? w1 : w0, (uint64_t)p.experts * p.n_out, (uint64_t)p.K, BF))
     return HB_ERR_UNSUPPORTED;
-  constexpr int STAGE_BYTES = (DUAL ? 2 : 1) * BF * BK * 2 + BT * BK * 2;
+  constexpr int STAGE_BYTES = (DUAL ? 2 : 1) * BF * BK * 2 + XR * BK * 2;
   static_assert((2 * STAGES + 6) * 8 + 12 <= 256, "the barriers and the tensor-memory slot fit their 256 bytes");
   const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + 4 * ((size_t)p.experts + 2);
   if (smem > 227 * 1024) return HB_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(grouped_gemm_tc_kernel<DUAL, STAGES, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(grouped_gemm_tc_kernel<DUAL, STAGES, BT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return (int)e;
   int dev = 0, sms = 0;
@@ -503,10 +538,27 @@ int launch(const void* x, const void* w0, const void* w1, const Params& p, int m
   // one persistent block per SM; with fewer tiles than SMs, as many blocks as tiles and their pieces can use
   const long long upper = (long long)max_tiles * ((p.n_out + BF - 1) / BF) * (p.scratch ? MAX_PIECES : 1);
   const int grid = (int)(upper < sms ? upper : sms);
-  grouped_gemm_tc_kernel<DUAL, STAGES, BT><<<grid, THREADS, smem, stream>>>(maps, p);
+  if constexpr (PAIR) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid < 2 ? 2 : grid & ~1); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, grouped_gemm_tc_kernel<DUAL, STAGES, BT, PAIR>, maps, p);
+  } else {
+    grouped_gemm_tc_kernel<DUAL, STAGES, BT, PAIR><<<grid, THREADS, smem, stream>>>(maps, p);
+  }
   HB_LAUNCH_CHECK();
   return HB_OK;
 }
+
+// Two blocks a tile (cta_group::2) where experts have many rows: each brings its own 128 rows of a weight and half the tokens, so a
+// stage brings 28 KB where it brought 40 (DUAL 44 and 56, of 128 tokens 40 and 48). us, one block / two, up with gather and down: 2,048
+// tokens, 2 of 8 experts of 2,048 x 4,096 (512 rows each) 132 / 127.5, 73.3 / 68.5; 1,024 (256) 91.4 / 86.4, 50.3 / 47.2; 600, 4 of
+// 16 of 1,024 x 2,048 (150) 45.3 / 49.3, 22.9 / 25.8; 512 (128) 65.2 / 68.2, 39.4 / 40.6: fewer, larger tiles fill the last round worse.
+bool pairs(int rows, int experts) { return rows >= (long long)PAIR_ROWS * experts; }
 
 }  // namespace
 
@@ -534,7 +586,8 @@ extern "C" int hb_moe_gate_up_tc(const void* xs, const int* sorted_entry, const 
   if (max_tiles > 65535) return HB_ERR_UNSUPPORTED;
   Params p{offsets, sorted_entry, scores, act, status, experts, inter, hidden, rows, nullptr, nullptr, limit, 0};
   return few ? launch<true, 5, BT_SHORT>(xs, w_gate, w_up, p, max_tiles, stream)
-             : launch<true, 4, BT_LONG>(xs, w_gate, w_up, p, max_tiles, stream);
+         : pairs(rows, experts) ? launch<true, 5, BT_LONG, true>(xs, w_gate, w_up, p, max_tiles, stream)
+                                : launch<true, 4, BT_LONG>(xs, w_gate, w_up, p, max_tiles, stream);
 }
 
 // down projection on tensor cores: act [rows, inter] -> y float32 [rows, hidden].
@@ -557,7 +610,8 @@ extern "C" int hb_moe_down_tc(const void* act, const void* w_down, const int* of
   const bool room = scratch && counters && n_counters >= sms && scratch_floats >= (long long)sms * bt * BF;
   Params p{offsets, nullptr, nullptr, y, status, experts, hidden, inter, rows, room ? scratch : nullptr, counters, 0.f, 0};
   return few ? launch<false, 8, BT_SHORT>(act, w_down, nullptr, p, max_tiles, stream)
-             : launch<false, 5, BT_LONG>(act, w_down, nullptr, p, max_tiles, stream);
+         : pairs(rows, experts) ? launch<false, 7, BT_LONG, true>(act, w_down, nullptr, p, max_tiles, stream)
+                                : launch<false, 5, BT_LONG>(act, w_down, nullptr, p, max_tiles, stream);
 }
 
 // an expert's up stack alone with the squared relu: xs [rows, hidden] sorted rows -> act bfloat16 [rows, inter]
@@ -573,7 +627,8 @@ extern "C" int hb_moe_up_relu2_tc(const void* xs, const void* w_up, const int* o
   if (max_tiles > 65535) return HB_ERR_UNSUPPORTED;
   Params p{offsets, nullptr, nullptr, act, status, experts, inter, hidden, rows, nullptr, nullptr, 0.f, 1};
   return few ? launch<false, 8, BT_SHORT>(xs, w_up, nullptr, p, max_tiles, stream)
-             : launch<false, 5, BT_LONG>(xs, w_up, nullptr, p, max_tiles, stream);
+         : pairs(rows, experts) ? launch<false, 7, BT_LONG, true>(xs, w_up, nullptr, p, max_tiles, stream)
+                                : launch<false, 5, BT_LONG>(xs, w_up, nullptr, p, max_tiles, stream);
 }
 
 extern "C" long long hb_moe_down_tc_scratch_floats(int sms) { return (long long)sms * BT_LONG * BF; }

@@ -116,6 +116,62 @@ __device__ __forceinline__ void commit_if(uint32_t mine, uint64_t* bar) {
       "setp.ne.b32 e, %1, 0;\n"
       "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(smem_u32(bar)), "r"(mine) : "memory");
 }
+// ---- two blocks of a cluster on one product (cta_group::2): each has its half of A's rows, of B's rows and of the sums' rows, the
+// even one issues. Barriers of the even block are named by their address there (even_block), commits reach both blocks.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t even_block(const void* smem) {
+  uint32_t at;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(smem)), "r"(0));
+  return at;
+}
+__device__ __forceinline__ void arrive_even(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair_if(uint32_t mine, uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred e;\n"
+      "setp.ne.b32 e, %5, 0;\n"
+      "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n}"
+      ::"r"(smem_dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(mine) : "memory");
+}
+__device__ __forceinline__ void mma_pair_if(uint32_t mine, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred e, p;\n"
+      "setp.ne.b32 e, %5, 0;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(mine) : "memory");
+}
+__device__ __forceinline__ void commit_pair_if(uint32_t mine, uint64_t* bar) {
+  asm volatile(
+      "{\n.reg .pred e;\n.reg .b16 both;\n"
+      "setp.ne.b32 e, %1, 0;\n"
+      "mov.b16 both, 3;\n"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n}"
+      ::"r"(smem_u32(bar)), "r"(mine) : "memory");
+}
+__device__ __forceinline__ void alloc_pair(uint32_t* slot_in_smem, uint32_t columns) {      // a warp of either block
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_in_smem)),
+               "r"(columns) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void dealloc_pair(uint32_t taddr, uint32_t columns) {            // the same warps
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_if(uint32_t mine, uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred e;\n"
+      "setp.ne.b32 e, %5, 0;\n"
+      "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n}"
+      ::"r"(smem_dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(mine) : "memory");
+}
 __device__ __forceinline__ void ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
   asm volatile(
