@@ -241,7 +241,7 @@ int hb_delta_out_norm(const float* o, const void* gate, int gate_dtype, const vo
 // A request's state row: [heads][vdim + 1][dim] float32 (S column by column, then n), then m [heads] at m_off.
 int hb_mlstm_gates(const float* z, const float* bias_i, const float* bias_f, float cap, float* state,
                    long long state_stride, long long m_off, const int* cu_seqlens, const int* slots, float* keep,
-                   float* take, float* floor_, int n_seqs, int heads, cudaStream_t stream);
+                   float* take, float* floor_, int n_tokens, int n_seqs, int heads, cudaStream_t stream);
 int hb_mlstm_recurrence(const void* proj, int proj_dtype, long long ld, int q_off, int k_off, int v_off, float q_scale,
                         const float* keep, const float* take, float* state, long long state_stride,
                         const int* cu_seqlens, const int* slots, float* o, float* nq, int n_seqs, int heads, int dim,

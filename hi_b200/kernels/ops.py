@@ -90,7 +90,7 @@ _SIGNATURES = {
     "hb_mamba2_prep": [P, I, c_longlong, I, I, P, P, P, c_longlong, c_longlong, P, P, P, P, P, P, P, P, P, P, I, I, I, I,
                        I, I, P],
     "hb_mamba2_out": [P, P, P, I, c_longlong, P, P, F, P, I, I, I, I, I, P],
-    "hb_mlstm_gates": [P, P, P, F, P, c_longlong, c_longlong, P, P, P, P, P, I, I, P],
+    "hb_mlstm_gates": [P, P, P, F, P, c_longlong, c_longlong, P, P, P, P, P, I, I, I, P],
     "hb_mlstm_recurrence": [P, I, c_longlong, I, I, I, F, P, P, P, c_longlong, P, P, P, P, I, I, I, I, I, P],
     "hb_mlstm_out_norm": [P, P, P, P, I, c_longlong, I, P, I, F, P, I, c_longlong, I, I, P],
 }
@@ -925,7 +925,7 @@ def mlstm_gates(z: torch.Tensor, bias_i: Optional[torch.Tensor], bias_f: Optiona
     keep, take, floor = (torch.empty((n, heads), dtype=torch.float32, device=z.device) for _ in range(3))
     _check(lib().hb_mlstm_gates(_ptr(z), _ptr(bias_i), _ptr(bias_f), float(cap), _ptr(state), state.stride(0),
                                 heads * (vdim + 1) * dim, _ptr(cu_seqlens), _ptr(slots), _ptr(keep), _ptr(take),
-                                _ptr(floor), slots.numel(), heads, _stream()), "mlstm_gates")
+                                _ptr(floor), n, slots.numel(), heads, _stream()), "mlstm_gates")
     return keep, take, floor
 
 
