@@ -248,11 +248,19 @@ __global__ void delta_conv_update_kernel(const void* proj, int proj_dtype, long 
   float* conv = state + (size_t)slots[s] * state_stride + conv_off;
   for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
     // row i of the new state is input (n - (K-1) + i) of the portion; a negative one is row (n + i) of the
-    // old state, which lies behind every row written so far
-    for (int i = 0; i < K - 1; ++i) {
-      const int rel = n - (K - 1) + i;
-      conv[(size_t)i * C + c] = rel >= 0 ? ldf(proj, proj_dtype, (size_t)(start + rel) * ld + chan_off + c)
-                                         : conv[(size_t)(n + i) * C + c];
+    // old state, which lies behind every row written so far. The rows are asked for four at a time: one by one each waited for
+    // the store before it (one token of 5 requests, 6,144 channels, 4 taps 3.9 -> 2.0 us, with blocks for all channels).
+    for (int i0 = 0; i0 < K - 1; i0 += 4) {
+      float row[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int i = i0 + j, rel = n - (K - 1) + i;
+        if (i < K - 1)
+          row[j] = rel >= 0 ? ldf(proj, proj_dtype, (size_t)(start + rel) * ld + chan_off + c) : conv[(size_t)(n + i) * C + c];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j < K - 1) conv[(size_t)(i0 + j) * C + c] = row[j];
     }
   }
 }
@@ -734,7 +742,8 @@ extern "C" int hb_delta_conv_update(const void* proj, int proj_dtype, long long 
   if (!proj || !state || !cu_seqlens || !slots || channels <= 0 || taps_n < 1 || n_seqs < 0) return HB_ERR_BAD_ARG;
   if (n_seqs == 0 || taps_n == 1) return HB_OK;
   int per = (channels + 127) / 128;
-  if (per > 16) per = 16;
+  const int most = n_seqs < 32 ? 64 : 16;
+  if (per > most) per = most;
   delta_conv_update_kernel<<<dim3(n_seqs, per), 128, 0, stream>>>(proj, proj_dtype, ld, chan_off, state, state_stride,
                                                                   conv_off, cu_seqlens, slots, channels, taps_n);
   HB_LAUNCH_CHECK();
