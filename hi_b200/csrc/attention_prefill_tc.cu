@@ -822,7 +822,9 @@ int prefill_tc(const void* q, const void* k_pages, const void* v_pages, const in
          window, skip_single, page_size < BKEYS ? page_size : BKEYS, scale * 1.4426950408889634f, key_splits, part_acc, part_ml, sink, head_bias,
          turn_inside, v_pairs, v_interleaved, v_inv_freq, softcap, slopes, sink_values, slopes ? 1 : 0, keep, pair ? *pair : Pair{}};
   const long long pool_rows = (long long)n_pages * nkv * page_size;
-  if (!pair && !turn_inside && sink != 2 && softcap <= 0.f && !slopes && keep == 0 && hd <= 128) {
+  // (a launch of more pairs than a grid holds goes one tile a block)
+  const long long pairs = ((max_new + 127LL) / 128 * (nh / nkv) + 1) / 2;
+  if (!pair && !turn_inside && sink != 2 && softcap <= 0.f && !slopes && keep == 0 && hd <= 128 && pairs <= 65535) {
     const PrefillPairArgs b{block_table, cu_seqlens, positions, (__nv_bfloat16*)out, status, table_stride, nh, nkv, page_size, chunk, window,
                             skip_single, a.box_rows, a.scale_log2, key_splits, part_acc, part_ml, sink, sink_values};
     return hb_prefill_pair_launch(q, k_pages, v_pages, b, n_tokens, pool_rows, n_seqs, max_new, hd, stream);
