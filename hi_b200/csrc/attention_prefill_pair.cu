@@ -21,6 +21,9 @@
 // begun before the last 32 keys of P are there 215 (64 keys: the same). Two warps that issue the products, one an item, 284: both
 // items then wait for their products at the same time. Rows stored by the lane that holds them, 32 lines an instruction: 2.5 us a
 // pair, by fours of lanes 1.4.
+// Keys are multiplied in steps of 16, those that any row of an item reads: what the pool holds on pages given back reaches no row, rows
+// behind the request's end are cleared, and a value that is not finite reaches rows of its request that come before it where a step of
+// theirs ends behind it (with one tile a block: where their tile did).
 // Every mbarrier wait is bounded; on a time-out a code goes to `status` and the block leaves through the common exit.
 #include <cuda.h>
 #include <cuda_bf16.h>
