@@ -2014,7 +2014,17 @@ def prefill_pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window
 
 
 @functools.lru_cache(maxsize=256)                  # a step's layers ask the same
-def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, rows: int, sms: int, least: int) -> int:
+def prefill_pair_idle_us(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, sms: int) -> float:
+    """By the same model, for how long the SMs of such a launch (one share) are idle on average: its longest blocks against all tiles
+    over all SMs; 0 for launches of less than 80 us: the host's calls take 40
+    with a second stream."""
+    runs = _pair_runs(portions, nh, nkv, chunk, window)
+    tile = 1.515 if hd <= 64 else 1.73
+    longest = max((t for t, _n in runs), default=0)
+    return max(0.0, tile * (longest - sum(t * n for t, n in runs) / sms)) if tile * longest >= 80.0 else 0.0
+
+
+def _pair_runs(portions, nh: int, nkv: int, chunk: int, window: int):
     runs = []                           # (key tiles, blocks), eight runs a portion at most
 
     def visible(first):
@@ -2030,6 +2040,12 @@ def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, 
             first, last = (a + b - 1) // group, min(a + b, items - 1) // group
             end = min(cached + 128 * (last + 1), cached + new) - 1
             runs.append((end // 128 - visible(cached + 128 * first) // 128 + 1, (b - a) * nkv))
+    return runs
+
+
+@functools.lru_cache(maxsize=256)                  # a step's layers ask the same
+def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, rows: int, sms: int, least: int) -> int:
+    runs = _pair_runs(portions, nh, nkv, chunk, window)
     if not runs:
         return 1
     numbers = rows * nh * hd

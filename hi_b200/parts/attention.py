@@ -1,6 +1,7 @@
 """The attention mixer: grouped-query attention over a paged cache, global or windowed."""
 from __future__ import annotations
 
+import threading
 from typing import Optional
 
 import numpy as np
@@ -15,6 +16,20 @@ from .spec import CacheSpec, PartSpec, TensorSpec
 
 DIFF_TC_MIN_TOKENS = 64      # new tokens of a request from which differential attention takes the tcgen05 kernel (its
                              # tile is 64 tokens by two maps)
+
+
+# Where a launch of portions leaves SMs idle for this long (us), the single tokens beside them are decoded on a second stream meanwhile:
+# they take the SMs that are done early (513 tokens behind 7,000, 200 and 129 others beside four single tokens, 40 heads: 141 -> 133 us; 197 such steps
+# 0.90 of the time, the worst 1.07).
+DECODE_ASIDE_IDLE_US = 8.0
+_aside = threading.local()             # a stream and two events per thread and device: joined before the call returns
+
+
+def _decode_aside(device):
+    kept = _aside.__dict__.setdefault("kept", {})
+    if device.index not in kept:
+        kept[device.index] = (torch.cuda.Stream(device=device), torch.cuda.Event(), torch.cuda.Event())
+    return kept[device.index]
 
 
 def _key_splits(ctx, nh: int, nkv: int, hd: int, chunk: int, sliding: int, keep: int, single: bool, pairs: bool, device) -> int:
@@ -69,12 +84,31 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
     if ctx.max_new > 1 and ops.prefill_attention_supported(q.dtype, nh, nkv, hd):
         # portions of prompts (single tokens of other requests ride along as one-row tiles)
         single = ctx.decode_rows is not None and decode_ok
+        pairs = ops.prefill_pairs(hd, softcap, slopes, keep)
         if tc:
+            shares = _key_splits(ctx, nh, nkv, hd, chunk, sliding, keep, single, pairs, q.device)
+            # (the merge of shared keys writes every row, so single tokens wait for it)
+            aside = single and pairs and shares == 1 and ops.prefill_pair_idle_us(
+                tuple((s, n) for s, n in zip(ctx.start_pos, ctx.n_new) if n > 1), nh, nkv, hd, chunk, sliding,
+                ops.sm_count(q.device)) >= DECODE_ASIDE_IDLE_US
+            if aside:
+                current = torch.cuda.current_stream()
+                stream, before, after = _decode_aside(q.device)
+                before.record(current)
             o = ops.prefill_attention_tc(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions,
-                                         ctx.n_seqs, ctx.max_new, chunk, sliding, scale, skip_single=single,
-                                         key_splits=_key_splits(ctx, nh, nkv, hd, chunk, sliding, keep, single,
-                                                                ops.prefill_pairs(hd, softcap, slopes, keep), q.device), sink=sink,
+                                         ctx.n_seqs, ctx.max_new, chunk, sliding, scale, skip_single=single, key_splits=shares, sink=sink,
                                          softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep)
+            if aside:
+                # other rows of the same output; nothing of the call's is freed before the streams have met again
+                stream.wait_event(before)
+                torch.cuda.set_stream(stream)
+                try:
+                    decode(ctx.decode_max_context, ctx.decode_rows, o)
+                finally:
+                    torch.cuda.set_stream(current)
+                    after.record(stream)
+                    current.wait_event(after)
+                return o
         else:
             o = ops.prefill_attention(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions,
                                       ctx.n_seqs, ctx.max_new, chunk, sliding, scale, skip_single=single, sink=sink,

@@ -91,3 +91,58 @@ def test_shares_of_pairs(portions, nh, nkv, hd, chunk, window, least, want):
     """Prompts from the start, short launches and those that fill the GPU stay in one share; few long pairs are shared out."""
     rows = sum(n for _c, n in portions)
     assert ops.prefill_pair_shares(portions, nh, nkv, hd, chunk, window, rows, 148, least) in want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("capture", [False, True])
+def test_single_tokens_decoded_aside(capture, monkeypatch):
+    """Single tokens beside portions that leave SMs idle go on a second stream: the same rows as one after the other, call after call
+    on memory that the calls before gave back, and in a captured step."""
+    from hi_b200.parts import attention as part
+    from hi_b200.parts.context import StepContext
+
+    g = torch.Generator(device=DEV).manual_seed(3)
+    nh, nkv, hd, page = 8, 2, 128, 64
+    lens, starts = [300, 1, 130, 1, 1], [6600, 900, 0, 3, 2500]
+    total = [c + n for c, n in zip(starts, lens)]
+    need = [-(-t // page) for t in total]
+    table, at = torch.zeros(len(lens), max(need), dtype=torch.int32, device=DEV), 0
+    for s, k in enumerate(need):
+        table[s, :k] = torch.arange(at, at + k)
+        at += k
+    kp, vp = (torch.randn(at, nkv, page, hd, device=DEV, generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(sum(lens), nh, hd, device=DEV, generator=g).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    cu = [0] + [sum(lens[: i + 1]) for i in range(len(lens))]
+    singles = [i for i, n in enumerate(lens) if n == 1]
+    ctx = StepContext(n_tokens=cu[-1], n_seqs=len(lens), tokens=i32([0] * cu[-1]),
+                      positions=torch.cat([torch.arange(c, c + n) for c, n in zip(starts, lens)]).int().to(DEV),
+                      seq_of_token=i32([s for s, n in enumerate(lens) for _ in range(n)]), cu_seqlens=i32(cu),
+                      slots=i32(list(range(len(lens)))), start_pos=starts, n_new=lens, slot_ids=list(range(len(lens))), page_size=page,
+                      max_context=max(total))
+    ctx.decode_rows = torch.tensor([cu[i] for i in singles], dtype=torch.int64, device=DEV)
+    ctx.decode_max_context = max(total[i] for i in singles)
+    monkeypatch.setattr(ops, "prefill_pair_shares", lambda *a: 1)
+    idle = ops.prefill_pair_idle_us(((6600, 300), (0, 130)), nh, nkv, hd, 0, 0, ops.sm_count(q.device))
+    assert idle >= part.DECODE_ASIDE_IDLE_US
+    call = lambda: part.attend_over_pages(q, kp, vp, table, ctx, nh, nkv, hd, 0, 0, hd ** -0.5)
+    with monkeypatch.context() as m:
+        m.setattr(part, "DECODE_ASIDE_IDLE_US", 1e9)
+        want = call()
+    if capture:
+        call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = call()
+        for _ in range(5):
+            got.zero_()
+            graph.replay()
+            assert torch.equal(got, want)
+    else:
+        for _ in range(20):
+            got = call()
+            again = torch.full_like(got, 3.0)          # (may take memory that the call gave back)
+            assert torch.equal(got, want) and float(again.float().mean()) == 3.0
+            del got, again
+    ops.check_tc_status()
