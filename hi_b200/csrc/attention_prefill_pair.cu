@@ -374,20 +374,18 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               wait(&p_ready[i], phase[i] & 1, 58 + i);
               if (!ok) break;
               tc::fence_after();
-              if (EARLY < BK) {
-                if (whole) {
-#pragma unroll
-                  for (int t = 0; t < EARLY / 16; ++t)
-                    tc::mma_a_tmem_if(mine, tmem_o[i], tmem_s[i] + t * 8, v + t * (2048 >> 4), idesc_pv, t == 0 ? more : 1u);
-                }
-                wait(&p_rest[i], phase[i] & 1, 70 + i);
-                if (!ok) break;
-                tc::fence_after();
-              }
               if (whole) {
 #pragma unroll
-                for (int t = EARLY < BK ? EARLY / 16 : 0; t < BK / 16; ++t)
+                for (int t = 0; t < EARLY / 16; ++t)
                   tc::mma_a_tmem_if(mine, tmem_o[i], tmem_s[i] + t * 8, v + t * (2048 >> 4), idesc_pv, t == 0 ? more : 1u);
+              }
+              wait(&p_rest[i], phase[i] & 1, 70 + i);
+              if (!ok) break;
+              tc::fence_after();
+              if (whole) {
+#pragma unroll
+                for (int t = EARLY / 16; t < BK / 16; ++t)
+                  tc::mma_a_tmem_if(mine, tmem_o[i], tmem_s[i] + t * 8, v + t * (2048 >> 4), idesc_pv, 1u);
               } else {
 #pragma unroll 1
                 for (int t = from; t <= to; ++t)
@@ -500,7 +498,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             tc::wait_st();
             tc::fence_before();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(EARLY < BK && 32 * (h + 1) == BK ? &p_rest[i] : &p_ready[i]);
+            if (lane == 0) tc::mbar_arrive(32 * (h + 1) == BK ? &p_rest[i] : &p_ready[i]);
           }
         }
         const float2 both = __fadd2_rn(part[0], part[1]);

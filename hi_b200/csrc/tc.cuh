@@ -69,29 +69,7 @@ __device__ __forceinline__ uint32_t elect_one() {
 __device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                    uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The same with A [128 rows x 16 k] read from tensor memory: row i is lane i, its 16 bfloat16 in 8
-// columns from `a_tmem` on, two per column with the lower k in the lower half.
-__device__ __forceinline__ void mma_a_tmem(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The same three, done by the lane whose `mine` is not zero (elect_one's answer) and by no branch: what one warp does between two
+// Products and commits, by the lane whose `mine` is not zero (elect_one's answer) and without a branch: what a warp does between two
 // products stands in the way of the next.
 __device__ __forceinline__ void mma_if(uint32_t mine, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -101,6 +79,8 @@ __device__ __forceinline__ void mma_if(uint32_t mine, uint32_t d_tmem, uint64_t 
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(mine) : "memory");
 }
+// The same with A [128 rows x 16 k] read from tensor memory: row i is lane i, its 16 bfloat16 in 8
+// columns from `a_tmem` on, two per column with the lower k in the lower half.
 __device__ __forceinline__ void mma_a_tmem_if(uint32_t mine, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                               uint32_t accumulate) {
   asm volatile(
