@@ -2010,7 +2010,7 @@ def prefill_pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window
     average; what it chooses takes 0.856 of the time of one share and 1.006 of the best. 40 heads of 128, us in one share and as
     chosen: 128 tokens behind 7,000 101 -> 33, 1,024 behind 16,384 438 -> 336, 150 behind 9,000 beside 700 behind 300 127 -> 85;
     2,048 alone stay in one (50, in two 99)."""
-    return _pair_shares(tuple(portions), nh, nkv, hd, chunk, window, rows, sms, least)
+    return _pair_shares(tuple(portions), nh, nkv, hd, chunk, window, rows, sms, min(least, PREFILL_MOST_SHARES), PREFILL_MOST_SHARES)
 
 
 @functools.lru_cache(maxsize=256)                  # a step's layers ask the same
@@ -2044,7 +2044,7 @@ def _pair_runs(portions, nh: int, nkv: int, chunk: int, window: int):
 
 
 @functools.lru_cache(maxsize=256)                  # a step's layers ask the same
-def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, rows: int, sms: int, least: int) -> int:
+def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, rows: int, sms: int, least: int, limit: int) -> int:
     runs = _pair_runs(portions, nh, nkv, chunk, window)
     if not runs:
         return 1
@@ -2061,7 +2061,7 @@ def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, 
                 most = max(most, turn * t)
         return fixed + tile * most + (merge + (share * k + whole) * numbers / 1e6 if k > 1 else 0.0)
 
-    best = min((k for k in (1, 2, 3, 4, 6, 8) if k >= least), key=cost)
+    best = min(range(least, limit + 1), key=cost)
     return best if least > 1 or cost(best) < min(0.93 * cost(1), cost(1) - 8.0) else 1
 
 

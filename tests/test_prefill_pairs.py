@@ -83,10 +83,10 @@ def test_pairs_of_query_tiles(nh, nkv, hd, page, chunk, window, lens, starts, si
 
 
 @pytest.mark.parametrize("portions,nh,nkv,hd,chunk,window,least,want", [
-    ([(0, 2048)], 40, 8, 128, 0, 0, 1, {1}), ([(7000, 128)], 40, 8, 128, 8192, 0, 1, {4, 6, 8}), ([(0, 128)], 8, 2, 64, 0, 0, 1, {1}),
-    ([(0, 2048)], 40, 8, 128, 0, 0, 2, {2, 3, 4, 6, 8}), ([(9000, 150), (300, 700)], 40, 8, 128, 0, 0, 1, {2, 3, 4}),
+    ([(0, 2048)], 40, 8, 128, 0, 0, 1, {1}), ([(7000, 128)], 40, 8, 128, 8192, 0, 1, {4, 5, 6, 7, 8}), ([(0, 128)], 8, 2, 64, 0, 0, 1, {1}),
+    ([(0, 2048)], 40, 8, 128, 0, 0, 2, {2, 3, 4, 5, 6, 7, 8}), ([(9000, 150), (300, 700)], 40, 8, 128, 0, 0, 1, {2, 3, 4}),
     ([(100000, 128)], 16, 4, 128, 0, 64, 1, {1}), ([], 40, 8, 128, 0, 0, 1, {1}), ([(500, 128)], 8, 2, 128, 0, 0, 1, {1}),
-    ([(20000, 4096)], 24, 24, 64, 0, 0, 1, {1}), ([(65000, 200)], 1, 1, 64, 0, 0, 1, {6, 8})])
+    ([(20000, 4096)], 24, 24, 64, 0, 0, 1, {1}), ([(65000, 200)], 1, 1, 64, 0, 0, 1, {6, 7, 8})])
 def test_shares_of_pairs(portions, nh, nkv, hd, chunk, window, least, want):
     """Prompts from the start, short launches and those that fill the GPU stay in one share; few long pairs are shared out."""
     rows = sum(n for _c, n in portions)
