@@ -285,16 +285,14 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       const int key = first + n * a.box_rows;
       return key <= last ? table[key / a.page_size] : -1;
     };
-    int pages = page_of(lane);
-    bool ok = true;
+    int pages = page_of(lane), tile = 0;
     __syncwarp();
-    for (int tile = 0; tile < n_tiles; ++tile) {
+    for (; tile < n_tiles; ++tile) {
       const int s = tile % STAGES, n = tile * boxes;
       if (n % 32 == 0 && n > 0) pages = page_of(n + lane);
       const int page = __shfl_sync(0xffffffffu, pages, (n + box) % 32);
       if (tile >= STAGES && !tc::mbar_wait_warp(&empty[s], (tile / STAGES - 1) & 1)) {
         if (lane == 0) atomicExch(a.status, 31);
-        ok = false;
         break;
       }
       const bool mine = box < boxes && page >= 0;
@@ -308,8 +306,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
       if (tile == min(n_tiles, STAGES) - 1) __syncthreads();         // the others may wait on the barriers
     }
-    // no copy is under way when the block ends, whoever gave up
-    for (int tile = max(0, n_tiles - STAGES); ok && tile < n_tiles; ++tile) tc::mbar_wait_warp(&full[tile % STAGES], (tile / STAGES) & 1);
+    // no copy is under way when the block ends, whoever gave up: this warp too waits for the tiles that it has asked for
+    for (int i = max(0, tile - STAGES); i < tile; ++i) tc::mbar_wait_warp(&full[i % STAGES], (i / STAGES) & 1);
     return;
   }
 
