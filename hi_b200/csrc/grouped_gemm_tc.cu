@@ -238,6 +238,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
 
   if (warp == 0) {                              // ---- TMA producer: the whole warp waits, one lane issues
     int s = 0, turn = 1;                        // (the first wait on a fresh barrier for the phase before it returns at once)
+    int issued = 0;
     bool ok = true;
     const uint32_t mine = tc::elect_one(), ring = tc::smem_u32(smem);
     const uint32_t bars = PAIR ? tc::even_block(full) : tc::smem_u32(full);
@@ -269,7 +270,17 @@ grouped_gemm_tc_kernel(const __grid_constant__ Maps maps, const Params p) {
           tc::tma_load_2d_if(mine, st + NW * W_BYTES, x_map, kb * BK, x_row, bar);
         }
         if (++s == STAGES) { s = 0; turn ^= 1; }
+        ++issued;
       }
+    }
+    // The block leaves when nothing reaches for its memory any more: the commits on every stage's `empty` have arrived, those of the even
+    // block here too (they come behind the products, which come behind the copies). Where a wait ran out those may never come: then the
+    // copies on their way are waited for, by the block whose barriers count them; the odd one of a pair stays for it below.
+    if (ok) {
+      for (int i = 0; i < STAGES && tc::mbar_wait_warp(&empty[s], turn); ++i)
+        if (++s == STAGES) { s = 0; turn ^= 1; }
+    } else if (rank == 0) {
+      for (int i = max(0, issued - STAGES); i < issued; ++i) tc::mbar_wait_warp(&full[i % STAGES], (i / STAGES) & 1);
     }
   } else if (warp == 1) {                       // ---- MMA issuer: the whole warp walks, one lane issues
     const uint32_t mine = tc::elect_one();
