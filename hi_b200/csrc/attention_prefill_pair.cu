@@ -303,10 +303,10 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
         if (ok) bid();
       }
-      if (lane == 0) {                          // no copy is under way when the block ends, whoever gave up
-        if (queries > 0) tc::mbar_wait(q_full, (queries - 1) & 1);
-        for (int i = max(0, n - STAGES); i < n; ++i) tc::mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
-      }
+      // nothing reaches for the block's memory when it ends: the commits on the last stages have arrived, which come behind their copies;
+      // where a wait ran out they may never come, and the copies on their way are waited for
+      if (!ok && queries > 0) tc::mbar_wait_warp(q_full, (queries - 1) & 1);
+      for (int i = max(0, n - STAGES); i < n; ++i) tc::mbar_wait_warp(ok ? &empty[i % STAGES] : &full[i % STAGES], (i / STAGES) & 1);
     } else if (warp == 9) {                     // ---- the products: the whole warp walks, one lane issues
       constexpr uint32_t idesc_qk = tc::idesc_bf16(BQ, BK, false);
       constexpr uint32_t idesc_pv = tc::idesc_bf16(BQ, HD, true);
