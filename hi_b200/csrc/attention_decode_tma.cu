@@ -46,11 +46,18 @@ constexpr int TILE = 64;     // keys per shared-memory tile
 constexpr int NWARPS = 4;    // that compute; one more warp brings the tiles in
 constexpr int COMP = NWARPS * 32;
 constexpr int ROWS = 16;     // query rows of the tile (heads of one kv group, padded)
+// How a token's splits come together: by hb_attention_merge; in the block that finishes last (the fused form); among the
+// blocks of a cluster, which read one another's shared memory.
+enum Merge { APART, FUSED_FORM, CLUSTER };
 // Tiles in flight and blocks an SM: rows of 128 two and three (three and two blocks are as fast where each has its best split), rows of
 // 64 three and four, or two and five where a split has no more than two tiles (us, two and five / three and four: 16 tokens of 4,000
-// keys, 40 heads on 8, 26.0 / 22.8; 10 of 10,000, 8 on 2, 15.7 / 13.9, 32 on 8 31.8 / 36.3; 30 of 108, 24 on 24, 8.6 / 10.8).
-template <int HD> constexpr int STAGES_OF = HD == 128 ? 2 : 3;
-template <int HD, int STAGES> constexpr int BLOCKS_OF = HD == 128 ? 3 : STAGES == 2 ? 5 : 4;
+// keys, 40 heads on 8, 26.0 / 22.8; 10 of 10,000, 8 on 2, 15.7 / 13.9, 32 on 8 31.8 / 36.3; 30 of 108, 24 on 24, 8.6 / 10.8). The fused
+// form encodes rows first and needs 122 and 168 registers for it: three tiles and three blocks of rows of 64, two of rows of 128. Held
+// to the others' 72 to 128 registers it spilled up to 224 bytes a thread (us, so / now: 8 tokens of 4,000 keys, 32 heads on 8, rows of 64,
+// 20.7 / 16.7; rows of 128, 40 on 8, 32 tokens of 2,048 45.7 / 38.8, 2 of 8,192 20.8 / 19.3, ops._fused_splits' cuts).
+template <int HD, Merge MERGE> constexpr int STAGES_OF = HD == 128 && MERGE != FUSED_FORM ? 2 : 3;
+template <int HD, int STAGES, Merge MERGE> constexpr int BLOCKS_OF =
+    MERGE == FUSED_FORM ? (HD == 128 ? 2 : 3) : HD == 128 ? 3 : STAGES == 2 ? 5 : 4;
 constexpr int HALF_BYTES = TILE * 128;   // a tile's 64 rows x 64 dims (128 bytes a row)
 
 struct Args {
@@ -181,9 +188,6 @@ __device__ __forceinline__ uint32_t tile_offset(int r, int d) {
   return (uint32_t)((d >> 6) * HALF_BYTES + r * 128 + ((((d & 63) >> 3) ^ (r & 7)) << 4));
 }
 
-// How a token's splits come together: by hb_attention_merge; in the block that finishes last (the fused form); among the
-// blocks of a cluster, which read one another's shared memory.
-enum Merge { APART, FUSED_FORM, CLUSTER };
 constexpr int MAX_CLUSTER = 8;
 
 // a barrier of the computing warps; and one over which they agree
@@ -217,7 +221,7 @@ __device__ __forceinline__ float4 load4_cluster(uint32_t at) {
 }
 
 template <int HD, int STAGES, Merge MERGE>
-__global__ void __launch_bounds__(COMP + 32, (BLOCKS_OF<HD, STAGES>))
+__global__ void __launch_bounds__(COMP + 32, (BLOCKS_OF<HD, STAGES, MERGE>))
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Args a,
                        const Fuse f) {
   constexpr bool FUSED = MERGE == FUSED_FORM;
@@ -675,7 +679,7 @@ inline void cluster_of(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, dim3 
 
 template <int HD>
 int clusters_at_once(int splits) {
-  constexpr int STAGES = STAGES_OF<HD>;
+  constexpr int STAGES = STAGES_OF<HD, CLUSTER>;
   constexpr size_t smem = smem_bytes<HD, STAGES>();
   cudaLaunchAttribute attr;
   cudaLaunchConfig_t cfg = {};
@@ -690,10 +694,10 @@ int clusters_at_once(int splits) {
   return n;
 }
 
-template <int HD, Merge MERGE, int STAGES = STAGES_OF<HD>>
+template <int HD, Merge MERGE, int STAGES = STAGES_OF<HD, MERGE>>
 int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, const Args& a, const Fuse& f,
            cudaStream_t stream) {
-  if constexpr (HD == 64 && STAGES == STAGES_OF<HD>)
+  if constexpr (HD == 64 && MERGE != FUSED_FORM && STAGES == STAGES_OF<HD, MERGE>)
     if (a.split_size <= 2 * TILE) return launch<HD, MERGE, 2>(k_pages, v_pages, n_pages, n_tokens, a, f, stream);
   const uint64_t pool_rows = (uint64_t)n_pages * a.nkv * a.page_size;
   CUtensorMap mk, mv;

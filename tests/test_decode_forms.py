@@ -1,0 +1,63 @@
+"""The decode attention by TMA: what its forms are compiled to, how they are cut, and the results at the cuts."""
+import os
+import re
+import subprocess
+
+import pytest
+import torch
+
+from hi_b200.kernels import build, ops
+
+DEV = "cuda:0"
+
+
+def test_the_fused_form_keeps_its_registers(tmp_path):
+    """Its blocks an SM leave it the registers that it needs: held to the other forms' it spilled up to 224 bytes a thread."""
+    source = os.path.join(build.CSRC, "attention_decode_tma.cu")
+    out = subprocess.run([build._nvcc(), *build.ARCH_FLAGS, *build.NVCC_FLAGS, "-Xptxas", "-v", "-I", build.CSRC, "-c", source, "-o",
+                          str(tmp_path / "x.o")], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, check=True).stdout
+    spills = {name: int(n) for name, n in re.findall(r"Function properties for (\S+)\s+\d+ bytes stack frame, (\d+) bytes spill stores", out)}
+    fused = {name: n for name, n in spills.items() if "attn_decode_tma_kernel" in name and "MergeE1E" in name}
+    assert len(fused) == 2 and not any(fused.values()), spills
+
+
+@pytest.mark.parametrize("hd,resident", [(64, 444), (128, 296)])
+def test_the_fused_form_is_cut_for_its_own_merge_and_blocks(hd, resident):
+    for groups in (1, 2, 8, 40, 100, 148, 149, 200, 222, 223, 256):
+        for tiles in (1, 2, 3, 4, 7, 16, 33, 125, 1024, 4096):
+            size, splits = ops._fused_splits(tiles, groups, hd)
+            assert size % 64 == 0 and (splits - 1) * size < 64 * tiles <= splits * size and splits <= 48
+            assert splits == 1 or size >= 128
+            assert splits * groups <= resident or (splits <= 4 and 2 * groups > resident)
+    want = {64: {(63, 64): {4, 5, 6}, (1, 256): {1}, (5, 256): {1}}, 128: {(128, 64): {4}, (32, 256): {1}, (1024, 32): {8, 9}, (128, 16): range(13, 19)}}
+    for (tiles, groups), splits in want[hd].items():
+        assert ops._fused_splits(tiles, groups, hd)[1] in splits, (tiles, groups)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nh,nkv,hd", [(6, 2, 64), (16, 1, 128)])
+@pytest.mark.parametrize("size", [64, 192, 256, 448])           # one tile a split; as many as are in flight; one more; the ring goes round
+def test_fused_decode_at_the_ends_of_its_ring(nh, nkv, hd, size, monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(size + hd)
+    lens = [1, 64, 65, 193, 448, 449, 1000]
+    need = [-(-k // 64) for k in lens]
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    kp, vp, qkv = rnd(sum(need), nkv, 64, hd), rnd(sum(need), nkv, 64, hd), rnd(len(lens), (nh + 2 * nkv) * hd)
+    table, at = torch.full((len(lens), max(need)), -1, dtype=torch.int32, device=DEV), 0
+    for i, k in enumerate(need):
+        table[i, :k] = torch.arange(at, at + k)
+        at += k
+    pos = torch.tensor([k - 1 for k in lens], dtype=torch.int32, device=DEV)
+    seq = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    monkeypatch.setattr(ops, "_fused_splits", lambda *a: (size, -(-max(lens) // size)))
+    k1, v1 = kp.clone(), vp.clone()
+    got = ops.decode_attention_fused(qkv, nh, nkv, hd, pos, None, False, False, 1e-6, None, seq, table, k1, v1, 0, 0, hd ** -0.5, max(lens))
+    ops.check_tc_status()
+    q, k_new, v_new = (x.view(len(lens), -1, hd) for x in qkv.split([nh * hd, nkv * hd, nkv * hd], dim=1))
+    for i, k in enumerate(lens):
+        rows = lambda t, new: torch.cat([t[table[i, : need[i]].long()].transpose(1, 2).reshape(-1, nkv, hd)[: k - 1], new[i: i + 1]]).double() \
+            .repeat_interleave(nh // nkv, dim=1)
+        p = torch.softmax(torch.einsum("hd,khd->hk", q[i].double(), rows(kp, k_new)) * hd ** -0.5, dim=1)
+        want = torch.einsum("hk,khd->hd", p, rows(vp, v_new))
+        # weights and the result in bfloat16, 2^-9 each, of the largest value
+        assert float((got[i].double() - want).abs().max()) <= 2 ** -7 * float(want.abs().max()), (i, k)
