@@ -29,10 +29,16 @@ def test_splits_meet_in_a_cluster(nh, nkv, hd, lens, page, chunk, sink, splits, 
     pos = torch.tensor([k - 1 for k in lens], dtype=torch.int32)
     args = [t.to(DEV) for t in (q, kp, vp, table, torch.arange(n, dtype=torch.int32), pos)]
     call = lambda: ops.decode_attention(*args, chunk, 0, hd ** -0.5, max(lens), sink=sink)
-    assert ops._decode_splits(min(max(lens), chunk or max(lens)), n * nkv)[1] == splits
+    # every number of splits from 1 to 9 runs for rows of either length, whatever the model of the time would choose
+    longest = min(max(lens), chunk or max(lens))
+    size = -(-(-(-longest // 64)) // splits) * 64
+    assert -(-longest // size) == splits
+    asked = []
+    monkeypatch.setattr(ops, "_decode_splits", lambda *a: (asked.append(a), (size, splits))[1])
     before = ops.CALLS.get("attention_merge", 0)
     got = call()
     assert ops.CALLS.get("attention_merge", 0) - before == (splits > 8)
+    assert asked == [(longest, n * nkv, hd, 0)]
     assert torch.equal(got, call())                        # the blocks of a cluster finish in any order: the sum has one
     monkeypatch.setattr(ops, "DECODE_CLUSTER", 1)
     apart = call()
