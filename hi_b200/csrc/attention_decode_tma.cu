@@ -50,14 +50,18 @@ constexpr int ROWS = 16;     // query rows of the tile (heads of one kv group, p
 // blocks of a cluster, which read one another's shared memory.
 enum Merge { APART, FUSED_FORM, CLUSTER };
 // Tiles in flight and blocks an SM: rows of 128 two and three (three and two blocks are as fast where each has its best split), rows of
-// 64 three and four, or two and five where a split has no more than two tiles (us, two and five / three and four: 16 tokens of 4,000
-// keys, 40 heads on 8, 26.0 / 22.8; 10 of 10,000, 8 on 2, 15.7 / 13.9, 32 on 8 31.8 / 36.3; 30 of 108, 24 on 24, 8.6 / 10.8). The fused
+// 64 three and four (two and five are slower while one round holds the launch; us, two and five / three and four: 16 tokens of 3,943
+// keys, 40 heads on 8, 26.4 / 22.9; 10 of 8,619, 32 on 8, 33.9 / 28.7). Launches of more blocks of rows of 64 than that: where a split has
+// no more than two tiles, or of up to five and in fewer rounds so, two and six, without a warp for the loads: 128 threads of 80 registers (34 tokens
+// of 80 keys, 24 heads on 24: 9.3, 11.8 with the warp; 64 of 91 15.7, 17.6; 36 of 191 12.1, 14.4; 47 of 280, two rounds either way, 20.3 / 17.6). The fused
 // form encodes rows first and needs 122 and 168 registers for it: three tiles and three blocks of rows of 64, two of rows of 128. Held
 // to the others' 72 to 128 registers it spilled up to 224 bytes a thread (us, so / now: 8 tokens of 4,000 keys, 32 heads on 8, rows of 64,
 // 20.7 / 16.7; rows of 128, 40 on 8, 32 tokens of 2,048 45.7 / 38.8, 2 of 8,192 20.8 / 19.3, ops._fused_splits' cuts).
 template <int HD, Merge MERGE> constexpr int STAGES_OF = HD == 128 && MERGE != FUSED_FORM ? 2 : 3;
-template <int HD, int STAGES, Merge MERGE> constexpr int BLOCKS_OF =
-    MERGE == FUSED_FORM ? (HD == 128 ? 2 : 3) : HD == 128 ? 3 : STAGES == 2 ? 5 : 4;
+template <int HD, int STAGES, Merge MERGE, bool LOADER> constexpr int BLOCKS_OF =
+    !LOADER ? 6 : MERGE == FUSED_FORM ? (HD == 128 ? 2 : 3) : HD == 128 ? 3 : 4;
+template <bool LOADER> constexpr int THREADS_OF = COMP + (LOADER ? 32 : 0);
+constexpr int ROUND_64 = 4 * 148, ROUND_64_SHORT = 6 * 148;    // blocks of rows of 64 that live at a time, with the loads' warp and without
 constexpr int HALF_BYTES = TILE * 128;   // a tile's 64 rows x 64 dims (128 bytes a row)
 
 struct Args {
@@ -220,8 +224,9 @@ __device__ __forceinline__ float4 load4_cluster(uint32_t at) {
   return v;
 }
 
-template <int HD, int STAGES, Merge MERGE>
-__global__ void __launch_bounds__(COMP + 32, (BLOCKS_OF<HD, STAGES, MERGE>))
+// Without LOADER no warp is there for the loads alone: the first of the computing warps asks for the tiles.
+template <int HD, int STAGES, Merge MERGE, bool LOADER>
+__global__ void __launch_bounds__(THREADS_OF<LOADER>, (BLOCKS_OF<HD, STAGES, MERGE, LOADER>))
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Args a,
                        const Fuse f) {
   constexpr bool FUSED = MERGE == FUSED_FORM;
@@ -266,7 +271,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if (first > pos) {                                          // this token has fewer splits
     if (MERGE == CLUSTER) {                                   // (the barrier of a cluster counts the threads still there)
       if (split == 0)
-        for (int i = tid; i < G * HD; i += COMP + 32) a.out[qh0 * HD + i] = __float2bfloat16_rn(0.f);
+        for (int i = tid; i < G * HD; i += THREADS_OF<LOADER>) a.out[qh0 * HD + i] = __float2bfloat16_rn(0.f);
     } else if (!merge_inside && a.max_splits > 1 && tid < G) {
       float* ml = a.part_ml + ((th0 + tid) * a.max_splits + split) * 2;
       ml[0] = -INFINITY; ml[1] = 0.f;
@@ -277,42 +282,53 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int n_tiles = (last - first + TILE) / TILE;
 
   // The last warp brings the tiles in: for every page under a tile (one, or 64 / page_size of them) that holds a key of the range,
-  // the page's rows of K and of V, 64 dims per copy and lane. The ids of 32 pages are asked for at a time.
-  if (warp == NWARPS) {
+  // the page's rows of K and of V, 64 dims per copy and lane. The ids of 32 pages are asked for at a time. Without LOADER the first warp
+  // does it: the first tiles here, each later one when all warps are through with the tile in its place.
+  const int boxes = TILE / a.box_rows;             // box_rows: min(page_size, 64)
+  const int box = lane / (2 * HALVES), half = lane % HALVES, is_v = lane / HALVES % 2;      // of this lane's copy
+  auto page_of = [&](int n) {                      // of box n of the range
+    const int key = first + n * a.box_rows;
+    return key <= last ? table[key / a.page_size] : -1;
+  };
+  int pages = -1, asked = 0;                       // tiles asked for
+  auto bring = [&]() {                             // the next tile; false: its place was not given back in time
+    const int tile = asked, s = tile % STAGES, n = tile * boxes;
+    if (n % 32 == 0 && n > 0) pages = page_of(n + lane);
+    const int page = __shfl_sync(0xffffffffu, pages, (n + box) % 32);
+    if (tile >= STAGES && !tc::mbar_wait_warp(&empty[s], (tile / STAGES - 1) & 1)) {
+      if (lane == 0) atomicExch(a.status, 31);
+      return false;
+    }
+    const bool mine = box < boxes && page >= 0;
+    const uint32_t copies = __popc(__ballot_sync(0xffffffffu, mine));
+    if (lane == 0) tc::mbar_expect_tx(&full[s], copies * a.box_rows * 128);
+    __syncwarp();
+    if (mine) {
+      const int at = first + tile * TILE + box * a.box_rows;
+      tc::tma_load_2d((is_v ? v_s : k_s) + s * KV_BYTES + half * HALF_BYTES + box * a.box_rows * 128, is_v ? &map_v : &map_k,
+                      half * 64, (page * a.nkv + kvh) * a.page_size + at % a.page_size, &full[s]);
+    }
+    ++asked;
+    return true;
+  };
+  // no copy is under way when the block ends, whoever gave up: the warp that asked waits for its last tiles in any case
+  auto settle = [&]() {
+    for (int i = max(0, asked - STAGES); i < asked; ++i) tc::mbar_wait_warp(&full[i % STAGES], (i / STAGES) & 1);
+  };
+  if (warp == (LOADER ? NWARPS : 0)) {
+    pages = page_of(lane);
     if (lane == 0) {
       for (int s = 0; s < STAGES; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], NWARPS); }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const int boxes = TILE / a.box_rows;           // box_rows: min(page_size, 64)
-    const int box = lane / (2 * HALVES), half = lane % HALVES, is_v = lane / HALVES % 2;    // of this lane's copy
-    auto page_of = [&](int n) {                    // of box n of the range
-      const int key = first + n * a.box_rows;
-      return key <= last ? table[key / a.page_size] : -1;
-    };
-    int pages = page_of(lane), tile = 0;
     __syncwarp();
-    for (; tile < n_tiles; ++tile) {
-      const int s = tile % STAGES, n = tile * boxes;
-      if (n % 32 == 0 && n > 0) pages = page_of(n + lane);
-      const int page = __shfl_sync(0xffffffffu, pages, (n + box) % 32);
-      if (tile >= STAGES && !tc::mbar_wait_warp(&empty[s], (tile / STAGES - 1) & 1)) {
-        if (lane == 0) atomicExch(a.status, 31);
-        break;
-      }
-      const bool mine = box < boxes && page >= 0;
-      const uint32_t copies = __popc(__ballot_sync(0xffffffffu, mine));
-      if (lane == 0) tc::mbar_expect_tx(&full[s], copies * a.box_rows * 128);
-      __syncwarp();
-      if (mine) {
-        const int at = first + tile * TILE + box * a.box_rows;
-        tc::tma_load_2d((is_v ? v_s : k_s) + s * KV_BYTES + half * HALF_BYTES + box * a.box_rows * 128, is_v ? &map_v : &map_k,
-                        half * 64, (page * a.nkv + kvh) * a.page_size + at % a.page_size, &full[s]);
-      }
-      if (tile == min(n_tiles, STAGES) - 1) __syncthreads();         // the others may wait on the barriers
+    while (asked < min(n_tiles, STAGES)) bring();
+    if constexpr (LOADER) {
+      __syncthreads();                             // the others may wait on the barriers
+      while (asked < n_tiles && bring()) {}
+      settle();
+      return;
     }
-    // no copy is under way when the block ends, whoever gave up: this warp too waits for the tiles that it has asked for
-    for (int i = max(0, tile - STAGES); i < tile; ++i) tc::mbar_wait_warp(&full[i % STAGES], (i / STAGES) & 1);
-    return;
   }
 
   // the query rows of this kv group
@@ -481,7 +497,11 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(&empty[buf]);   // this warp is done with the buffer
+    if constexpr (!LOADER)
+      if (warp == 0 && asked < n_tiles && !bring()) { ok = false; break; }
   }
+  if constexpr (!LOADER)
+    if (!ok && warp == 0) settle();                // (else it has seen them all land)
   ok = comp_and(ok);        // every warp is done with the tiles; and they agree on whether all of them arrived
   // fused form: the blocks of a (token, kv head) count themselves in; the last one combines the splits
   const bool counted = merge_inside && n_splits > 1;
@@ -685,20 +705,23 @@ int clusters_at_once(int splits) {
   cudaLaunchConfig_t cfg = {};
   cluster_of(cfg, attr, dim3(splits, 1, 1), smem, nullptr);
   int n = 0;
-  if (cudaFuncSetAttribute(attn_decode_tma_kernel<HD, STAGES, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  if (cudaFuncSetAttribute(attn_decode_tma_kernel<HD, STAGES, CLUSTER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<HD, STAGES, CLUSTER>, &cfg) != cudaSuccess) {
+      cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<HD, STAGES, CLUSTER, true>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return n;
 }
 
-template <int HD, Merge MERGE, int STAGES = STAGES_OF<HD, MERGE>>
+template <int HD, Merge MERGE, int STAGES = STAGES_OF<HD, MERGE>, bool LOADER = true>
 int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, const Args& a, const Fuse& f,
            cudaStream_t stream) {
-  if constexpr (HD == 64 && MERGE != FUSED_FORM && STAGES == STAGES_OF<HD, MERGE>)
-    if (a.split_size <= 2 * TILE) return launch<HD, MERGE, 2>(k_pages, v_pages, n_pages, n_tokens, a, f, stream);
+  if constexpr (HD == 64 && MERGE == APART && STAGES == 3) {
+    const long long blocks = (long long)a.max_splits * a.nkv * n_tokens;
+    if (blocks > ROUND_64 && (a.split_size <= 2 * TILE || (a.split_size <= 5 * TILE && (blocks - 1) / ROUND_64_SHORT < (blocks - 1) / ROUND_64)))
+      return launch<HD, MERGE, 2, false>(k_pages, v_pages, n_pages, n_tokens, a, f, stream);
+  }
   const uint64_t pool_rows = (uint64_t)n_pages * a.nkv * a.page_size;
   CUtensorMap mk, mv;
   if (!tc::make_map_bf16(&mk, k_pages, pool_rows, HD, a.box_rows) || !tc::make_map_bf16(&mv, v_pages, pool_rows, HD, a.box_rows))
@@ -709,18 +732,18 @@ int launch(const void* k_pages, const void* v_pages, int n_pages, int n_tokens, 
   static_assert((size_t)STAGES * KV_BYTES >= (size_t)ROWS * HD * sizeof(float), "o_s aliases the K tiles");
   // the fused merge keeps [G][splits] weights and [G] sums where the V tiles were
   if (FUSED && (size_t)(a.nh / a.nkv) * (2 * a.max_splits + 1) * sizeof(float) > (size_t)STAGES * KV_BYTES) return HB_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<HD, STAGES, MERGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<HD, STAGES, MERGE, LOADER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   dim3 grid(a.max_splits, a.nkv, n_tokens);
   if (MERGE == CLUSTER) {
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = {};
     cluster_of(cfg, attr, grid, smem, stream);
-    cudaLaunchKernelEx(&cfg, attn_decode_tma_kernel<HD, STAGES, MERGE>, mk, mv, a, f);
+    cudaLaunchKernelEx(&cfg, attn_decode_tma_kernel<HD, STAGES, MERGE, LOADER>, mk, mv, a, f);
     HB_LAUNCH_CHECK();
     return HB_OK;
   }
-  attn_decode_tma_kernel<HD, STAGES, MERGE><<<grid, COMP + 32, smem, stream>>>(mk, mv, a, f);
+  attn_decode_tma_kernel<HD, STAGES, MERGE, LOADER><<<grid, THREADS_OF<LOADER>, smem, stream>>>(mk, mv, a, f);
   HB_LAUNCH_CHECK();
   return HB_OK;
 }

@@ -1389,9 +1389,11 @@ def _decode_splits(longest: int, groups: int, hd: int = 0, device: int = -1) -> 
     8 requests x 8,192 keys: 6 splits (one wave of 384 blocks) 57 us, 13 splits (two waves) 63 us;
     one request x 32,768 keys: 32 splits 33 us, 47 splits 36 us.
     The cut moves results by rounding only. With ``hd`` and ``device``: for the kernel whose tiles come by TMA; rows
-    of 128 have a model of their own there (:func:`_tma_splits`)."""
+    of 128 and of 64 have models of their own there (:func:`_tma_splits`, :func:`_tma_splits_64`)."""
     if hd == 128:
         return _tma_splits(-(-longest // 64), groups, device, DECODE_CLUSTER + 1 if _decode_splits(longest, groups)[1] > DECODE_CLUSTER else 1)
+    if hd == 64:
+        return _tma_splits_64(-(-longest // 64), groups, device)
     best = (None, 1, longest)
     for s in range(1, max(1, -(-longest // ATTENTION_SPLIT)) + 1):
         size = -(-(-(-longest // s)) // 64) * 64
@@ -1420,6 +1422,28 @@ def _tma_splits(tiles: int, groups: int, device: int, least: int) -> Tuple[int, 
         if real > 1:
             met = real <= DECODE_CLUSTER and groups <= _decode_clusters(device, 128, real)
             cost += 0.023 * real if met else 3.4 + 0.000215 * real * groups
+        if best[0] is None or cost < best[0]:
+            best = (cost, 64 * size, real)
+    return best[1], best[2]
+
+
+def _tma_splits_64(tiles: int, groups: int, device: int) -> Tuple[int, int]:
+    """The same for rows of 64, of which 592 blocks live at a time (888 of the form for short splits of many blocks:
+    ``launch`` of attention_decode_tma.cu): no more splits than one round holds, as contexts are seldom all as long as the longest
+    and a second round that a few blocks start costs as much as a full one. Fitted to 522 steps of 1 to 64 tokens, up to 16,384 keys, in up
+    to 18 cuts each: what it takes is 1.014 of the best cut's time on average, 1.21 at worst; :func:`_decode_splits`'s own 1.023 and 1.68 (12 tokens
+    of 12,056 keys, 40 heads on 8, 9 splits / 6: 54.8 / 43.2 us; 64 of 991, 32 on 8, 4 / 1: 28.6 / 19.3)."""
+    best = (None, 64 * tiles, 1)
+    for s in range(1, max(1, min(tiles // 2, 48, 592 // groups)) + 1):
+        size = -(-tiles // s)
+        real = -(-tiles // size)
+        blocks = real * groups
+        met = 1 < real <= DECODE_CLUSTER and groups <= _decode_clusters(device, 64, real)
+        short = not met and blocks > 592 and (size <= 2 or size <= 5 and (blocks - 1) // 888 < (blocks - 1) // 592)
+        waves = -(-blocks // (888 if short else 592))
+        cost = max(waves * (5.17 + 0.514 * size), 0.00127 * groups * tiles + 0.329 * size + 5.35 * waves)
+        if real > 1:
+            cost += 0.147 * real + 0.00258 * blocks if met else 1.39 + 0.084 * real + 0.00146 * blocks
         if best[0] is None or cost < best[0]:
             best = (cost, 64 * size, real)
     return best[1], best[2]

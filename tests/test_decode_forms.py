@@ -61,3 +61,39 @@ def test_fused_decode_at_the_ends_of_its_ring(nh, nkv, hd, size, monkeypatch):
         want = torch.einsum("hk,khd->hd", p, rows(vp, v_new))
         # weights and the result in bfloat16, 2^-9 each, of the largest value
         assert float((got[i].double() - want).abs().max()) <= 2 ** -7 * float(want.abs().max()), (i, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,nh,nkv,longest,size", [
+    (25, 24, 24, 128, 128), (64, 20, 10, 65, 128), (40, 24, 24, 64, 64),         # 600 to 960 blocks of one or two tiles: no warp for the loads
+    (31, 24, 24, 140, 192), (50, 30, 15, 320, 320), (56, 24, 24, 300, 320),      # of three to five in a round less: places are given back
+    (38, 16, 16, 300, 128), (47, 24, 24, 321, 384), (13, 24, 24, 300, 128)])     # several short splits a token; with the warp again
+def test_rows_of_64_in_launches_of_many_blocks(n, nh, nkv, longest, size, monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(n + longest)
+    lens = [max(1, longest - 7 * i % longest) for i in range(n)]
+    need = -(-longest // 32)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    kp, vp, q = rnd(n * need, nkv, 32, 64), rnd(n * need, nkv, 32, 64), rnd(n, nh, 64)
+    table = torch.randperm(n * need, device=DEV, generator=g).int().view(n, need)
+    pos = torch.tensor([k - 1 for k in lens], dtype=torch.int32, device=DEV)
+    for i, k in enumerate(lens):                                # pages that a token does not reach are given back
+        table[i, -(-k // 32):] = -1
+    monkeypatch.setattr(ops, "_decode_splits", lambda *a: (size, -(-longest // size)))
+    got = ops.decode_attention(q, kp, vp, table, torch.arange(n, dtype=torch.int32, device=DEV), pos, 0, 0, 0.125, longest)
+    ops.check_tc_status()
+    for i, k in enumerate(lens):
+        rows = lambda t: t[table[i, : -(-k // 32)].long()].transpose(1, 2).reshape(-1, nkv, 64)[:k].double().repeat_interleave(nh // nkv, dim=1)
+        p = torch.softmax(torch.einsum("hd,khd->hk", q[i].double(), rows(kp)) * 0.125, dim=1)
+        want = torch.einsum("hk,khd->hd", p, rows(vp))
+        # weights and the result in bfloat16, 2^-9 each, of the largest value
+        assert float((got[i].double() - want).abs().max()) <= 2 ** -7 * float(want.abs().max()), (i, k)
+
+
+@pytest.mark.parametrize("hd,groups,tiles,splits", [(64, 96, 189, {6}), (64, 512, 16, {1}), (64, 8, 125, range(8, 25)), (64, 720, 2, {1})])
+def test_rows_of_64_are_cut_for_one_round(hd, groups, tiles, splits, monkeypatch):
+    fit = {2: 296, 3: 187, 4: 142, 5: 112, 6: 93, 7: 78, 8: 71}
+    monkeypatch.setattr(ops, "_decode_clusters", lambda device, hd, real: fit[real])
+    ops._decode_splits.cache_clear()
+    size, real = ops._decode_splits(64 * tiles, groups, hd, 99)
+    ops._decode_splits.cache_clear()
+    assert real in splits and size % 64 == 0 and (real - 1) * size < 64 * tiles <= real * size
