@@ -87,6 +87,10 @@ int hb_attention_decode_tma_rows(const void* q, const void* k_pages, const void*
                                  const long long* rows, int step_tokens, cudaStream_t stream);
 // clusters of `splits` blocks that run at a time
 int hb_attention_decode_clusters(int hd, int splits);
+// On the host alone, without a stream: the shares of the keys for a launch of attention_prefill_pair.cu, and how long it leaves SMs idle
+int hb_prefill_pair_shares(const int* portions, int n, int nh, int nkv, int hd, int chunk, int window, long long rows, int sms, int least,
+                           int most);
+double hb_prefill_pair_idle_us(const int* portions, int n, int nh, int nkv, int hd, int chunk, int window, int sms, double from);
 
 // hb_qkv_post, hb_attention_decode_tma_rows and hb_attention_merge in one launch (attention_decode_tma.cu)
 int hb_attention_decode_fused(const void* qkv, const float* inv_freq, int rot_pairs, int interleaved, int qk_norm,

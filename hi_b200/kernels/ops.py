@@ -42,6 +42,7 @@ _SIGNATURES = {
     "hb_attention_merge_rows": [P, P, P, I, I, I, I, I, I, P, P, I, P],
     "hb_attention_decode_rows": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P, I, P, P],
     "hb_attention_decode_clusters": [I, I],
+    "hb_prefill_pair_shares": [P, I, I, I, I, I, I, c_longlong, I, I, I],
     "hb_attention_decode_tma_rows": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, I, P, P, P, P, I, P],
     "hb_attention_decode": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, P, P],
     "hb_attention_decode_fused": [P, P, I, I, I, F, I, F, F, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P, P, P, P, P, I, F, I, I, P],
@@ -116,6 +117,8 @@ def lib():
             fn.restype = c_int
         handle.hb_recurrence_chunked_scratch_floats.argtypes = [I, I, I, I, I, I, I, c_longlong]
         handle.hb_recurrence_chunked_scratch_floats.restype = c_longlong
+        handle.hb_prefill_pair_idle_us.argtypes = [P, I, I, I, I, I, I, I, ctypes.c_double]
+        handle.hb_prefill_pair_idle_us.restype = ctypes.c_double
         handle.hb_moe_down_tc_scratch_floats.argtypes = [I]
         handle.hb_moe_down_tc_scratch_floats.restype = c_longlong
         _lib = handle
@@ -2056,7 +2059,9 @@ def prefill_pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window
     and 30 us). Fitted to 3,745 launches (1 to 3 portions of 64 to 2,048 tokens behind up to 65,000) in 1 to 8 shares: 5 % off on
     average; what it chooses takes 0.856 of the time of one share and 1.006 of the best. 40 heads of 128, us in one share and as
     chosen: 128 tokens behind 7,000 101 -> 33, 1,024 behind 16,384 438 -> 336, 150 behind 9,000 beside 700 behind 300 127 -> 85;
-    2,048 alone stay in one (50, in two 99)."""
+    2,048 alone stay in one (50, in two 99). ``least``: where :func:`prefill_key_splits` shares out long runs of keys the model, which takes
+    every tile for as long as any other, still says one now and then; of 14 such launches (1 to 3 portions behind 33,000 to 90,000) 13 took 0.73 to
+    0.95 of the time with at least two, one 1.07. The search is in the library (attention_plan.cu)."""
     return _pair_shares(tuple(portions), nh, nkv, hd, chunk, window, rows, sms, min(least, PREFILL_MOST_SHARES), PREFILL_MOST_SHARES)
 
 
@@ -2065,51 +2070,22 @@ def prefill_pair_idle_us(portions, nh: int, nkv: int, hd: int, chunk: int, windo
     """By the same model, for how long the SMs of such a launch (one share) are idle on average: its longest blocks against all tiles
     over all SMs; 0 for launches of less than 80 us: the host's calls take 40
     with a second stream."""
-    runs = _pair_runs(portions, nh, nkv, chunk, window)
-    tile = 1.515 if hd <= 64 else 1.73
-    longest = max((t for t, _n in runs), default=0)
-    return max(0.0, tile * (longest - sum(t * n for t, n in runs) / sms)) if tile * longest >= 80.0 else 0.0
+    idle = lib().hb_prefill_pair_idle_us(_portion_numbers(portions), len(portions), nh, nkv, hd, chunk, window, sms, 80.0)
+    if idle < 0:
+        raise KernelError(f"prefill attention: no time for portions {portions} of {nh} heads on {nkv}")
+    return idle
 
 
-def _pair_runs(portions, nh: int, nkv: int, chunk: int, window: int):
-    runs = []                           # (key tiles, blocks), eight runs a portion at most
-
-    def visible(first):
-        lo = first // chunk * chunk if chunk else 0
-        return max(lo, first - window + 1) if window else lo
-
-    group = nh // nkv
-    for cached, new in portions:
-        items = -(-new // 128) * group
-        pairs = -(-items // 2)
-        for i in range(min(8, pairs)):
-            a, b = pairs * i // min(8, pairs), pairs * (i + 1) // min(8, pairs)
-            first, last = (a + b - 1) // group, min(a + b, items - 1) // group
-            end = min(cached + 128 * (last + 1), cached + new) - 1
-            runs.append((end // 128 - visible(cached + 128 * first) // 128 + 1, (b - a) * nkv))
-    return runs
+def _portion_numbers(portions):
+    return (I * (2 * len(portions)))(*(x for portion in portions for x in portion))
 
 
 @functools.lru_cache(maxsize=256)                  # a step's layers ask the same
 def _pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, rows: int, sms: int, least: int, limit: int) -> int:
-    runs = _pair_runs(portions, nh, nkv, chunk, window)
-    if not runs:
-        return 1
-    numbers = rows * nh * hd
-    fixed, tile, merge, share, whole = (7.75, 1.515, 1.46, 0.6, 6.2) if hd <= 64 else (8.4, 1.73, 1.27, 0.63, 4.05)
-
-    def cost(k):
-        tiles = sorted(((-(-t // k) + 0.5, n * k) for t, n in runs), reverse=True)
-        most, before, turn = max(tiles[0][0], sum(t * n for t, n in tiles) / sms), 0, 0
-        for t, n in tiles:
-            before += n
-            if sms * turn < before:                 # the last of the turns that start within these blocks
-                turn = (before - 1) // sms + 1
-                most = max(most, turn * t)
-        return fixed + tile * most + (merge + (share * k + whole) * numbers / 1e6 if k > 1 else 0.0)
-
-    best = min(range(least, limit + 1), key=cost)
-    return best if least > 1 or cost(best) < min(0.93 * cost(1), cost(1) - 8.0) else 1
+    shares = lib().hb_prefill_pair_shares(_portion_numbers(portions), len(portions), nh, nkv, hd, chunk, window, rows, sms, least, limit)
+    if shares < 1:
+        raise KernelError(f"prefill attention: no shares for portions {portions} of {nh} heads on {nkv}")
+    return shares
 
 
 # --------------------------------------------------------------------------- experts
