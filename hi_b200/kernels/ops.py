@@ -1383,8 +1383,6 @@ def sigmoid_prefill_attention_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages
     return sigmoid_merge(part_acc, positions, q.dtype, v_inv_freq, v_interleaved)
 
 
-@functools.lru_cache(maxsize=1024)           # a step's layers ask the same (a search over every number of splits)
-@functools.lru_cache(maxsize=4096)                 # a step's layers ask the same
 def _decode_splits(longest: int, groups: int, hd: int = 0, device: int = -1) -> Tuple[int, int]:
     """How to cut ``longest`` keys for ``groups`` (token, kv head) pairs: the number of splits
     that minimises waves x (tiles per block + a block's fixed cost) + a cost per split (the
@@ -1392,20 +1390,26 @@ def _decode_splits(longest: int, groups: int, hd: int = 0, device: int = -1) -> 
     8 requests x 8,192 keys: 6 splits (one wave of 384 blocks) 57 us, 13 splits (two waves) 63 us;
     one request x 32,768 keys: 32 splits 33 us, 47 splits 36 us.
     The cut moves results by rounding only. With ``hd`` and ``device``: for the kernel whose tiles come by TMA; rows
-    of 128 and of 64 have models of their own there (:func:`_tma_splits`, :func:`_tma_splits_64`)."""
+    of 128 and of 64 have models of their own there (:func:`_tma_splits`, :func:`_tma_splits_64`). All of them see tiles of
+    64 keys only, so a generation asks anew at every 64th token, and its layers once."""
+    return _splits_of_tiles(-(-longest // 64), groups, hd, device)
+
+
+@functools.lru_cache(maxsize=4096)
+def _splits_of_tiles(tiles: int, groups: int, hd: int, device: int) -> Tuple[int, int]:
     if hd == 128:
-        return _tma_splits(-(-longest // 64), groups, device, DECODE_CLUSTER + 1 if _decode_splits(longest, groups)[1] > DECODE_CLUSTER else 1)
+        return _tma_splits(tiles, groups, device, DECODE_CLUSTER + 1 if _splits_of_tiles(tiles, groups, 0, -1)[1] > DECODE_CLUSTER else 1)
     if hd == 64:
-        return _tma_splits_64(-(-longest // 64), groups, device)
-    best = (None, 1, longest)
-    for s in range(1, max(1, -(-longest // ATTENTION_SPLIT)) + 1):
-        size = -(-(-(-longest // s)) // 64) * 64
-        real = -(-longest // size)
+        return _tma_splits_64(tiles, groups, device)
+    best = (None, 1, tiles)
+    for s in range(1, max(1, -(-tiles // (ATTENTION_SPLIT // 64))) + 1):
+        size = -(-tiles // s)
+        real = -(-tiles // size)
         waves = -(-(real * groups) // DECODE_RESIDENT_BLOCKS)
-        cost = waves * (size // 64 + 1.5) + 0.2 * real + 0.3 * max(0, real - 32)   # past 32 the merge reads in turns
+        cost = waves * (size + 1.5) + 0.2 * real + 0.3 * max(0, real - 32)   # past 32 the merge reads in turns
         if best[0] is None or cost < best[0]:
             best = (cost, real, size)
-    return best[2], best[1]
+    return 64 * best[2], best[1]
 
 
 def _tma_splits(tiles: int, groups: int, device: int, least: int) -> Tuple[int, int]:

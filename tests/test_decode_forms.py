@@ -89,11 +89,21 @@ def test_rows_of_64_in_launches_of_many_blocks(n, nh, nkv, longest, size, monkey
         assert float((got[i].double() - want).abs().max()) <= 2 ** -7 * float(want.abs().max()), (i, k)
 
 
+def test_a_cut_is_searched_for_once_in_64_tokens(monkeypatch):
+    monkeypatch.setattr(ops, "_decode_clusters", lambda *a: 50)
+    ops._splits_of_tiles.cache_clear()
+    for hd in (0, 64, 128):
+        cuts = {ops._decode_splits(longest, 24, hd, 99) for longest in range(961, 1025)}
+        assert len(cuts) == 1 and ops._decode_splits(1025, 24, hd, 99)[0] * ops._decode_splits(1025, 24, hd, 99)[1] >= 1025
+    assert ops._splits_of_tiles.cache_info().misses == 8           # (rows of 128 ask the general rule too)
+    ops._splits_of_tiles.cache_clear()
+
+
 @pytest.mark.parametrize("hd,groups,tiles,splits", [(64, 96, 189, {6}), (64, 512, 16, {1}), (64, 8, 125, range(8, 25)), (64, 720, 2, {1})])
 def test_rows_of_64_are_cut_for_one_round(hd, groups, tiles, splits, monkeypatch):
     fit = {2: 296, 3: 187, 4: 142, 5: 112, 6: 93, 7: 78, 8: 71}
     monkeypatch.setattr(ops, "_decode_clusters", lambda device, hd, real: fit[real])
-    ops._decode_splits.cache_clear()
+    ops._splits_of_tiles.cache_clear()
     size, real = ops._decode_splits(64 * tiles, groups, hd, 99)
-    ops._decode_splits.cache_clear()
+    ops._splits_of_tiles.cache_clear()
     assert real in splits and size % 64 == 0 and (real - 1) * size < 64 * tiles <= real * size
