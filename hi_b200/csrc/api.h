@@ -119,12 +119,12 @@ int hb_attention_prefill_tc_reshaped(const void* q, const void* k_pages, const v
                                      int n_tokens, int n_pages, int n_seqs, int max_new, int nh, int nkv, int hd,
                                      int page_size, int chunk, int window, int keep, float scale, int skip_single, int sink,
                                      float softcap, const float* slopes, const float* sink_values, int key_splits,
-                                     float* part_acc, float* part_ml, int* status, cudaStream_t stream);
+                                     float* part_acc, float* part_ml, int one_tile, int* status, cudaStream_t stream);
 int hb_attention_prefill_tc(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                             int table_stride, const int* cu_seqlens, const int* positions, void* out, int n_tokens,
                             int n_pages, int n_seqs, int max_new, int nh, int nkv, int hd, int page_size, int chunk,
                             int window, float scale, int skip_single, int sink, const float* head_bias, int key_splits,
-                            float* part_acc, float* part_ml, int* status, cudaStream_t stream);   // sink == 2 as above
+                            float* part_acc, float* part_ml, int one_tile, int* status, cudaStream_t stream);   // sink == 2 as above
 // differential attention: both maps of a head in one block, their difference normed and gated in the epilogue
 int hb_diff_prefill_tc(const void* q, const void* k_pages, const void* v_pages, const int* block_table, int table_stride,
                        const int* cu_seqlens, const int* positions, void* out, int n_tokens, int n_pages, int n_seqs,

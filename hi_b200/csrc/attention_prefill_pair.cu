@@ -12,8 +12,8 @@
 //
 // Measured (B200, one tile a block and two blocks an SM / this, us): 2,048 tokens of 40 heads of 128 on 8 69.3 / 44.7, 4,096 207 / 153,
 // 1,024 behind 16,384 424 / 336, 600 beside 700 behind 300 and 400 behind 100 49 / 35, 2,048 behind 8,192 in a window of 1,024 92 / 61,
-// 24 heads on 24 49 / 37; prompts of 160 to 300 tokens, which are a block's latency, 9.2 to 11.1 / 10.6 to 12.1 (an eager call
-// takes the host 17).
+// 24 heads on 24 49 / 37. Short launches whose last 128 keys are half empty are a block's latency and stay one tile a block
+// (ops.prefill_one_tile).
 // What bounds it: a pair of 128-key tiles takes 3,000 cycles where its products take 2,048 and its exponentials, 16 a cycle, as many:
 // a chain of softmax (1,550), the last 32 keys' P V and Q K^T (640) and the hand-overs between them (about 350 from the last
 // product to the softmax's first load, 200 back). What mattered on the way there, in us for 256 tokens behind 16,384: one lane that

@@ -1,6 +1,7 @@
 // Prefill attention on the 5th-generation tensor cores (tcgen05), bfloat16: portions of prompts of
 // at least a tile of new tokens against the paged cache. Plain softmax rows of 64 and 128 values go two query tiles a block
-// (attention_prefill_pair.cu); here are rows of 192, reshaped scores, kept first tokens, sigmoid weights and differential
+// (attention_prefill_pair.cu) but for short launches whose last 128 keys are half empty (ops.prefill_one_tile); here are those, rows of 192,
+// reshaped scores, kept first tokens, sigmoid weights and differential
 // attention. One block = 128 consecutive new tokens of one request and one query head:
 //   warp 0      one lane issues TMA loads: the Q tile once, then K and V tiles of 64 key positions
 //               (one box per page, 128-byte swizzle): K into a ring of three and a tile ahead of V,
@@ -737,18 +738,19 @@ int prefill_tc(const void* q, const void* k_pages, const void* v_pages, const in
                int nh, int nkv, int hd, int page_size, int chunk, int window, float scale, int skip_single, int sink,
                const float* head_bias, int key_splits, float* part_acc, float* part_ml, int* status, int turn_inside,
                const float* v_inv_freq, int v_pairs, int v_interleaved, float softcap, const float* slopes,
-               const float* sink_values, int keep, const Pair* pair, cudaStream_t stream);
+               const float* sink_values, int keep, const Pair* pair, int one_tile, cudaStream_t stream);
 }  // namespace
 
+// one_tile: plain softmax rows of 64 and 128 too go one query tile a block (ops.prefill_one_tile says where that is faster)
 extern "C" int hb_attention_prefill_tc(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                        int table_stride, const int* cu_seqlens, const int* positions, void* out,
                                        int n_tokens, int n_pages, int n_seqs, int max_new, int nh, int nkv, int hd,
                                        int page_size, int chunk, int window, float scale, int skip_single,
                                        int sink, const float* head_bias, int key_splits, float* part_acc,
-                                       float* part_ml, int* status, cudaStream_t stream) {
+                                       float* part_ml, int one_tile, int* status, cudaStream_t stream) {
   return prefill_tc(q, k_pages, v_pages, block_table, table_stride, cu_seqlens, positions, out, n_tokens, n_pages, n_seqs,
                     max_new, nh, nkv, hd, page_size, chunk, window, scale, skip_single, sink, head_bias, key_splits,
-                    part_acc, part_ml, status, 0, nullptr, 0, 0, 0.f, nullptr, nullptr, 0, nullptr, stream);
+                    part_acc, part_ml, status, 0, nullptr, 0, 0, 0.f, nullptr, nullptr, 0, nullptr, one_tile, stream);
 }
 
 // The same with reshaped scores (see Args): a cap, a distance bias per head, a sink with a score per head.
@@ -758,10 +760,10 @@ extern "C" int hb_attention_prefill_tc_reshaped(const void* q, const void* k_pag
                                                 int max_new, int nh, int nkv, int hd, int page_size, int chunk,
                                                 int window, int keep, float scale, int skip_single, int sink, float softcap,
                                                 const float* slopes, const float* sink_values, int key_splits,
-                                                float* part_acc, float* part_ml, int* status, cudaStream_t stream) {
+                                                float* part_acc, float* part_ml, int one_tile, int* status, cudaStream_t stream) {
   return prefill_tc(q, k_pages, v_pages, block_table, table_stride, cu_seqlens, positions, out, n_tokens, n_pages, n_seqs,
                     max_new, nh, nkv, hd, page_size, chunk, window, scale, skip_single, sink, nullptr, key_splits,
-                    part_acc, part_ml, status, 0, nullptr, 0, 0, softcap, slopes, sink_values, keep, nullptr, stream);
+                    part_acc, part_ml, status, 0, nullptr, 0, 0, softcap, slopes, sink_values, keep, nullptr, one_tile, stream);
 }
 
 // Sigmoid weights with the result written by the kernel itself: `out` [n_tokens, nh, hd] bfloat16 takes every
@@ -778,7 +780,7 @@ extern "C" int hb_sigmoid_prefill_tc(const void* q, const void* k_pages, const v
   if (v_pairs > 0 && !v_interleaved && 2 * v_pairs != hd) return HB_ERR_UNSUPPORTED;
   return prefill_tc(q, k_pages, v_pages, block_table, table_stride, cu_seqlens, positions, out, n_tokens, n_pages, n_seqs,
                     max_new, nh, nkv, hd, page_size, chunk, window, scale, skip_single, 2, head_bias, 1, nullptr, nullptr,
-                    status, 1, v_inv_freq, v_pairs, v_interleaved, 0.f, nullptr, nullptr, 0, nullptr, stream);
+                    status, 1, v_inv_freq, v_pairs, v_interleaved, 0.f, nullptr, nullptr, 0, nullptr, 1, stream);
 }
 
 // Differential attention: q [n_tokens, nh, hd] holds the two maps of head a as heads 2a and 2a + 1, both over the same
@@ -797,7 +799,7 @@ extern "C" int hb_diff_prefill_tc(const void* q, const void* k_pages, const void
   const Pair pair{lambda, eps, mul, vdim, vec ? 1 : 0, (const __nv_bfloat16*)gate, gate_stride};
   return prefill_tc(q, k_pages, v_pages, block_table, table_stride, cu_seqlens, positions, out, n_tokens, n_pages, n_seqs,
                     max_new, nh, nkv, hd, page_size, chunk, window, scale, skip_single, 0, nullptr, 1, nullptr, nullptr,
-                    status, 0, nullptr, 0, 0, 0.f, nullptr, nullptr, keep, &pair, stream);
+                    status, 0, nullptr, 0, 0, 0.f, nullptr, nullptr, keep, &pair, 1, stream);
 }
 
 namespace {
@@ -806,7 +808,7 @@ int prefill_tc(const void* q, const void* k_pages, const void* v_pages, const in
                int nh, int nkv, int hd, int page_size, int chunk, int window, float scale, int skip_single, int sink,
                const float* head_bias, int key_splits, float* part_acc, float* part_ml, int* status, int turn_inside,
                const float* v_inv_freq, int v_pairs, int v_interleaved, float softcap, const float* slopes,
-               const float* sink_values, int keep, const Pair* pair, cudaStream_t stream) {
+               const float* sink_values, int keep, const Pair* pair, int one_tile, cudaStream_t stream) {
   if (sink == 2 && (softcap > 0.f || slopes || sink_values)) return HB_ERR_UNSUPPORTED;
   if (!q || !k_pages || !v_pages || !block_table || !cu_seqlens || !positions || !out || !status) return HB_ERR_BAD_ARG;
   if (n_tokens < 0 || n_pages <= 0 || n_seqs < 0 || max_new < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 ||
@@ -824,7 +826,7 @@ int prefill_tc(const void* q, const void* k_pages, const void* v_pages, const in
   const long long pool_rows = (long long)n_pages * nkv * page_size;
   // (a launch of more pairs than a grid holds goes one tile a block)
   const long long pairs = ((max_new + 127LL) / 128 * (nh / nkv) + 1) / 2;
-  if (!pair && !turn_inside && sink != 2 && softcap <= 0.f && !slopes && keep == 0 && hd <= 128 && pairs <= 65535) {
+  if (!one_tile && !pair && !turn_inside && sink != 2 && softcap <= 0.f && !slopes && keep == 0 && hd <= 128 && pairs <= 65535) {
     const PrefillPairArgs b{block_table, cu_seqlens, positions, (__nv_bfloat16*)out, status, table_stride, nh, nkv, page_size, chunk, window,
                             skip_single, a.box_rows, a.scale_log2, key_splits, part_acc, part_ml, sink, sink_values};
     return hb_prefill_pair_launch(q, k_pages, v_pages, b, n_tokens, pool_rows, n_seqs, max_new, hd, stream);

@@ -48,9 +48,9 @@ _SIGNATURES = {
     "hb_attention_decode_fused": [P, P, I, I, I, F, I, F, F, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P, P, P, P, P, I, F, I, I, P],
     "hb_attention_prefill": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, I, P],
     "hb_attention_prefill_reshaped": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, F, P, P, P, P, P],
-    "hb_attention_prefill_tc": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, I, P, I, P, P, P, P],
-    "hb_attention_prefill_tc_reshaped": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, I, I, F, P, P, I, P, P, P,
-                                         P],
+    "hb_attention_prefill_tc": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, I, P, I, P, P, I, P, P],
+    "hb_attention_prefill_tc_reshaped": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, I, I, F, P, P, I, P, P, I,
+                                         P, P],
     "hb_sigmoid_prefill_tc": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P, I, I, P, P],
     "hb_sigmoid_merge": [P, P, P, I, I, P, I, I, I, I, I, P],
     "hb_router_topk": [P, I, P, I, P, I, I, I, I, I, F, P, P, P, P],
@@ -1377,7 +1377,7 @@ def sigmoid_prefill_attention_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages
     _check(lib().hb_attention_prefill_tc(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
                                          block_table.shape[1], _ptr(cu_seqlens), _ptr(positions), _ptr(part_acc), n, n_pages,
                                          n_seqs, int(max_new), nh, nkv, hd, page_size, int(chunk), int(window),
-                                         float(scale), int(skip_single), 2, _ptr(head_bias), 1, _ptr(part_acc), None,
+                                         float(scale), int(skip_single), 2, _ptr(head_bias), 1, _ptr(part_acc), None, 1,
                                          _ptr(_tc_status(q.device)), _stream()), "attention_prefill_tc")
     TC_USED[0] = True
     return sigmoid_merge(part_acc, positions, q.dtype, v_inv_freq, v_interleaved)
@@ -1744,11 +1744,11 @@ def prefill_attention_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.
                          window: int, scale: float, skip_single: bool = False,
                          out: Optional[torch.Tensor] = None, key_splits: int = 1, sink: bool = False,
                          softcap: float = 0.0, slopes: Optional[torch.Tensor] = None,
-                         sink_values: Optional[torch.Tensor] = None, keep: int = 0) -> torch.Tensor:
+                         sink_values: Optional[torch.Tensor] = None, keep: int = 0, one_tile: bool = False) -> torch.Tensor:
     """As :func:`prefill_attention`, on tcgen05 (S, P V and O in tensor memory, TMA page loads).
     ``key_splits`` > 1: that many blocks share the key tiles of every (query tile, head) and a
     merge kernel combines their rows (see :func:`prefill_key_splits`). ``softcap``, ``slopes``, ``sink_values``, ``keep``:
-    as :func:`paged_attention`."""
+    as :func:`paged_attention`. ``one_tile``: one query tile a block also where two are the rule (:func:`prefill_pairs`)."""
     _need(q, "q", torch.bfloat16); _need(k_pages, "k_pages", q.dtype); _need(v_pages, "v_pages", q.dtype)
     for t, nm in ((block_table, "block_table"), (cu_seqlens, "cu_seqlens"), (positions, "positions")):
         _need(t, nm, torch.int32)
@@ -1778,14 +1778,14 @@ def prefill_attention_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.
             _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.shape[1], _ptr(cu_seqlens),
             _ptr(positions), _ptr(out), n, n_pages, n_seqs, int(max_new), nh, nkv, hd, page_size, int(chunk), int(window),
             int(keep), float(scale), int(skip_single), int(sink), float(softcap), _ptr(slopes), _ptr(sink_values), key_splits,
-            _ptr(part_acc), _ptr(part_ml), _ptr(_tc_status(q.device)), _stream()), "attention_prefill_tc")
+            _ptr(part_acc), _ptr(part_ml), int(one_tile), _ptr(_tc_status(q.device)), _stream()), "attention_prefill_tc")
     else:
         _check(lib().hb_attention_prefill_tc(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
                                              block_table.shape[1], _ptr(cu_seqlens), _ptr(positions), _ptr(out), n, n_pages,
                                              n_seqs, int(max_new), nh, nkv, hd, page_size, int(chunk), int(window),
                                              float(scale), int(skip_single), int(sink), None, key_splits,
                                              _ptr(part_acc) if part_acc is not None else None,
-                                             _ptr(part_ml) if part_ml is not None else None, _ptr(_tc_status(q.device)),
+                                             _ptr(part_ml) if part_ml is not None else None, int(one_tile), _ptr(_tc_status(q.device)),
                                              _stream()),
                "attention_prefill_tc")
     TC_USED[0] = True
@@ -2052,6 +2052,17 @@ def prefill_pairs(hd: int, softcap: float = 0.0, slopes=None, keep: int = 0) -> 
     """Whether the tcgen05 prefill attention takes two query tiles a block (``attention_prefill_pair.cu``): plain softmax rows of 64
     or 128 values. Rows of 192, reshaped scores and windows that keep first tokens go one tile a block."""
     return hd <= 128 and not softcap and slopes is None and keep == 0
+
+
+def prefill_one_tile(portions, nh: int, nkv: int, chunk: int, window: int) -> bool:
+    """Whether such rows still go one query tile a block, in one share: launches of one round of blocks, one on an SM, whose longest context
+    has three, five or seven tiles of 64 keys, so that half of the last 128 that two tiles a block would take is empty. Of 170 launches of one to three
+    portions in up to 480 keys, two tiles a block against one: 1.13, 1.10 and 1.06 of the time there (16 heads on 4, rows of 64: 192 tokens
+    9.5 / 7.8 us), 0.98 to 1.01 where the number is even, 0.75 to 0.98 where there are more blocks than SMs. Not five tiles of as many key
+    heads as heads, whose pairs are neighbours in tokens: portions of 163, 109 and 96, 24 heads on 24 of 64, 10.3 / 11.9."""
+    tiles = -(-max((cached + new for cached, new in portions), default=0) // 64)
+    return (tiles in (3, 7) or (tiles == 5 and nkv < nh)) and not 0 < chunk < 64 * tiles and not 0 < window < 64 * tiles and \
+        nh * sum(-(-new // 128) for _cached, new in portions) <= 148
 
 
 def prefill_pair_shares(portions, nh: int, nkv: int, hd: int, chunk: int, window: int, rows: int, sms: int, least: int = 1) -> int:

@@ -32,16 +32,13 @@ def _decode_aside(device):
     return kept[device.index]
 
 
-def _key_splits(ctx, nh: int, nkv: int, hd: int, chunk: int, sliding: int, keep: int, single: bool, pairs: bool, device) -> int:
+def _key_splits(portions, rows: int, nh: int, nkv: int, hd: int, chunk: int, sliding: int, keep: int, pairs: bool, device) -> int:
     """Portions far into long contexts on a layer that sees every key: all blocks of the
     tensor-core prefill kernel then have about the same many key tiles, and a partly filled
     last round of blocks is worth splitting the keys for (ops.prefill_key_splits). Everything else: what a model of
     the kernel's time says (ops.prefill_shares; for the kernel of two query tiles a block ops.prefill_pair_shares, which then
     also says into how many)."""
-    if keep:
-        return 1
-    portions = [(s, n) for s, n in zip(ctx.start_pos, ctx.n_new) if n > 1 or not single]
-    if not portions:
+    if keep or not portions:
         return 1
     sms, least = ops.sm_count(device), 1
     if not chunk and not sliding:
@@ -53,8 +50,8 @@ def _key_splits(ctx, nh: int, nkv: int, hd: int, chunk: int, sliding: int, keep:
                 return shares
             least = min(shares, 2)
     if pairs:
-        return ops.prefill_pair_shares(portions, nh, nkv, hd, chunk, sliding, ctx.n_tokens, sms, least)
-    return ops.prefill_shares(portions, nh, hd, chunk, sliding, ctx.n_tokens, sms)
+        return ops.prefill_pair_shares(portions, nh, nkv, hd, chunk, sliding, rows, sms, least)
+    return ops.prefill_shares(portions, nh, hd, chunk, sliding, rows, sms)
 
 
 def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, hd: int, chunk: int, sliding: int,
@@ -86,18 +83,19 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
         single = ctx.decode_rows is not None and decode_ok
         pairs = ops.prefill_pairs(hd, softcap, slopes, keep)
         if tc:
-            shares = _key_splits(ctx, nh, nkv, hd, chunk, sliding, keep, single, pairs, q.device)
+            portions = [(s, n) for s, n in zip(ctx.start_pos, ctx.n_new) if n > 1 or not single]
+            one_tile = pairs and ops.prefill_one_tile(portions, nh, nkv, chunk, sliding)
+            shares = 1 if one_tile else _key_splits(portions, ctx.n_tokens, nh, nkv, hd, chunk, sliding, keep, pairs, q.device)
             # (the merge of shared keys writes every row, so single tokens wait for it)
-            aside = single and pairs and shares == 1 and ops.prefill_pair_idle_us(
-                tuple((s, n) for s, n in zip(ctx.start_pos, ctx.n_new) if n > 1), nh, nkv, hd, chunk, sliding,
-                ops.sm_count(q.device)) >= DECODE_ASIDE_IDLE_US
+            aside = single and pairs and shares == 1 and not one_tile and ops.prefill_pair_idle_us(
+                tuple(portions), nh, nkv, hd, chunk, sliding, ops.sm_count(q.device)) >= DECODE_ASIDE_IDLE_US
             if aside:
                 current = torch.cuda.current_stream()
                 stream, before, after = _decode_aside(q.device)
                 before.record(current)
             o = ops.prefill_attention_tc(q, k_pages, v_pages, block_table, ctx.cu_seqlens, positions,
                                          ctx.n_seqs, ctx.max_new, chunk, sliding, scale, skip_single=single, key_splits=shares, sink=sink,
-                                         softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep)
+                                         softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep, one_tile=one_tile)
             if aside:
                 # other rows of the same output; nothing of the call's is freed before the streams have met again
                 stream.wait_event(before)

@@ -151,6 +151,49 @@ def test_single_tokens_decoded_aside(capture, monkeypatch):
     ops.check_tc_status()
 
 
+@pytest.mark.parametrize("portions,nh,nkv,chunk,window,want", [
+    ([(0, 160)], 40, 8, 0, 0, True), ([(0, 161), (0, 105)], 16, 4, 0, 0, True), ([(5, 315)], 16, 4, 8192, 4096, True), ([(0, 448)], 8, 8, 0, 0, True),
+    ([(0, 128)], 40, 8, 0, 0, False), ([(0, 200)], 40, 8, 0, 0, False), ([(0, 449)], 8, 2, 0, 0, False), ([(0, 513)], 8, 2, 0, 0, False),
+    ([(0, 300)], 40, 8, 0, 0, True), ([(0, 300), (0, 130)], 40, 8, 0, 0, False), ([(0, 300)], 8, 2, 256, 0, False), ([(0, 300)], 8, 2, 0, 100, False),
+    ([], 8, 2, 0, 0, False), ([(400, 140), (0, 150)], 8, 2, 0, 0, False), ([(0, 300)], 8, 8, 0, 0, False), ([(0, 180)], 8, 8, 0, 0, True)])
+def test_short_launches_that_go_one_query_tile_a_block(portions, nh, nkv, chunk, window, want):
+    """One round of blocks whose last 128 keys are half empty: two tiles a block took 1.05 to 1.2 of the time there."""
+    assert ops.prefill_one_tile(portions, nh, nkv, chunk, window) is want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nh,nkv,hd,lens,sink", [(8, 2, 128, [160, 1, 131], False), (4, 2, 64, [300, 17], True)])
+def test_one_query_tile_a_block_gives_the_same_rows(nh, nkv, hd, lens, sink, monkeypatch):
+    from hi_b200.parts import attention as part
+    from hi_b200.parts.context import StepContext
+
+    g = torch.Generator(device=DEV).manual_seed(hd)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    need = -(-max(lens) // 64)
+    kp, vp, q = rnd(len(lens) * need, nkv, 64, hd), rnd(len(lens) * need, nkv, 64, hd), rnd(sum(lens), nh, hd)
+    table = torch.arange(len(lens) * need, dtype=torch.int32, device=DEV).view(len(lens), need)
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    ctx = StepContext(n_tokens=cu[-1], n_seqs=len(lens), tokens=i32([0] * cu[-1]), positions=torch.cat([torch.arange(n) for n in lens]).int().to(DEV),
+                      seq_of_token=i32([s for s, n in enumerate(lens) for _ in range(n)]), cu_seqlens=i32(cu), slots=i32(list(range(len(lens)))),
+                      start_pos=[0] * len(lens), n_new=lens, slot_ids=list(range(len(lens))), page_size=64, max_context=max(lens))
+    ctx.decode_rows, ctx.decode_max_context = (torch.tensor([cu[lens.index(1)]], device=DEV), 1) if 1 in lens else (None, 0)
+    sinks = torch.randn(nh, device=DEV, generator=g) if sink else None
+    call = lambda: part.attend_over_pages(q, kp, vp, table, ctx, nh, nkv, hd, 0, 0, hd ** -0.5, sink_values=sinks)
+    seen, real = [], ops.prefill_attention_tc
+    monkeypatch.setattr(ops, "prefill_attention_tc", lambda *a, **k: (seen.append(k["one_tile"]), real(*a, **k))[1])
+    one = call()
+    monkeypatch.setattr(ops, "prefill_one_tile", lambda *a: False)
+    two = call()
+    ops.check_tc_status()
+    assert seen == [True, False]
+    rows = lambda t, s: t[table[s].long()].transpose(1, 2).reshape(-1, nkv, hd)[: lens[s]].cpu()
+    want = reference(q.cpu(), [rows(kp, s) for s in range(len(lens))], [rows(vp, s) for s in range(len(lens))], [0] * len(lens), lens, 0, 0, hd ** -0.5,
+                     None if sinks is None else sinks.cpu())
+    for got in (one, two):      # as in the test of the pairs
+        assert float((got.double().cpu() - want).abs().max()) <= 2e-2
+
+
 def shares_in_plain_python(portions, nh, nkv, hd, chunk, window, rows, sms, least, most=8):
     """The model as it reads: runs of neighbouring pairs, and for every number of shares the longest block, the average SM and the turns."""
     runs, group = [], nh // nkv
