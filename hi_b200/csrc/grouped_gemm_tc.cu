@@ -592,9 +592,10 @@ extern "C" int hb_moe_gate_up_tc(const void* xs, const int* sorted_entry, const 
   if (hidden % 8 != 0 || inter % 8 != 0 || hidden <= 0 || inter <= 0) return HB_ERR_UNSUPPORTED;
   if (rows == 0) return HB_OK;
   const bool few = rows <= SHORT_STEP_ROWS;
-  const int bt = few ? BT_SHORT : DUAL_SLOT_T;      // (or more: dual_tokens)
-  const int max_tiles = (rows + bt - 1) / bt + (experts < rows ? experts : rows);
-  if (max_tiles > 65535) return HB_ERR_UNSUPPORTED;
+  const int most = few ? BT_SHORT : BT_LONG, bt = few ? BT_SHORT : DUAL_SLOT_T;      // tokens of a tile: that or fewer (dual_tokens)
+  const int with_rows = experts < rows ? experts : rows;
+  if ((rows + most - 1) / most + with_rows > 65535) return HB_ERR_UNSUPPORTED;       // as the other products
+  const int max_tiles = (rows + bt - 1) / bt + with_rows;
   Params p{offsets, sorted_entry, scores, act, status, experts, inter, hidden, rows, nullptr, nullptr, limit, 0};
   return few ? launch<true, 5, BT_SHORT>(xs, w_gate, w_up, p, max_tiles, stream)
          : pairs(rows, experts) ? launch<true, 5, BT_LONG, true>(xs, w_gate, w_up, p, max_tiles, stream)

@@ -40,3 +40,19 @@ def test_pairs_of_blocks(experts, hidden, inter, counts):
     want = torch.einsum("rk,rfk->rf", act.double(), wd.double()[of])
     assert float((down.double() - want).abs().max()) <= inter * 2 ** -23 * float(want.abs().max())
     assert torch.equal(down, again)              # whichever piece comes last
+
+
+def test_as_many_rows_as_the_other_products_take():
+    """8.4 million rows are 43,751 tiles of 192 tokens, which all three products take, and more than 65,535 of 128."""
+    rows, hidden = 8_400_000, 8
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x, scores = torch.randn(rows, hidden, device=DEV, generator=g).bfloat16(), torch.rand(rows, device=DEV, generator=g)
+    wg, wu = (torch.randn(1, hidden, hidden, device=DEV, generator=g).bfloat16() for _ in range(2))
+    entry = torch.arange(rows, dtype=torch.int32, device=DEV)
+    plan = ops.MoePlan(torch.tensor([0, rows], dtype=torch.int32, device=DEV), entry, entry, torch.tensor([1, 0], dtype=torch.int32, device=DEV))
+    act = ops.moe_gate_up_tc(x, plan, 1, wg, wu, scores)
+    ops.check_tc_status()
+    gate, up = (scores[:, None] * (x.float() @ w[0].float().t()) for w in (wg, wu))
+    want = torch.nn.functional.silu(gate) * up
+    # one rounding to bfloat16 on sums of eight products in float32
+    assert bool(((act.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all())
