@@ -118,8 +118,10 @@ __device__ __forceinline__ bool find_tile(const int* offsets, int experts, int t
 // The most tokens of a tile in a long DUAL launch: 192, or 128 where that takes less time. A tile of up to 128 leaves its slot to the
 // next one's accumulators, a larger one has both and the next waits until it is in registers; a stage brings less with it, but the
 // weights come once more. By the rounds over the SMs times what a stage brings (32 KB of weights, the box of tokens) and, for the
-// larger tiles, 480 KB a tile for that wait (us, 192 / 128: 2,048 tokens, 2 of 8 experts of 2,048 x 4,096, up product with gather, 136
-// / 128; 4 of 16 of 1,024 x 2,048 91 / 78; 1 of 16 of 2,048 x 8,192, where weights come from HBM, 196 / 208). One warp asks.
+// larger tiles, 480 KB a round for that wait (us, 192 / 128: 2,048 tokens, 2 of 8 experts of 2,048 x 4,096, up product with gather, 136
+// / 128; 4 of 16 of 1,024 x 2,048 91 / 78; 1 of 16 of 2,048 x 8,192, where weights come from HBM, 196 / 208). Pairs of blocks, which bring 44
+// and 40 KB a stage, are chosen for by the same numbers: over 103 launches of 256 to 900 rows an expert that takes 1.010 of the better one's
+// time, with 44 and 40 KB exactly the same choices, with another wait 1.016 to 1.047; always 128 1.032, always 192 1.098. One warp asks.
 __device__ __forceinline__ int dual_tokens(const int* offsets, int experts, int f_tiles, int num_kb, int blocks) {
   int few = 0, many = 0, large = 0;
   for (int e = threadIdx.x & 31; e < experts; e += 32) {
