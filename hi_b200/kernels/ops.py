@@ -1513,13 +1513,13 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                      max_context: int, sink: bool = False, softcap: float = 0.0,
                      slopes: Optional[torch.Tensor] = None, sink_values: Optional[torch.Tensor] = None,
                      keep: int = 0, parts: bool = False, rows: Optional[torch.Tensor] = None,
-                     out: Optional[torch.Tensor] = None):
+                     out: Optional[torch.Tensor] = None, most_keys: int = 0):
     """Attention for a batch of single decoded tokens (every row of ``q`` is one request's
     token), bfloat16, split over runs of ``ATTENTION_SPLIT`` keys. The splits' partial results meet in
     a cluster's shared memory or in scratch memory. ``softcap``, ``slopes``, ``sink_values``: as :func:`paged_attention`
     (the kernel that loads its tiles by cp.async takes them). With ``rows`` (int64, distinct) only those tokens of the
     step are decoded, from where they lie in ``q`` to where they lie in ``out`` [N, nh, hd] (not with ``parts``); a row outside
-    the step is left out and found by :func:`check_tc_status`."""
+    the step is left out and found by :func:`check_tc_status`. ``most_keys`` > 0: no split has more keys than that."""
     if rows is not None:
         rows, seq_of_token, positions = rows.contiguous(), seq_of_token.contiguous(), positions.contiguous()
     _need(q, "q", torch.bfloat16); _need(k_pages, "k_pages", q.dtype); _need(v_pages, "v_pages", q.dtype)
@@ -1553,6 +1553,9 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         (page_size % 64 == 0 or page_size in (16, 32))
     split_size, splits = _decode_splits(longest, n * nkv, hd, q.get_device()) if tma else \
         _decode_splits(longest, n * nkv * -(-(nh // nkv) // 16))
+    if 0 < most_keys < split_size:
+        split_size = -(-(-(-longest // 64)) // -(-longest // most_keys)) * 64
+        splits = -(-longest // split_size)
     if rows is None:
         out = None if parts else torch.empty_like(q)
     part_acc = part_ml = None

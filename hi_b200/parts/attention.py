@@ -19,9 +19,13 @@ DIFF_TC_MIN_TOKENS = 64      # new tokens of a request from which differential a
 
 
 # Where a launch of portions leaves SMs idle for this long (us), the single tokens beside them are decoded on a second stream meanwhile:
-# they take the SMs that are done early (513 tokens behind 7,000, 200 and 129 others beside four single tokens, 40 heads: 141 -> 133 us; 197 such steps
-# 0.90 of the time, the worst 1.07).
+# they take the SMs that are done early (513 tokens behind 7,000, 200 and 129 others beside four single tokens, 40 heads, graph replays back to
+# back: 136 -> 116 us).
 DECODE_ASIDE_IDLE_US = 8.0
+# Splits there are not longer than this: the rules for the cut count on all SMs, of which the portions hold most, and a long split that starts
+# late is a tail. 70 such steps took 0.971 of the time without the limit (0.72 to 1.02), and 0.876 of one after the other (0.68 to 0.98, without
+# it up to 1.06); 16 single tokens of up to 8,335 keys beside 301 behind 3,042 and 551 behind 5,897, 32 heads on 8: 153 -> 121 us.
+DECODE_ASIDE_KEYS = 2048
 _aside = threading.local()             # a stream and two events per thread and device: joined before the call returns
 
 
@@ -68,10 +72,10 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
     positions = ctx.positions
     decode_ok = ops.decode_attention_supported(q.dtype, nh, nkv, hd)
 
-    def decode(longest, rows=None, out=None):
+    def decode(longest, rows=None, out=None, most_keys=0):
         return ops.decode_attention(q, k_pages, v_pages, block_table, ctx.seq_of_token, positions, chunk, sliding, scale, longest,
                                     sink=sink, softcap=softcap, slopes=slopes, sink_values=sink_values, keep=keep, rows=rows,
-                                    out=out)
+                                    out=out, most_keys=most_keys)
 
     if ctx.max_new == 1 and decode_ok:
         # every token of the step is one request's decoded token: the tensor-core kernel
@@ -101,7 +105,7 @@ def attend_over_pages(q, k_pages, v_pages, block_table, ctx, nh: int, nkv: int, 
                 stream.wait_event(before)
                 torch.cuda.set_stream(stream)
                 try:
-                    decode(ctx.decode_max_context, ctx.decode_rows, o)
+                    decode(ctx.decode_max_context, ctx.decode_rows, o, DECODE_ASIDE_KEYS)
                 finally:
                     torch.cuda.set_stream(current)
                     after.record(stream)

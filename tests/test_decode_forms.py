@@ -107,3 +107,24 @@ def test_rows_of_64_are_cut_for_one_round(hd, groups, tiles, splits, monkeypatch
     size, real = ops._decode_splits(64 * tiles, groups, hd, 99)
     ops._splits_of_tiles.cache_clear()
     assert real in splits and size % 64 == 0 and (real - 1) * size < 64 * tiles <= real * size
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("longest,most,splits,size", [(10752, 2048, 6, 1792), (4097, 2048, 3, 1408), (2048, 2048, 1, 2048), (1000, 100, 8, 128), (130, 64, 3, 64)])
+def test_no_split_is_longer_than_asked(longest, most, splits, size, monkeypatch):
+    monkeypatch.setattr(ops, "_decode_splits", lambda keys, *a: (-(-keys // 64) * 64, 1))
+    g = torch.Generator(device=DEV).manual_seed(longest)
+    pages = -(-longest // 64)
+    q, kp, vp = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((1, 4, 64), (pages, 2, 64, 64), (pages, 2, 64, 64)))
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    args = (q, kp, vp, torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1), i32(0), i32(longest - 1), 0, 0, 0.125, longest)
+    acc, ml = ops.decode_attention(*args, parts=True, most_keys=most)
+    assert acc.shape == (1, 4, splits, 64)
+    for s in range(splits):                                     # every split its own run of keys: the sums of the weights by it
+        keys = kp.transpose(1, 2).reshape(-1, 2, 64)[:longest][s * size:(s + 1) * size].double().repeat_interleave(2, dim=1)
+        want = torch.logsumexp(torch.einsum("hd,khd->hk", q[0].double(), keys) * 0.125, dim=1)
+        got = ml[0, :, s, 0].double() + ml[0, :, s, 1].double().log()
+        assert float((got - want).abs().max()) <= 1e-4         # float32 sums of up to 2,048 terms
+    whole = ops.decode_attention(*args)
+    assert float((ops.decode_attention(*args, most_keys=most).float() - whole.float()).abs().max()) <= 2 ** -7 * float(whole.abs().max())
+    ops.check_tc_status()
