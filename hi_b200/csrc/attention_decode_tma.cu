@@ -53,8 +53,8 @@ enum Merge { APART, FUSED_FORM, CLUSTER };
 // 64 three and four (two and five are slower while one round holds the launch; us, two and five / three and four: 16 tokens of 3,943
 // keys, 40 heads on 8, 26.4 / 22.9; 10 of 8,619, 32 on 8, 33.9 / 28.7). Launches of more blocks of rows of 64 than that: where a split has
 // no more than two tiles, or of up to five and in fewer rounds so, two and six, without a warp for the loads: 128 threads of 80 registers (34 tokens
-// of 80 keys, 24 heads on 24: 9.3, 11.8 with the warp; 64 of 91 15.7, 17.6; 36 of 191 12.1, 14.4; 47 of 280, two rounds either way, 20.3 / 17.6). The fused
-// form encodes rows first and needs 122 and 168 registers for it: three tiles and three blocks of rows of 64, two of rows of 128. Held
+// of 80 keys, 24 heads on 24: 9.3, 11.8 with the warp; 64 of 91 15.7, 17.6; 36 of 191 12.1, 14.4). The fused
+// form encodes rows first and needs 128 and 168 registers for it: three tiles and three blocks of rows of 64, two of rows of 128. Held
 // to the others' 72 to 128 registers it spilled up to 224 bytes a thread (us, so / now: 8 tokens of 4,000 keys, 32 heads on 8, rows of 64,
 // 20.7 / 16.7; rows of 128, 40 on 8, 32 tokens of 2,048 45.7 / 38.8, 2 of 8,192 20.8 / 19.3, ops._fused_splits' cuts).
 template <int HD, Merge MERGE> constexpr int STAGES_OF = HD == 128 && MERGE != FUSED_FORM ? 2 : 3;

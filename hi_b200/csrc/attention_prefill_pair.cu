@@ -10,7 +10,7 @@
 // S and O of both items take all of tensor memory, so one block lives on an SM; when a work's loads are under way, the block takes the
 // next one that has not started (cluster launch control), and its Q and first K arrive while the last tiles of this one are worked at.
 //
-// Measured (B200, one tile a block and two blocks an SM / this, us): 2,048 tokens of 40 heads of 128 on 8 69.3 / 44.7, 4,096 207 / 153,
+// Measured (B200, one tile a block and two blocks an SM / this, us): 2,048 tokens of 40 heads of 128 on 8 69.3 / 44.7, 4,096 205 / 141,
 // 1,024 behind 16,384 424 / 336, 600 beside 700 behind 300 and 400 behind 100 49 / 35, 2,048 behind 8,192 in a window of 1,024 92 / 61,
 // 24 heads on 24 49 / 37. Short launches whose last 128 keys are half empty are a block's latency and stay one tile a block
 // (ops.prefill_one_tile).
