@@ -1441,7 +1441,7 @@ def _tma_splits_64(tiles: int, groups: int, device: int) -> Tuple[int, int]:
     to 18 cuts each: what it takes is 1.014 of the best cut's time on average, 1.21 at worst; :func:`_decode_splits`'s own 1.023 and 1.68 (12 tokens
     of 12,056 keys, 40 heads on 8, 9 splits / 6: 54.8 / 43.2 us; 64 of 991, 32 on 8, 4 / 1: 28.6 / 19.3)."""
     best = (None, 64 * tiles, 1)
-    for s in range(1, max(1, min(tiles // 2, 48, 592 // groups)) + 1):
+    for s in range(1, max(1, min(tiles // 2, 48, 592 // max(groups, 1))) + 1):
         size = -(-tiles // s)
         real = -(-tiles // size)
         blocks = real * groups
@@ -1467,7 +1467,7 @@ def _fused_splits(tiles: int, groups: int, hd: int) -> Tuple[int, int]:
     all tiles loaded by one thread. 8 tokens of 8,192 keys, 40 heads of 128 on 8, 4 / 6 splits: 40.3 / 43.4 us; 32 of 2,048, 1 / 3: 38.8 / 50.4."""
     resident, block, tile, read, last, start, fixed, each, pair = \
         (444, 6.2, 0.445, 0.00116, 0.326, 5.2, 2.08, 0.0665, 0.00246) if hd <= 64 else (296, 7.93, 0.594, 0.00245, 0.332, 7.72, 2.42, 0.0748, 0.0)
-    most = 4 if 2 * groups > resident else resident // groups
+    most = 4 if 2 * groups > resident else resident // max(groups, 1)
     best = (None, 64 * tiles, 1)
     for s in range(1, max(1, min(tiles // 2, 48, most)) + 1):
         size = -(-tiles // s)

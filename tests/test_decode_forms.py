@@ -128,3 +128,18 @@ def test_no_split_is_longer_than_asked(longest, most, splits, size, monkeypatch)
     whole = ops.decode_attention(*args)
     assert float((ops.decode_attention(*args, most_keys=most).float() - whole.float()).abs().max()) <= 2 ** -7 * float(whole.abs().max())
     ops.check_tc_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hd", [64, 128])
+def test_no_tokens_to_decode(hd):
+    e = lambda *s, dtype=torch.bfloat16: torch.empty(*s, dtype=dtype, device=DEV)
+    pages, none, table = torch.zeros(2, 2, 64, hd, dtype=torch.bfloat16, device=DEV), e(0, dtype=torch.int32), torch.zeros(1, 1, dtype=torch.int32, device=DEV)
+    with pytest.raises(ops.KernelError, match="bad argument"):
+        ops.decode_attention(e(0, 4, hd), pages, pages, e(0, 1, dtype=torch.int32), none, none, 0, 0, 0.125, 100)
+    with pytest.raises(ops.KernelError, match="bad argument"):
+        ops.decode_attention_fused(e(0, 8 * hd), 4, 2, hd, none, None, False, False, 1e-6, None, none, e(0, 1, dtype=torch.int32), pages, pages, 0, 0, 0.125, 100)
+    q, out = torch.ones(3, 4, hd, dtype=torch.bfloat16, device=DEV), torch.full((3, 4, hd), 7.0, dtype=torch.bfloat16, device=DEV)
+    three = torch.zeros(3, dtype=torch.int32, device=DEV)
+    assert ops.decode_attention(q, pages, pages, table, three, three, 0, 0, 0.125, 100, rows=e(0, dtype=torch.int64), out=out) is out
+    assert bool((out == 7.0).all())
