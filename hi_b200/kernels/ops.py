@@ -1608,9 +1608,9 @@ def decode_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
 
 FUSED_COUNTERS = 1 << 18     # (token, kv head) pairs the fused decode kernel has counters for
 # The fused kernel pays for what it saves in launches with work at the head and the tail of every
-# block; once the blocks fill the machine several times over that shows. Measured at 8,192 keys, 8 kv
-# heads: 2 / 8 / 16 requests 32.8 / 69.6 / 110.6 us against 38.9 / 76.7 / 117.8 us for the three
-# kernels; 32 requests equal; 64 requests 364 against 352 us.
+# block; once the blocks fill the machine several times over that shows. Measured at 8,192 keys, 40 heads of 128 on 8 kv
+# heads, L2 flushed: 2 / 8 / 16 / 32 requests 26.6 / 62.4 / 105.4 / 179.1 us against 30.8 / 63.9 / 105.9 / 182.7 us for the three
+# kernels; 64 requests 336.9 against 331.7 us.
 FUSED_MAX_GROUPS = 256       # (token, kv head) pairs up to which a decode step takes the fused kernel
 _fused_counters: dict = {}   # device -> int32 zeros that the fused kernel leaves at zero
 
